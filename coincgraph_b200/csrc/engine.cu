@@ -210,7 +210,9 @@ enum SmallIdx : int {
     kCoopR = 28,
     kHugeF = 29,  // hub deletion groups served by the whole grid, per arena
     kHugeR = 30,
-    kSmallCount = 32
+    kCompactBig = 31,  // rows to compact above kWarpMove slots, per arena
+    kCompactBigR = 32,
+    kSmallCount = 64
 };
 
 constexpr uint32_t kBigRowCap = 65536;
@@ -1748,11 +1750,14 @@ struct cig_handle {
         p = prof_begin(forward ? CIG_STAGE_MUTATE : CIG_STAGE_MUTATE_REV);
         unsigned long long *stats = with_stats ? status->counters : nullptr;
         uint32_t *ccount = small + (forward ? kCompactCount : kCompactCountR);
+        const CompactList cl{compact, ccount, small + (forward ? kCompactBig : kCompactBigR),
+                             static_cast<uint32_t>(bcap)};
         uint32_t *ocount = small + (forward ? kOrderedCount : kOrderedCountR);
         // Flat path: rows whose deletion requests are all distinct.
         uint32_t *icount = small + (forward ? kIndexedCount : kIndexedCountR);
         if (!zeroed) {
             CK(cudaMemsetAsync(ccount, 0, sizeof(uint32_t), cs));
+            CK(cudaMemsetAsync(cl.big_count, 0, sizeof(uint32_t), cs));
             CK(cudaMemsetAsync(ocount, 0, sizeof(uint32_t), cs));
             CK(cudaMemsetAsync(icount, 0, sizeof(uint32_t), cs));
         }
@@ -1783,15 +1788,15 @@ struct cig_handle {
         }
         prof_end(ps);
         launch(del_apply, grid_for(nd), 256, A.view(), A.desc, sorted, m, firstpos, stats);
-        launch(del_finish, persistent_grid(), 256, A.desc, sorted, grp, gtype, firstpos, compact, ccount, stats);
+        launch(del_finish, persistent_grid(), 256, A.desc, sorted, grp, gtype, firstpos, cl, stats);
         // Ordered path: rows with repeated requests for a destination.
         launch(mutate_delete, persistent_grid(), kMutWarps * 32, A.view(), A.desc, sorted, grp, ordered, ocount,
-               matched, big, bcount, compact, ccount, stats, status);
-        launch(mutate_delete_big, sms * 4, kTpbMut, A.view(), A.desc, sorted, grp, big, bcount, matched, compact,
-               ccount, stats, status);
+               matched, big, bcount, cl, stats, status);
+        launch(mutate_delete_big, sms * 4, kTpbMut, A.view(), A.desc, sorted, grp, big, bcount, matched, cl, stats,
+               status);
         if (ix.keys) launch(idx_fix_ordered, persistent_grid(), 256, A.view(), A.desc, sorted, grp, ordered, ocount, ix,
                             status);
-        launch(compact_rows, sms * 4, kTpbMut, A.view(), A.desc, compact, ccount, ix, status);
+        launch(compact_rows, sms * 4, kTpbMut, A.view(), A.desc, cl, ix, status);
         prof_end(p);
         check_launch();
     }
@@ -1890,12 +1895,13 @@ struct cig_handle {
         const InBatch ib(in_batch);
         const uint32_t *ep = small + kEpoch;
         // frontier, affected and deletion-path counters of both arenas
-        static_assert(kSmallCount == 32 && kEpoch == 23, "phase_begin clears one 32-word counter block");
-        const uint32_t mask = (0x3Fu << kFr) | (1u << kBigF) | (1u << kBigR) | (1u << kCompactCount) |
-                              (1u << kOrderedCount) | (1u << kIndexedCount) | (1u << kInvalDone) |
-                              (1u << kCompactCountR) | (1u << kOrderedCountR) | (1u << kIndexedCountR) |
-                              (1u << kCoopF) | (1u << kCoopR) | (1u << kHugeF) | (1u << kHugeR);
-        launch(phase_begin, 1, 32, small + kEpoch, small, mask);
+        static_assert(kSmallCount == 64, "phase_begin clears one 64-word counter block");
+        const unsigned long long mask = (0x3Full << kFr) | (1ull << kBigF) | (1ull << kBigR) | (1ull << kCompactCount) |
+                              (1ull << kOrderedCount) | (1ull << kIndexedCount) | (1ull << kInvalDone) |
+                              (1ull << kCompactCountR) | (1ull << kOrderedCountR) | (1ull << kIndexedCountR) |
+                              (1ull << kCoopF) | (1ull << kCoopR) | (1ull << kHugeF) | (1ull << kHugeR) |
+                                        (1ull << kCompactBig) | (1ull << kCompactBigR);
+        launch(phase_begin, 1, kSmallCount, small + kEpoch, small, mask);
         int p = prof_begin(CIG_STAGE_SEED);
         if (nd)
             launch(seed_deletions<A>, grid_for(nd), 256, d_du, d_dv, static_cast<uint32_t>(nd), n, state,

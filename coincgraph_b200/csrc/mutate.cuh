@@ -272,14 +272,30 @@ __device__ __forceinline__ void write_slot(const AdjView &view, unsigned long lo
     *view.wptr(off) = value;
 }
 
+// Rows to compact, in one array: rows a warp serves from the front, longer
+// ones (kWarpMove) from the back, so that each kind is dealt to workers of its
+// own width without reading the other's descriptors.
+constexpr uint32_t kWarpMove = 1024;  // survivors of rows up to this length are moved by one warp
+struct CompactList {
+    uint32_t *rows;
+    uint32_t *count;      // from the front
+    uint32_t *big_count;  // from the back
+    uint32_t cap;
+};
+
 // Record the tombstones a row received; queue it for compaction when they
 // reach a quarter of its length.
 __device__ __forceinline__ void finish_row(RowDesc *desc, uint32_t u, const RowDesc &d, uint32_t removed,
-                                           uint32_t *compact, uint32_t *compact_count) {
+                                           const CompactList &cl) {
     if (!removed) return;
     const uint32_t tombs = rd_tombs(d) + removed;
     desc[u].meta = rd_meta(rd_cls(d), tombs);
-    if (4ull * tombs >= d.len || tombs >= kMaxTombs / 2) compact[atomicAdd(compact_count, 1u)] = u;
+    if (4ull * tombs >= d.len || tombs >= kMaxTombs / 2) {
+        if (d.len <= kWarpMove)
+            cl.rows[atomicAdd(cl.count, 1u)] = u;
+        else
+            cl.rows[cl.cap - 1u - atomicAdd(cl.big_count, 1u)] = u;
+    }
 }
 
 // ---------------------------------------------------------------- deletion
@@ -384,7 +400,7 @@ __device__ __forceinline__ uint32_t warp_tomb_global(const AdjView &view, const 
 __global__ void __launch_bounds__(kMutWarps * 32)
     mutate_delete(AdjView view, RowDesc *desc, const unsigned long long *keys, Groups gr, const uint32_t *list,
                   const uint32_t *list_count, uint32_t *matched, uint32_t *big, uint32_t *big_count,
-                  uint32_t *compact, uint32_t *compact_count, unsigned long long *stats, Status *st) {
+                  CompactList cl, unsigned long long *stats, Status *st) {
     const uint32_t lane = lane_id();
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
     const uint32_t nl = *list_count;
@@ -402,7 +418,7 @@ __global__ void __launch_bounds__(kMutWarps * 32)
         const uint32_t done = (ge - gs <= 32u) ? warp_tomb_regs(view, d, keys, gs, ge - gs)
                                                : warp_tomb_global(view, d, u, keys, gs, ge, matched);
         if (lane == 0) {
-            finish_row(desc, u, d, done, compact, compact_count);
+            finish_row(desc, u, d, done, cl);
             removed += done;
             changed += done != 0;
         }
@@ -427,8 +443,8 @@ __device__ __forceinline__ uint32_t filter_hash(uint32_t x) { return (x * 0x9E37
 
 __global__ void __launch_bounds__(kTpbMut)
     mutate_delete_big(AdjView view, RowDesc *desc, const unsigned long long *keys, Groups gr, const uint32_t *big,
-                      const uint32_t *big_count, uint32_t *matched, uint32_t *compact, uint32_t *compact_count,
-                      unsigned long long *stats, Status *st) {
+                      const uint32_t *big_count, uint32_t *matched, CompactList cl, unsigned long long *stats,
+                      Status *st) {
     __shared__ uint32_t skey[kBigKeys];
     __shared__ uint32_t scount[kBigKeys];
     __shared__ uint32_t filter[kFilterBits / 32];
@@ -554,7 +570,7 @@ __global__ void __launch_bounds__(kTpbMut)
         }
         if (tid == 0) {
             const uint32_t done = gm - left;
-            finish_row(desc, u, d, done, compact, compact_count);
+            finish_row(desc, u, d, done, cl);
             if (done && stats) {
                 atomicAdd(&stats[kCntRemoved], static_cast<unsigned long long>(done));
                 atomicAdd(&stats[kCntChanged], 1ull);
@@ -1036,15 +1052,14 @@ __global__ void del_apply(AdjView view, RowDesc *desc, const unsigned long long 
 
 // Queue flat rows whose tombstones reached a quarter of their length.
 __global__ void del_finish(const RowDesc *desc, const unsigned long long *keys, Groups gr, const uint8_t *gtype,
-                           const uint32_t *firstpos, uint32_t *compact, uint32_t *compact_count,
-                           unsigned long long *stats) {
+                           const uint32_t *firstpos, CompactList cl, unsigned long long *stats) {
     const uint32_t ng = *gr.count;
     const uint32_t rounded = (ng + 31u) & ~31u;
     uint32_t changed = 0;
     // Warp-aggregated appends and counts: ~10^5 rows per batch would
     // otherwise queue on one counter address.
     for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < rounded; g += gridDim.x * blockDim.x) {
-        bool want = false;
+        bool want = false, big = false;
         uint32_t u = 0;
         if (g < ng && gtype[g] != kGroupOrdered) {  // flat group (scanned or indexed)
             const uint32_t gs = gr.start[g];
@@ -1057,124 +1072,191 @@ __global__ void del_finish(const RowDesc *desc, const unsigned long long *keys, 
                 const RowDesc d = desc[u];
                 const uint32_t tombs = rd_tombs(d);
                 want = 4ull * tombs >= d.len || tombs >= kMaxTombs / 2;
+                big = want && d.len > kWarpMove;
+                want = want && !big;
             }
         }
-        warp_enqueue(want, u, compact, compact_count, 0xFFFFFFFFu, nullptr);
+        warp_enqueue(want, u, cl.rows, cl.count, 0xFFFFFFFFu, nullptr);
+        if (big) cl.rows[cl.cap - 1u - atomicAdd(cl.big_count, 1u)] = u;
     }
     if (stats) warp_count(&stats[kCntChanged], changed);
 }
 
-// ---------------------------------------------------------------- index upkeep
-// The live entries of an indexed row moved (compaction, relocation): the
-// first positions of its keys are recomputed over the row's first `len`
-// slots at `off` (two passes, reset then minimum).  Block-wide and warp-wide
-// forms; all threads of the block (warp) call.
-// One pass over the entries t, t + stride, ... of the row: `set` false
-// clears every key's first position, true lowers it to the entry's
-// position.  Four entries per thread at a time, their row reads and index
-// probes in flight together.
-__device__ __forceinline__ void idx_reposition_pass(const AdjView &view, const PosIndex &ix, uint32_t u,
-                                                    uint64_t off, uint32_t len, uint32_t t, uint32_t stride, bool set,
-                                                    Status *st) {
-    constexpr int N = 4;
-    for (uint32_t base = t; base < len; base += N * stride) {
-        uint32_t v[N];
-        bool live[N];
+// ---------------------------------------------------------------- moving survivors
+// The live entries of a row of `len` slots at `src_off` move, in order, to the
+// front of the block at `dst_off` (the same block: compaction in place), and
+// the position index follows (idx_move_n) where an entry's position changes.
+// Return the number of survivors.
+//
+// One warp, rows inside one segment: 256 entries per step, the row loads of
+// the next step in flight while this step is scanned, stored and indexed (in
+// place, this step's stores lie below the next step's loads).
+__device__ __forceinline__ uint32_t warp_move_live(const AdjView &view, const PosIndex &ix, uint32_t u,
+                                                   uint64_t src_off, uint32_t len, uint64_t dst_off, Status *st) {
+    if (!len) return 0u;
+    const uint32_t lane = lane_id();
+    const uint4 tomb4 = make_uint4(kTomb, kTomb, kTomb, kTomb);
+    const uint32_t *src = view.at(src_off);
+    uint32_t *dst = view.wptr(dst_off);
+    const bool indexed = idx_row(ix, u);
+    uint32_t w = 0;
+    uint4 next[2];
 #pragma unroll
-        for (int j = 0; j < N; ++j) {
-            const uint32_t k = base + j * stride;
-            live[j] = k < len;
-            v[j] = live[j] ? __ldcg(view.at(off + k)) : 0u;
+    for (uint32_t h = 0; h < 2; ++h) {
+        const uint32_t k = 128u * h + 4u * lane;
+        next[h] = k < len ? *reinterpret_cast<const uint4 *>(src + k) : tomb4;
+    }
+    for (uint32_t b0 = 0; b0 < len; b0 += 256u) {
+        uint4 cur[2] = {next[0], next[1]};
+#pragma unroll
+        for (uint32_t h = 0; h < 2; ++h) {
+            const uint32_t k = b0 + 256u + 128u * h + 4u * lane;
+            next[h] = k < len ? *reinterpret_cast<const uint4 *>(src + k) : tomb4;
         }
-        unsigned long long slot[N];
-        idx_find_n<N>(ix, u, v, live, slot, st);
 #pragma unroll
-        for (int j = 0; j < N; ++j) {
-            if (slot[j] == ~0ull) continue;
-            if (set)
-                atomicMin(&ix.val[slot[j]].x, base + j * stride);
-            else
-                atomicExch(&ix.val[slot[j]].x, kInf);
+        for (uint32_t h = 0; h < 2; ++h) {
+            const uint32_t k = b0 + 128u * h + 4u * lane;
+            const uint32_t v[4] = {cur[h].x, cur[h].y, cur[h].z, cur[h].w};
+            bool live[4];
+            uint32_t c = 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                live[j] = k + j < len && v[j] != kTomb;
+                c += live[j] ? 1u : 0u;
+            }
+            uint32_t incl = c;
+#pragma unroll
+            for (uint32_t o = 1; o < 32u; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(kFull, incl, o);
+                if (lane >= o) incl += t;
+            }
+            uint32_t pos = w + incl - c;
+            uint32_t p[4], q[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                p[j] = k + j;
+                q[j] = pos;
+                if (live[j]) {
+                    dst[pos++] = v[j];
+                    live[j] = p[j] != q[j];
+                }
+            }
+            if (indexed) idx_move_n<4>(ix, u, v, p, q, live, st);
+            w += __shfl_sync(kFull, incl, 31);
         }
     }
+    __syncwarp();
+    return w;
 }
 
-__device__ __forceinline__ void idx_reposition_block(const AdjView &view, const PosIndex &ix, uint32_t u,
-                                                     uint64_t off, uint32_t len, Status *st) {
-    idx_reposition_pass(view, ix, u, off, len, threadIdx.x, blockDim.x, false, st);
-    __syncthreads();
-    idx_reposition_pass(view, ix, u, off, len, threadIdx.x, blockDim.x, true, st);
-    __syncthreads();
-}
+// One block, rows of any length: tiles of kTpbMut x 8 slots, block scan,
+// survivors staged in shared memory and stored with coalesced writes.
+struct MoveSmem {
+    typename cub::BlockScan<uint32_t, kTpbMut>::TempStorage scan;
+    uint32_t stage[kTpbMut * kBigItems];
+};
 
-__device__ __forceinline__ void idx_reposition_warp(const AdjView &view, const PosIndex &ix, uint32_t u,
-                                                    uint64_t off, uint32_t len, Status *st) {
-    const uint32_t lane = lane_id();
-    __syncwarp();
-    idx_reposition_pass(view, ix, u, off, len, lane, 32u, false, st);
-    __syncwarp();
-    idx_reposition_pass(view, ix, u, off, len, lane, 32u, true, st);
-    __syncwarp();
+__device__ __forceinline__ uint32_t block_move_live(const AdjView &view, const PosIndex &ix, uint32_t u,
+                                                    uint64_t src_off, uint32_t len, uint64_t dst_off, MoveSmem &sm,
+                                                    Status *st) {
+    using BlockScan = cub::BlockScan<uint32_t, kTpbMut>;
+    const uint32_t tid = threadIdx.x;
+    const bool indexed = idx_row(ix, u);
+    uint32_t w = 0;
+    for (uint32_t base = 0; base < len; base += kTpbMut * kBigItems) {
+        const uint32_t k0 = base + tid * kBigItems;
+        uint32_t e[kBigItems];
+#pragma unroll
+        for (int h = 0; h < kBigItems; h += 4) {
+            if (k0 + h < len) {
+                const uint4 q = *reinterpret_cast<const uint4 *>(view.at(src_off + k0 + h));
+                e[h] = q.x;
+                e[h + 1] = q.y;
+                e[h + 2] = q.z;
+                e[h + 3] = q.w;
+            } else {
+                e[h] = e[h + 1] = e[h + 2] = e[h + 3] = kTomb;
+            }
+        }
+        uint32_t kc = 0;
+#pragma unroll
+        for (int s = 0; s < kBigItems; ++s) {
+            if (k0 + s >= len) e[s] = kTomb;
+            kc += e[s] != kTomb ? 1u : 0u;
+        }
+        uint32_t prefix, total;
+        BlockScan(sm.scan).ExclusiveSum(kc, prefix, total);
+        uint32_t pos = prefix;
+        uint32_t q[kBigItems];
+#pragma unroll
+        for (int s = 0; s < kBigItems; ++s) {
+            q[s] = w + pos;
+            if (e[s] != kTomb) sm.stage[pos++] = e[s];
+        }
+        __syncthreads();  // every load of this tile is done before any store
+        const uint32_t tile = min(static_cast<uint32_t>(kTpbMut * kBigItems), len - base);
+        if (src_off != dst_off || w != base || total != tile) {
+            for (uint32_t i = tid; i < total; i += kTpbMut) write_slot(view, dst_off + w + i, sm.stage[i]);
+            if (indexed) {
+#pragma unroll
+                for (int h = 0; h < kBigItems; h += 4) {
+                    const uint32_t v4[4] = {e[h], e[h + 1], e[h + 2], e[h + 3]};
+                    const uint32_t p4[4] = {k0 + h, k0 + h + 1, k0 + h + 2, k0 + h + 3};
+                    const uint32_t q4[4] = {q[h], q[h + 1], q[h + 2], q[h + 3]};
+                    bool moved[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) moved[j] = v4[j] != kTomb && p4[j] != q4[j];
+                    idx_move_n<4>(ix, u, v4, p4, q4, moved, st);
+                }
+            }
+        }
+        w += total;
+        __syncthreads();
+    }
+    return w;
 }
 
 // ---------------------------------------------------------------- compaction
 
-// Drop the tombstones of the queued rows in place (order kept).  One block
-// per row; tiles of kTpbMut x 8 slots, block scan, survivors staged in
-// shared memory and stored with coalesced writes.
-__global__ void __launch_bounds__(kTpbMut) compact_rows(AdjView view, RowDesc *desc, const uint32_t *list,
-                                                         const uint32_t *count, PosIndex ix, Status *st) {
-    using BlockScan = cub::BlockScan<uint32_t, kTpbMut>;
-    __shared__ typename BlockScan::TempStorage scan_tmp;
-    __shared__ uint32_t stage[kTpbMut * kBigItems];
-    const uint32_t tid = threadIdx.x;
-    const uint32_t nc = *count;
-    for (uint32_t c = blockIdx.x; c < nc; c += gridDim.x) {
-        const uint32_t u = list[c];
+// Drop the tombstones of the queued rows in place (order kept): a warp per
+// row of up to kWarpMove slots (nearly all of them: a row of four entries
+// compacts at its first deletion), a block per longer row.  A block for
+// every row left 255 of 256 threads idle on the short ones.
+__global__ void __launch_bounds__(kTpbMut) compact_rows(AdjView view, RowDesc *desc, CompactList cl, PosIndex ix,
+                                                         Status *st) {
+    __shared__ MoveSmem sm;
+    const uint32_t nb = *cl.big_count;
+    for (uint32_t c = blockIdx.x; c < nb; c += gridDim.x) {
+        const uint32_t u = cl.rows[cl.cap - 1u - c];
         const RowDesc d = desc[u];
-        uint32_t w = 0;
-        for (uint32_t base = 0; base < d.len; base += kTpbMut * kBigItems) {
-            const uint32_t k0 = base + tid * kBigItems;
-            uint32_t e[kBigItems];
-#pragma unroll
-            for (int h = 0; h < kBigItems; h += 4) {
-                if (k0 + h < d.len) {
-                    const uint4 q = *reinterpret_cast<const uint4 *>(view.at(d.off + k0 + h));
-                    e[h] = q.x;
-                    e[h + 1] = q.y;
-                    e[h + 2] = q.z;
-                    e[h + 3] = q.w;
-                } else {
-                    e[h] = e[h + 1] = e[h + 2] = e[h + 3] = kTomb;
-                }
-            }
-            uint32_t kc = 0;
-#pragma unroll
-            for (int s = 0; s < kBigItems; ++s) kc += (k0 + s < d.len && e[s] != kTomb) ? 1u : 0u;
-            uint32_t prefix, total;
-            BlockScan(scan_tmp).ExclusiveSum(kc, prefix, total);
-            uint32_t pos = prefix;
-#pragma unroll
-            for (int s = 0; s < kBigItems; ++s)
-                if (k0 + s < d.len && e[s] != kTomb) stage[pos++] = e[s];
-            __syncthreads();  // every load of this tile is done before any store
-            const uint32_t tile_valid = min(static_cast<uint32_t>(kTpbMut * kBigItems), d.len - base);
-            if (w != base || total != tile_valid)
-                for (uint32_t i = tid; i < total; i += kTpbMut) write_slot(view, d.off + w + i, stage[i]);
-            w += total;
-            __syncthreads();
-        }
-        if (tid == 0) desc[u] = RowDesc{d.off, w, rd_meta(rd_cls(d), 0)};
+        const uint32_t w = block_move_live(view, ix, u, d.off, d.len, d.off, sm, st);
+        if (threadIdx.x == 0) desc[u] = RowDesc{d.off, w, rd_meta(rd_cls(d), 0)};
         __syncthreads();
-        if (idx_row(ix, u)) idx_reposition_block(view, ix, u, d.off, w, st);
+    }
+    const uint32_t nc = *cl.count;
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < nc; c += warps) {
+        const uint32_t u = cl.rows[c];
+        const RowDesc d = desc[u];
+        const uint32_t w = warp_move_live(view, ix, u, d.off, d.len, d.off, st);
+        if (lane_id() == 0) desc[u] = RowDesc{d.off, w, rd_meta(rd_cls(d), 0)};
     }
 }
 
 // ---------------------------------------------------------------- addition
 
-// Addition plan: rows that outgrow their block get a class (sized for the
-// live entries plus the additions, since relocation drops tombstones) and a
-// rank in that class.
+// Addition plan.  A row whose block has room appends in place (kKeyNone).  A
+// row whose used slots would overflow its block while its live entries and
+// the additions fit (kKeyInPlace) drops its tombstones where it is.  A row
+// that outgrows its block gets a class (sized for the live entries plus the
+// additions) and a rank in that class; it moves as it is, tombstones and
+// all, when that fits the new block, which leaves every position, and so the
+// position index, as it was.  (Giving the second kind a fresh block of its
+// own class, as before, lost a block per overflow for good: 3.2 slots per
+// inserted edge on the s22 SSSP stream at a steady size.)
+constexpr unsigned long long kKeyOverflow = ~0ull - 1ull;  // degree overflow, reported by the apply kernel
+constexpr unsigned long long kKeyInPlace = ~0ull - 2ull;
+
 __global__ void plan_add(const RowDesc *desc, const unsigned long long *keys, Groups gr, unsigned long long *plan,
                          ArenaAlloc *al) {
     const uint32_t ng = *gr.count;
@@ -1191,10 +1273,12 @@ __global__ void plan_add(const RowDesc *desc, const unsigned long long *keys, Gr
             const unsigned long long used = static_cast<unsigned long long>(d.len) + (ge - gs);
             const unsigned long long live = static_cast<unsigned long long>(rd_live(d)) + (ge - gs);
             if (live > 0xFFFFFFFFull) {
-                p = kKeyNone - 1;  // degree overflow, reported by the apply kernel
-            } else if (rd_cls(d) == 0 || used > (1ull << rd_cls(d))) {
+                p = kKeyOverflow;
+            } else if (rd_cls(d) == 0 || live > (1ull << rd_cls(d))) {
                 cls = class_for(static_cast<uint32_t>(live));
                 move = true;
+            } else if (used > (1ull << rd_cls(d))) {
+                p = kKeyInPlace;
             }
         }
         // Ranks within a class, one atomic per class present in the warp
@@ -1283,7 +1367,7 @@ __global__ void __launch_bounds__(256, 4)
             const unsigned long long p = plan[g];
             const uint32_t gs = gr.start[g];
             const uint32_t a = gr.end[g] - gs;
-            if (p == kKeyNone - 1) {
+            if (p == kKeyOverflow) {
                 set_error(st, kErrInternal, g);
             } else if (a > kLaneAdds) {
                 coop = true;
@@ -1310,11 +1394,13 @@ __global__ void __launch_bounds__(256, 4)
                     if (indexed) idx_add_n<kLaneAdds>(ix, u, add, d.len, a, st);
                     desc[u] = RowDesc{d.off, d.len + a, d.meta};
                     changed += 1;
-                } else if (d.len > kLaneRow) {
+                } else if (d.len > kLaneRow || indexed) {
                     coop = true;
                 } else {
-                    const uint32_t cls = static_cast<uint32_t>(p >> 32);
-                    const unsigned long long off = alloc_offset(al, cls, static_cast<uint32_t>(p));
+                    // In place, or to a larger block.
+                    const bool moves = p != kKeyInPlace;
+                    const uint32_t cls = moves ? static_cast<uint32_t>(p >> 32) : rd_cls(d);
+                    const unsigned long long off = moves ? alloc_offset(al, cls, static_cast<uint32_t>(p)) : d.off;
                     // Old block (<= kLaneRow slots) and new block (<= 16 slots)
                     // each lie in one segment: one slot lookup apiece.
                     uint32_t row[kLaneRow];
@@ -1330,13 +1416,8 @@ __global__ void __launch_bounds__(256, 4)
                     for (uint32_t j = 0; j < kLaneAdds; ++j)
                         if (j < a) wp[w + j] = add[j];
                     desc[u] = RowDesc{off, w + a, rd_meta(cls, 0)};
-                    moved_entries += w;
-                    if (indexed) {
-                        for (uint32_t k = 0; k < w; ++k) idx_pos_reset(ix, u, __ldcg(wp + k), st);
-                        for (uint32_t k = 0; k < w; ++k) idx_pos_set(ix, u, __ldcg(wp + k), k);
-                        for (uint32_t j = 0; j < a; ++j) idx_add(ix, u, add[j], w + j, st);
-                    }
-                    moved += 1;
+                    moved += moves ? 1u : 0u;
+                    moved_entries += moves ? w : 0u;
                     changed += 1;
                 }
             }
@@ -1354,9 +1435,10 @@ __global__ void __launch_bounds__(256, 4)
 
 
 // The groups mutate_add left to whole warps (more than kLaneAdds appends, or
-// a moving row of more than kLaneRow entries), one warp per group over the
-// whole grid: rows of up to kWarpRowMax entries move here, larger ones go to
-// mutate_add_big.
+// a moving or compacting row of more than kLaneRow entries), one warp per
+// group over the whole grid: rows of up to kWarpRowMax entries move as they
+// are here, rows of up to kWarpMove entries drop their tombstones here,
+// larger ones go to mutate_add_big.
 __global__ void mutate_add_warp(AdjView view, RowDesc *desc, const unsigned long long *keys, Groups gr,
                                 const unsigned long long *plan, const ArenaAlloc *al, const uint32_t *vals,
                                 const uint32_t *coop_list, const uint32_t *coop_count, uint32_t *big,
@@ -1383,58 +1465,51 @@ __global__ void mutate_add_warp(AdjView view, RowDesc *desc, const unsigned long
             }
             if (lane == 0) desc[u] = RowDesc{d.off, d.len + a, d.meta};
         } else {
-            if (d.len > kWarpRowMax) {
+            const bool moves = p != kKeyInPlace;
+            const uint32_t cls = moves ? static_cast<uint32_t>(p >> 32) : rd_cls(d);
+            // Tombstones come along when they fit.
+            const bool whole = moves && static_cast<unsigned long long>(d.len) + a <= (1ull << cls);
+            if (d.len > (whole ? kWarpRowMax : kWarpMove)) {
                 if (lane == 0) big[atomicAdd(big_count, 1u)] = gb;
                 continue;
             }
-            const uint32_t cls = static_cast<uint32_t>(p >> 32);
-            const unsigned long long off = alloc_offset(al, cls, static_cast<uint32_t>(p));
-            // Copy the survivors in order, 256 entries per step: each lane
-            // issues two independent 16-byte loads (the old block lies in
-            // one segment and starts on a 16-byte boundary) before any
-            // store, so a zero-copy row costs one host round trip per
-            // 256 entries instead of one per 32.
-            const uint32_t *src = view.at(d.off);
-            uint32_t w = 0;
-            for (uint32_t b0 = 0; b0 < d.len; b0 += 256u) {
-                uint32_t e[8];
+            const unsigned long long off = moves ? alloc_offset(al, cls, static_cast<uint32_t>(p)) : d.off;
+            uint32_t w = d.len;
+            if (!whole) {
+                w = warp_move_live(view, ix, u, d.off, d.len, off, st);
+            } else if (d.len) {
+                // Old and new block each lie in one segment and start on a
+                // 16-byte boundary: 512 entries per step, four independent
+                // 16-byte loads per lane before any store (a zero-copy row
+                // costs one host round trip per step).
+                const uint32_t *src = view.at(d.off);
+                uint32_t *dst = view.wptr(off);
+                for (uint32_t b0 = 0; b0 < d.len; b0 += 512u) {
+                    uint4 q[4];
 #pragma unroll
-                for (uint32_t h = 0; h < 2; ++h) {
-                    const uint32_t k = b0 + 128u * h + 4u * lane;
-                    uint4 q = make_uint4(kTomb, kTomb, kTomb, kTomb);
-                    if (k < d.len) q = *reinterpret_cast<const uint4 *>(src + k);
-                    e[4 * h] = k < d.len ? q.x : kTomb;
-                    e[4 * h + 1] = k + 1u < d.len ? q.y : kTomb;
-                    e[4 * h + 2] = k + 2u < d.len ? q.z : kTomb;
-                    e[4 * h + 3] = k + 3u < d.len ? q.w : kTomb;
-                }
-#pragma unroll
-                for (uint32_t h = 0; h < 2; ++h) {
-                    uint32_t c = 0;
-#pragma unroll
-                    for (uint32_t j = 0; j < 4; ++j) c += e[4 * h + j] != kTomb ? 1u : 0u;
-                    uint32_t incl = c;
-#pragma unroll
-                    for (uint32_t o = 1; o < 32u; o <<= 1) {
-                        const uint32_t t = __shfl_up_sync(kFull, incl, o);
-                        if (lane >= o) incl += t;
+                    for (uint32_t h = 0; h < 4; ++h) {
+                        const uint32_t k = b0 + 128u * h + 4u * lane;
+                        if (k < d.len) q[h] = *reinterpret_cast<const uint4 *>(src + k);
                     }
-                    uint32_t pos = w + incl - c;
 #pragma unroll
-                    for (uint32_t j = 0; j < 4; ++j)
-                        if (e[4 * h + j] != kTomb) write_slot(view, off + pos++, e[4 * h + j]);
-                    w += __shfl_sync(kFull, incl, 31);
+                    for (uint32_t h = 0; h < 4; ++h) {
+                        const uint32_t k = b0 + 128u * h + 4u * lane;
+                        if (k < d.len) *reinterpret_cast<uint4 *>(dst + k) = q[h];
+                    }
                 }
+                __syncwarp();  // the last 16 bytes may reach past the row's end, where the appends go
             }
-            if (lane == 0) moved_entries += w;
-            for (uint32_t j = lane; j < a; j += 32u) write_slot(view, off + w + j, vals[key_low(keys[gs + j])]);
-            if (lane == 0) desc[u] = RowDesc{off, w + a, rd_meta(cls, 0)};
-            if (idx_row(ix, u)) {
-                // survivors moved: reposition them; then count the appended entries
-                idx_reposition_warp(view, ix, u, off, w, st);
-                for (uint32_t j = lane; j < a; j += 32u) idx_add(ix, u, vals[key_low(keys[gs + j])], w + j, st);
+            const bool indexed = idx_row(ix, u);
+            for (uint32_t j = lane; j < a; j += 32u) {
+                const uint32_t v = vals[key_low(keys[gs + j])];
+                write_slot(view, off + w + j, v);  // many additions may span segments
+                if (indexed) idx_add(ix, u, v, w + j, st);
             }
-            if (lane == 0) moved += 1;
+            if (lane == 0) {
+                desc[u] = RowDesc{off, w + a, rd_meta(cls, whole ? rd_tombs(d) : 0u)};
+                moved += moves ? 1u : 0u;
+                moved_entries += moves ? w : 0u;
+            }
         }
         if (lane == 0) changed += 1;
     }
@@ -1449,8 +1524,7 @@ __global__ void __launch_bounds__(kTpbMut)
     mutate_add_big(AdjView view, RowDesc *desc, const unsigned long long *keys, Groups gr,
                    const unsigned long long *plan, const ArenaAlloc *al, const uint32_t *vals, const uint32_t *big,
                    const uint32_t *big_count, unsigned long long *stats, PosIndex ix, Status *st) {
-    using BlockScan = cub::BlockScan<uint32_t, kTpbMut>;
-    __shared__ typename BlockScan::TempStorage scan_tmp;
+    __shared__ MoveSmem sm;
     if (ld_volatile(&st->err) & kErrArena) return;
     const uint32_t nb = *big_count;
     for (uint32_t b = blockIdx.x; b < nb; b += gridDim.x) {
@@ -1461,31 +1535,44 @@ __global__ void __launch_bounds__(kTpbMut)
         const uint32_t u = key_src(keys[gs]);
         const RowDesc d = desc[u];
         const uint32_t a = ge - gs;
-        const uint32_t cls = static_cast<uint32_t>(p >> 32);
-        const unsigned long long off = alloc_offset(al, cls, static_cast<uint32_t>(p));
-        uint32_t w = 0;
-        for (uint32_t base = 0; base < d.len; base += kTpbMut) {
-            const uint32_t k = base + threadIdx.x;
-            const uint32_t x = k < d.len ? *view.at(d.off + k) : kTomb;
-            uint32_t prefix, total;
-            BlockScan(scan_tmp).ExclusiveSum(x != kTomb ? 1u : 0u, prefix, total);
-            if (x != kTomb) write_slot(view, off + w + prefix, x);
-            w += total;
-            __syncthreads();
+        const bool moves = p != kKeyInPlace;
+        const uint32_t cls = moves ? static_cast<uint32_t>(p >> 32) : rd_cls(d);
+        const bool whole = moves && static_cast<unsigned long long>(d.len) + a <= (1ull << cls);
+        const unsigned long long off = moves ? alloc_offset(al, cls, static_cast<uint32_t>(p)) : d.off;
+        uint32_t w = d.len;
+        if (!whole) {
+            w = block_move_live(view, ix, u, d.off, d.len, off, sm, st);
+        } else {
+            // 16 entries per thread and step, resolved per 16 bytes (a block
+            // above one segment may lie in HBM and in host memory).
+            for (uint32_t b0 = 0; b0 < d.len; b0 += 16u * kTpbMut) {
+                uint4 q[4];
+#pragma unroll
+                for (uint32_t h = 0; h < 4; ++h) {
+                    const uint32_t k = b0 + 4u * (h * kTpbMut + threadIdx.x);
+                    if (k < d.len) q[h] = *reinterpret_cast<const uint4 *>(view.at(d.off + k));
+                }
+#pragma unroll
+                for (uint32_t h = 0; h < 4; ++h) {
+                    const uint32_t k = b0 + 4u * (h * kTpbMut + threadIdx.x);
+                    if (k < d.len) *reinterpret_cast<uint4 *>(view.wptr(off + k)) = q[h];
+                }
+            }
         }
-        for (uint32_t j = threadIdx.x; j < a; j += kTpbMut) write_slot(view, off + w + j, vals[key_low(keys[gs + j])]);
+        __syncthreads();  // moved before the appends behind them (and before their index entries)
+        const bool indexed = idx_row(ix, u);
+        for (uint32_t j = threadIdx.x; j < a; j += kTpbMut) {
+            const uint32_t v = vals[key_low(keys[gs + j])];
+            write_slot(view, off + w + j, v);
+            if (indexed) idx_add(ix, u, v, w + j, st);
+        }
         __syncthreads();
-        if (idx_row(ix, u)) {
-            idx_reposition_block(view, ix, u, off, w, st);
-            for (uint32_t j = threadIdx.x; j < a; j += kTpbMut) idx_add(ix, u, vals[key_low(keys[gs + j])], w + j, st);
-            __syncthreads();
-        }
         if (threadIdx.x == 0) {
-            desc[u] = RowDesc{off, w + a, rd_meta(cls, 0)};
+            desc[u] = RowDesc{off, w + a, rd_meta(cls, whole ? rd_tombs(d) : 0u)};
             if (stats) {
                 atomicAdd(&stats[kCntChanged], 1ull);
-                atomicAdd(&stats[kCntRelocated], 1ull);
-                atomicAdd(&stats[kCntMovedEntries], static_cast<unsigned long long>(w));
+                atomicAdd(&stats[kCntRelocated], moves ? 1ull : 0ull);
+                atomicAdd(&stats[kCntMovedEntries], moves ? static_cast<unsigned long long>(w) : 0ull);
             }
         }
     }

@@ -137,6 +137,38 @@ def heavy_delete_case() -> Case:
     return Case("heavydelete", n, xadj, adj, batches, source=0)
 
 
+def full_row_case() -> Case:
+    """Rows at and beside the block sizes and worker limits (lane 8, warp 1024
+    and 4096, segment 16384) that overflow while they hold tombstones: batch 0
+    appends as many entries as it deletes (a full row compacts in place),
+    batch 1 outgrows the block (the row moves, tombstones and all where they
+    fit), batch 2 repeats batch 0 on the moved rows; some entries are parallel
+    edges whose first occurrence goes."""
+    rng = np.random.default_rng(23)
+    n = 40000
+    sizes = [2, 3, 4, 5, 7, 8, 9, 15, 16, 17, 31, 32, 33, 255, 256, 257, 1023, 1024, 1025, 2048, 4095, 4096, 4097,
+             16384, 16385]
+    rows = [list(rng.integers(0, max(64, 2 * k), k) % n) for k in sizes]
+    src = np.repeat(np.arange(len(sizes)), sizes)
+    xadj, adj = _csr_from_edges(n, src, np.concatenate(rows))
+    batches = []
+    for k in range(3):
+        du, dv, au, av = [], [], [], []
+        for u, row in enumerate(rows):
+            gone = max(1, len(row) // 16)
+            come = gone + (len(row) if k == 1 and u % 2 else 1 if k == 1 else 0)
+            for i in sorted(rng.choice(len(row), gone, replace=False), reverse=True):
+                du.append(u)
+                dv.append(row[i])
+                row.remove(row[i])  # the first occurrence goes
+            new = list(rng.integers(0, n, come))
+            au += [u] * come
+            av += new
+            row += new
+        batches.append((_u32(du), _u32(dv), _u32(au), _u32(av)))
+    return Case("fullrow", n, xadj, adj, batches, source=0)
+
+
 def grid_case(side: int = 48, batches: int = 3, size: int = 150) -> Case:
     """Road-like high-diameter case: a side x side grid, local insertions."""
     g = gen.grid(side)

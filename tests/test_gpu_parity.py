@@ -13,7 +13,7 @@ import pytest
 
 import oracle
 from coincgraph_b200 import Engine
-from helpers import (ORACLE_MODE, adversarial_case, big_row_case, grid_case, heavy_delete_case, make_engine,
+from helpers import (ORACLE_MODE, adversarial_case, big_row_case, full_row_case, grid_case, heavy_delete_case, make_engine,
                      oracle_trace, rmat_case)
 
 pytestmark = pytest.mark.gpu
@@ -306,6 +306,17 @@ def test_position_index_modes(algo, mode, monkeypatch):
     run_case(heavy_delete_case(), algo, CACHES["zerocopy"])
     run_case_whole_batches(big_row_case(), algo, CACHES["mixed"])
     run_case_whole_batches(rmat_case(11, 3, 400, 400, seed_offset=17), algo, CACHES["resident"])
+
+
+@pytest.mark.parametrize("mode", ["default", "off", "all_rows"])
+@pytest.mark.parametrize("cache", ["resident", "zerocopy", "mixed"])
+def test_full_rows(cache, mode, monkeypatch):
+    """Rows that overflow their block while they hold tombstones: compacted in
+    place or moved with them, positions kept by the index or the scan."""
+    for k, v in INDEX_MODES.get(mode, {}).items():
+        monkeypatch.setenv(k, v)
+    run_case(full_row_case(), "sssp", CACHES[cache])
+    run_case_whole_batches(full_row_case(), "bfs", CACHES[cache])
 
 
 @pytest.mark.parametrize("algo", ["bfs", "sssp", "cc"])
