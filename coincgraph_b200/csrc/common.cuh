@@ -121,14 +121,17 @@ struct AdjView {
     }
 };
 
+// The barrier's arrival counter and its generation, which the waiting blocks
+// poll, lie in cache lines of their own: in one line with each other (and
+// with the error word) the polls delayed the arrivals.
 struct Status {
     uint32_t err;
     uint32_t err_info;
-    uint32_t barrier_count;
-    uint32_t barrier_gen;
-    unsigned long long counters[40];
     uint32_t cc_shift;  // CC: depth bits of a value (label << cc_shift | depth); 0 otherwise
     uint32_t cc_pad;
+    unsigned long long counters[40];
+    alignas(128) uint32_t barrier_count;
+    alignas(128) uint32_t barrier_gen;
 };
 
 enum Counter : int {
@@ -242,14 +245,24 @@ __device__ __forceinline__ void warp_count(unsigned long long *counter, uint32_t
 // Grid-wide barrier for cooperatively launched kernels.  Waits are bounded:
 // after ~2 s without progress the waiting block records kErrBarrier and
 // returns false; every later barrier then returns false at once.
+// One thread per block arrives and polls the generation; the error word and
+// the clock are looked at once per kBarrierPoll polls.
 constexpr long long kBarrierTimeoutCycles = 4000000000LL;
+constexpr uint32_t kBarrierPoll = 64;
+constexpr uint32_t kBarrierSleepNs = 20;
+
+__device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p) {
+    uint32_t v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
 
 __device__ __forceinline__ bool grid_barrier(Status *st) {
     __syncthreads();
     __shared__ uint32_t ok;
     if (threadIdx.x == 0) {
         ok = 1;
-        const uint32_t gen = atomicAdd(&st->barrier_gen, 0);
+        const uint32_t gen = ld_acquire(&st->barrier_gen);
         __threadfence();
         const uint32_t arrived = atomicAdd(&st->barrier_count, 1);
         if (arrived == gridDim.x - 1) {
@@ -258,13 +271,16 @@ __device__ __forceinline__ bool grid_barrier(Status *st) {
             atomicAdd(&st->barrier_gen, 1);
         } else {
             const long long start = clock64();
-            while (ld_volatile(&st->barrier_gen) == gen) {
-                if (ld_volatile(&st->err) & kErrBarrier) break;
-                if (clock64() - start > kBarrierTimeoutCycles) {
-                    set_error(st, kErrBarrier, blockIdx.x);
-                    break;
+            uint32_t polls = 0;
+            while (ld_acquire(&st->barrier_gen) == gen) {
+                if (++polls % kBarrierPoll == 0) {
+                    if (ld_volatile(&st->err) & kErrBarrier) break;
+                    if (clock64() - start > kBarrierTimeoutCycles) {
+                        set_error(st, kErrBarrier, blockIdx.x);
+                        break;
+                    }
                 }
-                __nanosleep(100);
+                __nanosleep(kBarrierSleepNs);
             }
         }
         __threadfence();

@@ -212,6 +212,7 @@ enum SmallIdx : int {
     kHugeR = 30,
     kCompactBig = 31,  // rows to compact above kWarpMove slots, per arena
     kCompactBigR = 32,
+    kPrAct = 33,  // 3 counters of vertices consumed per PageRank sweep, then 3 of its chunks
     kSmallCount = 64
 };
 
@@ -343,6 +344,8 @@ struct cig_handle {
     uint32_t *firstpos_r = nullptr, *indexed_groups_r = nullptr, *chunk_map_r = nullptr;
     uint8_t *gtype_r = nullptr;
     uint32_t *coopf = nullptr, *coopr = nullptr;  // addition groups served one warp each
+    BigRow *pr_chunks = nullptr;  // the sweeps' chunks of long rows (pr_chunk_cap entries)
+    uint64_t pr_chunk_cap() const { return 2 * fwd.seg_total * (kSegEdges / kPrChunk); }
     uint32_t *hugef = nullptr, *huger = nullptr;  // hub deletion groups served by the grid
     void *cub_r = nullptr;
     size_t cub_r_bytes = 0;
@@ -974,6 +977,7 @@ struct cig_handle {
         for (auto &e : bev) cudaEventDestroy(e);
         bev.clear();
         free_queries();
+        dfree(pr_chunks);
         if (side) cudaStreamSynchronize(side);
         if (fork_ev) cudaEventDestroy(fork_ev);
         if (join_ev) cudaEventDestroy(join_ev);
@@ -1299,6 +1303,7 @@ struct cig_handle {
 
     void upload_alloc(DevArena &a, const Layout &L) {
         ArenaAlloc h{};
+            dmalloc(pr_chunks, pr_chunk_cap());
         h.seg_bump = a.seg_used;
         h.seg_total = a.seg_total;
         std::memcpy(h.cur_next, L.cur_next, sizeof(h.cur_next));
@@ -1414,8 +1419,10 @@ struct cig_handle {
         auto a = pr_arrays<T>();
         const T eps = static_cast<T>(opt.pr_epsilon);
         const int p = prof_begin(CIG_STAGE_PR);
-        launch_coop(pr_converge<T>, kTpbPr, fwd.view(), a, eps, static_cast<uint32_t>(opt.pr_max_rounds), seg_hot,
-                    status);
+        CK(cudaMemsetAsync(small + kPrAct, 0, 6 * sizeof(uint32_t), stream));
+        const PrChunks ch{pr_chunks, small + kPrAct + 3, static_cast<uint32_t>(pr_chunk_cap())};
+        launch_coop(pr_converge<T>, kTpbPr, fwd.view(), a, eps, n, static_cast<uint32_t>(opt.pr_max_rounds), ch,
+                    small + kPrAct, seg_hot, status);
         prof_end(p);
         launch(pr_normalize_frontier<T>, persistent_grid(), 256, a);
         launch(pr_set_counts<T>, 1, 1, a);
@@ -2864,7 +2871,7 @@ struct cig_handle {
             if (inval_done) vs += (nn + 1) * sizeof(uint32_t);
             if (opt.algo == CIG_PR) {
                 const uint64_t es = pr64 ? sizeof(double) : sizeof(float);
-                vs += 2 * nn * es + (nn + 1) * es + 2 * nn * sizeof(uint32_t);
+                vs += 2 * nn * es + (nn + 1) * es + 2 * nn * sizeof(uint32_t) + pr_chunk_cap() * sizeof(BigRow);
                 if (!pr64) vs += nn * sizeof(float) + nn * sizeof(double) + 2 * w * sizeof(uint32_t) +
                                  std::max<uint32_t>(pr_hubs, 1) * sizeof(double);
             } else {

@@ -235,12 +235,86 @@ __device__ __forceinline__ uint32_t spread_rank() {
 // Op must provide: __device__ bool edge(bool valid, uint32_t x, P payload, uint32_t y) const;
 // returning true when the edge changed state.
 // edge() is called by all 32 lanes of a warp together (valid=false on padding lanes).
+//
+// The warp tiers: each lane brings at most one row of at most one segment.
+// No block-wide synchronisation, so warps go through their rows at their own
+// pace.
+template <int TPB, class Op, class P>
+__device__ __forceinline__ void expand_rows_warp(const AdjView &view, bool has, uint32_t x, P payload, uint64_t off,
+                                                 uint32_t deg, const Op &op, ExpandSmem<TPB, P> &sm,
+                                                 ExpandCounters &cnt) {
+    const uint32_t lane = lane_id();
+    // Tier 2: warp-wide rows (32 <= deg, always inside one segment).
+    bool med = has && deg >= 32u;
+    uint32_t mmask;
+    while ((mmask = __ballot_sync(kFull, med)) != 0u) {
+        const uint32_t leader = __ffs(mmask) - 1;
+        const uint32_t wx = __shfl_sync(kFull, x, leader);
+        const P wp = __shfl_sync(kFull, payload, leader);
+        const uint32_t wdeg = __shfl_sync(kFull, deg, leader);
+        const uint64_t woff = __shfl_sync(kFull, static_cast<unsigned long long>(off), leader);
+        if (lane == leader) med = false;
+        sweep_row<32u>(view, view.at(woff), wdeg, lane, wx, wp, op, cnt);
+    }
+
+    // Tier 3: small rows gathered through a warp scan.
+    const uint32_t mydeg = (has && deg < 32u) ? deg : 0u;
+    uint32_t incl = mydeg;
+#pragma unroll
+    for (uint32_t o = 1; o < 32u; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += t;
+    }
+    const uint32_t total = __shfl_sync(kFull, incl, 31);
+    if (total == 0) return;
+    const uint32_t wb = (threadIdx.x >> 5) * 32u;
+    sm.f_scan[wb + lane] = incl - mydeg;
+    sm.f_x[wb + lane] = x;
+    sm.f_payload[wb + lane] = payload;
+    sm.f_ptr[wb + lane] = mydeg ? view.at(off) : nullptr;
+    __syncwarp();
+    // Two entries per lane per step: both row reads, then (for ops with
+    // peek) both state reads, are in flight together.
+    for (uint32_t base = 0; base < total; base += 64u) {
+        uint32_t ox[2], y[2];
+        P pl[2];
+        bool valid[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const uint32_t e = base + 32u * j + lane;
+            valid[j] = e < total;
+            ox[j] = 0;
+            y[j] = 0;
+            pl[j] = 0;
+            if (valid[j]) {
+                // Last lane whose exclusive prefix is <= e owns edge e.
+                uint32_t lo = 0, hi = 32;
+                while (hi - lo > 1) {
+                    const uint32_t mid = (lo + hi) >> 1;
+                    if (sm.f_scan[wb + mid] <= e)
+                        lo = mid;
+                    else
+                        hi = mid;
+                }
+                ox[j] = sm.f_x[wb + lo];
+                pl[j] = sm.f_payload[wb + lo];
+                y[j] = __ldg(sm.f_ptr[wb + lo] + (e - sm.f_scan[wb + lo]));
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            y[j] = valid[j] ? view.vid(y[j]) : 0u;
+            valid[j] = valid[j] && y[j] != kTomb;
+        }
+        cnt.hits += edges_n<2>(op, valid, ox, pl, y);
+    }
+    __syncwarp();
+}
+
 template <int TPB, class Op, class P>
 __device__ __forceinline__ void expand_rows(const AdjView &view, bool has, uint32_t x, P payload,
                                             uint64_t off, uint32_t deg, const Op &op, ExpandSmem<TPB, P> &sm,
                                             ExpandCounters &cnt, const Defer &defer = Defer{nullptr, nullptr, 0, 0}) {
-    const uint32_t lane = lane_id();
-    const uint32_t warp = threadIdx.x >> 5;
     if (has) {
         cnt.rows += 1;
         cnt.edges += deg;
@@ -283,72 +357,7 @@ __device__ __forceinline__ void expand_rows(const AdjView &view, bool has, uint3
         }
         __syncthreads();
     }
-
-    // Tier 2: warp-wide rows (32 <= deg < TPB, always inside one segment).
-    bool med = has && deg >= 32u && deg < static_cast<uint32_t>(TPB);
-    uint32_t mmask;
-    while ((mmask = __ballot_sync(kFull, med)) != 0u) {
-        const uint32_t leader = __ffs(mmask) - 1;
-        const uint32_t wx = __shfl_sync(kFull, x, leader);
-        const P wp = __shfl_sync(kFull, payload, leader);
-        const uint32_t wdeg = __shfl_sync(kFull, deg, leader);
-        const uint64_t woff = __shfl_sync(kFull, static_cast<unsigned long long>(off), leader);
-        if (lane == leader) med = false;
-        sweep_row<32u>(view, view.at(woff), wdeg, lane, wx, wp, op, cnt);
-    }
-
-    // Tier 3: small rows gathered through a warp scan.
-    const uint32_t mydeg = (has && deg < 32u) ? deg : 0u;
-    uint32_t incl = mydeg;
-#pragma unroll
-    for (uint32_t o = 1; o < 32u; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(kFull, incl, o);
-        if (lane >= o) incl += t;
-    }
-    const uint32_t total = __shfl_sync(kFull, incl, 31);
-    if (total == 0) return;
-    const uint32_t wb = warp * 32u;
-    sm.f_scan[wb + lane] = incl - mydeg;
-    sm.f_x[wb + lane] = x;
-    sm.f_payload[wb + lane] = payload;
-    sm.f_ptr[wb + lane] = mydeg ? view.at(off) : nullptr;
-    __syncwarp();
-    // Two entries per lane per step: both row reads, then (for ops with
-    // peek) both state reads, are in flight together.
-    for (uint32_t base = 0; base < total; base += 64u) {
-        uint32_t ox[2], y[2];
-        P pl[2];
-        bool valid[2];
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const uint32_t e = base + 32u * j + lane;
-            valid[j] = e < total;
-            ox[j] = 0;
-            y[j] = 0;
-            pl[j] = 0;
-            if (valid[j]) {
-                // Last lane whose exclusive prefix is <= e owns edge e.
-                uint32_t lo = 0, hi = 32;
-                while (hi - lo > 1) {
-                    const uint32_t mid = (lo + hi) >> 1;
-                    if (sm.f_scan[wb + mid] <= e)
-                        lo = mid;
-                    else
-                        hi = mid;
-                }
-                ox[j] = sm.f_x[wb + lo];
-                pl[j] = sm.f_payload[wb + lo];
-                y[j] = __ldg(sm.f_ptr[wb + lo] + (e - sm.f_scan[wb + lo]));
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            y[j] = valid[j] ? view.vid(y[j]) : 0u;
-            valid[j] = valid[j] && y[j] != kTomb;
-        }
-        cnt.hits += edges_n<2>(op, valid, ox, pl, y);
-    }
-    __syncwarp();
+    expand_rows_warp<TPB>(view, has && deg < static_cast<uint32_t>(TPB), x, payload, off, deg, op, sm, cnt);
 }
 
 // Expand the deferred rows: chunk g of the concatenated chunk sequence goes

@@ -8,8 +8,9 @@
 // first withdraws the old contributions of every touched source over its old
 // row, mutates the topology, then re-adds them over the new row.
 //
-// Differences: one persistent cooperative kernel runs consume and scatter
-// rounds with grid barriers (no host count read per round); the rank is
+// Differences: one persistent cooperative kernel converges (no host count
+// read per round): queue rounds while few vertices hold a residual above
+// epsilon, sweeps over all vertices once many do (pr_converge); the rank is
 // FP32 with a per-vertex Kahan compensation term (or FP64 throughout); the
 // batch reports the FP64 L1 norm of the residual.
 //
@@ -25,6 +26,7 @@
 
 #include "common.cuh"
 #include "expand.cuh"
+#include "traverse.cuh"  // BigList
 
 namespace cig {
 
@@ -183,39 +185,263 @@ __global__ void pr_init(PrArrays<T> a, uint32_t n) {
 
 constexpr int kTpbPr = 256;
 
-// Persistent converge loop (Runtime::Converge, pr_residual.cuh:171-187):
-// each round consumes the queued residuals (Consume, :54-71), then scatters
-// them (Scatter, :74-100); the queue of round r is q[r&1] with cnt[r%3].
-// On exit `final_round` holds the round whose queue is still pending.
+// Sweep payload: the contribution's bits, in a word of its own width.
 template <class T>
-__global__ void __launch_bounds__(kTpbPr) pr_converge(AdjView fwd, PrArrays<T> a, T eps, uint32_t max_rounds,
+struct PrBits;
+template <>
+struct PrBits<float> {
+    using type = uint32_t;
+    static __device__ __forceinline__ type to(float c) { return __float_as_uint(c); }
+    static __device__ __forceinline__ float from(type b) { return __uint_as_float(b); }
+};
+template <>
+struct PrBits<double> {
+    using type = unsigned long long;
+    static __device__ __forceinline__ type to(double c) { return static_cast<type>(__double_as_longlong(c)); }
+    static __device__ __forceinline__ double from(type b) { return __longlong_as_double(static_cast<long long>(b)); }
+};
+
+// Add in memory without a result (an atomicAdd whose result is unused was
+// still issued as one that returns it).
+__device__ __forceinline__ void red_add(float *p, float x) {
+    asm volatile("red.relaxed.gpu.global.add.f32 [%0], %1;" ::"l"(p), "f"(x) : "memory");
+}
+__device__ __forceinline__ void red_add(double *p, double x) {
+    asm volatile("red.relaxed.gpu.global.add.f64 [%0], %1;" ::"l"(p), "d"(x) : "memory");
+}
+
+// Sweeps: add to the residual, with no result to wait for (the sweep over
+// the vertices finds what crossed epsilon).  The hub lookups of a thread's
+// entries are in flight together (peek).
+template <class T>
+struct PrSweepOp {
+    PrArrays<T> a;
+    __device__ __forceinline__ int32_t peek(uint32_t y) const { return hub_slot(a, y); }
+    __device__ __forceinline__ bool edge_peeked(bool valid, uint32_t, typename PrBits<T>::type c, uint32_t y,
+                                                int32_t h) const {
+        if (valid) {
+            if (h >= 0)
+                red_add(a.res_hub + h, static_cast<double>(PrBits<T>::from(c)));
+            else
+                red_add(a.res + y, PrBits<T>::from(c));
+        }
+        return valid;
+    }
+    __device__ __forceinline__ bool edge(bool valid, uint32_t x, typename PrBits<T>::type c, uint32_t y) const {
+        return edge_peeked(valid, x, c, y, valid ? peek(y) : -1);
+    }
+};
+
+// v's residual while others add to it: true when it is above epsilon.
+template <class T>
+__device__ __forceinline__ bool res_above(const PrArrays<T> &a, uint32_t v, int32_t h, T eps, bool &finite) {
+    if (h >= 0) {
+        const double r = __ldcg(a.res_hub + h);
+        finite = isfinite(r);
+        return fabs(r) > static_cast<double>(eps);
+    }
+    const T r = __ldcg(a.res + v);
+    finite = pr_finite(r);
+    return pr_abs(r) > eps;
+}
+
+// Take it, leaving zero.
+template <class T>
+__device__ __forceinline__ double res_exchange(const PrArrays<T> &a, uint32_t v, int32_t h) {
+    if (h >= 0)
+        return __longlong_as_double(
+            static_cast<long long>(atomicExch(reinterpret_cast<unsigned long long *>(a.res_hub + h), 0ull)));
+    using B = typename PrBits<T>::type;
+    return static_cast<double>(PrBits<T>::from(atomicExch(reinterpret_cast<B *>(a.res + v), B{0})));
+}
+
+// An FP64 residual enters an FP32 rank as two compensated adds (its float
+// part and the rest), so nothing of it is lost.  Returns alpha * r / deg.
+template <class T>
+__device__ __forceinline__ T rank_consume(const PrArrays<T> &a, uint32_t v, double r, uint32_t deg) {
+    const T hi = static_cast<T>(r);
+    rank_add(a, v, hi);
+    if (sizeof(T) == 4) {
+        const T lo = static_cast<T>(r - static_cast<double>(hi));
+        if (lo != T(0)) rank_add(a, v, lo);
+    }
+    return deg ? static_cast<T>(kAlphaD * r / static_cast<double>(deg)) : T(0);
+}
+
+// Rows of at least this many entries are pushed by the whole grid, a warp
+// per chunk of as many entries.
+constexpr uint32_t kPrChunk = 512;
+
+// The chunks a sweep leaves to the whole grid; `cap` covers every slot of the
+// arena (2 * slots / kPrChunk), so it cannot run out.
+struct PrChunks {
+    BigRow *rows;
+    uint32_t *cnt;  // 3 counters
+    uint32_t cap;
+};
+
+// Share of the vertices above which a round's queue is left for sweeps.
+constexpr uint32_t kPrSweepShare = 16;
+
+// Sweeps over all vertices until none holds a residual above epsilon.  Every
+// vertex above it is consumed and pushed in one go, its residual taken with
+// an exchange while other vertices add to it: what reaches a vertex before
+// its turn is pushed on in the same sweep (Gauss-Seidel rather than Jacobi
+// order), which needs about 0.6 of the pushes and half the rounds.  Against
+// the queue rounds a push is an add without a result (no threshold test,
+// queue claim or append per edge), and the consume pass with its barrier is
+// gone.  Warps take tiles of vertices and push their rows without waiting for
+// one another; the chunks of rows of kPrChunk entries and more are pushed by
+// the whole grid after a barrier, in sweeps that have any.  (With block-wide
+// rows inside the sweep nearly half of all warp time was spent at block
+// barriers.)  Tiles shrink with n so that every warp gets a few.
+// `act` and `ch.cnt`: three counters each (sweep s uses s mod 3, clears
+// (s+1) mod 3, which was last read before the previous barrier).
+// Returns false on a barrier error; `done` tells whether it converged.
+template <class T>
+__device__ __forceinline__ bool pr_sweeps(const AdjView &fwd, const PrArrays<T> &a, T eps, uint32_t n,
+                                          uint32_t max_sweeps, const PrChunks &ch, uint32_t *act, uint32_t *seg_hot,
+                                          ExpandSmem<kTpbPr, typename PrBits<T>::type> &sm, ExpandCounters &cnt,
+                                          uint32_t &sweeps, bool &done, Status *st) {
+    using B = typename PrBits<T>::type;
+    const PrSweepOp<T> op{a};
+    const uint32_t lane = lane_id();
+    const uint32_t warps = (gridDim.x * kTpbPr) >> 5;
+    const uint32_t wid = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    uint32_t tile = 32;
+    while (tile > 8 && n < 4ull * warps * tile) tile >>= 1;
+    done = false;
+    for (sweeps = 0;; ++sweeps) {
+        if (sweeps && ld_volatile(act + (sweeps + 2) % 3) == 0) {
+            done = true;
+            return true;
+        }
+        if (sweeps >= max_sweeps) return true;
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            act[(sweeps + 1) % 3] = 0;
+            ch.cnt[(sweeps + 1) % 3] = 0;
+        }
+        uint32_t *ch_cnt = ch.cnt + sweeps % 3;
+        uint32_t mine = 0;
+        for (uint64_t base = static_cast<uint64_t>(wid) * tile; base < n; base += static_cast<uint64_t>(warps) * tile) {
+            const uint32_t v = static_cast<uint32_t>(base) + lane;
+            const bool in = lane < tile && v < n && v >= static_cast<uint32_t>(base);
+            bool has = false;
+            uint32_t deg = 0;
+            uint64_t off = 0;
+            T c = T(0);
+            if (in) {
+                const int32_t h = hub_slot(a, v);
+                bool finite = true;
+                has = res_above(a, v, h, eps, finite);
+                if (!finite) set_error(st, kErrNonFinite, v);
+                if (has) {
+                    const RowDesc d = fwd.desc[v];
+                    ++mine;
+                    c = rank_consume(a, v, res_exchange(a, v, h), rd_live(d));
+                    deg = d.len;
+                    off = d.off;
+                    has = deg > 0 && c != T(0);
+                    if (has) {
+                        cnt.rows += 1;
+                        cnt.edges += deg;
+                        if (fwd.cached(off)) cnt.edges_cached += deg;
+                        if (seg_hot && sweeps == 0) atomicAdd(seg_hot + (off >> kSegShift), deg);
+                    }
+                }
+            }
+            uint32_t bigs = __ballot_sync(kFull, has && deg >= kPrChunk);
+            while (bigs) {
+                const uint32_t l = __ffs(bigs) - 1;
+                bigs &= bigs - 1;
+                const uint32_t ldeg = __shfl_sync(kFull, deg, l), lv = __shfl_sync(kFull, v, l);
+                const uint64_t loff = __shfl_sync(kFull, static_cast<unsigned long long>(off), l);
+                const B lc = __shfl_sync(kFull, PrBits<T>::to(c), l);
+                const uint32_t k = (ldeg + kPrChunk - 1) / kPrChunk;
+                uint32_t at = 0;
+                if (lane == 0) at = atomicAdd(ch_cnt, k);
+                at = __shfl_sync(kFull, at, 0);
+                for (uint32_t i = lane; i < k; i += 32u) {
+                    if (at + i < ch.cap)
+                        ch.rows[at + i] = BigRow{loff + static_cast<uint64_t>(i) * kPrChunk,
+                                                 static_cast<unsigned long long>(lc), lv,
+                                                 min(kPrChunk, ldeg - i * kPrChunk)};
+                    else
+                        set_error(st, kErrQueue, at + i);
+                }
+            }
+            expand_rows_warp<kTpbPr>(fwd, has && deg < kPrChunk, v, PrBits<T>::to(c), off, deg, op, sm, cnt);
+        }
+        mine = __reduce_add_sync(kFull, mine);
+        if (lane == 0 && mine) atomicAdd(act + sweeps % 3, mine);
+        if (!grid_barrier(st)) return false;
+        const uint32_t nch = min(ld_volatile(ch_cnt), ch.cap);
+        if (nch) {
+            for (uint32_t i = wid; i < nch; i += warps) {
+                const BigRow r = ch.rows[i];
+                // A chunk starts a multiple of kPrChunk into a block that covers
+                // whole segments or lies in one: it never straddles two.
+                sweep_row<32u>(fwd, fwd.at(r.off), r.deg, lane, r.x, static_cast<B>(r.payload), op, cnt);
+            }
+            if (!grid_barrier(st)) return false;
+        }
+    }
+}
+
+// Persistent converge loop (Runtime::Converge, pr_residual.cuh:171-187).
+// Queue rounds: each consumes the queued residuals (Consume, :54-71), then
+// scatters them (Scatter, :74-100); the queue of round r is q[r&1] with
+// cnt[r%3].  A queue of more than n / kPrSweepShare vertices is left for
+// sweeps (pr_sweeps), which run to the end.  On exit `final_round` holds the
+// round whose queue is still pending.
+template <class T>
+__global__ void __launch_bounds__(kTpbPr, 4) pr_converge(AdjView fwd, PrArrays<T> a, T eps, uint32_t n,
+                                                      uint32_t max_rounds, PrChunks ch, uint32_t *act,
                                                       uint32_t *seg_hot, Status *st) {
-    __shared__ ExpandSmem<kTpbPr> sm;
+    using B = typename PrBits<T>::type;
+    __shared__ union {
+        ExpandSmem<kTpbPr> rounds;
+        ExpandSmem<kTpbPr, B> sweeps;
+    } sm;
     ExpandCounters cnt;
-    uint32_t r = 0;
+    uint32_t r = 0, sweeps = 0;
     for (;; ++r) {
         const uint32_t n_in = ld_volatile(a.cnt + (r % 3));
         if (n_in == 0 || r >= max_rounds) break;
-        if (blockIdx.x == 0 && threadIdx.x == 0) a.cnt[(r + 2) % 3] = 0;
         const uint32_t *in = (r & 1) ? a.q1 : a.q0;
+        if (n_in > n / kPrSweepShare) {
+            for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_in; i += gridDim.x * blockDim.x)
+                a.queued[__ldcg(in + i)] = 0u;
+            bool done = false;
+            if (!pr_sweeps(fwd, a, eps, n, max_rounds - r, ch, act, seg_hot, sm.sweeps, cnt, sweeps, done, st)) break;
+            // The pending queue: empty, or (round bound) rebuilt in q0.
+            if (blockIdx.x == 0 && threadIdx.x < 3) a.cnt[threadIdx.x] = 0;
+            if (!done) {
+                if (!grid_barrier(st)) break;
+                const uint32_t rounded = (n + 31u) & ~31u;
+                for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < rounded; v += gridDim.x * blockDim.x) {
+                    bool want = false;
+                    if (v < n) {
+                        const int32_t h = hub_slot(a, v);
+                        want = h >= 0 ? fabs(__ldcg(a.res_hub + h)) > static_cast<double>(eps)
+                                      : pr_abs(__ldcg(a.res + v)) > eps;
+                        if (want) a.queued[v] = 1u;
+                    }
+                    warp_enqueue(want, v, a.q0, a.cnt, a.cap, st);
+                }
+            }
+            sweeps += r;
+            r = 0;
+            break;
+        }
+        if (blockIdx.x == 0 && threadIdx.x == 0) a.cnt[(r + 2) % 3] = 0;
         for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_in; i += gridDim.x * blockDim.x) {
             const uint32_t v = __ldcg(in + i);
             a.queued[v] = 0u;
             T c = T(0);
             double r64 = 0.0;
             bool finite = true;
-            if (res_take(a, v, eps, r64, finite)) {
-                // An FP64 residual enters an FP32 rank as two compensated adds
-                // (its float part and the rest), so nothing of it is lost.
-                const T hi = static_cast<T>(r64);
-                rank_add(a, v, hi);
-                if (sizeof(T) == 4) {
-                    const T lo = static_cast<T>(r64 - static_cast<double>(hi));
-                    if (lo != T(0)) rank_add(a, v, lo);
-                }
-                const uint32_t deg = rd_live(fwd.desc[v]);  // out-degree: live entries only
-                if (deg) c = static_cast<T>(kAlphaD * r64 / static_cast<double>(deg));
-            }
+            if (res_take(a, v, eps, r64, finite)) c = rank_consume(a, v, r64, rd_live(fwd.desc[v]));
             if (!finite) set_error(st, kErrNonFinite, v);
             a.contrib[i] = c;
         }
@@ -234,14 +460,14 @@ __global__ void __launch_bounds__(kTpbPr) pr_converge(AdjView fwd, PrArrays<T> a
                 has = deg > 0 && __ldcg(a.contrib + i) != T(0);
                 if (has && seg_hot) atomicAdd(seg_hot + (off >> kSegShift), deg);
             }
-            expand_rows<kTpbPr>(fwd, has, v, i, off, deg, op, sm, cnt);
+            expand_rows<kTpbPr>(fwd, has, v, i, off, deg, op, sm.rounds, cnt);
         }
         if (!grid_barrier(st)) break;
     }
     flush_counters(st, cnt, kCntPr);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         *a.final_round = r;
-        atomicAdd(&st->counters[kCntPrRounds], static_cast<unsigned long long>(r));
+        atomicAdd(&st->counters[kCntPrRounds], static_cast<unsigned long long>(r + sweeps));
     }
 }
 
@@ -296,7 +522,7 @@ __global__ void pr_amend_contrib(const RowDesc *desc, PrArrays<T> a, const uint3
 }
 
 template <class T>
-__global__ void __launch_bounds__(kTpbPr) pr_amend_scatter(AdjView fwd, PrArrays<T> a, const uint32_t *list,
+__global__ void __launch_bounds__(kTpbPr, 4) pr_amend_scatter(AdjView fwd, PrArrays<T> a, const uint32_t *list,
                                                            const uint32_t *count, const T *contrib, T eps,
                                                            Status *st) {
     __shared__ ExpandSmem<kTpbPr> sm;
@@ -347,7 +573,7 @@ struct PrAmendOp {
 };
 
 template <class T>
-__global__ void __launch_bounds__(kTpbPr) pr_amend_scatter64(AdjView fwd, const uint32_t *list, const uint32_t *count,
+__global__ void __launch_bounds__(kTpbPr, 4) pr_amend_scatter64(AdjView fwd, const uint32_t *list, const uint32_t *count,
                                                              const double *contrib, double *acc, Status *st) {
     __shared__ ExpandSmem<kTpbPr> sm;
     ExpandCounters cnt;

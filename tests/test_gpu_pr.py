@@ -63,3 +63,27 @@ def test_pr_reference_check_at_default_error():
             assert g.pr_check(rank, res, 1e-6)["ok"] == 1.0
             if ref is not None:
                 assert ref.pr_check(rank, res, 1e-6)
+
+
+@pytest.mark.parametrize("fp64", [False, True])
+@pytest.mark.parametrize("make", [lambda: rmat_case(9, 1, 50, 50, seed_offset=22), big_row_case])
+def test_pr_round_bound_keeps_the_pending_queue(make, fp64):
+    """A solve cut off by pr_max_rounds leaves every vertex above epsilon
+    queued: empty batches then carry it on to the same fixed point (rows on
+    both sides of the sweeps' chunk length, and rows over several segments)."""
+    case = make()
+    g = oracle.Graph(case.n, case.xadj, case.adj)
+    du, dv, au, av = case.batches[0]
+    g.delete(du, dv)
+    g.add(au, av)
+    x, ok = g.pagerank(1e-15, 100000)
+    assert ok
+    with Engine("pr", pr_epsilon=1e-9, pr_max_rounds=3, flags=FLAG_PR_FP64 if fp64 else 0) as eng:
+        eng.load_csr(case.n, case.xadj, case.adj)
+        eng.init()
+        s = eng.apply_batch(du, dv, au, av)
+        assert s["pr_rounds"] <= 3 and s["pr_residual_l1"] > case.n * 1e-9
+        for _ in range(120):
+            s = eng.apply_batch([], [], [], [])
+        assert s["pr_residual_l1"] <= case.n * 1e-9 * 1.01
+        assert max_rel(eng.pagerank(fp64=fp64)[0], x) <= 1e-6
