@@ -676,8 +676,7 @@ __device__ __forceinline__ uint32_t del_index_key(const AdjView &view, RowDesc *
     write_slot(view, d.off + e.x, kTomb);
     if (count_tomb) atomicAdd(&desc[u].meta, 1u << 6);
     if (e.y == 1u) {
-        ix.val[s] = make_uint2(kInf, 0u);
-        ix.keys[s] = kIdxDeleted;
+        ix.val[s] = make_uint2(kInf, 0u);  // the key keeps its slot for the next time it is inserted
     } else {
         uint32_t q = e.x + 1;
         while (q < d.len && *view.at(d.off + q) != v) ++q;
@@ -731,8 +730,7 @@ __device__ __forceinline__ uint32_t del_index_keys(const AdjView &view, RowDesc 
         write_slot(view, d[j].off + e[j].x, kTomb);
         atomicAdd(&desc[u].meta, 1u << 6);
         if (e[j].y == 1u) {
-            ix.val[slot[j]] = make_uint2(kInf, 0u);
-            ix.keys[slot[j]] = kIdxDeleted;
+            ix.val[slot[j]] = make_uint2(kInf, 0u);  // the key keeps its slot
         } else {
             uint32_t q = e[j].x + 1;
             while (q < d[j].len && *view.at(d[j].off + q) != v) ++q;
@@ -879,7 +877,6 @@ __global__ void idx_fix_ordered(AdjView view, const RowDesc *desc, const unsigne
                     ++live;
                 }
             ix.val[s] = make_uint2(first, live);
-            if (!live) ix.keys[s] = kIdxDeleted;
         }
     }
 }

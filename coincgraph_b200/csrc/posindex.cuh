@@ -11,14 +11,18 @@
 // the number of live occurrences.  Deletions look positions up; appends,
 // relocations and compactions keep the entries current.
 //
-// Table: keys (u << 32 | v), EMPTY / DELETED sentinels, linear probing with
+// Table: keys (u << 32 | v), an EMPTY sentinel, linear probing with
 // a bounded probe length (kIdxProbe; running past it is reported as
 // kErrInternal, never a fault).  Values {pos, count} start as {kInf, 0} in
 // every slot, so an insert is a key CAS followed by atomicMin / atomicAdd
-// with no initialisation race.  A slot is never reused after DELETED (so a
-// probe never meets an EMPTY slot before its key); the host sizes the table
-// with room for as many inserts as it has entries and rebuilds it before the
-// keys inserted since the last build can take the load factor past one half.
+// with no initialisation race.  A key whose last occurrence is deleted keeps
+// its slot with {kInf, 0}, as an absent key, and is found there when it is
+// inserted again.  (Marked deleted, every delete and re-insert of an edge
+// left one more slot for its next probe to pass: a batch of 1,000 + 1,000
+// recurring edges on R-MAT s16 went from 320 to 600 us within 1,000 batches.)
+// The host sizes the table with room for as many inserts as it has entries
+// and rebuilds it before the keys inserted since the last build can take the
+// load factor past one half.
 #pragma once
 
 #include "common.cuh"
@@ -26,7 +30,6 @@
 namespace cig {
 
 constexpr unsigned long long kIdxEmpty = ~0ull;
-constexpr unsigned long long kIdxDeleted = ~0ull - 1ull;
 constexpr uint32_t kIdxCls = 5;       // default: rows in blocks of >= 32 slots are indexed
 constexpr uint32_t kIdxProbe = 4096;  // probe bound
 
