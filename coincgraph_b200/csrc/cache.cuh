@@ -38,11 +38,7 @@ enum SegCtl : int {
     kCtlNewLast = 2,    // segments created since the last service
     kCtlVictims = 3,    // cold resident segments found this service
     kCtlAdmits = 4,     // hot host segments found this service
-    kCtlEvictNeed = 5,  // evictions this service
-    kCtlReserve = 6,    // free slots kept for new segments
-    kCtlThreshold = 7,  // victims: bucket below this ...
-    kCtlExtra = 8,      // ... plus this many from the threshold bucket
-    kCtlExtraTaken = 9,
+    kCtlExtraTaken = 5, // victims taken from the threshold bucket
     kCtlHist = 16,      // kScoreBuckets counters of resident scores
     kCtlCount = 16 + kScoreBuckets
 };
@@ -67,11 +63,10 @@ __device__ __forceinline__ void seg_touch(uint32_t *hot, uint64_t off, uint32_t 
     if (hot && len) atomicAdd(hot + (off >> kSegShift), len);
 }
 
-// Slots for the segments the allocator created since the last call.
-// One thread; a handful of segments per batch.
-__global__ void seg_assign_new(SegTable t, const unsigned long long *seg_bump, Status *st) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const uint32_t bump = static_cast<uint32_t>(min(*seg_bump, static_cast<unsigned long long>(t.nsegs)));
+// Slots for the segments the allocator created since the last call (`bump`:
+// its bump pointer).  One thread; a handful of segments per batch.
+__device__ __forceinline__ void seg_assign_new(const SegTable &t, unsigned long long seg_bump, Status *st) {
+    const uint32_t bump = static_cast<uint32_t>(min(seg_bump, static_cast<unsigned long long>(t.nsegs)));
     const uint32_t seen = t.ctl[kCtlBumpSeen];
     uint32_t top = t.ctl[kCtlFreeTop];
     for (uint32_t s = seen; s < bump; ++s) {
@@ -88,73 +83,14 @@ __global__ void seg_assign_new(SegTable t, const unsigned long long *seg_bump, S
     t.ctl[kCtlBumpSeen] = max(seen, bump);
 }
 
+// Clear the per-batch counters, before the batch's first allocation; one
+// thread per word (at least kCtlCount threads).
+__device__ __forceinline__ void seg_ctl_clear(uint32_t *ctl) {
+    const uint32_t i = threadIdx.x;
+    if (i < kCtlCount && i != kCtlFreeTop && i != kCtlBumpSeen) ctl[i] = 0u;
+}
+
 __device__ __forceinline__ uint32_t score_bucket(uint32_t sc) { return 32u - __clz(sc); }
-
-// Decay scores, histogram the resident ones (evictable: below cold_score)
-// and list admission candidates among hot host segments.  Grid-stride.
-__global__ void seg_rescore(SegTable t, uint32_t bump) {
-    __shared__ uint32_t hist[kScoreBuckets];
-    for (uint32_t b = threadIdx.x; b < kScoreBuckets; b += blockDim.x) hist[b] = 0;
-    __syncthreads();
-    for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < bump; s += gridDim.x * blockDim.x) {
-        const uint32_t h = t.hot[s];
-        if (h) t.hot[s] = 0;
-        const uint32_t sc = (t.score[s] >> 1) + min(h, 1u << 24);
-        t.score[s] = sc;
-        if (t.seg_slot[s] >= 0) {
-            if (sc < t.cold_score) atomicAdd(hist + score_bucket(sc), 1u);
-        } else if (sc >= t.admit_score) {
-            const uint32_t i = atomicAdd(t.ctl + kCtlAdmits, 1u);
-            if (i < kMaxAdmit) t.admits[i] = s;
-        }
-    }
-    __syncthreads();
-    for (uint32_t b = threadIdx.x; b < kScoreBuckets; b += blockDim.x)
-        if (hist[b]) atomicAdd(t.ctl + kCtlHist + b, hist[b]);
-}
-
-// How many to evict: enough to keep `reserve` slots free for new segments
-// (twice the last batches' count, 16..1024) plus the admissions; the
-// coldest first: whole buckets below a threshold, then part of it.
-__global__ void seg_plan(SegTable t) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const uint32_t reserve = min(1024u, max(16u, 2u * t.ctl[kCtlNewLast]));
-    t.ctl[kCtlNewLast] = 0;
-    t.ctl[kCtlReserve] = reserve;
-    const uint32_t want = reserve + min(t.ctl[kCtlAdmits], kMaxAdmit);
-    const uint32_t top = t.ctl[kCtlFreeTop];
-    uint32_t need = min(want > top ? want - top : 0u, kMaxEvict);
-    uint32_t below = 0, b = 0;
-    for (; b < static_cast<uint32_t>(kScoreBuckets); ++b) {
-        const uint32_t c = t.ctl[kCtlHist + b];
-        if (below + c >= need) break;
-        below += c;
-    }
-    if (b == static_cast<uint32_t>(kScoreBuckets)) need = below;  // fewer evictable segments than wanted
-    t.ctl[kCtlThreshold] = b;
-    t.ctl[kCtlExtra] = need - below;
-    t.ctl[kCtlExtraTaken] = 0;
-    t.ctl[kCtlEvictNeed] = need;
-}
-
-// The victims chosen by seg_plan.  Grid-stride over segments.
-__global__ void seg_pick(SegTable t, uint32_t bump) {
-    const uint32_t thr = t.ctl[kCtlThreshold], extra = t.ctl[kCtlExtra], need = t.ctl[kCtlEvictNeed];
-    if (!need) return;
-    for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < bump; s += gridDim.x * blockDim.x) {
-        const int32_t slot = t.seg_slot[s];
-        if (slot < 0) continue;
-        const uint32_t sc = t.score[s];
-        if (sc >= t.cold_score) continue;
-        const uint32_t b = score_bucket(sc);
-        bool take = b < thr;
-        if (!take && b == thr && extra) take = atomicAdd(t.ctl + kCtlExtraTaken, 1u) < extra;
-        if (take) {
-            const uint32_t i = atomicAdd(t.ctl + kCtlVictims, 1u);
-            if (i < need) t.victims[i] = static_cast<uint32_t>(slot);
-        }
-    }
-}
 
 // One block copies one 64 KiB segment: each thread has eight 16-byte loads
 // in flight before it stores them, so a copy from host memory (about 2 us
@@ -176,39 +112,105 @@ __device__ __forceinline__ void copy_segment(uint4 *dst, const uint4 *src) {
     }
 }
 
-// One block per victim slot: write back if dirty, unmap, free the slot.
-__global__ void seg_evict(SegTable t, const uint32_t *cache, uint32_t *host, Status *st) {
-    const uint32_t nv = min(t.ctl[kCtlEvictNeed], t.ctl[kCtlVictims]);
-    for (uint32_t v = blockIdx.x; v < nv; v += gridDim.x) {
-        const uint32_t slot = t.victims[v];
-        const int32_t seg = t.slot_seg[slot];
-        if (seg < 0) continue;
-        if (t.seg_dirty[seg])
-            copy_segment(reinterpret_cast<uint4 *>(host + (static_cast<uint64_t>(seg) << kSegShift)),
-                         reinterpret_cast<const uint4 *>(cache + (static_cast<uint64_t>(slot) << kSegShift)));
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            __threadfence_system();
-            t.seg_dirty[seg] = 0;
-            t.seg_slot[seg] = -1;
-            t.slot_seg[slot] = -1;
-            const uint32_t pos = atomicAdd(t.ctl + kCtlFreeTop, 1u);
-            if (pos < t.nslots)
-                t.free_slots[pos] = slot;
-            else
-                set_error(st, kErrInternal, pos);
-            atomicAdd(&st->counters[kCntSegEvicted], 1ull);
-        }
-        __syncthreads();
-    }
-}
-
-// One block per admission candidate while free slots above the reserve
-// last: copy the host segment into a slot and map it.
-__global__ void seg_admit(SegTable t, uint32_t *cache, const uint32_t *host, Status *st) {
+// The service of one batch (cooperative launch), in four steps with a grid
+// barrier between them; a batch with nothing to evict or admit ends after the
+// first.  (Five kernels and two memsets before: 16 to 25 us of launches for
+// what is mostly one pass over the scores.)  The counters of seg_ctl_clear
+// are zero at launch, kCtlNewLast counts this batch's new segments.
+//   1. decay the scores, histogram the resident ones that may go (below
+//      cold_score), list hot host segments as admission candidates;
+//   2. choose the victims: enough to keep `reserve` slots free for new
+//      segments (twice the last batch's count, 16..1024) plus the admissions,
+//      the coldest first: whole buckets below a threshold, then part of it;
+//   3. a block per victim: write back if dirty, unmap, free the slot;
+//   4. a block per candidate while free slots above the reserve last: copy
+//      the host segment into a slot and map it.
+__global__ void __launch_bounds__(256) seg_service(SegTable t, uint32_t bump, uint32_t *cache, uint32_t *host,
+                                                   Status *st) {
+    __shared__ uint32_t hist[kScoreBuckets];
+    __shared__ uint32_t s_reserve, s_need, s_thr, s_extra;
     __shared__ int32_t slot_s;
-    const uint32_t na = min(t.ctl[kCtlAdmits], kMaxAdmit);
-    const uint32_t reserve = t.ctl[kCtlReserve];
+    const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, gthreads = gridDim.x * blockDim.x;
+    for (uint32_t b = threadIdx.x; b < kScoreBuckets; b += blockDim.x) hist[b] = 0;
+    __syncthreads();
+    for (uint32_t s = gtid; s < bump; s += gthreads) {
+        const uint32_t h = t.hot[s];
+        if (h) t.hot[s] = 0;
+        const uint32_t sc = (t.score[s] >> 1) + min(h, 1u << 24);
+        t.score[s] = sc;
+        if (t.seg_slot[s] >= 0) {
+            if (sc < t.cold_score) atomicAdd(hist + score_bucket(sc), 1u);
+        } else if (sc >= t.admit_score) {
+            const uint32_t i = atomicAdd(t.ctl + kCtlAdmits, 1u);
+            if (i < kMaxAdmit) t.admits[i] = s;
+        }
+    }
+    __syncthreads();
+    for (uint32_t b = threadIdx.x; b < kScoreBuckets; b += blockDim.x)
+        if (hist[b]) atomicAdd(t.ctl + kCtlHist + b, hist[b]);
+    if (!grid_barrier(st)) return;
+    const uint32_t na = min(ld_volatile(t.ctl + kCtlAdmits), kMaxAdmit);
+    if (threadIdx.x == 0) {  // every block comes to the same plan
+        const uint32_t reserve = min(1024u, max(16u, 2u * ld_volatile(t.ctl + kCtlNewLast)));
+        const uint32_t want = reserve + na;
+        const uint32_t top = ld_volatile(t.ctl + kCtlFreeTop);
+        uint32_t need = min(want > top ? want - top : 0u, kMaxEvict);
+        uint32_t below = 0, b = 0;
+        if (need)
+            for (; b < static_cast<uint32_t>(kScoreBuckets); ++b) {
+                const uint32_t c = ld_volatile(t.ctl + kCtlHist + b);
+                if (below + c >= need) break;
+                below += c;
+            }
+        if (b == static_cast<uint32_t>(kScoreBuckets)) need = below;  // fewer evictable segments than wanted
+        s_reserve = reserve;
+        s_need = need;
+        s_thr = b;
+        s_extra = need - below;
+    }
+    __syncthreads();
+    const uint32_t need = s_need, reserve = s_reserve;
+    if (!need && !na) return;
+    if (need) {
+        for (uint32_t s = gtid; s < bump; s += gthreads) {
+            const int32_t slot = t.seg_slot[s];
+            if (slot < 0) continue;
+            const uint32_t sc = t.score[s];
+            if (sc >= t.cold_score) continue;
+            const uint32_t b = score_bucket(sc);
+            bool take = b < s_thr;
+            if (!take && b == s_thr && s_extra) take = atomicAdd(t.ctl + kCtlExtraTaken, 1u) < s_extra;
+            if (take) {
+                const uint32_t i = atomicAdd(t.ctl + kCtlVictims, 1u);
+                if (i < need) t.victims[i] = static_cast<uint32_t>(slot);
+            }
+        }
+        if (!grid_barrier(st)) return;
+        const uint32_t nv = min(need, ld_volatile(t.ctl + kCtlVictims));
+        for (uint32_t v = blockIdx.x; v < nv; v += gridDim.x) {
+            const uint32_t slot = t.victims[v];
+            const int32_t seg = t.slot_seg[slot];
+            if (seg < 0) continue;
+            if (t.seg_dirty[seg])
+                copy_segment(reinterpret_cast<uint4 *>(host + (static_cast<uint64_t>(seg) << kSegShift)),
+                             reinterpret_cast<const uint4 *>(cache + (static_cast<uint64_t>(slot) << kSegShift)));
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                __threadfence_system();
+                t.seg_dirty[seg] = 0;
+                t.seg_slot[seg] = -1;
+                t.slot_seg[slot] = -1;
+                const uint32_t pos = atomicAdd(t.ctl + kCtlFreeTop, 1u);
+                if (pos < t.nslots)
+                    t.free_slots[pos] = slot;
+                else
+                    set_error(st, kErrInternal, pos);
+                atomicAdd(&st->counters[kCntSegEvicted], 1ull);
+            }
+            __syncthreads();
+        }
+        if (!grid_barrier(st)) return;
+    }
     for (uint32_t a = blockIdx.x; a < na; a += gridDim.x) {
         const uint32_t seg = t.admits[a];
         if (threadIdx.x == 0 && t.seg_slot[seg] < 0) {

@@ -212,9 +212,26 @@ enum SmallIdx : int {
     kHugeR = 30,
     kCompactBig = 31,  // rows to compact above kWarpMove slots, per arena
     kCompactBigR = 32,
+    kPullBig = 39,  // in-rows of the pull repair left to the whole grid
+    // cleared by phase_begin for the addition phase (kInsertMask)
+    kAddBlockF = 40,  // addition groups served by a block, per arena
+    kAddBlockR = 41,
+    kAddWarpF = 42,   // ... by a warp
+    kAddWarpR = 43,
+    kPushBig = 44,    // 3 counters of the push closure's deferred hub rows
+    kPlanDoneF = 47,  // blocks of plan_add that are done, per arena (each launch leaves 0)
+    kPlanDoneR = 48,
     kPrAct = 33,  // 3 counters of vertices consumed per PageRank sweep, then 3 of its chunks
     kSmallCount = 64
 };
+
+constexpr unsigned long long kInsertMask = 0x7Full << kAddBlockF;
+// The counters of a deletion phase, of both arenas.
+constexpr unsigned long long kDeleteMask =
+    (1ull << kBigF) | (1ull << kBigR) | (7ull << kBigRows) | (1ull << kCompactCount) | (1ull << kOrderedCount) |
+    (1ull << kIndexedCount) | (1ull << kInvalDone) | (1ull << kCompactCountR) | (1ull << kOrderedCountR) |
+    (1ull << kIndexedCountR) | (1ull << kCoopF) | (1ull << kCoopR) | (1ull << kHugeF) | (1ull << kHugeR) |
+    (1ull << kCompactBig) | (1ull << kCompactBigR) | (1ull << kPullBig);
 
 constexpr uint32_t kBigRowCap = 65536;
 
@@ -327,6 +344,8 @@ struct cig_handle {
     uint32_t pr_hubs = 0;
     double *pr_res_hub = nullptr;
     float *pr_comp = nullptr;
+    BigRow *pr_chunks = nullptr;  // the sweeps' chunks of long rows (pr_chunk_cap entries)
+    uint64_t pr_chunk_cap() const { return 2 * fwd.seg_total * (kSegEdges / kPrChunk); }
     uint32_t *pr_queued = nullptr;
     bool pr64 = false;
 
@@ -344,8 +363,6 @@ struct cig_handle {
     uint32_t *firstpos_r = nullptr, *indexed_groups_r = nullptr, *chunk_map_r = nullptr;
     uint8_t *gtype_r = nullptr;
     uint32_t *coopf = nullptr, *coopr = nullptr;  // addition groups served one warp each
-    BigRow *pr_chunks = nullptr;  // the sweeps' chunks of long rows (pr_chunk_cap entries)
-    uint64_t pr_chunk_cap() const { return 2 * fwd.seg_total * (kSegEdges / kPrChunk); }
     uint32_t *hugef = nullptr, *huger = nullptr;  // hub deletion groups served by the grid
     void *cub_r = nullptr;
     size_t cub_r_bytes = 0;
@@ -600,11 +617,9 @@ struct cig_handle {
     Frontier frontier() const { return Frontier{q0, q1, small + kFr, n + 1}; }
 
     BigRow *big_rows = nullptr;
-    // Deferred hub rows; the counters are cleared before every launch that uses them.
-    BigList big_list() {
-        CK(cudaMemsetAsync(small + kBigRows, 0, 3 * sizeof(uint32_t), stream));
-        return BigList{big_rows, small + kBigRows, kBigRowCap, tune.split};
-    }
+    // Deferred hub rows; the counters (three from `counter` on) are cleared by
+    // the phase's begin.
+    BigList big_list(int counter) const { return BigList{big_rows, small + counter, kBigRowCap, tune.split}; }
 
     template <class K>
     int coop_blocks(K kernel, int tpb) const {
@@ -645,8 +660,11 @@ struct cig_handle {
     // void* argument array of a cooperative launch requires.
     template <class... P>
     void launch_coop(void (*kernel)(P...), int tpb, typename Identity<P>::type... args) {
+        launch_coop_blocks(kernel, coop_blocks(kernel, tpb), tpb, args...);
+    }
+    template <class... P>
+    void launch_coop_blocks(void (*kernel)(P...), int blocks, int tpb, typename Identity<P>::type... args) {
         void *argv[] = {static_cast<void *>(&args)...};
-        const int blocks = coop_blocks(kernel, tpb);
         if (capturing) {
             // Captured as a kernel node with the cooperative attribute: the
             // graph launch keeps the co-residency guarantee of the grid.
@@ -960,6 +978,7 @@ struct cig_handle {
         dfree(pr_hub_prefix);
         dfree(pr_res_hub);
         dfree(pr_comp);
+        dfree(pr_chunks);
         dfree(pr_queued);
         free_batch();
         dfree(tmp_u32);
@@ -977,7 +996,6 @@ struct cig_handle {
         for (auto &e : bev) cudaEventDestroy(e);
         bev.clear();
         free_queries();
-        dfree(pr_chunks);
         if (side) cudaStreamSynchronize(side);
         if (fork_ev) cudaEventDestroy(fork_ev);
         if (join_ev) cudaEventDestroy(join_ev);
@@ -1286,6 +1304,7 @@ struct cig_handle {
                 pr_hubs = nh;
             }
             dmalloc(pr_queued, n);
+            dmalloc(pr_chunks, pr_chunk_cap());
             dmalloc(aff_stamp, n);
             CK(cudaMemset(aff_stamp, 0, n * sizeof(uint32_t)));
         } else {
@@ -1303,7 +1322,6 @@ struct cig_handle {
 
     void upload_alloc(DevArena &a, const Layout &L) {
         ArenaAlloc h{};
-            dmalloc(pr_chunks, pr_chunk_cap());
         h.seg_bump = a.seg_used;
         h.seg_total = a.seg_total;
         std::memcpy(h.cur_next, L.cur_next, sizeof(h.cur_next));
@@ -1368,6 +1386,7 @@ struct cig_handle {
     void static_solve() {
         launch(init_state<A>, persistent_grid(), 256, state, n, source, cc_shift);
         CK(cudaMemsetAsync(small + kFr, 0, 3 * sizeof(uint32_t), stream));
+        CK(cudaMemsetAsync(small + kPushBig, 0, 3 * sizeof(uint32_t), stream));
         if (A == kCc)
             launch(enqueue_all_nonempty, persistent_grid(), 256, fwd.desc, n, frontier(), status);
         else
@@ -1381,9 +1400,13 @@ struct cig_handle {
     template <int A>
     void run_push() {
         const int p = prof_begin(CIG_STAGE_PUSH);
-        launch_coop(push_closure<A>, kTpb, fwd.view(), state, qstamp, tags, frontier(), big_list(), n + 2,
-                    local_sweeps, seg_hot, status);
+        run_push_part<A>(SeedEdges{nullptr, nullptr, 0u, n}, kPartRounds);
         prof_end(p);
+    }
+    template <int A>
+    void run_push_part(const SeedEdges &seeds, uint32_t parts) {
+        launch_coop(push_closure<A>, kTpb, fwd.view(), state, qstamp, tags, frontier(), seeds, parts, big_list(kPushBig),
+                    n + 2, local_sweeps, seg_hot, status);
     }
     uint32_t local_sweeps = 8;  // block-local hops per closure round (CIG_LOCAL_SWEEPS; 0 = off)
     // Share of the initially resident slots given to the last segments of the
@@ -1441,7 +1464,7 @@ struct cig_handle {
         auto a = pr_arrays<T>();
         const T eps = static_cast<T>(opt.pr_epsilon);
         ++epoch;
-        CK(cudaMemsetAsync(small + kTouched, 0, sizeof(uint32_t), stream));
+        launch(phase_begin, 1, kSmallCount, nullptr, small, kDeleteMask | kInsertMask | (1ull << kTouched), seg_ctl);
         if (nd + na)
             launch(collect_touched, grid_for(nd + na), 256, d_du, static_cast<uint32_t>(nd), d_au,
                                                                   static_cast<uint32_t>(na), n, aff_stamp, epoch,
@@ -1586,15 +1609,8 @@ struct cig_handle {
     // engine stream after the insertion phase.
     void cache_service() {
         if (!refresh) return;
-        const SegTable t = seg_table();
-        CK(cudaMemsetAsync(seg_ctl + kCtlVictims, 0, 2 * sizeof(uint32_t), stream));
-        CK(cudaMemsetAsync(seg_ctl + kCtlHist, 0, kScoreBuckets * sizeof(uint32_t), stream));
-        launch(seg_rescore, grid_for(fwd.seg_total), 256, t, static_cast<uint32_t>(fwd.seg_total));
-        launch(seg_plan, 1, 32, t);
-        launch(seg_pick, grid_for(fwd.seg_total), 256, t, static_cast<uint32_t>(fwd.seg_total));
-        launch(seg_evict, static_cast<int>(std::min<uint64_t>(kMaxEvict, sms * 4)), 256, t, fwd.dev, fwd.host_dptr,
-               status);
-        launch(seg_admit, static_cast<int>(kMaxAdmit), 256, t, fwd.dev, fwd.host_dptr, status);
+        launch_coop_blocks(seg_service, sms, 256, seg_table(), static_cast<uint32_t>(fwd.seg_total), fwd.dev,
+                           fwd.host_dptr, status);
         check_launch();
     }
 
@@ -1717,9 +1733,9 @@ struct cig_handle {
         prof[CIG_STAGE_GROUP].hits += 2 * na;
     }
 
-    // `zeroed`: the phase's counters were cleared by phase_begin.
+    // The phase's counters were cleared by phase_begin.
     void mutate_delete_arena(DevArena &A, const uint32_t *d_du, const uint32_t *d_dv, uint64_t nd, bool forward,
-                             bool with_stats, bool zeroed = false) {
+                             bool with_stats) {
         if (nd == 0) return;
         reserve_chunk_map(nd);  // before the map's address is taken below
         const uint32_t m = static_cast<uint32_t>(nd);
@@ -1752,7 +1768,6 @@ struct cig_handle {
             sorted = sort_keys(keys, tmp, nd);
             grp = build_groups(sorted, nd, groups, forward ? gendf : gendr, gcount);
         }
-        if (!zeroed) CK(cudaMemsetAsync(bcount, 0, sizeof(uint32_t), cs));
         prof_end(p);
         p = prof_begin(forward ? CIG_STAGE_MUTATE : CIG_STAGE_MUTATE_REV);
         unsigned long long *stats = with_stats ? status->counters : nullptr;
@@ -1762,13 +1777,28 @@ struct cig_handle {
         uint32_t *ocount = small + (forward ? kOrderedCount : kOrderedCountR);
         // Flat path: rows whose deletion requests are all distinct.
         uint32_t *icount = small + (forward ? kIndexedCount : kIndexedCountR);
-        if (!zeroed) {
-            CK(cudaMemsetAsync(ccount, 0, sizeof(uint32_t), cs));
-            CK(cudaMemsetAsync(cl.big_count, 0, sizeof(uint32_t), cs));
-            CK(cudaMemsetAsync(ocount, 0, sizeof(uint32_t), cs));
-            CK(cudaMemsetAsync(icount, 0, sizeof(uint32_t), cs));
-        }
         const PosIndex ix = pos_index(forward);
+        uint32_t *wide = forward ? coopf : coopr;
+        uint32_t *huge = forward ? hugef : huger;
+        uint32_t *wcount = small + (forward ? kCoopF : kCoopR);
+        uint32_t *hcount = small + (forward ? kHugeF : kHugeR);
+        if (ix.keys && ixb[forward ? 0 : 1].cls <= kIdxCls) {
+            // Every row above kIdxCls at the last build is indexed: no flat
+            // scan.  Grids follow the batch: at most one group per request.
+            const DelLists dl{wide, wcount, huge, hcount, big, bcount};
+            uint32_t *hot = forward ? seg_hot : nullptr;
+            const int ps = prof_begin(CIG_STAGE_DEL_SCAN);
+            launch(del_lane, std::min(grid_for(nd), persistent_grid()), 256, A.view(), A.desc, sorted, grp, ix, dl, cl,
+                   matched, hot, stats, status->counters, status);
+            launch(del_wide, std::min(grid_for(nd, kMutWarps), sms * 3), kMutWarps * 32, A.view(), A.desc, sorted, grp,
+                   ix, dl, cl, matched, hot, stats, status->counters, status);
+            prof_end(ps);
+            launch(del_rest, std::min(grid_for(nd, kMutWarps), sms * 4), kTpbMut, A.view(), A.desc, sorted, grp, ix,
+                   dl, cl, matched, hot, stats, status->counters, status);
+            prof_end(p);
+            check_launch();
+            return;
+        }
         launch(del_classify, persistent_grid(), 256, A.desc, sorted, grp, chunks, gtype, ordered, ocount, ix,
                indexed_groups, icount, m, firstpos, matched);
         CK(cub::DeviceScan::InclusiveSum(scan_tmp, scan_tmp_bytes, chunks, chunk_end, static_cast<int>(nd), cs));
@@ -1778,16 +1808,7 @@ struct cig_handle {
                chunk_map, m, firstpos, status->counters, forward ? seg_hot : nullptr);
         if (ix.keys) {
             // groups of more than kLaneKeys keys: one warp each, hub groups the
-            // whole grid (del_index_wide); the warp list is the arena's
-            // addition warp-group list, free during deletions
-            uint32_t *wide = forward ? coopf : coopr;
-            uint32_t *huge = forward ? hugef : huger;
-            uint32_t *wcount = small + (forward ? kCoopF : kCoopR);
-            uint32_t *hcount = small + (forward ? kHugeF : kHugeR);
-            if (!zeroed) {
-                CK(cudaMemsetAsync(wcount, 0, sizeof(uint32_t), cs));
-                CK(cudaMemsetAsync(hcount, 0, sizeof(uint32_t), cs));
-            }
+            // whole grid (del_index_wide)
             launch(del_index, persistent_grid(), 256, A.view(), A.desc, sorted, grp, indexed_groups, icount, firstpos,
                    ix, wide, wcount, huge, hcount, stats, status);
             launch(del_index_wide, persistent_grid(), 256, A.view(), A.desc, sorted, grp, wide, wcount, huge, hcount,
@@ -1818,7 +1839,6 @@ struct cig_handle {
         uint32_t *big = forward ? bigf : bigr;
         unsigned long long *plan = forward ? pf : prr;
         uint32_t *gcount = small + (forward ? kGcF : kGcR);
-        uint32_t *bcount = small + (forward ? kBigF : kBigR);
         int p = prof_begin(CIG_STAGE_GROUP);
         unsigned long long *sorted;
         Groups grp;
@@ -1833,24 +1853,19 @@ struct cig_handle {
             sorted = sort_keys(keys, tmp, na);
             grp = build_groups(sorted, na, groups, forward ? gendf : gendr, gcount);
         }
-        CK(cudaMemsetAsync(bcount, 0, sizeof(uint32_t), cs));
         prof_end(p);
         p = prof_begin(forward ? CIG_STAGE_ADD : CIG_STAGE_ADD_REV);
-        launch(plan_add, persistent_grid(), 256, A.desc, sorted, grp, plan, A.alloc);
-        launch(alloc_classes, 1, 64, A.alloc, status);
-        if (forward && refresh) launch(seg_assign_new, 1, 32, seg_table(), &A.alloc->seg_bump, status);
+        const int lane_grid = std::min(grid_for(na), persistent_grid());  // at most one group per request
+        launch(plan_add, lane_grid, 256, A.desc, sorted, grp, plan, A.alloc, forward && refresh, seg_table(),
+               small + (forward ? kPlanDoneF : kPlanDoneR), status);
         unsigned long long *stats = with_stats ? status->counters : nullptr;
         const uint32_t *vals = forward ? d_av : d_au;
         const PosIndex ix = pos_index(forward);
-        uint32_t *coop = forward ? coopf : coopr;
-        uint32_t *ccount = small + (forward ? kCoopF : kCoopR);
-        CK(cudaMemsetAsync(ccount, 0, sizeof(uint32_t), cs));
-        launch(mutate_add, persistent_grid(), 256, A.view(), A.desc, sorted, grp, plan, A.alloc, vals, coop, ccount,
-               stats, ix, status);
-        launch(mutate_add_warp, persistent_grid(), 256, A.view(), A.desc, sorted, grp, plan, A.alloc, vals, coop,
-               ccount, big, bcount, stats, ix, status);
-        launch(mutate_add_big, sms * 2, kTpbMut, A.view(), A.desc, sorted, grp, plan, A.alloc, vals, big, bcount,
-               stats, ix, status);
+        const AddLists ls{forward ? coopf : coopr, small + (forward ? kAddWarpF : kAddWarpR), big,
+                          small + (forward ? kAddBlockF : kAddBlockR)};
+        launch(mutate_add, lane_grid, 256, A.view(), A.desc, sorted, grp, plan, A.alloc, vals, ls, stats, ix, status);
+        launch(mutate_add_wide, std::min(grid_for(na, kTpbMut / 32), sms * 2), kTpbMut, A.view(), A.desc, sorted, grp,
+               plan, A.alloc, vals, ls, stats, ix, status);
         prof_end(p);
         check_launch();
     }
@@ -1901,55 +1916,49 @@ struct cig_handle {
     void delete_phase_dev(const uint32_t *d_du, const uint32_t *d_dv, uint64_t nd, bool push = true) {
         const InBatch ib(in_batch);
         const uint32_t *ep = small + kEpoch;
-        // frontier, affected and deletion-path counters of both arenas
         static_assert(kSmallCount == 64, "phase_begin clears one 64-word counter block");
-        const unsigned long long mask = (0x3Full << kFr) | (1ull << kBigF) | (1ull << kBigR) | (1ull << kCompactCount) |
-                              (1ull << kOrderedCount) | (1ull << kIndexedCount) | (1ull << kInvalDone) |
-                              (1ull << kCompactCountR) | (1ull << kOrderedCountR) | (1ull << kIndexedCountR) |
-                              (1ull << kCoopF) | (1ull << kCoopR) | (1ull << kHugeF) | (1ull << kHugeR) |
-                                        (1ull << kCompactBig) | (1ull << kCompactBigR);
-        launch(phase_begin, 1, kSmallCount, small + kEpoch, small, mask);
-        int p = prof_begin(CIG_STAGE_SEED);
-        if (nd)
-            launch(seed_deletions<A>, grid_for(nd), 256, d_du, d_dv, static_cast<uint32_t>(nd), n, state,
-                                                                aff_stamp, ep, list, small + kAff, n + 1, status);
-        prof_end(p);
-        check_launch();
-        fork_arenas([&] { mutate_delete_arena(fwd, d_du, d_dv, nd, true, true, true); },
-                    [&] { mutate_delete_arena(rev, d_du, d_dv, nd, false, false, true); });
-        p = prof_begin(CIG_STAGE_INVAL);
-        launch_coop(inval_closure<A>, kTpb, fwd.view(), state, aff_stamp, ep, list, small + kAff, n + 1,
-                    big_list(), n + 2, local_sweeps, inval_done, small + kInvalDone, small + kAffTotal, seg_hot,
-                    status);
-        prof_end(p);
-        p = prof_begin(CIG_STAGE_PULL);
-        launch(reset_affected<A>, persistent_grid(), 256, list, small + kAffTotal, state, cc_shift);
-        const BigList pull_big = big_list();
-        // One resident wave (__launch_bounds__(kTpb, 4)): a second wave of
-        // blocks would start its few rows only after the first wave ends.
-        launch(pull_repair<A>, sms * 4, kTpb, rev.view(), state, aff_stamp, ep, list, small + kAffTotal, pull_big,
-               status);
-        launch(pull_deferred<A>, persistent_grid(), kTpb, rev.view(), state, aff_stamp, ep, pull_big, status);
-        launch(enqueue_affected<A>, persistent_grid(), 256, list, small + kAffTotal, state, frontier(), status);
-        prof_end(p);
+        launch(phase_begin, 1, kSmallCount, small + kEpoch, small, kDeleteMask | kInsertMask | (0x3Full << kFr),
+               seg_ctl);
+        fork_arenas([&] { mutate_delete_arena(fwd, d_du, d_dv, nd, true, true); },
+                    [&] { mutate_delete_arena(rev, d_du, d_dv, nd, false, false); });
+        const SeedEdges seeds{d_du, d_dv, static_cast<uint32_t>(nd), n};
+        auto closure = [&](uint32_t parts) {
+            launch_coop(repair_closure<A>, kTpb, fwd.view(), rev.view(), seeds, parts, state, aff_stamp, ep, list,
+                        small + kAff, n + 1, big_list(kBigRows), small + kPullBig, n + 2, local_sweeps, inval_done,
+                        small + kInvalDone, small + kAffTotal, frontier(), seg_hot, status);
+        };
+        if (prof_on) {  // stage by stage (the rows are mutated by now; the seeds read only values)
+            const std::pair<int, uint32_t> stages[] = {
+                {CIG_STAGE_SEED, kPartSeed}, {CIG_STAGE_INVAL, kPartRounds}, {CIG_STAGE_PULL, kPartPull}};
+            for (const auto &sg : stages) {
+                const int p = prof_begin(sg.first);
+                closure(sg.second);
+                prof_end(p);
+            }
+        } else {
+            closure(kPartAll);
+        }
         check_launch();
         if (push) run_push<A>();
     }
 
-    // `fresh` false: keep the frontier the deletion phase left queued.
+    // `fresh` false: keep the frontier the deletion phase left queued (its
+    // begin cleared the insertion counters too).
     template <int A>
     void insert_phase_dev(const uint32_t *d_au, const uint32_t *d_av, uint64_t na, bool fresh = true) {
         const InBatch ib(in_batch);
-        if (fresh) CK(cudaMemsetAsync(small + kFr, 0, 3 * sizeof(uint32_t), stream));
+        if (fresh) launch(phase_begin, 1, kSmallCount, nullptr, small, kInsertMask | (7ull << kFr), seg_ctl);
         fork_arenas([&] { mutate_add_arena(fwd, d_au, d_av, na, true, true); },
                     [&] { mutate_add_arena(rev, d_au, d_av, na, false, false); });
-        int p = prof_begin(CIG_STAGE_SEED);
-        if (na)
-            launch(seed_insertions<A>, grid_for(na), 256, d_au, d_av, static_cast<uint32_t>(na), n, state,
-                                                                 qstamp, tags, frontier(), status);
-        prof_end(p);
-        check_launch();
-        run_push<A>();
+        const SeedEdges seeds{d_au, d_av, static_cast<uint32_t>(na), n};
+        if (prof_on) {
+            const int p = prof_begin(CIG_STAGE_SEED);
+            run_push_part<A>(seeds, kPartSeed);
+            prof_end(p);
+            run_push<A>();
+        } else {
+            run_push_part<A>(seeds, kPartAll);
+        }
     }
 
     // Copy host update arrays into the device batch buffers (pinned staging).

@@ -27,6 +27,7 @@
 #include <cub/block/block_radix_sort.cuh>
 #include <cub/block/block_scan.cuh>
 
+#include "cache.cuh"
 #include "common.cuh"
 #include "posindex.cuh"
 
@@ -441,135 +442,147 @@ constexpr uint32_t kFilterBits = 4096;
 
 __device__ __forceinline__ uint32_t filter_hash(uint32_t x) { return (x * 0x9E3779B1u) >> 20; }  // 12 bits
 
+struct OrderedSmem {
+    uint32_t skey[kBigKeys];
+    uint32_t scount[kBigKeys];
+    uint32_t filter[kFilterBits / 32];
+    uint8_t cand_bits[kTpbMut];
+    uint8_t del_bits[kTpbMut];
+    uint16_t cand_run[kTpbMut * kBigItems];
+    uint32_t g_run[kTpbMut * kBigItems];
+    uint32_t cand_warp[kTpbMut / 32];
+    uint32_t left;
+};
+
+// One row by one block; returns the tombstones written (all threads call;
+// `matched` of a group above kBigKeys must be zero).
+__device__ __forceinline__ uint32_t block_tomb_ordered(const AdjView &view, const RowDesc &d, uint32_t u,
+                                                       const unsigned long long *keys, uint32_t gs, uint32_t ge,
+                                                       uint32_t *matched, OrderedSmem &sm) {
+    const uint32_t tid = threadIdx.x;
+    const uint32_t gm = ge - gs;
+    const bool in_smem = gm <= kBigKeys;
+    const unsigned long long uhi = static_cast<unsigned long long>(u) << kKeyShift;
+    for (uint32_t i = tid; i < kFilterBits / 32; i += kTpbMut) sm.filter[i] = 0;
+    if (tid == 0) sm.left = gm;
+    __syncthreads();
+    for (uint32_t j = tid; j < gm; j += kTpbMut) {
+        const uint32_t x = key_low(keys[gs + j]);
+        if (in_smem) {
+            sm.skey[j] = x;
+            sm.scount[j] = 0;
+        }
+        const uint32_t h = filter_hash(x);
+        atomicOr(&sm.filter[h >> 5], 1u << (h & 31u));
+    }
+    __syncthreads();
+    for (uint32_t base = 0; base < d.len; base += kTpbMut * kBigItems) {
+        const uint32_t k0 = base + tid * kBigItems;
+        uint32_t e[kBigItems];
+#pragma unroll
+        for (int h = 0; h < kBigItems; h += 4) {
+            if (k0 + h < d.len) {
+                const uint4 q = *reinterpret_cast<const uint4 *>(view.at(d.off + k0 + h));
+                e[h] = q.x;
+                e[h + 1] = q.y;
+                e[h + 2] = q.z;
+                e[h + 3] = q.w;
+            } else {
+                e[h] = e[h + 1] = e[h + 2] = e[h + 3] = kTomb;
+            }
+        }
+        uint32_t cb = 0;
+#pragma unroll
+        for (int s = 0; s < kBigItems; ++s) {
+            if (k0 + s >= d.len || e[s] == kTomb) continue;
+            const uint32_t h = filter_hash(e[s]);
+            if (!((sm.filter[h >> 5] >> (h & 31u)) & 1u)) continue;
+            if (in_smem) {
+                uint32_t lo = 0, hi = gm;
+                while (lo < hi) {
+                    const uint32_t mid = (lo + hi) >> 1;
+                    if (sm.skey[mid] < e[s])
+                        lo = mid + 1;
+                    else
+                        hi = mid;
+                }
+                if (lo < gm && sm.skey[lo] == e[s]) {
+                    cb |= 1u << s;
+                    sm.cand_run[tid * kBigItems + s] = static_cast<uint16_t>(lo);
+                }
+            } else {
+                uint32_t run, req;
+                if (find_run(keys, gs, ge, uhi | e[s], run, req)) {
+                    cb |= 1u << s;
+                    sm.g_run[tid * kBigItems + s] = run;
+                }
+            }
+        }
+        sm.cand_bits[tid] = static_cast<uint8_t>(cb);
+        sm.del_bits[tid] = 0;
+        const uint32_t wmask = __ballot_sync(kFull, cb != 0);
+        if ((tid & 31u) == 0) sm.cand_warp[tid >> 5] = wmask;
+        if (__syncthreads_or(cb != 0)) {
+            if (tid == 0) {
+                // Visit only the threads that hold candidates, in position order.
+                uint32_t l = sm.left;
+                for (uint32_t wi = 0; wi < kTpbMut / 32; ++wi) {
+                    for (uint32_t tm = sm.cand_warp[wi]; tm; tm &= tm - 1) {
+                        const uint32_t t = wi * 32 + __ffs(tm) - 1;
+                        uint32_t b = sm.cand_bits[t];
+                        uint32_t dbits = 0;
+                        while (b) {
+                            const uint32_t s = __ffs(b) - 1;
+                            b &= b - 1;
+                            bool del;
+                            if (in_smem) {
+                                const uint32_t r = sm.cand_run[t * kBigItems + s];
+                                uint32_t e2 = r + 1;
+                                while (e2 < gm && sm.skey[e2] == sm.skey[r]) ++e2;
+                                del = sm.scount[r] < e2 - r;
+                                sm.scount[r] += 1;
+                            } else {
+                                const uint32_t r = sm.g_run[t * kBigItems + s];
+                                uint32_t e2 = r + 1;
+                                while (e2 < ge && keys[e2] == keys[r]) ++e2;
+                                del = matched[r] < e2 - r;
+                                matched[r] += 1;
+                            }
+                            if (del) {
+                                dbits |= 1u << s;
+                                --l;
+                            }
+                        }
+                        sm.del_bits[t] = static_cast<uint8_t>(dbits);
+                    }
+                }
+                sm.left = l;
+            }
+            __syncthreads();
+            const uint32_t db = sm.del_bits[tid];
+#pragma unroll
+            for (int s = 0; s < kBigItems; ++s)
+                if ((db >> s) & 1u) write_slot(view, d.off + k0 + s, kTomb);
+        }
+        __syncthreads();
+        if (sm.left == 0) break;
+    }
+    return gm - sm.left;
+}
+
 __global__ void __launch_bounds__(kTpbMut)
     mutate_delete_big(AdjView view, RowDesc *desc, const unsigned long long *keys, Groups gr, const uint32_t *big,
                       const uint32_t *big_count, uint32_t *matched, CompactList cl, unsigned long long *stats,
                       Status *st) {
-    __shared__ uint32_t skey[kBigKeys];
-    __shared__ uint32_t scount[kBigKeys];
-    __shared__ uint32_t filter[kFilterBits / 32];
-    __shared__ uint8_t cand_bits[kTpbMut];
-    __shared__ uint8_t del_bits[kTpbMut];
-    __shared__ uint16_t cand_run[kTpbMut * kBigItems];
-    __shared__ uint32_t g_run[kTpbMut * kBigItems];
-    __shared__ uint32_t cand_warp[kTpbMut / 32];
-    __shared__ uint32_t left;
-    const uint32_t tid = threadIdx.x;
+    __shared__ OrderedSmem sm;
     const uint32_t nb = *big_count;
     for (uint32_t b = blockIdx.x; b < nb; b += gridDim.x) {
         const uint32_t gs = gr.start[big[b]];
         const uint32_t ge = gr.end[big[b]];
-        const uint32_t gm = ge - gs;
-        const bool in_smem = gm <= kBigKeys;
         const uint32_t u = key_src(keys[gs]);
         const RowDesc d = desc[u];
-        const unsigned long long uhi = static_cast<unsigned long long>(u) << kKeyShift;
-        for (uint32_t i = tid; i < kFilterBits / 32; i += kTpbMut) filter[i] = 0;
-        if (tid == 0) left = gm;
-        __syncthreads();
-        for (uint32_t j = tid; j < gm; j += kTpbMut) {
-            const uint32_t x = key_low(keys[gs + j]);
-            if (in_smem) {
-                skey[j] = x;
-                scount[j] = 0;
-            }
-            const uint32_t h = filter_hash(x);
-            atomicOr(&filter[h >> 5], 1u << (h & 31u));
-        }
-        __syncthreads();
-        for (uint32_t base = 0; base < d.len; base += kTpbMut * kBigItems) {
-            const uint32_t k0 = base + tid * kBigItems;
-            uint32_t e[kBigItems];
-#pragma unroll
-            for (int h = 0; h < kBigItems; h += 4) {
-                if (k0 + h < d.len) {
-                    const uint4 q = *reinterpret_cast<const uint4 *>(view.at(d.off + k0 + h));
-                    e[h] = q.x;
-                    e[h + 1] = q.y;
-                    e[h + 2] = q.z;
-                    e[h + 3] = q.w;
-                } else {
-                    e[h] = e[h + 1] = e[h + 2] = e[h + 3] = kTomb;
-                }
-            }
-            uint32_t cb = 0;
-#pragma unroll
-            for (int s = 0; s < kBigItems; ++s) {
-                if (k0 + s >= d.len || e[s] == kTomb) continue;
-                const uint32_t h = filter_hash(e[s]);
-                if (!((filter[h >> 5] >> (h & 31u)) & 1u)) continue;
-                if (in_smem) {
-                    uint32_t lo = 0, hi = gm;
-                    while (lo < hi) {
-                        const uint32_t mid = (lo + hi) >> 1;
-                        if (skey[mid] < e[s])
-                            lo = mid + 1;
-                        else
-                            hi = mid;
-                    }
-                    if (lo < gm && skey[lo] == e[s]) {
-                        cb |= 1u << s;
-                        cand_run[tid * kBigItems + s] = static_cast<uint16_t>(lo);
-                    }
-                } else {
-                    uint32_t run, req;
-                    if (find_run(keys, gs, ge, uhi | e[s], run, req)) {
-                        cb |= 1u << s;
-                        g_run[tid * kBigItems + s] = run;
-                    }
-                }
-            }
-            cand_bits[tid] = static_cast<uint8_t>(cb);
-            del_bits[tid] = 0;
-            const uint32_t wmask = __ballot_sync(kFull, cb != 0);
-            if ((tid & 31u) == 0) cand_warp[tid >> 5] = wmask;
-            if (__syncthreads_or(cb != 0)) {
-                if (tid == 0) {
-                    // Visit only the threads that hold candidates, in position order.
-                    uint32_t l = left;
-                    for (uint32_t wi = 0; wi < kTpbMut / 32; ++wi) {
-                        for (uint32_t tm = cand_warp[wi]; tm; tm &= tm - 1) {
-                            const uint32_t t = wi * 32 + __ffs(tm) - 1;
-                            uint32_t b = cand_bits[t];
-                            uint32_t dbits = 0;
-                            while (b) {
-                                const uint32_t s = __ffs(b) - 1;
-                                b &= b - 1;
-                                bool del;
-                                if (in_smem) {
-                                    const uint32_t r = cand_run[t * kBigItems + s];
-                                    uint32_t e2 = r + 1;
-                                    while (e2 < gm && skey[e2] == skey[r]) ++e2;
-                                    del = scount[r] < e2 - r;
-                                    scount[r] += 1;
-                                } else {
-                                    const uint32_t r = g_run[t * kBigItems + s];
-                                    uint32_t e2 = r + 1;
-                                    while (e2 < ge && keys[e2] == keys[r]) ++e2;
-                                    del = matched[r] < e2 - r;
-                                    matched[r] += 1;
-                                }
-                                if (del) {
-                                    dbits |= 1u << s;
-                                    --l;
-                                }
-                            }
-                            del_bits[t] = static_cast<uint8_t>(dbits);
-                        }
-                    }
-                    left = l;
-                }
-                __syncthreads();
-                const uint32_t db = del_bits[tid];
-#pragma unroll
-                for (int s = 0; s < kBigItems; ++s)
-                    if ((db >> s) & 1u) write_slot(view, d.off + k0 + s, kTomb);
-            }
-            __syncthreads();
-            if (left == 0) break;
-        }
-        if (tid == 0) {
-            const uint32_t done = gm - left;
+        const uint32_t done = block_tomb_ordered(view, d, u, keys, gs, ge, matched, sm);
+        if (threadIdx.x == 0) {
             finish_row(desc, u, d, done, cl);
             if (done && stats) {
                 atomicAdd(&stats[kCntRemoved], static_cast<unsigned long long>(done));
@@ -660,21 +673,16 @@ constexpr uint32_t kLaneKeys = 4;
 constexpr uint32_t kHugeKeys = 256;
 constexpr uint32_t kApplied = 0x80000000u;  // firstpos flag: tombstone already written
 
-// `count_tomb`: add the tombstone to the row's descriptor here (callers that
-// serve many keys of one row add their warp's total once instead).
-__device__ __forceinline__ uint32_t del_index_key(const AdjView &view, RowDesc *desc, const RowDesc &d, uint32_t u,
-                                                  uint32_t v, uint32_t *fp, const PosIndex &ix, Status *st,
-                                                  bool count_tomb = true) {
-    const unsigned long long s = idx_find(ix, (static_cast<unsigned long long>(u) << 32) | v);
-    if (s == ~0ull) return 0u;  // not in the row: a missing delete
-    const uint2 e = ix.val[s];
+// One occurrence of v, found in slot s with entry e, is deleted: its
+// tombstone, and the entry moves to the next occurrence or is dropped.
+__device__ __forceinline__ uint32_t del_index_take(const AdjView &view, const RowDesc &d, uint32_t v,
+                                                   unsigned long long s, const uint2 &e, const PosIndex &ix,
+                                                   Status *st) {
     if (e.y == 0u || e.x >= d.len) {
         if (e.y != 0u) set_error(st, kErrInternal, 0x1d2u);
         return 0u;
     }
-    *fp = e.x | kApplied;
     write_slot(view, d.off + e.x, kTomb);
-    if (count_tomb) atomicAdd(&desc[u].meta, 1u << 6);
     if (e.y == 1u) {
         ix.val[s] = make_uint2(kInf, 0u);  // the key keeps its slot for the next time it is inserted
     } else {
@@ -683,6 +691,17 @@ __device__ __forceinline__ uint32_t del_index_key(const AdjView &view, RowDesc *
         if (q >= d.len) set_error(st, kErrInternal, 0x1d3u);
         ix.val[s] = make_uint2(q < d.len ? q : kInf, e.y - 1u);
     }
+    return 1u;
+}
+
+// Returns 1 when (u, v) was in the row; *pos is its position.
+__device__ __forceinline__ uint32_t del_index_key(const AdjView &view, const RowDesc &d, uint32_t u, uint32_t v,
+                                                  const PosIndex &ix, Status *st, uint32_t *pos = nullptr) {
+    const unsigned long long s = idx_find(ix, (static_cast<unsigned long long>(u) << 32) | v);
+    if (s == ~0ull) return 0u;  // not in the row: a missing delete
+    const uint2 e = ix.val[s];
+    if (!del_index_take(view, d, v, s, e, ix, st)) return 0u;
+    if (pos) *pos = e.x | kApplied;
     return 1u;
 }
 
@@ -722,21 +741,9 @@ __device__ __forceinline__ uint32_t del_index_keys(const AdjView &view, RowDesc 
             e[j] = ix.val[slot[j]];
         }
         const uint32_t u = static_cast<uint32_t>(key[j] >> 32), v = static_cast<uint32_t>(key[j]);
-        if (e[j].y == 0u || e[j].x >= d[j].len) {
-            if (e[j].y != 0u) set_error(st, kErrInternal, 0x1d2u);
-            continue;
-        }
+        if (!del_index_take(view, d[j], v, slot[j], e[j], ix, st)) continue;
         firstpos[ks[j]] = e[j].x | kApplied;
-        write_slot(view, d[j].off + e[j].x, kTomb);
         atomicAdd(&desc[u].meta, 1u << 6);
-        if (e[j].y == 1u) {
-            ix.val[slot[j]] = make_uint2(kInf, 0u);  // the key keeps its slot
-        } else {
-            uint32_t q = e[j].x + 1;
-            while (q < d[j].len && *view.at(d[j].off + q) != v) ++q;
-            if (q >= d[j].len) set_error(st, kErrInternal, 0x1d3u);
-            ix.val[slot[j]] = make_uint2(q < d[j].len ? q : kInf, e[j].y - 1u);
-        }
         ++removed;
     }
     return removed;
@@ -820,7 +827,7 @@ __global__ void del_index_wide(AdjView view, RowDesc *desc, const unsigned long 
         const RowDesc d = desc[u];
         uint32_t tombs = 0;
         for (uint32_t j = lane; j < nk; j += 32u)
-            tombs += del_index_key(view, desc, d, u, key_low(keys[gs + j]), firstpos + gs + j, ix, st, false);
+            tombs += del_index_key(view, d, u, key_low(keys[gs + j]), ix, st, firstpos + gs + j);
         tombs = __reduce_add_sync(kFull, tombs);
         if (lane == 0 && tombs) atomicAdd(&desc[u].meta, tombs << 6);
         removed += lane == 0 ? tombs : 0u;
@@ -842,7 +849,7 @@ __global__ void del_index_wide(AdjView view, RowDesc *desc, const unsigned long 
             for (; c < prefix + chunks; c += warps) {
                 const uint32_t j = static_cast<uint32_t>(c - prefix) * 32u + lane;
                 if (j < nk)
-                    tombs += del_index_key(view, desc, d, u, key_low(keys[gs + j]), firstpos + gs + j, ix, st, false);
+                    tombs += del_index_key(view, d, u, key_low(keys[gs + j]), ix, st, firstpos + gs + j);
             }
             tombs = __reduce_add_sync(kFull, tombs);
             if (lane == 0 && tombs) atomicAdd(&desc[u].meta, tombs << 6);
@@ -1219,9 +1226,8 @@ __device__ __forceinline__ uint32_t block_move_live(const AdjView &view, const P
 // row of up to kWarpMove slots (nearly all of them: a row of four entries
 // compacts at its first deletion), a block per longer row.  A block for
 // every row left 255 of 256 threads idle on the short ones.
-__global__ void __launch_bounds__(kTpbMut) compact_rows(AdjView view, RowDesc *desc, CompactList cl, PosIndex ix,
-                                                         Status *st) {
-    __shared__ MoveSmem sm;
+__device__ __forceinline__ void compact_listed(const AdjView &view, RowDesc *desc, const CompactList &cl,
+                                               const PosIndex &ix, MoveSmem &sm, Status *st) {
     const uint32_t nb = *cl.big_count;
     for (uint32_t c = blockIdx.x; c < nb; c += gridDim.x) {
         const uint32_t u = cl.rows[cl.cap - 1u - c];
@@ -1240,6 +1246,347 @@ __global__ void __launch_bounds__(kTpbMut) compact_rows(AdjView view, RowDesc *d
     }
 }
 
+__global__ void __launch_bounds__(kTpbMut) compact_rows(AdjView view, RowDesc *desc, CompactList cl, PosIndex ix,
+                                                         Status *st) {
+    __shared__ MoveSmem sm;
+    compact_listed(view, desc, cl, ix, sm, st);
+}
+
+// ---------------------------------------------------------------- indexed deletion
+// Deletion phase of an arena whose position index covers every row above
+// kIdxCls at its last build: three kernels in a chain.  (The flat scan of an
+// unindexed arena takes thirteen; on small batches their launches were most
+// of the phase.)
+//   del_lane: a lane per group.  Indexed rows take the positions of up to
+//     kLaneKeys distinct keys from the index; rows of up to kLaneDelRow slots
+//     are read into registers, lose the requested entries and are written
+//     back without tombstones.  The rest is listed for
+//   del_wide: a warp per group: more keys on an indexed row (hub groups of
+//     more than kHugeKeys: the whole grid), repeated requests, and unindexed
+//     rows (ones that grew since the build) of up to kWarpRowMax slots, in
+//     position order; the warp compacts its row when it is due.
+//   del_rest: a block per longer row, then the queued compactions.
+constexpr uint32_t kLaneDelRow = 16;
+
+// Work lists of the phase (each as long as the arena's groups).
+struct DelLists {
+    uint32_t *wide;
+    uint32_t *wide_count;
+    uint32_t *huge;
+    uint32_t *huge_count;
+    uint32_t *big;
+    uint32_t *big_count;
+};
+
+__global__ void __launch_bounds__(256, 4)
+    del_lane(AdjView view, RowDesc *desc, const unsigned long long *keys, Groups gr, PosIndex ix, DelLists dl,
+             CompactList cl, uint32_t *matched, uint32_t *seg_hot, unsigned long long *stats, unsigned long long *scan_stats, Status *st) {
+    const uint32_t ng = *gr.count;
+    const uint32_t rounded = (ng + 31u) & ~31u;
+    uint32_t removed = 0, changed = 0, scanned = 0, scanned_cached = 0;
+    for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < rounded; g += gridDim.x * blockDim.x) {
+        bool wide = false, huge = false, compact = false, compact_big = false;
+        uint32_t u = 0;
+        if (g < ng) {
+            const uint32_t gs = gr.start[g];
+            const uint32_t nk = gr.end[g] - gs;
+            uint32_t v[kLaneKeys];
+            bool dup = false;
+#pragma unroll
+            for (uint32_t j = 0; j < kLaneKeys; ++j) {
+                const unsigned long long k = j < nk ? keys[gs + j] : 0ull;
+                if (j == 0) u = key_src(k);
+                v[j] = key_low(k);
+                if (j && j < nk) dup |= v[j] == v[j - 1];
+            }
+            const RowDesc d = desc[u];
+            const bool indexed = idx_row(ix, u);
+            if (nk > kLaneKeys || (indexed ? dup : d.len > kLaneDelRow)) {
+                huge = indexed && nk > kHugeKeys;  // del_wide looks for repeated requests before it uses the index
+                wide = !huge;
+                if (huge) matched[gs] = rd_tombs(d);  // for del_rest: did the row lose any
+            } else if (indexed) {
+                unsigned long long slot[kLaneKeys], seen[kLaneKeys];
+                uint2 e[kLaneKeys];
+#pragma unroll
+                for (uint32_t j = 0; j < kLaneKeys; ++j) {
+                    const unsigned long long key = (static_cast<unsigned long long>(u) << 32) | v[j];
+                    slot[j] = idx_mix(key) & ix.mask;
+                    seen[j] = kIdxEmpty;
+                    if (j < nk) {
+                        seen[j] = *reinterpret_cast<volatile unsigned long long *>(ix.keys + slot[j]);
+                        e[j] = ix.val[slot[j]];
+                    }
+                }
+                uint32_t tombs = 0;
+#pragma unroll
+                for (uint32_t j = 0; j < kLaneKeys; ++j) {
+                    if (j >= nk) continue;
+                    const unsigned long long key = (static_cast<unsigned long long>(u) << 32) | v[j];
+                    if (seen[j] != key) {
+                        if (seen[j] == kIdxEmpty) continue;  // not in the row: a missing delete
+                        slot[j] = idx_find_from(ix, key, (slot[j] + 1) & ix.mask, 1);
+                        if (slot[j] == ~0ull) continue;
+                        e[j] = ix.val[slot[j]];
+                    }
+                    tombs += del_index_take(view, d, v[j], slot[j], e[j], ix, st);
+                }
+                if (tombs) {
+                    const uint32_t t = rd_tombs(d) + tombs;
+                    desc[u].meta = rd_meta(rd_cls(d), t);
+                    compact = 4ull * t >= d.len || t >= kMaxTombs / 2;
+                    compact_big = compact && d.len > kWarpMove;
+                    compact = compact && !compact_big;
+                    removed += tombs;
+                    ++changed;
+                }
+            } else if (d.len) {
+                // A block of at most one segment.
+                uint32_t e[kLaneDelRow];
+                const uint32_t *src = view.at(d.off);
+#pragma unroll
+                for (uint32_t h = 0; h < kLaneDelRow; h += 4) {
+                    uint4 q = make_uint4(kTomb, kTomb, kTomb, kTomb);
+                    if (h < d.len) q = *reinterpret_cast<const uint4 *>(src + h);
+                    e[h] = h < d.len ? q.x : kTomb;
+                    e[h + 1] = h + 1 < d.len ? q.y : kTomb;
+                    e[h + 2] = h + 2 < d.len ? q.z : kTomb;
+                    e[h + 3] = h + 3 < d.len ? q.w : kTomb;
+                }
+                scanned += d.len;
+                if (view.cached(d.off)) scanned_cached += d.len;
+                seg_touch(seg_hot, d.off, d.len);
+                // Each request takes the first live occurrence; a repeated
+                // one the next.
+                uint32_t gone = 0;
+#pragma unroll
+                for (uint32_t j = 0; j < kLaneKeys; ++j) {
+                    bool open = j < nk;
+#pragma unroll
+                    for (uint32_t k = 0; k < kLaneDelRow; ++k)
+                        if (open && e[k] == v[j] && v[j] != kTomb) {
+                            e[k] = kTomb;
+                            open = false;
+                            ++gone;
+                        }
+                }
+                if (gone) {
+                    uint32_t *wp = view.wptr(d.off);
+                    uint32_t w = 0;
+#pragma unroll
+                    for (uint32_t k = 0; k < kLaneDelRow; ++k)
+                        if (e[k] != kTomb) {
+                            if (w != k) wp[w] = e[k];
+                            ++w;
+                        }
+                    desc[u] = RowDesc{d.off, w, rd_meta(rd_cls(d), 0)};
+                    removed += gone;
+                    ++changed;
+                }
+            }
+        }
+        warp_enqueue(wide, g, dl.wide, dl.wide_count, ng, st);
+        warp_enqueue(huge, g, dl.huge, dl.huge_count, ng, st);
+        warp_enqueue(compact, u, cl.rows, cl.count, cl.cap, st);
+        if (compact_big) cl.rows[cl.cap - 1u - atomicAdd(cl.big_count, 1u)] = u;
+    }
+    if (stats) {
+        warp_count(&stats[kCntRemoved], removed);
+        warp_count(&stats[kCntChanged], changed);
+    }
+    warp_count(&scan_stats[kCntDelScanned], scanned);
+    warp_count(&scan_stats[kCntDelScannedCached], scanned_cached);
+}
+
+// The index entries of an ordered group (repeated requests on an indexed row)
+// recounted from the row; thread `t` of `stride`.
+__device__ __forceinline__ void idx_recount_group(const AdjView &view, const RowDesc &d, uint32_t u,
+                                                  const unsigned long long *keys, uint32_t gs, uint32_t ge,
+                                                  uint32_t t, uint32_t stride, const PosIndex &ix) {
+    for (uint32_t j = gs + t; j < ge; j += stride) {
+        if (j > gs && keys[j] == keys[j - 1]) continue;  // one pass per distinct key
+        const uint32_t v = key_low(keys[j]);
+        const unsigned long long s = idx_find(ix, (static_cast<unsigned long long>(u) << 32) | v);
+        if (s == ~0ull) continue;
+        uint32_t first = kInf, live = 0;
+        for (uint32_t q = 0; q < d.len; ++q)
+            if (*view.at(d.off + q) == v) {
+                if (first == kInf) first = q;
+                ++live;
+            }
+        ix.val[s] = make_uint2(first, live);
+    }
+}
+
+__device__ __forceinline__ bool warp_has_repeats(const unsigned long long *keys, uint32_t gs, uint32_t ge) {
+    bool any = false;
+    for (uint32_t i = gs + lane_id(); i + 1 < ge; i += 32u) any |= keys[i] == keys[i + 1];
+    return __any_sync(kFull, any);
+}
+
+__global__ void __launch_bounds__(kMutWarps * 32, 3)
+    del_wide(AdjView view, RowDesc *desc, const unsigned long long *keys, Groups gr, PosIndex ix, DelLists dl,
+             CompactList cl, uint32_t *matched, uint32_t *seg_hot, unsigned long long *stats,
+             unsigned long long *scan_stats, Status *st) {
+    const uint32_t lane = lane_id();
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    uint32_t removed = 0, changed = 0, scanned = 0, scanned_cached = 0;  // lane 0 counts
+    const uint32_t nw = *dl.wide_count;
+    for (uint32_t i = wid; i < nw; i += warps) {
+        const uint32_t g = dl.wide[i];
+        const uint32_t gs = gr.start[g], ge = gr.end[g];
+        const uint32_t u = key_src(keys[gs]);
+        const RowDesc d = desc[u];
+        const bool indexed = idx_row(ix, u);
+        uint32_t tombs = 0;
+        if (indexed && !warp_has_repeats(keys, gs, ge)) {
+            for (uint32_t j = gs + lane; j < ge; j += 32u)
+                tombs += del_index_key(view, d, u, key_low(keys[j]), ix, st);
+            tombs = __reduce_add_sync(kFull, tombs);
+        } else if (d.len > kWarpRowMax) {
+            if (lane == 0) dl.big[atomicAdd(dl.big_count, 1u)] = g;
+            continue;
+        } else if (d.len) {
+            if (ge - gs <= 32u) {
+                tombs = warp_tomb_regs(view, d, keys, gs, ge - gs);
+            } else {
+                for (uint32_t j = gs + lane; j < ge; j += 32u) matched[j] = 0u;
+                __syncwarp();
+                tombs = warp_tomb_global(view, d, u, keys, gs, ge, matched);
+            }
+            __syncwarp();
+            if (lane == 0) {
+                scanned += d.len;
+                if (view.cached(d.off)) scanned_cached += d.len;
+                seg_touch(seg_hot, d.off, d.len);
+            }
+            if (indexed) {
+                idx_recount_group(view, d, u, keys, gs, ge, lane, 32u, ix);
+                __syncwarp();
+            }
+        }
+        if (!tombs) continue;
+        const uint32_t t = rd_tombs(d) + tombs;
+        const bool compact = 4ull * t >= d.len || t >= kMaxTombs / 2;
+        if (compact && d.len <= kWarpMove) {
+            __syncwarp();
+            const uint32_t w = warp_move_live(view, ix, u, d.off, d.len, d.off, st);
+            if (lane == 0) desc[u] = RowDesc{d.off, w, rd_meta(rd_cls(d), 0)};
+        } else if (lane == 0) {
+            desc[u].meta = rd_meta(rd_cls(d), t);
+            if (compact) cl.rows[cl.cap - 1u - atomicAdd(cl.big_count, 1u)] = u;
+        }
+        if (lane == 0) {
+            removed += tombs;
+            ++changed;
+        }
+    }
+    // Hub groups: chunk c of their concatenated 32-key chunks goes to warp c
+    // mod warps; every warp walks the (short) list in the same order.  A
+    // group with repeated requests goes to the block path whole.
+    const uint32_t nh = *dl.huge_count;
+    uint64_t prefix = 0;
+    for (uint32_t h = 0; h < nh; ++h) {
+        const uint32_t g = dl.huge[h];
+        const uint32_t gs = gr.start[g], ge = gr.end[g];
+        if (warp_has_repeats(keys, gs, ge)) {
+            if (wid == 0 && lane == 0) dl.big[atomicAdd(dl.big_count, 1u)] = g;
+            continue;
+        }
+        const uint32_t nk = ge - gs;
+        const uint64_t chunks = (nk + 31u) / 32u;
+        uint64_t c = prefix + (wid + warps - static_cast<uint32_t>(prefix % warps)) % warps;
+        if (c < prefix + chunks) {
+            const uint32_t u = key_src(keys[gs]);
+            const RowDesc d = desc[u];  // only `meta` changes meanwhile
+            uint32_t tombs = 0;
+            for (; c < prefix + chunks; c += warps) {
+                const uint32_t j = static_cast<uint32_t>(c - prefix) * 32u + lane;
+                if (j < nk) tombs += del_index_key(view, d, u, key_low(keys[gs + j]), ix, st);
+            }
+            tombs = __reduce_add_sync(kFull, tombs);
+            if (lane == 0 && tombs) {
+                atomicAdd(&desc[u].meta, tombs << 6);
+                removed += tombs;
+            }
+        }
+        prefix += chunks;
+    }
+    if (stats) {
+        warp_count(&stats[kCntRemoved], removed);
+        warp_count(&stats[kCntChanged], changed);
+    }
+    warp_count(&scan_stats[kCntDelScanned], scanned);
+    warp_count(&scan_stats[kCntDelScannedCached], scanned_cached);
+}
+
+// Rows left by the two kernels before: ordered groups on rows above
+// kWarpRowMax, hub groups' rows that are due for compaction, and the queued
+// compactions.
+__global__ void __launch_bounds__(kTpbMut)
+    del_rest(AdjView view, RowDesc *desc, const unsigned long long *keys, Groups gr, PosIndex ix, DelLists dl,
+             CompactList cl, uint32_t *matched, uint32_t *seg_hot, unsigned long long *stats,
+             unsigned long long *scan_stats, Status *st) {
+    __shared__ OrderedSmem om;
+    __shared__ MoveSmem sm;
+    const uint32_t tid = threadIdx.x;
+    const uint32_t nb = *dl.big_count;
+    for (uint32_t b = blockIdx.x; b < nb; b += gridDim.x) {
+        const uint32_t gs = gr.start[dl.big[b]], ge = gr.end[dl.big[b]];
+        const uint32_t u = key_src(keys[gs]);
+        const RowDesc d = desc[u];
+        if (ge - gs > kBigKeys)
+            for (uint32_t j = gs + tid; j < ge; j += kTpbMut) matched[j] = 0u;
+        __syncthreads();
+        const uint32_t done = block_tomb_ordered(view, d, u, keys, gs, ge, matched, om);
+        __syncthreads();
+        if (idx_row(ix, u)) {
+            idx_recount_group(view, d, u, keys, gs, ge, tid, kTpbMut, ix);
+            __syncthreads();
+        }
+        const uint32_t t = rd_tombs(d) + done;
+        uint32_t len = d.len, tombs = t;
+        if (done && (4ull * t >= d.len || t >= kMaxTombs / 2)) {
+            len = block_move_live(view, ix, u, d.off, d.len, d.off, sm, st);
+            tombs = 0;
+        }
+        if (tid == 0 && done) {
+            desc[u] = RowDesc{d.off, len, rd_meta(rd_cls(d), tombs)};
+            if (stats) {
+                atomicAdd(&stats[kCntRemoved], static_cast<unsigned long long>(done));
+                atomicAdd(&stats[kCntChanged], 1ull);
+            }
+        }
+        if (tid == 0) {
+            seg_touch(seg_hot, d.off, d.len);
+            atomicAdd(&scan_stats[kCntDelScanned], static_cast<unsigned long long>(d.len));
+            if (view.cached(d.off)) atomicAdd(&scan_stats[kCntDelScannedCached], static_cast<unsigned long long>(d.len));
+        }
+        __syncthreads();
+    }
+    const uint32_t nh = *dl.huge_count;
+    for (uint32_t h = blockIdx.x; h < nh; h += gridDim.x) {
+        const uint32_t gs = gr.start[dl.huge[h]], ge = gr.end[dl.huge[h]];
+        bool rep = false;  // then it was in the list above
+        for (uint32_t i = gs + tid; i + 1 < ge; i += kTpbMut) rep |= keys[i] == keys[i + 1];
+        if (__syncthreads_or(rep)) continue;
+        const uint32_t u = key_src(keys[gs]);
+        const RowDesc d = desc[u];
+        const uint32_t t = rd_tombs(d);
+        const uint32_t before = matched[gs];
+        __syncthreads();
+        if (t == before) continue;
+        if (4ull * t >= d.len || t >= kMaxTombs / 2) {
+            const uint32_t w = block_move_live(view, ix, u, d.off, d.len, d.off, sm, st);
+            if (tid == 0) desc[u] = RowDesc{d.off, w, rd_meta(rd_cls(d), 0)};
+        }
+        if (tid == 0 && stats) atomicAdd(&stats[kCntChanged], 1ull);
+        __syncthreads();
+    }
+    compact_listed(view, desc, cl, ix, sm, st);
+}
+
 // ---------------------------------------------------------------- addition
 
 // Addition plan.  A row whose block has room appends in place (kKeyNone).  A
@@ -1254,49 +1601,8 @@ __global__ void __launch_bounds__(kTpbMut) compact_rows(AdjView view, RowDesc *d
 constexpr unsigned long long kKeyOverflow = ~0ull - 1ull;  // degree overflow, reported by the apply kernel
 constexpr unsigned long long kKeyInPlace = ~0ull - 2ull;
 
-__global__ void plan_add(const RowDesc *desc, const unsigned long long *keys, Groups gr, unsigned long long *plan,
-                         ArenaAlloc *al) {
-    const uint32_t ng = *gr.count;
-    const uint32_t rounded = (ng + 31u) & ~31u;
-    const uint32_t lane = lane_id();
-    for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < rounded; g += gridDim.x * blockDim.x) {
-        unsigned long long p = kKeyNone;
-        bool move = false;
-        uint32_t cls = 0;
-        if (g < ng) {
-            const uint32_t gs = gr.start[g];
-            const uint32_t ge = gr.end[g];
-            const RowDesc d = desc[key_src(keys[gs])];
-            const unsigned long long used = static_cast<unsigned long long>(d.len) + (ge - gs);
-            const unsigned long long live = static_cast<unsigned long long>(rd_live(d)) + (ge - gs);
-            if (live > 0xFFFFFFFFull) {
-                p = kKeyOverflow;
-            } else if (rd_cls(d) == 0 || live > (1ull << rd_cls(d))) {
-                cls = class_for(static_cast<uint32_t>(live));
-                move = true;
-            } else if (used > (1ull << rd_cls(d))) {
-                p = kKeyInPlace;
-            }
-        }
-        // Ranks within a class, one atomic per class present in the warp
-        // (tens of thousands of moving rows share a handful of classes).
-        const uint32_t movers = __ballot_sync(kFull, move);
-        if (move) {
-            const uint32_t peers = __match_any_sync(movers, cls);
-            const uint32_t leader = __ffs(peers) - 1;
-            uint32_t base = 0;
-            if (lane == leader) base = atomicAdd(&al->demand[cls], static_cast<uint32_t>(__popc(peers)));
-            base = __shfl_sync(peers, base, leader);
-            p = (static_cast<unsigned long long>(cls) << 32) | (base + __popc(peers & lanemask_lt()));
-        }
-        if (g < ng) plan[g] = p;
-    }
-}
-
-// Serve this batch's demand per class (one thread per class).
-__global__ void alloc_classes(ArenaAlloc *al, Status *st) {
-    const uint32_t c = threadIdx.x;
-    if (c >= kNumClasses) return;
+// Serve this batch's demand of one class.
+__device__ __forceinline__ void alloc_class(ArenaAlloc *al, uint32_t c, Status *st) {
     const uint32_t need = al->demand[c];
     al->demand[c] = 0;
     al->avail[c] = 0;
@@ -1333,25 +1639,91 @@ __global__ void alloc_classes(ArenaAlloc *al, Status *st) {
     }
 }
 
+// The last block to finish hands out the blocks (one thread per class) and
+// gives the new segments cache slots: two launches less in the chain.
+__global__ void plan_add(const RowDesc *desc, const unsigned long long *keys, Groups gr, unsigned long long *plan,
+                         ArenaAlloc *al, bool assign, SegTable seg, uint32_t *blocks_done, Status *st) {
+    const uint32_t ng = *gr.count;
+    const uint32_t rounded = (ng + 31u) & ~31u;
+    const uint32_t lane = lane_id();
+    for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < rounded; g += gridDim.x * blockDim.x) {
+        unsigned long long p = kKeyNone;
+        bool move = false;
+        uint32_t cls = 0;
+        if (g < ng) {
+            const uint32_t gs = gr.start[g];
+            const uint32_t ge = gr.end[g];
+            const RowDesc d = desc[key_src(keys[gs])];
+            const unsigned long long used = static_cast<unsigned long long>(d.len) + (ge - gs);
+            const unsigned long long live = static_cast<unsigned long long>(rd_live(d)) + (ge - gs);
+            if (live > 0xFFFFFFFFull) {
+                p = kKeyOverflow;
+            } else if (rd_cls(d) == 0 || live > (1ull << rd_cls(d))) {
+                cls = class_for(static_cast<uint32_t>(live));
+                move = true;
+            } else if (used > (1ull << rd_cls(d))) {
+                p = kKeyInPlace;
+            }
+        }
+        // Ranks within a class, one atomic per class present in the warp
+        // (tens of thousands of moving rows share a handful of classes).
+        const uint32_t movers = __ballot_sync(kFull, move);
+        if (move) {
+            const uint32_t peers = __match_any_sync(movers, cls);
+            const uint32_t leader = __ffs(peers) - 1;
+            uint32_t base = 0;
+            if (lane == leader) base = atomicAdd(&al->demand[cls], static_cast<uint32_t>(__popc(peers)));
+            base = __shfl_sync(peers, base, leader);
+            p = (static_cast<unsigned long long>(cls) << 32) | (base + __popc(peers & lanemask_lt()));
+        }
+        if (g < ng) plan[g] = p;
+    }
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(blocks_done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (uint32_t c = threadIdx.x; c < kNumClasses; c += blockDim.x) alloc_class(al, c, st);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        *blocks_done = 0;
+        if (assign) seg_assign_new(seg, *reinterpret_cast<volatile unsigned long long *>(&al->seg_bump), st);
+    }
+}
+
 // Addition phase.  mutate_add gives each lane a group of its own when the
 // lane can serve it alone (at most kLaneAdds appends, and a moving row of at
 // most kLaneRow slots, read into registers with independent loads: rows in
 // host memory cost one round trip, not one per entry), so the common
-// one-request groups run 32 to a warp.  The other groups are appended to a
-// list that mutate_add_warp serves one warp per group over the whole grid
-// (rows above kWarpRowMax that must move go on to the block path,
-// mutate_add_big).  Serving them inside the warp that found them left the
+// one-request groups run 32 to a warp.  The other groups are listed for
+// mutate_add_wide, which serves them one warp per group over the whole grid
+// (a block per row of more than kWarpRowMax slots that must move, or than
+// kWarpMove that must drop its tombstones).  Serving them inside the warp that found them left the
 // busiest warps a serial queue of up to 32 row copies while most of the grid
 // had no group at all.  `vals` is add_v for the forward arena and add_u for
 // the reverse arena.  A moving row is copied without its tombstones.
 constexpr uint32_t kLaneAdds = 8;
 constexpr uint32_t kLaneRow = 8;
 
+// Groups for whole warps and for whole blocks.
+struct AddLists {
+    uint32_t *warp;
+    uint32_t *warp_count;
+    uint32_t *block;
+    uint32_t *block_count;
+};
+
+// A moving row keeps its tombstones when they fit the new block.
+__device__ __forceinline__ bool moves_whole(unsigned long long p, const RowDesc &d, uint32_t a) {
+    return p != kKeyInPlace && static_cast<unsigned long long>(d.len) + a <= (1ull << static_cast<uint32_t>(p >> 32));
+}
+
 __global__ void __launch_bounds__(256, 4)
     mutate_add(AdjView view, RowDesc *desc, const unsigned long long *keys, Groups gr,
                            const unsigned long long *plan, const ArenaAlloc *al, const uint32_t *vals,
-                           uint32_t *coop_list, uint32_t *coop_count, unsigned long long *stats, PosIndex ix,
-                           Status *st) {
+                           AddLists ls, unsigned long long *stats, PosIndex ix, Status *st) {
     if (ld_volatile(&st->err) & kErrArena) return;
     const uint32_t lane = lane_id();
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
@@ -1359,19 +1731,21 @@ __global__ void __launch_bounds__(256, 4)
     uint32_t changed = 0, moved = 0, moved_entries = 0;  // per lane
     for (uint32_t base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32u; base < ng; base += warps * 32u) {
         const uint32_t g = base + lane;
-        bool coop = false;
+        bool coop = false, block = false;
         if (g < ng) {
             const unsigned long long p = plan[g];
             const uint32_t gs = gr.start[g];
             const uint32_t a = gr.end[g] - gs;
+            const uint32_t u = key_src(keys[gs]);
+            const RowDesc d = desc[u];
+            const bool indexed = idx_row(ix, u);
             if (p == kKeyOverflow) {
                 set_error(st, kErrInternal, g);
+            } else if (p != kKeyNone && d.len > (moves_whole(p, d, a) ? kWarpRowMax : kWarpMove)) {
+                block = true;
             } else if (a > kLaneAdds) {
                 coop = true;
             } else {
-                const uint32_t u = key_src(keys[gs]);
-                const RowDesc d = desc[u];
-                const bool indexed = idx_row(ix, u);
                 // The appended values first, with independent loads (the
                 // stores below could alias them as far as the compiler knows).
                 uint32_t add[kLaneAdds];
@@ -1419,9 +1793,8 @@ __global__ void __launch_bounds__(256, 4)
                 }
             }
         }
-        // Groups a lane cannot serve alone go to the warp-per-group kernel,
-        // which spreads them over every warp of the grid.
-        warp_enqueue(coop, g, coop_list, coop_count, ng, st);
+        warp_enqueue(coop, g, ls.warp, ls.warp_count, ng, st);
+        warp_enqueue(block, g, ls.block, ls.block_count, ng, st);
     }
     if (stats) {
         warp_count(&stats[kCntChanged], changed);
@@ -1431,22 +1804,69 @@ __global__ void __launch_bounds__(256, 4)
 }
 
 
-// The groups mutate_add left to whole warps (more than kLaneAdds appends, or
-// a moving or compacting row of more than kLaneRow entries), one warp per
-// group over the whole grid: rows of up to kWarpRowMax entries move as they
-// are here, rows of up to kWarpMove entries drop their tombstones here,
-// larger ones go to mutate_add_big.
-__global__ void mutate_add_warp(AdjView view, RowDesc *desc, const unsigned long long *keys, Groups gr,
-                                const unsigned long long *plan, const ArenaAlloc *al, const uint32_t *vals,
-                                const uint32_t *coop_list, const uint32_t *coop_count, uint32_t *big,
-                                uint32_t *big_count, unsigned long long *stats, PosIndex ix, Status *st) {
+// The groups mutate_add listed: a block per long row, then a warp per group.
+__global__ void __launch_bounds__(kTpbMut, 2)
+    mutate_add_wide(AdjView view, RowDesc *desc, const unsigned long long *keys, Groups gr,
+                    const unsigned long long *plan, const ArenaAlloc *al, const uint32_t *vals, AddLists ls,
+                    unsigned long long *stats, PosIndex ix, Status *st) {
+    __shared__ MoveSmem sm;
     if (ld_volatile(&st->err) & kErrArena) return;
+    const uint32_t nb = *ls.block_count;
+    for (uint32_t b = blockIdx.x; b < nb; b += gridDim.x) {
+        const uint32_t g = ls.block[b];
+        const unsigned long long p = plan[g];
+        const uint32_t gs = gr.start[g];
+        const uint32_t ge = gr.end[g];
+        const uint32_t u = key_src(keys[gs]);
+        const RowDesc d = desc[u];
+        const uint32_t a = ge - gs;
+        const bool moves = p != kKeyInPlace;
+        const uint32_t cls = moves ? static_cast<uint32_t>(p >> 32) : rd_cls(d);
+        const bool whole = moves_whole(p, d, a);
+        const unsigned long long off = moves ? alloc_offset(al, cls, static_cast<uint32_t>(p)) : d.off;
+        uint32_t w = d.len;
+        if (!whole) {
+            w = block_move_live(view, ix, u, d.off, d.len, off, sm, st);
+        } else {
+            // 16 entries per thread and step, resolved per 16 bytes (a block
+            // above one segment may lie in HBM and in host memory).
+            for (uint32_t b0 = 0; b0 < d.len; b0 += 16u * kTpbMut) {
+                uint4 q[4];
+#pragma unroll
+                for (uint32_t h = 0; h < 4; ++h) {
+                    const uint32_t k = b0 + 4u * (h * kTpbMut + threadIdx.x);
+                    if (k < d.len) q[h] = *reinterpret_cast<const uint4 *>(view.at(d.off + k));
+                }
+#pragma unroll
+                for (uint32_t h = 0; h < 4; ++h) {
+                    const uint32_t k = b0 + 4u * (h * kTpbMut + threadIdx.x);
+                    if (k < d.len) *reinterpret_cast<uint4 *>(view.wptr(off + k)) = q[h];
+                }
+            }
+        }
+        __syncthreads();  // moved before the appends behind them (and before their index entries)
+        const bool indexed = idx_row(ix, u);
+        for (uint32_t j = threadIdx.x; j < a; j += kTpbMut) {
+            const uint32_t v = vals[key_low(keys[gs + j])];
+            write_slot(view, off + w + j, v);
+            if (indexed) idx_add(ix, u, v, w + j, st);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            desc[u] = RowDesc{off, w + a, rd_meta(cls, whole ? rd_tombs(d) : 0u)};
+            if (stats) {
+                atomicAdd(&stats[kCntChanged], 1ull);
+                atomicAdd(&stats[kCntRelocated], moves ? 1ull : 0ull);
+                atomicAdd(&stats[kCntMovedEntries], moves ? static_cast<unsigned long long>(w) : 0ull);
+            }
+        }
+    }
     const uint32_t lane = lane_id();
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    const uint32_t nc = *coop_count;
+    const uint32_t nc = *ls.warp_count;
     uint32_t changed = 0, moved = 0, moved_entries = 0;  // lane 0 counts
     for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nc; i += warps) {
-        const uint32_t gb = coop_list[i];
+        const uint32_t gb = ls.warp[i];
         const unsigned long long p = plan[gb];
         const uint32_t gs = gr.start[gb];
         const uint32_t ge = gr.end[gb];
@@ -1464,12 +1884,7 @@ __global__ void mutate_add_warp(AdjView view, RowDesc *desc, const unsigned long
         } else {
             const bool moves = p != kKeyInPlace;
             const uint32_t cls = moves ? static_cast<uint32_t>(p >> 32) : rd_cls(d);
-            // Tombstones come along when they fit.
-            const bool whole = moves && static_cast<unsigned long long>(d.len) + a <= (1ull << cls);
-            if (d.len > (whole ? kWarpRowMax : kWarpMove)) {
-                if (lane == 0) big[atomicAdd(big_count, 1u)] = gb;
-                continue;
-            }
+            const bool whole = moves_whole(p, d, a);
             const unsigned long long off = moves ? alloc_offset(al, cls, static_cast<uint32_t>(p)) : d.off;
             uint32_t w = d.len;
             if (!whole) {
@@ -1514,64 +1929,6 @@ __global__ void mutate_add_warp(AdjView view, RowDesc *desc, const unsigned long
         warp_count(&stats[kCntChanged], changed);
         warp_count(&stats[kCntRelocated], moved);
         warp_count(&stats[kCntMovedEntries], moved_entries);
-    }
-}
-
-__global__ void __launch_bounds__(kTpbMut)
-    mutate_add_big(AdjView view, RowDesc *desc, const unsigned long long *keys, Groups gr,
-                   const unsigned long long *plan, const ArenaAlloc *al, const uint32_t *vals, const uint32_t *big,
-                   const uint32_t *big_count, unsigned long long *stats, PosIndex ix, Status *st) {
-    __shared__ MoveSmem sm;
-    if (ld_volatile(&st->err) & kErrArena) return;
-    const uint32_t nb = *big_count;
-    for (uint32_t b = blockIdx.x; b < nb; b += gridDim.x) {
-        const uint32_t g = big[b];
-        const unsigned long long p = plan[g];
-        const uint32_t gs = gr.start[g];
-        const uint32_t ge = gr.end[g];
-        const uint32_t u = key_src(keys[gs]);
-        const RowDesc d = desc[u];
-        const uint32_t a = ge - gs;
-        const bool moves = p != kKeyInPlace;
-        const uint32_t cls = moves ? static_cast<uint32_t>(p >> 32) : rd_cls(d);
-        const bool whole = moves && static_cast<unsigned long long>(d.len) + a <= (1ull << cls);
-        const unsigned long long off = moves ? alloc_offset(al, cls, static_cast<uint32_t>(p)) : d.off;
-        uint32_t w = d.len;
-        if (!whole) {
-            w = block_move_live(view, ix, u, d.off, d.len, off, sm, st);
-        } else {
-            // 16 entries per thread and step, resolved per 16 bytes (a block
-            // above one segment may lie in HBM and in host memory).
-            for (uint32_t b0 = 0; b0 < d.len; b0 += 16u * kTpbMut) {
-                uint4 q[4];
-#pragma unroll
-                for (uint32_t h = 0; h < 4; ++h) {
-                    const uint32_t k = b0 + 4u * (h * kTpbMut + threadIdx.x);
-                    if (k < d.len) q[h] = *reinterpret_cast<const uint4 *>(view.at(d.off + k));
-                }
-#pragma unroll
-                for (uint32_t h = 0; h < 4; ++h) {
-                    const uint32_t k = b0 + 4u * (h * kTpbMut + threadIdx.x);
-                    if (k < d.len) *reinterpret_cast<uint4 *>(view.wptr(off + k)) = q[h];
-                }
-            }
-        }
-        __syncthreads();  // moved before the appends behind them (and before their index entries)
-        const bool indexed = idx_row(ix, u);
-        for (uint32_t j = threadIdx.x; j < a; j += kTpbMut) {
-            const uint32_t v = vals[key_low(keys[gs + j])];
-            write_slot(view, off + w + j, v);
-            if (indexed) idx_add(ix, u, v, w + j, st);
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            desc[u] = RowDesc{off, w + a, rd_meta(cls, whole ? rd_tombs(d) : 0u)};
-            if (stats) {
-                atomicAdd(&stats[kCntChanged], 1ull);
-                atomicAdd(&stats[kCntRelocated], moves ? 1ull : 0ull);
-                atomicAdd(&stats[kCntMovedEntries], moves ? static_cast<unsigned long long>(w) : 0ull);
-            }
-        }
     }
 }
 

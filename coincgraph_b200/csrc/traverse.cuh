@@ -11,11 +11,12 @@
 //
 // Per batch (reference flow: include/framework/framework.cuh:2752-2894 for
 // deletions, :2139-2348 for insertions):
-//   deletion:  seed_deletions -> inval_closure -> reset_affected -> pull_repair
-//              -> enqueue_affected -> push_closure
-//   insertion: seed_insertions -> push_closure
+//   deletion:  repair_closure (seeds, invalidation rounds, reset, pull repair,
+//              re-queue), then push_closure
+//   insertion: push_closure (seeds, relaxation rounds)
 #pragma once
 
+#include "cache.cuh"
 #include "common.cuh"
 #include "expand.cuh"
 
@@ -325,13 +326,63 @@ struct LocalPushOp {
     }
 };
 
+// Insertion seeds (SeedAddedEdgeFrontier, framework.cuh:238-294): relax every
+// inserted edge with the value of its source after the topology update.
+struct SeedEdges {
+    const uint32_t *u;
+    const uint32_t *v;
+    uint32_t count;
+    uint32_t n;  // ids at or above are ignored
+};
+
+template <int A>
+__device__ __forceinline__ void seed_insertions(const SeedEdges &e, unsigned long long *state, uint32_t *qstamp,
+                                                uint32_t tag, uint32_t ccs, const Frontier &fr, Status *st) {
+    uint32_t seeds = 0;
+    const uint32_t rounded = (e.count + 31u) & ~31u;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < rounded; i += gridDim.x * blockDim.x) {
+        bool want = false;
+        uint32_t v = 0;
+        if (i < e.count) {
+            const uint32_t u = e.u[i];
+            v = e.v[i];
+            if (u < e.n && v < e.n) {
+                const uint32_t du = val_of(__ldcg(state + u));
+                const unsigned long long sv = __ldcg(state + v);
+                if (du != kInf) {
+                    const uint32_t nd = relax_value<A>(du, u, v, ccs);
+                    const unsigned long long cand = pack(nd, u);
+                    if (cand < sv) {
+                        const unsigned long long old = atomicMin(state + v, cand);
+                        if (nd < val_of(old)) want = atomicExch(qstamp + v, tag) != tag;
+                    }
+                }
+            }
+        }
+        warp_enqueue(want, v, fr.q0, fr.cnt, fr.cap, st);
+        seeds += want ? 1u : 0u;
+    }
+    warp_count(&st->counters[kCntSeeds], seeds);
+}
+
+// Parts of a closure kernel to run: all in one launch (a kernel of their own
+// each cost a launch in a chain whose kernels mostly take a few
+// microseconds), or one at a time for the stage profiler.
+enum ClosurePart : uint32_t { kPartSeed = 1, kPartRounds = 2, kPartPull = 4, kPartAll = 7 };
+
 template <int A>
 __global__ void __launch_bounds__(kTpb, 4) push_closure(AdjView fwd, unsigned long long *state, uint32_t *qstamp,
-                                                     TagState *tags, Frontier fr, BigList big, uint32_t max_rounds,
-                                                     uint32_t max_sweeps, uint32_t *seg_hot, Status *st) {
+                                                     TagState *tags, Frontier fr, SeedEdges seeds, uint32_t parts,
+                                                     BigList big, uint32_t max_rounds, uint32_t max_sweeps,
+                                                     uint32_t *seg_hot, Status *st) {
     __shared__ ExpandSmem<kTpb> sm;
     __shared__ uint32_t lq[2][kLocalCap];
     __shared__ uint32_t lq_n[2];
+    if ((parts & kPartSeed) && seeds.count) {
+        seed_insertions<A>(seeds, state, qstamp, tags->next_tag, (A == kCc) ? st->cc_shift : 0u, fr, st);
+        if ((parts & kPartRounds) && !grid_barrier(st)) return;
+    }
+    if (!(parts & kPartRounds)) return;
     ExpandCounters cnt;
     // next_tag itself belongs to the seeds queued before this launch.
     const uint32_t tag0 = tags->next_tag + 1;
@@ -532,18 +583,113 @@ struct LocalInvalOp {
     }
 };
 
+// Deletion seeds (reset_del_edges, include/framework/variants/driver.cuh:
+// 371-411), evaluated on the values before the batch.
 template <int A>
-__global__ void __launch_bounds__(kTpb, 4) inval_closure(AdjView fwd, unsigned long long *state, uint32_t *aff_stamp,
-                                                      const uint32_t *epoch_p, uint32_t *list, uint32_t *cnt3,
-                                                      uint32_t cap, BigList big, uint32_t max_rounds,
-                                                      uint32_t max_sweeps, uint32_t *done, uint32_t *done_cnt,
-                                                      uint32_t *aff_total, uint32_t *seg_hot, Status *st) {
+__device__ __forceinline__ void seed_deletions(const SeedEdges &e, const unsigned long long *state,
+                                               uint32_t *aff_stamp, uint32_t epoch, uint32_t ccs, uint32_t *list,
+                                               uint32_t *count, uint32_t cap, Status *st) {
+    const uint32_t rounded = (e.count + 31u) & ~31u;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < rounded; i += gridDim.x * blockDim.x) {
+        bool want = false;
+        uint32_t v = 0;
+        if (i < e.count) {
+            const uint32_t u = e.u[i];
+            v = e.v[i];
+            if (u < e.n && v < e.n) {
+                const unsigned long long sv = __ldcg(state + v);
+                bool dep;
+                if (A == kCc) {
+                    const uint32_t lu = val_of(__ldcg(state + u)) >> ccs;
+                    const uint32_t vv = val_of(sv);
+                    dep = u != v && (par_of(sv) == u || (cc_saturated(vv, ccs) && lu == (vv >> ccs) && (vv >> ccs) < v));
+                } else {
+                    dep = par_of(sv) == u && val_of(sv) != kInf;
+                }
+                if (dep && __ldcg(aff_stamp + v) != epoch) want = atomicExch(aff_stamp + v, epoch) != epoch;
+            }
+        }
+        warp_enqueue(want, v, list, count, cap, st);
+    }
+}
+
+// Repair of the invalidated vertices: value <- initial value
+// (reset_affected_values, driver.cuh:418-433: unreached for BFS/SSSP, its own
+// id for CC), pull over their in-rows, queue every one that has a value (all
+// of them for CC).  In-rows of at least big.split entries are left to the
+// whole grid after a barrier.
+template <int A>
+__device__ __forceinline__ void pull_repair(const AdjView &rev, unsigned long long *state, const uint32_t *aff_stamp,
+                                            uint32_t epoch, uint32_t ccs, const uint32_t *list, uint32_t n,
+                                            const Frontier &fr, const Defer &df, ExpandSmem<kTpb> &sm, Status *st) {
+    const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, gthreads = gridDim.x * blockDim.x;
+    for (uint32_t i = gtid; i < n; i += gthreads) {
+        const uint32_t v = __ldcg(list + i);
+        state[v] = (A == kCc) ? pack(v << ccs, kInf) : kInf64;
+        prefetch_l2(rev.desc + v);
+    }
+    if (!grid_barrier(st)) return;
+    ExpandCounters c;
+    const PullOp<A> op{ccs, state, aff_stamp, epoch};
+    for (uint32_t base = 0; base < n; base += gridDim.x * kTpb) {
+        const uint32_t i = base + spread_rank<kTpb>() * gridDim.x + blockIdx.x;
+        bool has = i < n;
+        uint32_t v = 0, deg = 0;
+        uint64_t off = 0;
+        if (has) {
+            v = __ldcg(list + i);
+            const RowDesc d = rev.desc[v];
+            deg = d.len;
+            off = d.off;
+            has = deg > 0;
+        }
+        expand_rows<kTpb>(rev, has, v, 0u, off, deg, op, sm, c, df);
+    }
+    if (!grid_barrier(st)) return;
+    const uint32_t nbig = min(ld_volatile(df.count), df.cap);
+    if (nbig) {
+        expand_deferred<kTpb>(rev, df.rows, nbig, op, c);
+        if (!grid_barrier(st)) return;
+    }
+    const uint32_t rounded = (n + 31u) & ~31u;
+    for (uint32_t i = gtid; i < rounded; i += gthreads) {
+        bool want = false;
+        uint32_t v = 0;
+        if (i < n) {
+            v = __ldcg(list + i);
+            want = (A == kCc) || val_of(__ldcg(state + v)) != kInf;
+        }
+        warp_enqueue(want, v, fr.q0, fr.cnt, fr.cap, st);
+    }
+    flush_counters(st, c, kCntPull);
+}
+
+// The deletion phase's closure (cooperative launch): seeds, invalidation
+// rounds, repair.  `pull_big`: counter of the in-rows left to the whole grid.
+template <int A>
+__global__ void __launch_bounds__(kTpb, 2) repair_closure(AdjView fwd, AdjView rev, SeedEdges seeds, uint32_t parts,
+                                                          unsigned long long *state, uint32_t *aff_stamp,
+                                                          const uint32_t *epoch_p, uint32_t *list, uint32_t *cnt3,
+                                                          uint32_t cap, BigList big, uint32_t *pull_big,
+                                                          uint32_t max_rounds, uint32_t max_sweeps, uint32_t *done,
+                                                          uint32_t *done_cnt, uint32_t *aff_total, Frontier fr,
+                                                          uint32_t *seg_hot, Status *st) {
     __shared__ ExpandSmem<kTpb> sm;
     __shared__ uint32_t lq[2][kLocalCap];
     __shared__ uint32_t lq_n[2];
     ExpandCounters c;
     const uint32_t ccs = (A == kCc) ? st->cc_shift : 0u;
     const uint32_t epoch = *epoch_p;
+    if ((parts & kPartSeed) && seeds.count) {
+        seed_deletions<A>(seeds, state, aff_stamp, epoch, ccs, list, cnt3, cap, st);
+        if ((parts & kPartRounds) && !grid_barrier(st)) return;
+    }
+    const Defer pull_df{big.rows, pull_big, big.cap, big.split};
+    if (!(parts & kPartRounds)) {
+        const uint32_t n = (parts & kPartPull) ? *aff_total : 0u;
+        if (n) pull_repair<A>(rev, state, aff_stamp, epoch, ccs, list, n, fr, pull_df, sm, st);
+        return;
+    }
     uint32_t lo = 0, hi = ld_volatile(cnt3 + 0);
     uint32_t r = 0;
     for (;; ++r) {
@@ -651,141 +797,22 @@ __global__ void __launch_bounds__(kTpb, 4) inval_closure(AdjView fwd, unsigned l
         atomicAdd(&st->counters[kCntRounds], static_cast<unsigned long long>(r));
         atomicAdd(&st->counters[kCntAffected], static_cast<unsigned long long>(hi));
     }
-}
-
-// Deletion seeds (reset_del_edges, include/framework/variants/driver.cuh:
-// 371-411), evaluated on the values before the batch.
-template <int A>
-__global__ void seed_deletions(const uint32_t *du, const uint32_t *dv, uint32_t nd, uint32_t n,
-                               const unsigned long long *state, uint32_t *aff_stamp, const uint32_t *epoch_p,
-                               uint32_t *list, uint32_t *count, uint32_t cap, Status *st) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t epoch = *epoch_p;
-    bool want = false;
-    uint32_t v = 0;
-    if (i < nd) {
-        const uint32_t u = du[i];
-        v = dv[i];
-        if (u < n && v < n) {
-            const unsigned long long sv = __ldcg(state + v);
-            bool dep;
-            if (A == kCc) {
-                const uint32_t ccs = st->cc_shift;
-                const uint32_t lu = val_of(__ldcg(state + u)) >> ccs;
-                const uint32_t vv = val_of(sv);
-                dep = u != v && (par_of(sv) == u || (cc_saturated(vv, ccs) && lu == (vv >> ccs) && (vv >> ccs) < v));
-            } else {
-                dep = par_of(sv) == u && val_of(sv) != kInf;
-            }
-            if (dep && __ldcg(aff_stamp + v) != epoch) want = atomicExch(aff_stamp + v, epoch) != epoch;
-        }
+    if ((parts & kPartPull) && hi) {
+        // the list is complete once every block has appended its share of `done`
+        if (max_sweeps && !grid_barrier(st)) return;
+        pull_repair<A>(rev, state, aff_stamp, epoch, ccs, list, hi, fr, pull_df, sm, st);
     }
-    if (__any_sync(kFull, i < nd)) warp_enqueue(want, v, list, count, cap, st);
 }
 
-// Start of a deletion phase: advance the batch epoch (the "invalidated in
-// this batch" marker of aff_stamp, kept on the device so that a captured
-// batch graph needs no new arguments) and clear the counters of `counters`
-// (64 words) whose bit is set in `mask`, in place of one memset each.
-// Launched with 64 threads.
-__global__ void phase_begin(uint32_t *epoch, uint32_t *counters, unsigned long long mask) {
-    if (threadIdx.x == 0) *epoch += 1u;
+// Start of a phase: advance the batch epoch (the "invalidated in this batch"
+// marker of aff_stamp, kept on the device so that a captured batch graph
+// needs no new arguments; null: keep it), clear the counters of `counters` (64
+// words) whose bit is set in `mask` and the segment table's per-batch ones
+// (null: no table), in place of one memset each.  Launched with 64 threads.
+__global__ void phase_begin(uint32_t *epoch, uint32_t *counters, unsigned long long mask, uint32_t *seg_ctl) {
+    if (epoch && threadIdx.x == 0) *epoch += 1u;
     if (threadIdx.x < 64u && ((mask >> threadIdx.x) & 1u)) counters[threadIdx.x] = 0u;
-}
-
-// value <- initial value for every invalidated vertex (reset_affected_values,
-// driver.cuh:418-433): unreached for BFS/SSSP, its own id for CC.
-template <int A>
-__global__ void reset_affected(const uint32_t *list, const uint32_t *total, unsigned long long *state,
-                               uint32_t ccs) {
-    const uint32_t n = *total;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t v = list[i];
-        state[v] = (A == kCc) ? pack(v << ccs, kInf) : kInf64;
-    }
-}
-
-template <int A>
-__global__ void __launch_bounds__(kTpb, 4) pull_repair(AdjView rev, unsigned long long *state, const uint32_t *aff_stamp,
-                                                    const uint32_t *epoch_p, const uint32_t *list,
-                                                    const uint32_t *total, BigList big, Status *st) {
-    __shared__ ExpandSmem<kTpb> sm;
-    ExpandCounters c;
-    const uint32_t n = *total;
-    PullOp<A> op{(A == kCc) ? st->cc_shift : 0u, state, aff_stamp, *epoch_p};
-    const Defer df{big.rows, big.cnt, big.cap, big.split};
-    for (uint32_t base = 0; base < n; base += gridDim.x * kTpb) {
-        const uint32_t i = base + spread_rank<kTpb>() * gridDim.x + blockIdx.x;
-        bool has = i < n;
-        uint32_t v = 0, deg = 0;
-        uint64_t off = 0;
-        if (has) {
-            v = list[i];
-            const RowDesc d = rev.desc[v];
-            deg = d.len;
-            off = d.off;
-            has = deg > 0;
-        }
-        expand_rows<kTpb>(rev, has, v, 0u, off, deg, op, sm, c, df);
-    }
-    flush_counters(st, c, kCntPull);
-}
-
-// The in-rows that pull_repair deferred, expanded by the whole grid.
-template <int A>
-__global__ void __launch_bounds__(kTpb) pull_deferred(AdjView rev, unsigned long long *state, const uint32_t *aff_stamp,
-                                                      const uint32_t *epoch_p, BigList big, Status *st) {
-    ExpandCounters c;
-    PullOp<A> op{(A == kCc) ? st->cc_shift : 0u, state, aff_stamp, *epoch_p};
-    expand_deferred<kTpb>(rev, big.rows, min(*big.cnt, big.cap), op, c);
-    flush_counters(st, c, kCntPull);
-}
-
-// Queue every repaired vertex that has a value (all of them for CC).
-template <int A>
-__global__ void enqueue_affected(const uint32_t *list, const uint32_t *total, const unsigned long long *state,
-                                 Frontier fr, Status *st) {
-    const uint32_t n = *total;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    const uint32_t rounded = (n + 31u) & ~31u;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < rounded; i += stride) {
-        bool want = false;
-        uint32_t v = 0;
-        if (i < n) {
-            v = list[i];
-            want = (A == kCc) || val_of(__ldcg(state + v)) != kInf;
-        }
-        warp_enqueue(want, v, fr.q0, fr.cnt, fr.cap, st);
-    }
-}
-
-// Insertion seeds (SeedAddedEdgeFrontier, framework.cuh:238-294): relax every
-// inserted edge with the value of its source after the topology update.
-template <int A>
-__global__ void seed_insertions(const uint32_t *au, const uint32_t *av, uint32_t na, uint32_t n,
-                                unsigned long long *state, uint32_t *qstamp, const TagState *tags, Frontier fr,
-                                Status *st) {
-    const uint32_t tag = tags->next_tag;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    bool want = false;
-    uint32_t v = 0;
-    if (i < na) {
-        const uint32_t u = au[i];
-        v = av[i];
-        if (u < n && v < n) {
-            const uint32_t du = val_of(__ldcg(state + u));
-            if (du != kInf) {
-                const uint32_t nd = relax_value<A>(du, u, v, (A == kCc) ? st->cc_shift : 0u);
-                const unsigned long long cand = pack(nd, u);
-                if (cand < __ldcg(state + v)) {
-                    const unsigned long long old = atomicMin(state + v, cand);
-                    if (nd < val_of(old)) want = atomicExch(qstamp + v, tag) != tag;
-                }
-            }
-        }
-    }
-    if (__any_sync(kFull, i < na)) warp_enqueue(want, v, fr.q0, fr.cnt, fr.cap, st);
-    if (want) atomicAdd(&st->counters[kCntSeeds], 1ull);
+    if (seg_ctl) seg_ctl_clear(seg_ctl);
 }
 
 // Static-solve initialisation (InitGraph, framework.cuh:991-1041).

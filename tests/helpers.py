@@ -169,6 +169,21 @@ def full_row_case() -> Case:
     return Case("fullrow", n, xadj, adj, batches, source=0)
 
 
+def recurring_case() -> Case:
+    """The same edges deleted and inserted again, batch after batch, some of
+    them twice in the row and some requested when they are absent, in an
+    indexed row of 300 entries and a short one."""
+    rng = np.random.default_rng(31)
+    n = 500
+    src = np.concatenate([np.zeros(300, np.int64), np.ones(10, np.int64), rng.integers(0, n, 2000)])
+    dst = rng.integers(0, n, len(src))
+    xadj, adj = _csr_from_edges(n, src, dst)
+    u = np.concatenate([np.zeros(40, np.uint32), np.ones(4, np.uint32)])
+    v = np.concatenate([adj[:40], adj[300:304]])
+    batches = [(u, v, u, v)] * 6 + [(u, v, _u32([]), _u32([])), (u, v, u, v), (u, v, u, v)]
+    return Case("recurring", n, xadj, adj, batches, source=0)
+
+
 def grid_case(side: int = 48, batches: int = 3, size: int = 150) -> Case:
     """Road-like high-diameter case: a side x side grid, local insertions."""
     g = gen.grid(side)

@@ -13,8 +13,8 @@ import pytest
 
 import oracle
 from coincgraph_b200 import Engine
-from helpers import (ORACLE_MODE, adversarial_case, big_row_case, full_row_case, grid_case, heavy_delete_case, make_engine,
-                     oracle_trace, rmat_case)
+from helpers import (ORACLE_MODE, adversarial_case, big_row_case, full_row_case, grid_case, heavy_delete_case,
+                     make_engine, oracle_trace, recurring_case, rmat_case)
 
 pytestmark = pytest.mark.gpu
 
@@ -306,6 +306,15 @@ def test_position_index_modes(algo, mode, monkeypatch):
     run_case(heavy_delete_case(), algo, CACHES["zerocopy"])
     run_case_whole_batches(big_row_case(), algo, CACHES["mixed"])
     run_case_whole_batches(rmat_case(11, 3, 400, 400, seed_offset=17), algo, CACHES["resident"])
+
+
+@pytest.mark.parametrize("mode", ["default", "off", "all_rows"])
+def test_recurring_edges(mode, monkeypatch):
+    """Keys that leave the index and come back to it."""
+    for k, v in INDEX_MODES.get(mode, {}).items():
+        monkeypatch.setenv(k, v)
+    run_case(recurring_case(), "sssp", 1.0)
+    run_case_whole_batches(recurring_case(), "bfs", 0.0)
 
 
 @pytest.mark.parametrize("mode", ["default", "off", "all_rows"])
