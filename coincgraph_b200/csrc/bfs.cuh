@@ -1,0 +1,698 @@
+// bfs.cuh - BFS queries: waves of up to 64 sources as bitmasks, and the
+// single-source form as bitmaps.
+//
+// Both are level-synchronous persistent kernels that switch direction
+// (Beamer, Asanovic and Patterson, "Direction-optimizing breadth-first
+// search", SC 2012): small frontiers are queues whose out-rows are expanded
+// (top-down), large ones are masks that every incomplete vertex gathers over
+// its in-row (bottom-up).  A wave keeps per vertex the 64-bit mask of sources
+// that reached it and of those that did so in the last round (MS-BFS: Then et
+// al., "The More the Merrier: Efficient Multi-Source Graph Traversal", VLDB
+// 2014).
+//
+// Depths of a wave are kept bit-sliced: plane p of vertex v holds, for every
+// source, bit p of its depth, so recording a level for any number of sources
+// is one OR per set bit of the level, and the k x n result is written once,
+// in rows, from a few planes (depths stay below 16, four planes, on R-MAT).
+// A word per vertex and source instead took a 4 n k byte fill, scattered
+// 4-byte stores and a transpose that read it all again.
+#pragma once
+
+#include "common.cuh"
+#include "expand.cuh"
+#include "traverse.cuh"
+
+namespace cig {
+
+constexpr uint32_t kMsWidth = 64;
+constexpr int kTpbMs = 256;
+constexpr uint32_t kBfsPlanes = 4;      // planes cleared before the wave; the kernel clears further ones as levels need them
+constexpr uint32_t kBfsChunk = 1024;     // in-rows of at least this many entries are gathered by several warps
+constexpr uint32_t kBfsWarpRow = 256;    // ... of at least this many by a warp, shorter ones by eight lanes
+constexpr uint32_t kBfsMaxPlanes = 32;  // depths are below 2^32
+
+struct MsFrontier {
+    uint32_t *q0;
+    uint32_t *q1;
+    uint32_t *cnt;                // 3 round counters, as for the push closure
+    unsigned long long *mask0;    // source masks read in even rounds
+    unsigned long long *mask1;    // ... in odd rounds
+    uint32_t cap;
+};
+
+// Bottom-up rounds: when the frontier holds more than `on` vertices (or, once
+// bottom-up, more than `off`), or when its out-rows hold more than `edges_on`
+// entries: a few hub vertices are a small frontier whose expansion costs as
+// much as the whole graph's (on R-MAT the round after the hubs; a top-down
+// edge costs an atomic or two, a bottom-up entry a load).  The chunks of long in-rows (`tasks`, listed
+// at the first bottom-up round) are gathered by warps of their own into
+// `acc`; the last to arrive completes the vertex.
+struct BfsPull {
+    AdjView rev;  // in-edges (desc null: no bottom-up)
+    uint32_t on, off;
+    uint32_t edges_on;
+    BigRow *tasks;              // off, len, x = vertex, payload = chunks of the row << 32 | row's place in acc
+    uint32_t task_cap;
+    unsigned long long *acc;    // zero between rounds
+    uint32_t *arrived;          // zero between rounds
+    uint32_t *bigbits;          // bit v: v's in-row is in `tasks`
+    uint32_t *ctl;              // BfsCtl, zero at launch
+};
+enum BfsCtl : int { kBfsTasks = 0, kBfsBigRows = 1, kBfsFill = 2, kBfsRounds = 3, kBfsEdges = 4 /* 3 counters */ };
+
+// Top-down edge of a wave: the bits that have not reached y do so now.
+struct MsBfsOp {
+    unsigned long long *visit;
+    unsigned long long *mask_out;
+    WarpBuf buf;
+
+    __device__ __forceinline__ unsigned long long peek(uint32_t y) const { return __ldcg(visit + y); }
+    __device__ __forceinline__ bool edge_peeked(bool valid, uint32_t, unsigned long long m, uint32_t y,
+                                                unsigned long long seen) const {
+        bool want = false, hit = false;
+        const unsigned long long cand = m & ~seen;
+        if (valid && cand) {
+            const unsigned long long nb = cand & ~atomicOr(visit + y, cand);
+            if (nb) {
+                hit = true;
+                want = atomicOr(mask_out + y, nb) == 0ull;
+            }
+        }
+        buf.add(want, y);
+        return hit;
+    }
+    __device__ __forceinline__ bool edge(bool valid, uint32_t x, unsigned long long m, uint32_t y) const {
+        return edge_peeked(valid, x, m, y, valid ? peek(y) : 0ull);
+    }
+};
+
+// Depth `level` for the sources in m at vertex v (one thread per vertex).
+__device__ __forceinline__ void planes_record(unsigned long long *planes, uint32_t n, uint32_t v, uint32_t level,
+                                              unsigned long long m) {
+    for (uint32_t b = level; b; b &= b - 1)
+        planes[static_cast<uint64_t>(__ffs(static_cast<int>(b)) - 1) * n + v] |= m;
+}
+
+// Warp-wide OR.
+__device__ __forceinline__ unsigned long long warp_or(unsigned long long x) {
+    const uint32_t lo = __reduce_or_sync(kFull, static_cast<uint32_t>(x));
+    const uint32_t hi = __reduce_or_sync(kFull, static_cast<uint32_t>(x >> 32));
+    return (static_cast<unsigned long long>(hi) << 32) | lo;
+}
+
+// OR of get(y) over the entries of a row (device-only arena), by one warp,
+// 256 entries per step, until it covers `missing`; *read counts the entries.
+template <class G>
+__device__ __forceinline__ unsigned long long warp_gather(const AdjView &rev, const uint32_t *rp, uint32_t len,
+                                                          unsigned long long missing, const G &get, uint32_t *read) {
+    const uint32_t lane = lane_id();
+    unsigned long long acc = 0;
+    for (uint32_t b0 = 0; b0 < len; b0 += 256u) {
+        uint4 q[2];
+#pragma unroll
+        for (uint32_t h = 0; h < 2; ++h) {
+            const uint32_t k = b0 + 128u * h + 4u * lane;
+            q[h] = k < len ? __ldg(reinterpret_cast<const uint4 *>(rp + k)) : make_uint4(kTomb, kTomb, kTomb, kTomb);
+        }
+        unsigned long long m[8];
+#pragma unroll
+        for (uint32_t h = 0; h < 2; ++h) {
+            const uint32_t k = b0 + 128u * h + 4u * lane;
+            const uint32_t y[4] = {rev.vid(q[h].x), rev.vid(q[h].y), rev.vid(q[h].z), rev.vid(q[h].w)};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) m[4 * h + j] = k + j < len && y[j] != kTomb ? get(y[j]) : 0ull;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc |= m[j];
+        *read += lane == 0 ? min(256u, len - b0) : 0u;
+        acc = warp_or(acc);
+        if ((acc & missing) == missing) break;
+    }
+    return acc;
+}
+
+// OR of get(y) over the first kBfsHead entries of the lane's own row, in
+// flight together.
+constexpr uint32_t kBfsHead = 8;
+template <class G>
+__device__ __forceinline__ unsigned long long lane_gather(const AdjView &rev, const uint32_t *rp, uint32_t len,
+                                                          const G &get) {
+    uint4 q[kBfsHead / 4];
+#pragma unroll
+    for (uint32_t h = 0; h < kBfsHead / 4; ++h)
+        q[h] = 4u * h < len ? __ldg(reinterpret_cast<const uint4 *>(rp + 4u * h))
+                            : make_uint4(kTomb, kTomb, kTomb, kTomb);
+    unsigned long long acc = 0;
+#pragma unroll
+    for (uint32_t h = 0; h < kBfsHead / 4; ++h) {
+        const uint32_t y[4] = {rev.vid(q[h].x), rev.vid(q[h].y), rev.vid(q[h].z), rev.vid(q[h].w)};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc |= 4u * h + j < len && y[j] != kTomb ? get(y[j]) : 0ull;
+    }
+    return acc;
+}
+
+// The rows of the lanes in `mask`, from entry kBfsHead on: eight lanes per
+// row, four rows at a time, 32 entries of each per step (a row per lane left
+// the warp waiting for its longest row, a row per warp for one chain of loads
+// after another).  ORs into the owners' `acc` until it covers `missing`.
+template <class G>
+__device__ __forceinline__ void groups_gather(const AdjView &rev, uint32_t mask, const RowDesc &d,
+                                              unsigned long long missing, const G &get, unsigned long long &acc,
+                                              uint32_t &read) {
+    const uint32_t lane = lane_id(), sub = lane & 7u;
+    while (mask) {  // warp-uniform
+        uint32_t m = mask;
+        for (uint32_t k = 0; k < (lane >> 3); ++k) m &= m - 1;
+        const bool on = m != 0;
+        const uint32_t src = on ? __ffs(m) - 1 : 0u;
+        const uint64_t off = __shfl_sync(kFull, static_cast<unsigned long long>(d.off), src);
+        const uint32_t len = __shfl_sync(kFull, d.len, src);
+        const unsigned long long want = __shfl_sync(kFull, missing, src);
+        unsigned long long a = __shfl_sync(kFull, acc, src);
+        const uint32_t *rp = rev.at(on ? off : 0ull);
+        uint32_t k = kBfsHead;
+        bool more = on && k < len;
+        while (__any_sync(kFull, more)) {
+            unsigned long long got = 0;
+            if (more) {
+                const uint32_t kk = k + 4u * sub;
+                const uint4 q = kk < len ? __ldg(reinterpret_cast<const uint4 *>(rp + kk))
+                                         : make_uint4(kTomb, kTomb, kTomb, kTomb);
+                const uint32_t y[4] = {rev.vid(q.x), rev.vid(q.y), rev.vid(q.z), rev.vid(q.w)};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) got |= kk + j < len && y[j] != kTomb ? get(y[j]) : 0ull;
+                k += 32u;
+            }
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) got |= __shfl_xor_sync(kFull, got, o);
+            a |= got;
+            more = on && k < len && (a & want) != want;
+        }
+        // the owner with rank g among the four takes group g's result
+        const uint32_t rank = __popc(mask & lanemask_lt());
+        const unsigned long long res = __shfl_sync(kFull, a, (rank & 3u) * 8u);
+        const uint32_t end = __shfl_sync(kFull, k, (rank & 3u) * 8u);
+        if (((mask >> lane) & 1u) && rank < 4u) {
+            acc = res;
+            read = min(end, d.len);
+        }
+        for (int t = 0; t < 4; ++t) mask &= mask - 1;  // 0 stays 0
+    }
+}
+
+// List the chunks of the long in-rows and mark their vertices.
+__device__ __forceinline__ void bfs_list_tasks(const BfsPull &pl, uint32_t n, Status *st) {
+    const uint32_t lane = lane_id();
+    const uint32_t rounded = (n + 31u) & ~31u;
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < rounded; v += gridDim.x * blockDim.x) {
+        uint32_t len = 0;
+        uint64_t off = 0;
+        if (v < n) {
+            const RowDesc d = pl.rev.desc[v];
+            len = d.len;
+            off = d.off;
+        }
+        uint32_t bigs = __ballot_sync(kFull, len >= kBfsChunk);
+        if (lane == 0) pl.bigbits[v >> 5] = bigs;
+        while (bigs) {
+            const uint32_t l = __ffs(bigs) - 1;
+            bigs &= bigs - 1;
+            const uint32_t llen = __shfl_sync(kFull, len, l), lv = __shfl_sync(kFull, v, l);
+            const uint64_t loff = __shfl_sync(kFull, static_cast<unsigned long long>(off), l);
+            const uint32_t chunks = (llen + kBfsChunk - 1) / kBfsChunk;
+            uint32_t at = 0, row = 0;
+            if (lane == 0) {
+                at = atomicAdd(pl.ctl + kBfsTasks, chunks);
+                row = atomicAdd(pl.ctl + kBfsBigRows, 1u);
+                if (at + chunks > pl.task_cap) set_error(st, kErrQueue, at);
+            }
+            at = __shfl_sync(kFull, at, 0);
+            row = __shfl_sync(kFull, row, 0);
+            for (uint32_t i = lane; i < chunks; i += 32u)
+                if (at + i < pl.task_cap)
+                    pl.tasks[at + i] = BigRow{loff + static_cast<uint64_t>(i) * kBfsChunk,
+                                              (static_cast<unsigned long long>(chunks) << 32) | row, lv,
+                                              min(kBfsChunk, llen - i * kBfsChunk)};
+        }
+    }
+}
+
+// Add the block's new frontier vertices to the round's counter: one atomic
+// per block (one per warp queued thousands on one address).  All threads call.
+__device__ __forceinline__ void block_add(uint32_t *counter, uint32_t mine, uint32_t *shared) {
+    mine = __reduce_add_sync(kFull, mine);
+    if (threadIdx.x == 0) *shared = 0;
+    __syncthreads();
+    if (lane_id() == 0 && mine) atomicAdd(shared, mine);
+    __syncthreads();
+    if (threadIdx.x == 0 && *shared) atomicAdd(counter, *shared);
+}
+
+// Does a top-down round over the queue hold more than pl.edges_on row
+// entries?  Looked at for queues of kBfsCount vertices and more (below, a
+// round is short anyway); one barrier, after which every block agrees.
+// `ok` false: barrier error.
+constexpr uint32_t kBfsCount = 256;
+__device__ __forceinline__ bool bfs_many_edges(const BfsPull &pl, const RowDesc *desc, const uint32_t *in,
+                                               uint32_t n_in, uint32_t r, uint32_t *shared, bool &ok, Status *st) {
+    if (!pl.rev.desc || n_in < kBfsCount) return false;
+    uint32_t mine = 0;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_in; i += gridDim.x * blockDim.x)
+        mine += min(desc[__ldcg(in + i)].len, 1u << 20);
+    block_add(pl.ctl + kBfsEdges + r % 3, mine, shared);
+    ok = grid_barrier(st);
+    return ld_volatile(pl.ctl + kBfsEdges + r % 3) > pl.edges_on;
+}
+
+// Bottom-up round of a wave: every vertex that misses source bits ORs the
+// frontier masks of its in-neighbours, stopping once nothing is missing.
+// Every in-row's first entries are gathered by its own lane, the rest of rows
+// below kBfsWarpRow by eight lanes, below kBfsChunk by a warp, longer ones by a
+// warp per chunk.  Bound by the gathers: 8 bytes of a 32-byte L2 sector per
+// entry.  Returns the new frontier vertices found by this thread.
+__device__ __forceinline__ uint32_t bfs_bottom_up(const BfsPull &pl, uint32_t n, unsigned long long full,
+                                                  unsigned long long *visit, unsigned long long *planes,
+                                                  const unsigned long long *m_in, unsigned long long *m_out,
+                                                  uint32_t level, ExpandCounters &cnt, unsigned long long &src_edges) {
+    const uint32_t lane = lane_id();
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t wid = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    auto get = [&](uint32_t u) { return m_in[u]; };
+    uint32_t found = 0;
+    const uint32_t nt = min(ld_volatile(pl.ctl + kBfsTasks), pl.task_cap);
+    for (uint32_t i = wid; i < nt; i += warps) {
+        const BigRow t = pl.tasks[i];
+        const unsigned long long vis = __ldcg(visit + t.x), missing = full & ~vis;
+        const uint32_t row = static_cast<uint32_t>(t.payload), chunks = static_cast<uint32_t>(t.payload >> 32);
+        uint32_t read = 0;
+        const unsigned long long acc =
+            missing ? warp_gather(pl.rev, pl.rev.at(t.off), t.deg, missing, get, &read) & missing : 0ull;
+        if (lane == 0) {
+            cnt.edges += read;
+            cnt.edges_cached += read;
+            cnt.rows += read ? 1u : 0u;
+            src_edges += static_cast<unsigned long long>(__popcll(missing)) * read;
+            if (acc) atomicOr(pl.acc + row, acc);
+            __threadfence();
+            if (atomicAdd(pl.arrived + row, 1u) == chunks - 1u) {
+                __threadfence();
+                const unsigned long long nb = atomicExch(pl.acc + row, 0ull);
+                pl.arrived[row] = 0u;
+                m_out[t.x] = nb;
+                if (nb) {
+                    visit[t.x] = vis | nb;
+                    planes_record(planes, n, t.x, level, nb);
+                    ++found;
+                    ++cnt.hits;
+                }
+            }
+        }
+    }
+    for (uint64_t base = static_cast<uint64_t>(wid) * 32u; base < n; base += static_cast<uint64_t>(warps) * 32u) {
+        const uint32_t v = static_cast<uint32_t>(base) + lane;
+        const bool mine = v < n && !((pl.bigbits[base >> 5] >> lane) & 1u);
+        const unsigned long long vis = mine ? __ldcg(visit + v) : full;
+        const unsigned long long missing = full & ~vis;
+        unsigned long long acc = 0;
+        RowDesc d{0, 0, 0};
+        if (missing) d = pl.rev.desc[v];
+        uint32_t read = 0;
+        if (d.len) {
+            acc = lane_gather(pl.rev, pl.rev.at(d.off), d.len, get);
+            read = min(d.len, kBfsHead);
+        }
+        const bool open = (acc & missing) != missing;
+        groups_gather(pl.rev, __ballot_sync(kFull, open && d.len > kBfsHead && d.len < kBfsWarpRow), d, missing, get,
+                      acc, read);
+        uint32_t meds = __ballot_sync(kFull, open && d.len >= kBfsWarpRow);
+        while (meds) {
+            const uint32_t l = __ffs(meds) - 1;
+            meds &= meds - 1;
+            const uint64_t loff = __shfl_sync(kFull, static_cast<unsigned long long>(d.off), l);
+            const uint32_t llen = __shfl_sync(kFull, d.len, l);
+            const unsigned long long lm = __shfl_sync(kFull, missing, l);
+            uint32_t r = 0;
+            const unsigned long long a = warp_gather(pl.rev, pl.rev.at(loff), llen, lm, get, &r);
+            r = __shfl_sync(kFull, r, 0);
+            if (lane == l) {
+                acc = a;
+                read = r;
+            }
+        }
+        cnt.edges += read;
+        cnt.edges_cached += read;
+        cnt.rows += read ? 1u : 0u;
+        src_edges += static_cast<unsigned long long>(__popcll(missing)) * read;
+        const unsigned long long nb = acc & missing;
+        if (mine) m_out[v] = nb;
+        if (nb) {
+            visit[v] = vis | nb;
+            planes_record(planes, n, v, level, nb);
+            ++found;
+            ++cnt.hits;
+        }
+    }
+    return found;
+}
+
+// One wave (cooperative launch).  Round r gives depth r + 1.  `full`: the
+// wave's source bits.  Planes 0..kBfsPlanes-1 are cleared before the launch.
+__global__ void __launch_bounds__(kTpbMs, 4) bfs_wave(AdjView fwd, uint32_t n, unsigned long long full,
+                                                      unsigned long long *visit, unsigned long long *planes,
+                                                      MsFrontier fr, BigList big, uint32_t max_rounds, BfsPull pl,
+                                                      Status *st) {
+    __shared__ ExpandSmem<kTpbMs, unsigned long long> sm;
+    __shared__ uint32_t s_new;
+    __shared__ uint32_t s_buf[kTpbMs / 32][kWarpBuf];
+    __shared__ uint32_t s_held[kTpbMs / 32];
+    if (threadIdx.x < kTpbMs / 32) s_held[threadIdx.x] = 0;
+    __syncthreads();
+    ExpandCounters cnt;
+    unsigned long long src_edges = 0;
+    // every block takes the same decisions from the same counts
+    bool pull = false, was_pull = false, listed = false;
+    const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, gthreads = gridDim.x * blockDim.x;
+    uint32_t r = 0;
+    for (;; ++r) {
+        const uint32_t n_in = ld_volatile(fr.cnt + (r % 3));
+        if (n_in == 0) break;
+        if (r >= max_rounds) {
+            if (gtid == 0) set_error(st, kErrRounds, r);
+            break;
+        }
+        if (gtid == 0) {
+            fr.cnt[(r + 2) % 3] = 0;
+            big.cnt[(r + 2) % 3] = 0;
+            pl.ctl[kBfsEdges + (r + 1) % 3] = 0;
+        }
+        uint32_t *in = (r & 1) ? fr.q1 : fr.q0;
+        uint32_t *out = (r & 1) ? fr.q0 : fr.q1;
+        uint32_t *out_cnt = fr.cnt + ((r + 1) % 3);
+        unsigned long long *m_in = (r & 1) ? fr.mask1 : fr.mask0;
+        unsigned long long *m_out = (r & 1) ? fr.mask0 : fr.mask1;
+        const uint32_t level = r + 1;
+        if (level >= (1u << kBfsPlanes) && (level & (level - 1)) == 0) {  // the first level that sets this plane
+            unsigned long long *plane = planes + static_cast<uint64_t>(31 - __clz(level)) * n;
+            for (uint32_t v = gtid; v < n; v += gthreads) plane[v] = 0ull;
+            if (!grid_barrier(st)) break;
+        }
+        was_pull = pull;
+        pull = pl.rev.desc && n_in > (was_pull ? pl.off : pl.on);
+        if (!pull && !was_pull) {
+            bool ok = true;
+            pull = bfs_many_edges(pl, fwd.desc, in, n_in, r, &s_new, ok, st);
+            if (!ok) break;
+        }
+        if (pull) {
+            if (!was_pull) {
+                // The queued vertices are not popped: record their depth here.
+                for (uint32_t i = gtid; i < n_in; i += gthreads) {
+                    const uint32_t x = __ldcg(in + i);
+                    planes_record(planes, n, x, r, __ldcg(m_in + x));
+                }
+                if (!listed) bfs_list_tasks(pl, n, st);
+                listed = true;
+                if (!grid_barrier(st)) break;
+            }
+            const uint32_t found =
+                bfs_bottom_up(pl, n, full, visit, planes, m_in, m_out, level, cnt, src_edges);
+            block_add(out_cnt, found, &s_new);
+            if (!grid_barrier(st)) break;
+            continue;
+        }
+        if (was_pull) {
+            // The frontier is the non-zero masks: queue it, and clear the
+            // masks of the round before for this one's.
+            const uint32_t rounded = (n + 31u) & ~31u;
+            for (uint32_t v = gtid; v < rounded; v += gthreads) {
+                bool want = false;
+                if (v < n) {
+                    want = m_in[v] != 0ull;
+                    m_out[v] = 0ull;
+                }
+                warp_enqueue(want, v, in, pl.ctl + kBfsFill, fr.cap, st);
+            }
+            if (!grid_barrier(st)) break;
+            if (gtid == 0) pl.ctl[kBfsFill] = 0;
+        }
+        const Defer df{big.rows, big.cnt + (r % 3), big.cap, big.split};
+        const MsBfsOp op{visit, m_out, WarpBuf{s_buf[threadIdx.x >> 5], s_held + (threadIdx.x >> 5), out, out_cnt, fr.cap, st}};
+        for (uint32_t base = 0; base < n_in; base += gridDim.x * kTpbMs) {
+            const uint32_t i = base + spread_rank<kTpbMs>() * gridDim.x + blockIdx.x;
+            bool has = i < n_in;
+            uint32_t x = 0, deg = 0;
+            uint64_t off = 0;
+            unsigned long long m = 0;
+            if (has) {
+                x = __ldcg(in + i);
+                // Nobody writes m_in this round: take the bits and clear them.
+                m = __ldcg(m_in + x);
+                m_in[x] = 0ull;
+                planes_record(planes, n, x, r, m);
+                const RowDesc d = fwd.desc[x];
+                deg = d.len;
+                off = d.off;
+                has = m != 0ull && deg > 0;
+                if (has) src_edges += static_cast<unsigned long long>(__popcll(m)) * deg;
+            }
+            expand_rows<kTpbMs>(fwd, has, x, m, off, deg, op, sm, cnt, df);
+        }
+        op.buf.flush();
+        if (!grid_barrier(st)) break;
+        const uint32_t nbig = min(ld_volatile(big.cnt + (r % 3)), big.cap);
+        if (nbig) {
+            expand_deferred<kTpbMs, unsigned long long>(fwd, big.rows, nbig, op, cnt);
+            op.buf.flush();
+            if (!grid_barrier(st)) break;
+        }
+    }
+    flush_counters(st, cnt, kCntPush);
+    for (int o = 16; o > 0; o >>= 1) src_edges += __shfl_down_sync(kFull, src_edges, o);
+    if (lane_id() == 0 && src_edges) atomicAdd(&st->counters[kCntSrcEdges], src_edges);
+    if (gtid == 0) {
+        pl.ctl[kBfsRounds] = r;
+        atomicAdd(&st->counters[kCntRounds], static_cast<unsigned long long>(r));
+    }
+}
+
+// Source-major depths from the planes: out[j * n + v], four vertices per
+// thread and 512-byte stores per warp where the rows are 16-byte aligned (n a
+// multiple of 4 and an aligned result), one vertex per thread otherwise; one
+// pass over `visit` and the planes in use.
+template <int V>
+__device__ __forceinline__ void bfs_depths_of(const unsigned long long *visit, const unsigned long long *planes,
+                                              uint32_t n, uint32_t k, uint32_t used, uint32_t v, uint32_t *out) {
+    unsigned long long vis[V], p[kBfsPlanes][V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) vis[i] = visit[v + i];
+#pragma unroll
+    for (uint32_t b = 0; b < kBfsPlanes; ++b)
+#pragma unroll
+        for (int i = 0; i < V; ++i) p[b][i] = b < used ? planes[static_cast<uint64_t>(b) * n + v + i] : 0ull;
+    for (uint32_t j = 0; j < k; ++j) {
+        uint32_t d[V];
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+            d[i] = 0;
+#pragma unroll
+            for (uint32_t b = 0; b < kBfsPlanes; ++b) d[i] |= (static_cast<uint32_t>(p[b][i] >> j) & 1u) << b;
+            for (uint32_t b = kBfsPlanes; b < used; ++b)
+                d[i] |= (static_cast<uint32_t>(planes[static_cast<uint64_t>(b) * n + v + i] >> j) & 1u) << b;
+            if (!((vis[i] >> j) & 1ull)) d[i] = kInf;
+        }
+        uint32_t *to = out + static_cast<uint64_t>(j) * n + v;
+        if constexpr (V == 4)
+            __stcs(reinterpret_cast<uint4 *>(to), make_uint4(d[0], d[1], d[2], d[3]));
+        else
+            __stcs(to, d[0]);
+    }
+}
+
+__global__ void bfs_depths(const unsigned long long *visit, const unsigned long long *planes, uint32_t n, uint32_t k,
+                           const uint32_t *ctl, uint32_t *out) {
+    const uint32_t used = 32u - __clz(ctl[kBfsRounds]);
+    const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, gthreads = gridDim.x * blockDim.x;
+    if ((n & 3u) == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
+        for (uint32_t q = gtid; q < n / 4; q += gthreads) bfs_depths_of<4>(visit, planes, n, k, used, 4 * q, out);
+    } else {
+        for (uint32_t v = gtid; v < n; v += gthreads) bfs_depths_of<1>(visit, planes, n, k, used, v, out);
+    }
+}
+
+// ---------------------------------------------------------------- one source
+// Visited and frontier vertices are bitmaps (n / 8 bytes: they stay in L2 and
+// largely in L1, where 8 bytes per vertex do not), depths go straight to the
+// result.
+struct OneBfsOp {
+    uint32_t *vis;
+    uint32_t *depth;
+    uint32_t level;
+    WarpBuf buf;
+
+    __device__ __forceinline__ uint32_t peek(uint32_t y) const { return __ldcg(vis + (y >> 5)); }
+    __device__ __forceinline__ bool edge_peeked(bool valid, uint32_t, uint32_t, uint32_t y, uint32_t word) const {
+        const uint32_t bit = 1u << (y & 31u);
+        bool want = false;
+        if (valid && !(word & bit)) want = !(atomicOr(vis + (y >> 5), bit) & bit);
+        if (want) depth[y] = level;
+        buf.add(want, y);
+        return want;
+    }
+    __device__ __forceinline__ bool edge(bool valid, uint32_t x, uint32_t p, uint32_t y) const {
+        return edge_peeked(valid, x, p, y, valid ? peek(y) : 0u);
+    }
+};
+
+__global__ void bfs_one_seed(const uint32_t *source, uint32_t *depth, uint32_t *vis, uint32_t *q0, uint32_t *cnt) {
+    const uint32_t s = source[0];
+    depth[s] = 0u;
+    vis[s >> 5] = 1u << (s & 31u);
+    q0[0] = s;
+    cnt[0] = 1u;
+}
+
+// Single-source BFS (cooperative launch); `vis` cleared and `depth` filled
+// with kInf before it, `bm0` / `bm1` the frontier bitmaps of bottom-up rounds
+// ((n + 31) / 32 words each).
+__global__ void __launch_bounds__(kTpbMs, 4) bfs_one(AdjView fwd, uint32_t n, uint32_t *depth, uint32_t *vis,
+                                                     uint32_t *bm0, uint32_t *bm1, MsFrontier fr, BigList big,
+                                                     uint32_t max_rounds, BfsPull pl, Status *st) {
+    __shared__ ExpandSmem<kTpbMs> sm;
+    __shared__ uint32_t s_new;
+    __shared__ uint32_t s_buf[kTpbMs / 32][kWarpBuf];
+    __shared__ uint32_t s_held[kTpbMs / 32];
+    if (threadIdx.x < kTpbMs / 32) s_held[threadIdx.x] = 0;
+    __syncthreads();
+    ExpandCounters cnt;
+    bool pull = false, was_pull = false;
+    const uint32_t lane = lane_id();
+    const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, gthreads = gridDim.x * blockDim.x;
+    const uint32_t warps = gthreads >> 5, wid = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    const uint32_t words = (n + 31u) / 32u;
+    uint32_t r = 0;
+    for (;; ++r) {
+        const uint32_t n_in = ld_volatile(fr.cnt + (r % 3));
+        if (n_in == 0) break;
+        if (r >= max_rounds) {
+            if (gtid == 0) set_error(st, kErrRounds, r);
+            break;
+        }
+        if (gtid == 0) {
+            fr.cnt[(r + 2) % 3] = 0;
+            big.cnt[(r + 2) % 3] = 0;
+            pl.ctl[kBfsEdges + (r + 1) % 3] = 0;
+        }
+        uint32_t *in = (r & 1) ? fr.q1 : fr.q0;
+        uint32_t *out = (r & 1) ? fr.q0 : fr.q1;
+        uint32_t *out_cnt = fr.cnt + ((r + 1) % 3);
+        uint32_t *cur = (r & 1) ? bm1 : bm0;
+        uint32_t *next = (r & 1) ? bm0 : bm1;
+        was_pull = pull;
+        pull = pl.rev.desc && n_in > (was_pull ? pl.off : pl.on);
+        if (!pull && !was_pull) {
+            bool ok = true;
+            pull = bfs_many_edges(pl, fwd.desc, in, n_in, r, &s_new, ok, st);
+            if (!ok) break;
+        }
+        if (pull) {
+            if (!was_pull) {  // the queue as a bitmap
+                for (uint32_t w = gtid; w < words; w += gthreads) cur[w] = 0u;
+                if (!grid_barrier(st)) break;
+                for (uint32_t i = gtid; i < n_in; i += gthreads) {
+                    const uint32_t x = __ldcg(in + i);
+                    atomicOr(cur + (x >> 5), 1u << (x & 31u));
+                }
+                if (!grid_barrier(st)) break;
+            }
+            auto get = [&](uint32_t u) { return static_cast<unsigned long long>((cur[u >> 5] >> (u & 31u)) & 1u); };
+            uint32_t found = 0;
+            for (uint32_t w = wid; w < words; w += warps) {
+                const uint32_t seen = __ldcg(vis + w);
+                const uint32_t v = 32u * w + lane;
+                RowDesc d{0, 0, 0};
+                if (v < n && !((seen >> lane) & 1u)) d = pl.rev.desc[v];
+                uint32_t read = 0;
+                unsigned long long hit = 0;
+                // Most vertices that have a parent in the frontier find one
+                // among the first entries.
+                if (d.len) {
+                    hit = lane_gather(pl.rev, pl.rev.at(d.off), d.len, get);
+                    read = min(d.len, kBfsHead);
+                }
+                const bool open = !hit;
+                groups_gather(pl.rev, __ballot_sync(kFull, open && d.len > kBfsHead && d.len < kBfsWarpRow), d, 1ull,
+                              get, hit, read);
+                uint32_t rest = __ballot_sync(kFull, open && d.len >= kBfsWarpRow);
+                while (rest) {
+                    const uint32_t l = __ffs(rest) - 1;
+                    rest &= rest - 1;
+                    const uint64_t loff = __shfl_sync(kFull, static_cast<unsigned long long>(d.off), l);
+                    const uint32_t llen = __shfl_sync(kFull, d.len, l);
+                    uint32_t rd = 0;
+                    const unsigned long long a = warp_gather(pl.rev, pl.rev.at(loff), llen, 1ull, get, &rd);
+                    rd = __shfl_sync(kFull, rd, 0);
+                    if (lane == l) {
+                        hit = a;
+                        read += rd;
+                    }
+                }
+                cnt.edges += read;
+                cnt.edges_cached += read;
+                cnt.rows += read ? 1u : 0u;
+                if (hit) {
+                    depth[v] = r + 1;
+                    ++cnt.hits;
+                    ++found;
+                }
+                const uint32_t nb = __ballot_sync(kFull, hit != 0ull);
+                if (lane == 0) {
+                    next[w] = nb;
+                    if (nb) vis[w] = seen | nb;
+                }
+            }
+            block_add(out_cnt, found, &s_new);
+            if (!grid_barrier(st)) break;
+            continue;
+        }
+        if (was_pull) {  // the bitmap as a queue
+            for (uint32_t w = wid; w < words; w += warps) {
+                const uint32_t bits = cur[w];
+                warp_enqueue((bits >> lane) & 1u, 32u * w + lane, in, pl.ctl + kBfsFill, fr.cap, st);
+            }
+            if (!grid_barrier(st)) break;
+            if (gtid == 0) pl.ctl[kBfsFill] = 0;
+        }
+        const Defer df{big.rows, big.cnt + (r % 3), big.cap, big.split};
+        const OneBfsOp op{vis, depth, r + 1,
+                          WarpBuf{s_buf[threadIdx.x >> 5], s_held + (threadIdx.x >> 5), out, out_cnt, fr.cap, st}};
+        for (uint32_t base = 0; base < n_in; base += gridDim.x * kTpbMs) {
+            const uint32_t i = base + spread_rank<kTpbMs>() * gridDim.x + blockIdx.x;
+            bool has = i < n_in;
+            uint32_t x = 0, deg = 0;
+            uint64_t off = 0;
+            if (has) {
+                x = __ldcg(in + i);
+                const RowDesc d = fwd.desc[x];
+                deg = d.len;
+                off = d.off;
+                has = deg > 0;
+            }
+            expand_rows<kTpbMs>(fwd, has, x, 0u, off, deg, op, sm, cnt, df);
+        }
+        op.buf.flush();
+        if (!grid_barrier(st)) break;
+        const uint32_t nbig = min(ld_volatile(big.cnt + (r % 3)), big.cap);
+        if (nbig) {
+            expand_deferred<kTpbMs>(fwd, big.rows, nbig, op, cnt);
+            op.buf.flush();
+            if (!grid_barrier(st)) break;
+        }
+    }
+    flush_counters(st, cnt, kCntPush);
+    const uint32_t edges = __reduce_add_sync(kFull, cnt.edges);  // one source: source edges = edges
+    if (lane == 0 && edges) atomicAdd(&st->counters[kCntSrcEdges], static_cast<unsigned long long>(edges));
+    if (gtid == 0) atomicAdd(&st->counters[kCntRounds], static_cast<unsigned long long>(r));
+}
+
+}  // namespace cig

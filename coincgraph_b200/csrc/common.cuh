@@ -204,6 +204,49 @@ __device__ __forceinline__ void warp_enqueue(bool want, uint32_t item, uint32_t 
     }
 }
 
+// Queue appends of one warp, collected in shared memory and written out with
+// one atomic per kWarpBuf items or so: in rounds of a million appends the
+// warps' atomics on the queue's one counter were what the round waited for.
+// All 32 lanes call; flush() once at the end of the warp's work.
+constexpr uint32_t kWarpBuf = 96;
+struct WarpBuf {
+    uint32_t *items;  // kWarpBuf words of this warp
+    uint32_t *held;   // items in it
+    uint32_t *queue;
+    uint32_t *count;
+    uint32_t capacity;
+    Status *st;
+
+    __device__ __forceinline__ void flush() const {
+        __syncwarp();
+        const uint32_t c = *held;
+        if (!c) return;
+        uint32_t base = 0;
+        if (lane_id() == 0) base = atomicAdd(count, c);
+        base = __shfl_sync(kFull, base, 0);
+        for (uint32_t i = lane_id(); i < c; i += 32u) {
+            if (base + i < capacity)
+                queue[base + i] = items[i];
+            else
+                set_error(st, kErrQueue, base + i);
+        }
+        __syncwarp();
+        if (lane_id() == 0) *held = 0;
+        __syncwarp();
+    }
+    __device__ __forceinline__ void add(bool want, uint32_t item) const {
+        const uint32_t mask = __ballot_sync(kFull, want);
+        if (!mask) return;
+        const uint32_t k = __popc(mask);
+        if (*held + k > kWarpBuf) flush();
+        const uint32_t at = *held;
+        if (want) items[at + __popc(mask & lanemask_lt())] = item;
+        __syncwarp();
+        if (lane_id() == 0) *held = at + k;
+        __syncwarp();
+    }
+};
+
 // Append up to N items per lane (item[j] where want[j]) with one warp scan
 // and one atomic per warp.
 template <int N>
@@ -289,6 +332,22 @@ __device__ __forceinline__ bool grid_barrier(Status *st) {
     __syncthreads();
     return ok != 0;
 }
+
+// Tiles of a round's items handed to the warps of a grid: the first by the
+// warp's number, further ones from a counter (zero at the round's start), so
+// that a warp that met long rows takes fewer.  The next tile is asked for
+// while the current one is worked on.
+struct TileFeed {
+    uint32_t *counter;
+    uint32_t warps;
+    uint32_t next;  // lane 0
+
+    __device__ __forceinline__ TileFeed(uint32_t *c, uint32_t w) : counter(c), warps(w), next(0) {}
+    __device__ __forceinline__ void ask() {
+        if (lane_id() == 0) next = atomicAdd(counter, 1u);
+    }
+    __device__ __forceinline__ uint32_t take() const { return warps + __shfl_sync(kFull, next, 0); }
+};
 
 // Edge weights of the reference samples: BFS 1 (samples/hybrid_bfs/
 // hybrid_bfs.cu:41-47), SSSP (src+dst)%128+1 (include/framework/variants/

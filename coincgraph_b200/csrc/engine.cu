@@ -647,7 +647,6 @@ struct cig_handle {
         uint32_t split = kSplitDeg; // rows of at least this many entries are expanded by the whole grid
         uint32_t pull_on = 32;      // BFS waves go bottom-up above n/pull_on frontier vertices (0: never)
         uint32_t pull_off = 64;     // ... and stay while at least n/pull_off
-        uint32_t pull_width = 16;   // waves of more sources stay top-down
     } tune;
 
     template <class... P>
@@ -2416,19 +2415,35 @@ struct cig_handle {
     uint64_t ms_out_cap = 0;
     BigRow *ms_big = nullptr;
 
-    // Bottom-up switch of a BFS wave of kw sources: frontier above n/pull_on
-    // vertices (then at least n/pull_off); needs the device in-edge arena.
-    // Only narrow waves pull: the thread-per-vertex bottom-up scan cut a
-    // 64-source wave's edge-scans 2.4x on RMAT s24 yet ran 14 % slower, while
-    // single-source waves ran 3.4x faster.
-    MsPull ms_pull(uint32_t kw) const {
-        MsPull p{};
-        if (opt.algo == CIG_PR || !rev.desc || !tune.pull_on || kw > tune.pull_width) return p;
+    // Long in-rows of bottom-up rounds (bfs.cuh): their chunks, partial masks
+    // and arrival counts; sized for every slot of the reverse arena.
+    BigRow *bfs_tasks = nullptr;
+    unsigned long long *bfs_acc = nullptr;
+    uint32_t *bfs_arrived = nullptr, *bfs_bigbits = nullptr;
+    BigRow *ms_chunks = nullptr;  // chunks of long rows of SSSP waves
+    uint64_t ms_chunk_cap() const { return 2 * fwd.seg_total * (kSegEdges / kMsChunk); }
+    uint64_t bfs_rows_cap() const { return rev.desc ? rev.seg_total * (kSegEdges / kBfsChunk) : 0; }
+
+    // Bottom-up switch of a BFS query: frontier above n/pull_on vertices
+    // (then at least n/pull_off); needs the device in-edge arena.
+    BfsPull bfs_pull(uint32_t kw) const {
+        BfsPull p{};
+        p.ctl = ms_small + 8;
+        if (opt.algo == CIG_PR || !rev.desc || !tune.pull_on) return p;
         p.rev = rev.view();
-        p.n = n;
-        p.full = kw >= 64 ? ~0ull : ((1ull << kw) - 1);
+#ifdef CIG_BOUNDS_CHECK
+        p.rev.bst = qstatus;
+#endif
         p.on = std::max<uint32_t>(1, n / tune.pull_on);
         p.off = std::max<uint32_t>(1, n / tune.pull_off);
+        // A bottom-up round passes over every vertex (and, in a wave, over
+        // most in-rows); a top-down edge costs about four times a vertex.
+        p.edges_on = kw == 1 ? n / 4 : n;
+        p.tasks = bfs_tasks;
+        p.task_cap = static_cast<uint32_t>(2 * bfs_rows_cap());
+        p.acc = bfs_acc;
+        p.arrived = bfs_arrived;
+        p.bigbits = bfs_bigbits;
         return p;
     }
 
@@ -2444,7 +2459,16 @@ struct cig_handle {
         dmalloc(ms_mask1, n);
         dmalloc(ms_q0, n + 1);
         dmalloc(ms_q1, n + 1);
-        dmalloc(ms_small, 8);
+        dmalloc(ms_small, 16);
+        dmalloc(ms_chunks, ms_chunk_cap());
+        if (rev.desc) {
+            dmalloc(bfs_tasks, 2 * bfs_rows_cap());
+            dmalloc(bfs_acc, bfs_rows_cap());
+            CK(cudaMemset(bfs_acc, 0, bfs_rows_cap() * sizeof(unsigned long long)));
+            dmalloc(bfs_arrived, bfs_rows_cap());
+            CK(cudaMemset(bfs_arrived, 0, bfs_rows_cap() * sizeof(uint32_t)));
+            dmalloc(bfs_bigbits, (n + 31) / 32);
+        }
         dmalloc(ms_src, kMsWidth);
         dmalloc(ms_big, kBigRowCap);
     }
@@ -2463,6 +2487,11 @@ struct cig_handle {
         dfree(ms_q0);
         dfree(ms_q1);
         dfree(ms_small);
+        dfree(ms_chunks);
+        dfree(bfs_tasks);
+        dfree(bfs_acc);
+        dfree(bfs_arrived);
+        dfree(bfs_bigbits);
         dfree(ms_src);
         dfree(ms_big);
         dfree(ms_out);
@@ -2492,6 +2521,38 @@ struct cig_handle {
         return v;
     }
 
+    // One SSSP wave of kw sources into wout (kw x n).
+    template <int A>
+    void sssp_wave(uint32_t kw, const MsFrontier &fr, const BigList &bl, uint32_t *wout) {
+        if (kw == 1) {  // distances straight into the result
+            CK(cudaMemsetAsync(wout, 0xFF, static_cast<size_t>(n) * sizeof(uint32_t), qstream));
+            ms_seed<<<1, kMsWidth, 0, qstream>>>(ms_src, 1u, wout, 1u, nullptr, fr, qstatus);
+            launch_coop_on(qstream, ms_closure<A>, kTpbMs, query_view(), wout, fr, bl, n + 2, qstatus);
+            --n_launch;  // no transpose
+        } else if (kw <= 4) {
+            sssp_wave_n<A, 1>(kw, fr, wout);
+        } else if (kw <= 8) {
+            sssp_wave_n<A, 2>(kw, fr, wout);
+        } else if (kw <= 16) {
+            sssp_wave_n<A, 4>(kw, fr, wout);
+        } else if (kw <= 32) {
+            sssp_wave_n<A, 8>(kw, fr, wout);
+        } else {
+            sssp_wave_n<A, 16>(kw, fr, wout);
+        }
+    }
+    template <int A, int LPE>
+    void sssp_wave_n(uint32_t kw, const MsFrontier &fr, uint32_t *wout) {
+        constexpr uint32_t row = 4 * LPE;
+        CK(cudaMemsetAsync(ms_dist, 0xFF, static_cast<size_t>(n) * row * sizeof(uint32_t), qstream));
+        ms_seed<<<1, kMsWidth, 0, qstream>>>(ms_src, kw, ms_dist, row, nullptr, fr, qstatus);
+        const MsChunks ch{ms_chunks, ms_small + 3, static_cast<uint32_t>(ms_chunk_cap()), ms_small + 8,
+                          ms_small + 11};
+        launch_coop_on(qstream, ms_wave<A, LPE>, kTpbMs, query_view(), n, ms_dist, fr, ch, n + 2, qstatus);
+        constexpr uint32_t rows = 512 / LPE;
+        ms_transpose<LPE><<<(n + rows - 1) / rows, 256, 0, qstream>>>(ms_dist, n, kw, wout);
+    }
+
     uint32_t query_launch(int algo, const uint32_t *sources, uint32_t k, uint32_t width, uint32_t *out) {
         const NvtxRange range("cig.query");
         if (!loaded) throw CigError(CIG_ERR_ARG, "load a graph first");
@@ -2509,30 +2570,46 @@ struct cig_handle {
         uint32_t waves = 0;
         for (uint32_t j0 = 0; j0 < k; j0 += width, ++waves) {
             const uint32_t kw = std::min(width, k - j0);
-            CK(cudaMemsetAsync(ms_dist, 0xFF, static_cast<size_t>(n) * width * sizeof(uint32_t), qstream));
-            CK(cudaMemsetAsync(ms_mask0, 0, n * sizeof(unsigned long long), qstream));
-            CK(cudaMemsetAsync(ms_mask1, 0, n * sizeof(unsigned long long), qstream));
-            if (algo == CIG_BFS)
-                CK(cudaMemsetAsync(ms_visit, 0, n * sizeof(unsigned long long), qstream));
-            CK(cudaMemsetAsync(ms_small, 0, 8 * sizeof(uint32_t), qstream));
+            uint32_t *wout = out + static_cast<uint64_t>(j0) * n;
+            CK(cudaMemsetAsync(ms_small, 0, 16 * sizeof(uint32_t), qstream));
             CK(cudaMemcpyAsync(ms_src, sources + j0, kw * sizeof(uint32_t), cudaMemcpyHostToDevice, qstream));
             const MsFrontier fr{ms_q0, ms_q1, ms_small, ms_mask0, ms_mask1, n + 1};
             const BigList bl{ms_big, ms_small + 3, kBigRowCap, tune.split};
-            ms_seed<<<1, kMsWidth, 0, qstream>>>(ms_src, kw, ms_dist, width, algo == CIG_BFS ? ms_visit : nullptr,
-                                                 fr, qstatus);
-            ++n_launch;
-            if (algo == CIG_BFS)
-                launch_coop_on(qstream, ms_closure<kBfs>, kTpbMs, query_view(), ms_dist, width, ms_visit, fr, bl, n + 2,
-                               ms_pull(kw), qstatus);
-            else if (opt.flags & CIG_FLAG_WEIGHT_U255)
-                launch_coop_on(qstream, ms_closure<kSsspU>, kTpbMs, query_view(), ms_dist, width,
-                               static_cast<unsigned long long *>(nullptr), fr, bl, n + 2, MsPull{}, qstatus);
-            else
-                launch_coop_on(qstream, ms_closure<kSssp>, kTpbMs, query_view(), ms_dist, width,
-                               static_cast<unsigned long long *>(nullptr), fr, bl, n + 2, MsPull{}, qstatus);
-            ms_transpose<<<(n + kMsTile - 1) / kMsTile, 256, 0, qstream>>>(ms_dist, n, width, kw,
-                                                                         out + static_cast<uint64_t>(j0) * n);
-            ++n_launch;
+            const size_t words = (n + 31) / 32;
+            if (algo == CIG_BFS && kw == 1) {
+                // One source: bitmaps, depths straight into the result.
+                uint32_t *vis = reinterpret_cast<uint32_t *>(ms_visit);
+                CK(cudaMemsetAsync(wout, 0xFF, static_cast<size_t>(n) * sizeof(uint32_t), qstream));
+                CK(cudaMemsetAsync(vis, 0, words * sizeof(uint32_t), qstream));
+                bfs_one_seed<<<1, 1, 0, qstream>>>(ms_src, wout, vis, ms_q0, ms_small);
+                launch_coop_on(qstream, bfs_one, kTpbMs, query_view(), n, wout, vis,
+                               reinterpret_cast<uint32_t *>(ms_mask0), reinterpret_cast<uint32_t *>(ms_mask1), fr, bl,
+                               n + 2, bfs_pull(kw), qstatus);
+                ++n_launch;
+                check_launch();
+                continue;
+            }
+            CK(cudaMemsetAsync(ms_mask0, 0, n * sizeof(unsigned long long), qstream));
+            CK(cudaMemsetAsync(ms_mask1, 0, n * sizeof(unsigned long long), qstream));
+            if (algo == CIG_BFS) {
+                // The planes live in the distance buffer (32 planes of 8 n
+                // bytes = 64 words per vertex).
+                static_assert(kBfsMaxPlanes * sizeof(unsigned long long) <= kMsWidth * sizeof(uint32_t),
+                              "planes fit the distance buffer");
+                unsigned long long *planes = reinterpret_cast<unsigned long long *>(ms_dist);
+                CK(cudaMemsetAsync(planes, 0, kBfsPlanes * n * sizeof(unsigned long long), qstream));
+                CK(cudaMemsetAsync(ms_visit, 0, n * sizeof(unsigned long long), qstream));
+                ms_seed<<<1, kMsWidth, 0, qstream>>>(ms_src, kw, nullptr, 0u, ms_visit, fr, qstatus);
+                const unsigned long long full = kw >= 64 ? ~0ull : ((1ull << kw) - 1);
+                launch_coop_on(qstream, bfs_wave, kTpbMs, query_view(), n, full, ms_visit, planes, fr, bl, n + 2,
+                               bfs_pull(kw), qstatus);
+                bfs_depths<<<sms * 8, 256, 0, qstream>>>(ms_visit, planes, n, kw, ms_small + 8, wout);
+            } else if (opt.flags & CIG_FLAG_WEIGHT_U255) {
+                sssp_wave<kSsspU>(kw, fr, bl, wout);
+            } else {
+                sssp_wave<kSssp>(kw, fr, bl, wout);
+            }
+            n_launch += 2;
             check_launch();
         }
         CK(cudaEventRecord(q_ev[2], qstream));
@@ -2902,8 +2979,9 @@ struct cig_handle {
                            static_cast<uint64_t>(bsnap_cap) * 41 * sizeof(unsigned long long);
         if (qstream)
             m->query_buffers = nn * kMsWidth * sizeof(uint32_t) + 3 * nn * sizeof(unsigned long long) +
-                               2 * (nn + 1) * sizeof(uint32_t) + sizeof(Status) + (8 + kMsWidth) * sizeof(uint32_t) +
-                               kBigRowCap * sizeof(BigRow);
+                               2 * (nn + 1) * sizeof(uint32_t) + sizeof(Status) + (16 + kMsWidth) * sizeof(uint32_t) +
+                               (kBigRowCap + ms_chunk_cap()) * sizeof(BigRow) +
+                               (rev.desc ? bfs_rows_cap() * (2 * sizeof(BigRow) + 12) + w * sizeof(uint32_t) : 0);
         m->total = m->edge_cache + m->segment_table + m->descriptors + m->reverse_arena + m->position_index +
                    m->vertex_state + m->batch_buffers + m->query_buffers;
         m->pinned_host = segs * kSegEdges * sizeof(uint32_t) + 4 * bcap * sizeof(uint32_t);

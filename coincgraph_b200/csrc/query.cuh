@@ -1,13 +1,14 @@
-// query.cuh - multi-source BFS and SSSP with 64-wide bitmask frontiers.
+// query.cuh - multi-source SSSP with 64-wide bitmask frontiers, and the
+// output side of the query waves (BFS: bfs.cuh).
 //
 // One wave serves up to 64 sources.  Per vertex the wave keeps a 64-bit mask
 // of the sources whose value at that vertex changed in the last round, so a
 // row is read once per round for all of those sources (the "MS-BFS" idea of
 // Then et al., "The More the Merrier: Efficient Multi-Source Graph
-// Traversal", VLDB 2014, applied to label-correcting SSSP as well).  Values
-// are stored vertex-major, `width` words per vertex (the wave width, 1..64),
-// so the sources of one vertex share cache lines; a transpose kernel writes
-// the k x n source-major result.
+// Traversal", VLDB 2014, applied to label-correcting SSSP).  Values
+// are stored vertex-major, 4 to 64 words per vertex (the wave's sources padded
+// to a power of two), so the sources of one vertex share cache lines; a
+// transpose kernel writes the k x n source-major result.
 //
 // The reference answers one source per engine run (BFS/SSSP Start,
 // include/framework/framework.cuh:1151-1182); these queries give the same
@@ -15,96 +16,45 @@
 // over the same adjacency (cache or zero-copy rows) and edge weights.
 #pragma once
 
+#include "bfs.cuh"
 #include "common.cuh"
 #include "expand.cuh"
 #include "traverse.cuh"
 
 namespace cig {
 
-constexpr uint32_t kMsWidth = 64;
-constexpr int kTpbMs = 256;
-
-struct MsFrontier {
-    uint32_t *q0;
-    uint32_t *q1;
-    uint32_t *cnt;                // 3 round counters, as for the push closure
-    unsigned long long *mask0;    // source masks read in even rounds
-    unsigned long long *mask1;    // ... in odd rounds
-    uint32_t cap;
-};
-
-// BFS: a source bit reaches y the first time any round carries it there;
-// `visit` holds the bits that already reached each vertex, so a bit is set
-// (and its depth written) exactly once.
-struct MsBfsOp {
-    uint32_t *dist;
-    uint32_t width;
-    unsigned long long *visit;
-    unsigned long long *mask_out;
-    uint32_t level;
-    uint32_t *q_out;
-    uint32_t *q_count;
-    uint32_t q_cap;
-    Status *st;
-
-    __device__ __forceinline__ bool edge(bool valid, uint32_t, unsigned long long m, uint32_t y) const {
-        bool want = false, hit = false;
-        if (valid) {
-            const unsigned long long cand = m & ~__ldcg(visit + y);
-            if (cand) {
-                const unsigned long long nb = cand & ~atomicOr(visit + y, cand);
-                if (nb) {
-                    hit = true;
-                    uint32_t *row = dist + static_cast<uint64_t>(y) * width;
-                    for (unsigned long long b = nb; b; b &= b - 1) row[__ffsll(static_cast<long long>(b)) - 1] = level;
-                    want = atomicOr(mask_out + y, nb) == 0ull;
-                }
-            }
-        }
-        warp_enqueue(want, y, q_out, q_count, q_cap, st);
-        return hit;
-    }
-};
-
-// SSSP (or BFS with unit weights): label-correcting relaxation per source
-// bit; a bit is carried to y for the next round when it lowered y's value.
+// One source (a wave of one: one word per vertex, the result itself).
 template <int A>
 struct MsRelaxOp {
     uint32_t *dist;
-    uint32_t width;
     unsigned long long *mask_out;
     uint32_t *q_out;
     uint32_t *q_count;
     uint32_t q_cap;
     Status *st;
 
-    __device__ __forceinline__ bool edge(bool valid, uint32_t x, unsigned long long m, uint32_t y) const {
-        bool want = false;
-        unsigned long long add = 0;
-        if (valid) {
-            const uint32_t w = edge_weight<A>(x, y);
-            const uint32_t *rx = dist + static_cast<uint64_t>(x) * width;
-            uint32_t *ry = dist + static_cast<uint64_t>(y) * width;
-            for (unsigned long long b = m; b; b &= b - 1) {
-                const int i = __ffsll(static_cast<long long>(b)) - 1;
-                const uint32_t nd = __ldcg(rx + i) + w;
-                if (nd < __ldcg(ry + i) && nd < atomicMin(ry + i, nd)) add |= 1ull << i;
-            }
-            if (add) want = atomicOr(mask_out + y, add) == 0ull;
-        }
+    __device__ __forceinline__ uint32_t peek(uint32_t y) const { return __ldcg(dist + y); }
+    __device__ __forceinline__ bool edge_peeked(bool valid, uint32_t x, uint32_t dx, uint32_t y, uint32_t dy) const {
+        const uint32_t nd = dx + edge_weight<A>(x, y);
+        const bool improved = valid && nd < dy && nd < atomicMin(dist + y, nd);
+        const bool want = improved && atomicOr(mask_out + y, 1ull) == 0ull;
         warp_enqueue(want, y, q_out, q_count, q_cap, st);
-        return add != 0ull;
+        return improved;
+    }
+    __device__ __forceinline__ bool edge(bool valid, uint32_t x, uint32_t dx, uint32_t y) const {
+        return edge_peeked(valid, x, dx, y, valid ? peek(y) : 0u);
     }
 };
 
-// Seeds of one wave: source j of the wave gets bit j, value 0, and its
-// vertex is queued once (several bits may share a vertex).
+// Seeds of one wave: source j of the wave gets bit j, value 0 (`dist`: SSSP)
+// or its visited bit (`visit`: BFS), and its vertex is queued once (several
+// bits may share a vertex).
 __global__ void ms_seed(const uint32_t *sources, uint32_t k, uint32_t *dist, uint32_t width,
                         unsigned long long *visit, MsFrontier fr, Status *st) {
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= k) return;
     const uint32_t s = sources[j];
-    dist[static_cast<uint64_t>(s) * width + j] = 0u;
+    if (dist) dist[static_cast<uint64_t>(s) * width + j] = 0u;
     if (visit) atomicOr(visit + s, 1ull << j);
     if (atomicOr(fr.mask0 + s, 1ull << j) == 0ull) {
         const uint32_t pos = atomicAdd(fr.cnt + 0, 1u);
@@ -115,69 +65,13 @@ __global__ void ms_seed(const uint32_t *sources, uint32_t k, uint32_t *dist, uin
     }
 }
 
-// Direction switching of the BFS wave (Beamer, Asanovic and Patterson,
-// "Direction-optimizing breadth-first search", SC 2012, on a bitmask
-// frontier): a round runs bottom-up when the frontier holds more than
-// `on` vertices (or, once bottom-up, at least `off`); 0 disables it.
-struct MsPull {
-    AdjView rev;             // in-edges (desc null: no bottom-up)
-    uint32_t n;
-    unsigned long long full; // the wave's source bits
-    uint32_t on, off;
-};
-
-// Bottom-up round: every vertex still missing source bits ORs the frontier
-// masks of its in-neighbours (stopping once nothing is missing) and takes
-// the new bits; one thread per vertex, so `visit` needs no atomics.
-__device__ __forceinline__ void ms_bottom_up(const MsPull &pl, uint32_t *dist, uint32_t width,
-                                             unsigned long long *visit, const unsigned long long *m_in,
-                                             unsigned long long *m_out, uint32_t level, uint32_t *q_out,
-                                             uint32_t *q_cnt, uint32_t cap, Status *st, ExpandCounters &cnt) {
-    const uint32_t rounded = (pl.n + 31u) & ~31u;
-    for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < rounded; w += gridDim.x * blockDim.x) {
-        bool want = false;
-        if (w < pl.n) {
-            const unsigned long long vis = __ldcg(visit + w);
-            const unsigned long long missing = pl.full & ~vis;
-            if (missing) {
-                const RowDesc d = pl.rev.desc[w];
-                unsigned long long acc = 0;
-                uint32_t k = 0;
-                for (; k < d.len && (acc & missing) != missing; ++k) {
-                    const uint32_t u = __ldg(pl.rev.at(d.off + k));
-                    if (u != kTomb) acc |= __ldcg(m_in + u);
-                }
-                cnt.edges += k;
-                cnt.edges_cached += k;
-                cnt.rows += d.len ? 1u : 0u;
-                const unsigned long long nb = acc & missing;
-                if (nb) {
-                    visit[w] = vis | nb;
-                    uint32_t *row = dist + static_cast<uint64_t>(w) * width;
-                    for (unsigned long long b = nb; b; b &= b - 1) row[__ffsll(static_cast<long long>(b)) - 1] = level;
-                    m_out[w] = nb;
-                    want = true;
-                    ++cnt.hits;
-                }
-            }
-        }
-        warp_enqueue(want, w, q_out, q_cnt, cap, st);
-    }
-}
-
-// Persistent multi-source closure (cooperative launch): round r expands the
-// vertices queued in round r-1 with the source bits that reached them.
-// BFS (kBfs with `visit`) is level-synchronous: round r writes depth r+1,
-// top-down or (with `pl`) bottom-up.
+// Single-source closure (cooperative launch): round r expands the vertices
+// queued in round r-1.
 template <int A>
-__global__ void __launch_bounds__(kTpbMs) ms_closure(AdjView fwd, uint32_t *dist, uint32_t width,
-                                                     unsigned long long *visit, MsFrontier fr, BigList big,
-                                                     uint32_t max_rounds, MsPull pl, Status *st) {
-    __shared__ ExpandSmem<kTpbMs, unsigned long long> sm;
+__global__ void __launch_bounds__(kTpbMs, 4) ms_closure(AdjView fwd, uint32_t *dist, MsFrontier fr, BigList big,
+                                                        uint32_t max_rounds, Status *st) {
+    __shared__ ExpandSmem<kTpbMs> sm;
     ExpandCounters cnt;
-    unsigned long long src_edges = 0;
-    bool pull = false;  // every block takes the same decisions from the same counts
-    const bool can_pull = A == kBfs && visit && pl.rev.desc && pl.on;
     uint32_t r = 0;
     for (;; ++r) {
         const uint32_t n_in = ld_volatile(fr.cnt + (r % 3));
@@ -194,82 +88,311 @@ __global__ void __launch_bounds__(kTpbMs) ms_closure(AdjView fwd, uint32_t *dist
         uint32_t *out = (r & 1) ? fr.q0 : fr.q1;
         unsigned long long *m_in = (r & 1) ? fr.mask1 : fr.mask0;
         unsigned long long *m_out = (r & 1) ? fr.mask0 : fr.mask1;
-        if (can_pull) pull = n_in > (pull ? pl.off : pl.on);
-        if (pull) {
-            ms_bottom_up(pl, dist, width, visit, m_in, m_out, r + 1, out, fr.cnt + ((r + 1) % 3), fr.cap, st, cnt);
-            if (!grid_barrier(st)) break;
-            // The frontier masks were read, not taken: clear them before
-            // the next round writes into this array.
-            for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_in; i += gridDim.x * blockDim.x)
-                m_in[__ldcg(in + i)] = 0ull;
-            if (!grid_barrier(st)) break;
-            continue;
-        }
         const Defer df{big.rows, big.cnt + (r % 3), big.cap, big.split};
+        const MsRelaxOp<A> op{dist, m_out, out, fr.cnt + ((r + 1) % 3), fr.cap, st};
         for (uint32_t base = 0; base < n_in; base += gridDim.x * kTpbMs) {
             const uint32_t i = base + spread_rank<kTpbMs>() * gridDim.x + blockIdx.x;
             bool has = i < n_in;
-            uint32_t x = 0, deg = 0;
+            uint32_t x = 0, dx = 0, deg = 0;
             uint64_t off = 0;
-            unsigned long long m = 0;
             if (has) {
                 x = __ldcg(in + i);
-                // Nobody writes m_in this round: take the bits and clear them.
-                m = __ldcg(m_in + x);
-                m_in[x] = 0ull;
+                m_in[x] = 0ull;  // nobody writes m_in this round
+                dx = __ldcg(dist + x);
                 const RowDesc d = fwd.desc[x];
                 deg = d.len;
                 off = d.off;
-                has = m != 0ull && deg > 0;
-                if (has) src_edges += static_cast<unsigned long long>(__popcll(m)) * deg;
+                has = deg > 0;
             }
-            // (Warp-only tiers, expand_rows_warp, measured the same for BFS and
-            // 12 % slower for SSSP waves than the block tiers.)
-            if (A == kBfs && visit) {
-                const MsBfsOp op{dist, width, visit, m_out, r + 1, out, fr.cnt + ((r + 1) % 3), fr.cap, st};
-                expand_rows<kTpbMs>(fwd, has, x, m, off, deg, op, sm, cnt, df);
-            } else {
-                const MsRelaxOp<A> op{dist, width, m_out, out, fr.cnt + ((r + 1) % 3), fr.cap, st};
-                expand_rows<kTpbMs>(fwd, has, x, m, off, deg, op, sm, cnt, df);
-            }
+            expand_rows<kTpbMs>(fwd, has, x, dx, off, deg, op, sm, cnt, df);
         }
         if (!grid_barrier(st)) break;
         const uint32_t nbig = min(ld_volatile(big.cnt + (r % 3)), big.cap);
         if (nbig) {
-            if (A == kBfs && visit) {
-                const MsBfsOp op{dist, width, visit, m_out, r + 1, out, fr.cnt + ((r + 1) % 3), fr.cap, st};
-                expand_deferred<kTpbMs, unsigned long long>(fwd, big.rows, nbig, op, cnt);
-            } else {
-                const MsRelaxOp<A> op{dist, width, m_out, out, fr.cnt + ((r + 1) % 3), fr.cap, st};
-                expand_deferred<kTpbMs, unsigned long long>(fwd, big.rows, nbig, op, cnt);
-            }
+            expand_deferred<kTpbMs>(fwd, big.rows, nbig, op, cnt);
             if (!grid_barrier(st)) break;
         }
     }
     flush_counters(st, cnt, kCntPush);
-    {
-        unsigned long long s = src_edges;
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(kFull, s, o);
-        if (lane_id() == 0 && s) atomicAdd(&st->counters[kCntSrcEdges], s);
-    }
+    warp_count(&st->counters[kCntSrcEdges], cnt.edges);  // one source
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&st->counters[kCntRounds], static_cast<unsigned long long>(r));
 }
 
-// Source-major output: out[j * n + v] = dist[v * width + j] for j < k,
-// through a shared-memory tile so that both sides are coalesced.
-constexpr uint32_t kMsTile = 32;
+// Waves of several sources.  A distance row holds the wave's sources padded to
+// `4 * LPE` words, so LPE lanes relax an edge with one 16-byte load of either
+// end's row each, and several edges' loads of a warp are in flight together.
+// (One lane relaxing an edge's sources in turn waited for two dependent loads
+// per source.)  While many vertices changed in the last round the frontier is
+// the non-zero masks: a round scans them, and an improved bit is an OR without
+// a result.  With a queue in those rounds too, the appends' atomics on its one
+// counter and the wait for every mask's old value took most of the time
+// (2.9 ms for 13 sources on R-MAT s19, a tenth of the L2's throughput).
+constexpr uint32_t kMsChunk = 256;  // rows of at least this many entries are expanded by the whole grid
+constexpr int kMsGroup = 4;         // edges per lane whose loads are in flight together
+constexpr uint32_t kMsScan = 64;    // rounds after more than n / kMsScan improvements scan the masks
 
-__global__ void ms_transpose(const uint32_t *dist, uint32_t n, uint32_t width, uint32_t k, uint32_t *out) {
-    __shared__ uint32_t tile[kMsTile][kMsWidth + 1];
-    const uint32_t v0 = blockIdx.x * kMsTile;
-    const uint32_t rows = min(kMsTile, n - v0);
-    // The tile's vertices are contiguous in `dist`: rows x width words.
-    const uint64_t base = static_cast<uint64_t>(v0) * width;
-    for (uint32_t e = threadIdx.x; e < rows * width; e += blockDim.x) tile[e / width][e % width] = dist[base + e];
+// Chunks of long rows met in a round (three counters, as for the frontier),
+// and the entries of a queue rebuilt from the masks (three counters).  A warp
+// per chunk: short, since the longest warp decides a round's time.
+struct MsChunks {
+    BigRow *rows;
+    uint32_t *cnt;
+    uint32_t cap;
+    uint32_t *fill;
+    uint32_t *tiles;  // three counters (TileFeed)
+};
+
+__device__ __forceinline__ void red_or(unsigned long long *p, unsigned long long x) {
+    asm volatile("red.relaxed.gpu.global.or.b64 [%0], %1;" ::"l"(p), "l"(x) : "memory");
+}
+
+template <int A, int LPE>
+struct MsWave {
+    uint32_t *dist;
+    unsigned long long *mask_out;
+    bool queue;  // append improved vertices
+    WarpBuf buf;
+
+    // Relax 32 edges, one per lane (x -> y for the sources in m; m = 0: none).
+    // Rows are read through L1: a value lowered meanwhile only costs a
+    // relaxation that fails, or one that its vertex repeats next round.
+    __device__ __forceinline__ uint32_t relax(uint32_t x, uint32_t y, unsigned long long m) const {
+        constexpr int kPer = 32 / LPE;                            // edges per step
+        constexpr int N = LPE < kMsGroup ? LPE : kMsGroup;        // steps in flight
+        constexpr uint64_t kRow = 4 * LPE;
+        const uint32_t lane = lane_id(), quad = lane % LPE;
+        uint32_t hits = 0;
+#pragma unroll
+        for (int s0 = 0; s0 < LPE; s0 += N) {
+            uint32_t xs[N], ys[N], bits[N];
+            uint4 dx[N], dy[N];
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                const int src = (s0 + j) * kPer + static_cast<int>(lane / LPE);
+                xs[j] = LPE == 1 ? x : __shfl_sync(kFull, x, src);
+                ys[j] = LPE == 1 ? y : __shfl_sync(kFull, y, src);
+                const unsigned long long ms = LPE == 1 ? m : __shfl_sync(kFull, m, src);
+                bits[j] = static_cast<uint32_t>(ms >> (4u * quad)) & 15u;
+            }
+#pragma unroll
+            for (int j = 0; j < N; ++j)
+                if (bits[j]) {
+                    dx[j] = *reinterpret_cast<const uint4 *>(dist + xs[j] * kRow + 4u * quad);
+                    dy[j] = *reinterpret_cast<const uint4 *>(dist + ys[j] * kRow + 4u * quad);
+                }
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                uint32_t add = 0;
+                if (bits[j]) {
+                    const uint32_t w = edge_weight<A>(xs[j], ys[j]);
+                    const uint32_t nd[4] = {dx[j].x + w, dx[j].y + w, dx[j].z + w, dx[j].w + w};
+                    const uint32_t od[4] = {dy[j].x, dy[j].y, dy[j].z, dy[j].w};
+                    uint32_t *row = dist + ys[j] * kRow + 4u * quad;
+                    uint32_t old[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        old[i] = ((bits[j] >> i) & 1u) && nd[i] < od[i] ? atomicMin(row + i, nd[i]) : 0u;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) add |= nd[i] < old[i] ? 1u << i : 0u;
+                    hits += add ? 1u : 0u;
+                }
+                const unsigned long long add64 = static_cast<unsigned long long>(add) << (4u * quad);
+                if (queue)
+                    buf.add(add && atomicOr(mask_out + ys[j], add64) == 0ull, ys[j]);
+                else if (add)
+                    red_or(mask_out + ys[j], add64);
+            }
+        }
+        return hits;
+    }
+};
+
+template <int A, int LPE>
+__global__ void __launch_bounds__(kTpbMs, 2) ms_wave(AdjView fwd, uint32_t n, uint32_t *dist, MsFrontier fr,
+                                                     MsChunks ch, uint32_t max_rounds, Status *st) {
+    __shared__ uint32_t s_scan[kTpbMs];
+    __shared__ uint32_t s_x[kTpbMs];
+    __shared__ unsigned long long s_m[kTpbMs];
+    __shared__ const uint32_t *s_ptr[kTpbMs];
+    __shared__ uint32_t s_buf[kTpbMs / 32][kWarpBuf];
+    __shared__ uint32_t s_held[kTpbMs / 32];
+    __shared__ uint32_t s_new;
+    if (threadIdx.x < kTpbMs / 32) s_held[threadIdx.x] = 0;
     __syncthreads();
-    for (uint32_t e = threadIdx.x; e < kMsTile * k; e += blockDim.x) {
-        const uint32_t j = e / kMsTile, vv = e % kMsTile;
-        if (vv < rows) out[static_cast<uint64_t>(j) * n + v0 + vv] = tile[vv][j];
+    ExpandCounters cnt;
+    unsigned long long src_edges = 0;
+    const uint32_t lane = lane_id(), wb = threadIdx.x & ~31u;
+    const uint32_t warps = (gridDim.x * kTpbMs) >> 5;
+    const uint32_t wid = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    bool scan = false;  // every block takes the same decisions from the same counts
+    uint32_t r = 0;
+    for (;; ++r) {
+        uint32_t n_in = ld_volatile(fr.cnt + (r % 3));  // queued vertices, or improvements of a scan round
+        if (n_in == 0) break;
+        if (r >= max_rounds) {
+            if (blockIdx.x == 0 && threadIdx.x == 0) set_error(st, kErrRounds, r);
+            break;
+        }
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            fr.cnt[(r + 2) % 3] = 0;
+            ch.cnt[(r + 2) % 3] = 0;
+            ch.fill[(r + 1) % 3] = 0;
+            ch.tiles[(r + 1) % 3] = 0;
+        }
+        uint32_t *in = (r & 1) ? fr.q1 : fr.q0;
+        uint32_t *out_cnt = fr.cnt + ((r + 1) % 3);
+        unsigned long long *m_in = (r & 1) ? fr.mask1 : fr.mask0;
+        unsigned long long *m_out = (r & 1) ? fr.mask0 : fr.mask1;
+        uint32_t *ch_cnt = ch.cnt + r % 3;
+        const bool was_scan = scan;
+        scan = n_in > n / kMsScan;
+        if (was_scan && !scan) {  // the masks as a queue
+            const uint32_t rounded = (n + 31u) & ~31u;
+            for (uint32_t v = blockIdx.x * kTpbMs + threadIdx.x; v < rounded; v += gridDim.x * kTpbMs)
+                warp_enqueue(v < n && m_in[v] != 0ull, v, in, ch.fill + r % 3, fr.cap, st);
+            if (!grid_barrier(st)) break;
+            n_in = ld_volatile(ch.fill + r % 3);
+        }
+        const MsWave<A, LPE> op{dist, m_out, !scan,
+                                WarpBuf{s_buf[threadIdx.x >> 5], s_held + (threadIdx.x >> 5), (r & 1) ? fr.q0 : fr.q1,
+                                        out_cnt, fr.cap, st}};
+        const uint32_t items = scan ? n : n_in;
+        uint32_t hits = 0;
+        uint32_t tile = 32;  // items per warp and step: few items spread over all warps
+        while (tile > (scan ? 8u : 1u) && items <= static_cast<uint64_t>(warps) * (scan ? 4u : 1u) * (tile / 2))
+            tile >>= 1;
+        TileFeed feed(ch.tiles + r % 3, warps);
+        for (uint64_t t = wid; t * tile < items; t = feed.take()) {
+            feed.ask();
+            const uint64_t i = t * tile + lane;
+            uint32_t x = 0, deg = 0;
+            uint64_t off = 0;
+            unsigned long long m = 0;
+            if (lane < tile && i < items) {
+                x = scan ? static_cast<uint32_t>(i) : __ldcg(in + i);
+                // Nobody writes m_in this round: take the bits and clear them.
+                m = __ldcg(m_in + x);
+                if (m) {
+                    m_in[x] = 0ull;
+                    const RowDesc d = fwd.desc[x];
+                    deg = d.len;
+                    off = d.off;
+                    if (deg) {
+                        src_edges += static_cast<unsigned long long>(__popcll(m)) * deg;
+                        cnt.rows += 1;
+                        cnt.edges += deg;
+                        if (fwd.cached(off)) cnt.edges_cached += deg;
+                    }
+                }
+            }
+            uint32_t bigs = __ballot_sync(kFull, deg >= kMsChunk);
+            while (bigs) {
+                const uint32_t l = __ffs(bigs) - 1;
+                bigs &= bigs - 1;
+                const uint32_t ldeg = __shfl_sync(kFull, deg, l), lx = __shfl_sync(kFull, x, l);
+                const uint64_t loff = __shfl_sync(kFull, static_cast<unsigned long long>(off), l);
+                const unsigned long long lm = __shfl_sync(kFull, m, l);
+                const uint32_t k = (ldeg + kMsChunk - 1) / kMsChunk;
+                uint32_t at = 0;
+                if (lane == 0) at = atomicAdd(ch_cnt, k);
+                at = __shfl_sync(kFull, at, 0);
+                for (uint32_t c = lane; c < k; c += 32u) {
+                    if (at + c < ch.cap)
+                        ch.rows[at + c] = BigRow{loff + static_cast<uint64_t>(c) * kMsChunk, lm, lx,
+                                                 min(kMsChunk, ldeg - c * kMsChunk)};
+                    else
+                        set_error(st, kErrQueue, at + c);
+                }
+            }
+            // The warp's rows concatenated, 32 edges per step; the next
+            // step's entries are read while this one's are relaxed.
+            const uint32_t mine = deg < kMsChunk ? deg : 0u;
+            uint32_t incl = mine;
+#pragma unroll
+            for (uint32_t o = 1; o < 32u; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(kFull, incl, o);
+                if (lane >= o) incl += t;
+            }
+            const uint32_t total = __shfl_sync(kFull, incl, 31);
+            if (!total) continue;
+            s_scan[wb + lane] = incl - mine;
+            s_x[wb + lane] = x;
+            s_m[wb + lane] = m;
+            s_ptr[wb + lane] = mine ? fwd.at(off) : nullptr;
+            __syncwarp();
+            auto fetch = [&](uint32_t e, uint32_t &owner) -> uint32_t {
+                owner = 0;
+                if (e >= total) return kTomb;
+                uint32_t lo = 0, hi = 32;  // the last lane whose edges start at or before e
+                while (hi - lo > 1) {
+                    const uint32_t mid = (lo + hi) >> 1;
+                    if (s_scan[wb + mid] <= e)
+                        lo = mid;
+                    else
+                        hi = mid;
+                }
+                owner = lo;
+                return __ldg(s_ptr[wb + lo] + (e - s_scan[wb + lo]));
+            };
+            uint32_t o_next, y_next = fetch(lane, o_next);
+            for (uint32_t e0 = 0; e0 < total; e0 += 32u) {
+                const uint32_t y = fwd.vid(y_next), o = o_next;
+                y_next = fetch(e0 + 32u + lane, o_next);
+                const bool live = y != kTomb;
+                hits += op.relax(s_x[wb + o], live ? y : 0u, live ? s_m[wb + o] : 0ull);
+            }
+            __syncwarp();
+        }
+        op.buf.flush();
+        if (scan) block_add(out_cnt, min(hits, 1024u), &s_new);
+        cnt.hits += hits;
+        if (!grid_barrier(st)) break;
+        const uint32_t nch = min(ld_volatile(ch_cnt), ch.cap);
+        if (nch) {
+            hits = 0;
+            for (uint32_t i = wid; i < nch; i += warps) {
+                const BigRow c = ch.rows[i];
+                const uint32_t *rp = fwd.at(c.off);  // a chunk lies in one segment
+                uint32_t y_next = lane < c.deg ? __ldg(rp + lane) : kTomb;
+                for (uint32_t e0 = 0; e0 < c.deg; e0 += 32u) {
+                    const uint32_t y = fwd.vid(y_next);
+                    y_next = e0 + 32u + lane < c.deg ? __ldg(rp + e0 + 32u + lane) : kTomb;
+                    const bool live = y != kTomb;
+                    hits += op.relax(c.x, live ? y : 0u, live ? c.payload : 0ull);
+                }
+            }
+            op.buf.flush();
+            if (scan) block_add(out_cnt, min(hits, 1024u), &s_new);
+            cnt.hits += hits;
+            if (!grid_barrier(st)) break;
+        }
+    }
+    flush_counters(st, cnt, kCntPush);
+    for (int o = 16; o > 0; o >>= 1) src_edges += __shfl_down_sync(kFull, src_edges, o);
+    if (lane == 0 && src_edges) atomicAdd(&st->counters[kCntSrcEdges], src_edges);
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&st->counters[kCntRounds], static_cast<unsigned long long>(r));
+}
+
+// Source-major output: out[j * n + v] = dist[v * 4 LPE + j] for j < k, through
+// a shared-memory tile: 16-byte reads, 128-byte stores.
+template <int LPE>
+__global__ void __launch_bounds__(256) ms_transpose(const uint32_t *dist, uint32_t n, uint32_t k, uint32_t *out) {
+    constexpr uint32_t kRow = 4 * LPE, kRows = 512 / LPE;
+    __shared__ uint32_t tile[kRows][kRow + 1];
+    const uint32_t v0 = blockIdx.x * kRows;
+    const uint32_t rows = min(kRows, n - v0);
+    for (uint32_t e = threadIdx.x; e < rows * LPE; e += 256u) {
+        const uint32_t v = e / LPE, q = e % LPE;
+        const uint4 d = *reinterpret_cast<const uint4 *>(dist + static_cast<uint64_t>(v0 + v) * kRow + 4u * q);
+        tile[v][4 * q] = d.x;
+        tile[v][4 * q + 1] = d.y;
+        tile[v][4 * q + 2] = d.z;
+        tile[v][4 * q + 3] = d.w;
+    }
+    __syncthreads();
+    for (uint32_t e = threadIdx.x; e < kRows * k; e += 256u) {
+        const uint32_t j = e / kRows, v = e % kRows;
+        if (v < rows) __stcs(out + static_cast<uint64_t>(j) * n + v0 + v, tile[v][j]);
     }
 }
 

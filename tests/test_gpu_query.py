@@ -11,7 +11,7 @@ import pytest
 import oracle
 from coincgraph_b200 import Engine, gen
 
-from helpers import big_row_case, rmat_case
+from helpers import big_row_case, grid_case, rmat_case
 
 pytestmark = pytest.mark.gpu
 
@@ -112,3 +112,38 @@ def test_query_rejects_bad_arguments(built):
             eng.query_bfs(np.array([g.n], dtype=np.uint32))
         # The handle stays usable after a rejected call.
         np.testing.assert_array_equal(eng.query_bfs([0])[0], eng.values())
+
+
+@pytest.mark.parametrize("pull", ["0", "32", "1000000"])  # never, default, as soon as two vertices are reached
+@pytest.mark.parametrize("make", [big_row_case, lambda: grid_case(33, 1, 40), lambda: rmat_case(10, 1, 50, 50)])
+def test_bfs_direction_and_depth_planes(built, make, pull, monkeypatch):
+    """Bottom-up and top-down rounds in every mix, in-rows on both sides of the
+    lane, warp and chunk limits, depths past the planes cleared at launch
+    (grid), a tail of the last bitmap word; waves of 1, 2 and 64 sources."""
+    monkeypatch.setenv("CIG_PULL_ON", pull)
+    monkeypatch.setenv("CIG_PULL_OFF", "2000000" if pull == "1000000" else "64")
+    case = make()
+    og = oracle.Graph(case.n, case.xadj, case.adj)
+    rng = np.random.default_rng(5)
+    src = np.concatenate([[0, case.n - 1], rng.integers(0, case.n, 62)]).astype(np.uint32)
+    ref = np.stack([og.sssp(int(s), oracle.BFS) for s in src])
+    with Engine("bfs", cache_gib=1.0) as eng:
+        eng.load_csr(case.n, case.xadj, case.adj)
+        eng.init()
+        for k in (64, 2, 1, 63):  # buffers of a wave are reused by the next
+            np.testing.assert_array_equal(eng.query_bfs(src[:k]), ref[:k])
+
+
+@pytest.mark.parametrize("k", [1, 2, 4, 5, 8, 9, 16, 17, 32, 33, 64])
+def test_sssp_wave_widths(built, k):
+    """Waves on both sides of every padded row width, rows on both sides of the
+    chunk length, host-resident and cached."""
+    case = big_row_case()
+    og = oracle.Graph(case.n, case.xadj, case.adj)
+    src = np.arange(k, dtype=np.uint32)
+    with Engine("sssp", cache_gib=65536 / 2**30) as eng:
+        eng.load_csr(case.n, case.xadj, case.adj)
+        eng.init()
+        got = eng.query_sssp(src)
+    for j in range(k):
+        np.testing.assert_array_equal(got[j], og.sssp(j, oracle.SSSP))
