@@ -90,6 +90,19 @@ __device__ __forceinline__ void seg_ctl_clear(uint32_t *ctl) {
     if (i < kCtlCount && i != kCtlFreeTop && i != kCtlBumpSeen) ctl[i] = 0u;
 }
 
+// Start of a phase: advance the batch epoch (the "invalidated in this batch"
+// marker of aff_stamp, kept on the device so that a captured batch graph
+// needs no new arguments; null: keep it), clear the counters of `counters` (64
+// words) whose bit is set in `mask` and the segment table's per-batch ones
+// (null: no table), in place of one memset each.  One block of at least 64
+// threads.
+__device__ __forceinline__ void begin_phase(uint32_t *epoch, uint32_t *counters, unsigned long long mask,
+                                            uint32_t *seg_ctl) {
+    if (epoch && threadIdx.x == 0) *epoch += 1u;
+    if (threadIdx.x < 64u && ((mask >> threadIdx.x) & 1u)) counters[threadIdx.x] = 0u;
+    if (seg_ctl) seg_ctl_clear(seg_ctl);
+}
+
 __device__ __forceinline__ uint32_t score_bucket(uint32_t sc) { return 32u - __clz(sc); }
 
 // One block copies one 64 KiB segment: each thread has eight 16-byte loads

@@ -233,6 +233,9 @@ constexpr unsigned long long kDeleteMask =
     (1ull << kIndexedCountR) | (1ull << kCoopF) | (1ull << kCoopR) | (1ull << kHugeF) | (1ull << kHugeR) |
     (1ull << kCompactBig) | (1ull << kCompactBigR) | (1ull << kPullBig);
 
+// A whole batch: frontier and affected counters too.
+constexpr unsigned long long kPhaseMask = kDeleteMask | kInsertMask | (0x3Full << kFr);
+
 constexpr uint32_t kBigRowCap = 65536;
 
 struct DevArena {
@@ -526,6 +529,7 @@ struct cig_handle {
     unsigned long long *kc = nullptr, *tc = nullptr;
     uint32_t *gaf = nullptr, *gar = nullptr, *gaendf = nullptr, *gaendr = nullptr;
     bool presorted = false;
+    bool begun = false;  // the whole-batch sort did the deletion phase's begin
     void *cub = nullptr;
     size_t cub_bytes = 0;
     uint32_t *stage = nullptr;  // pinned staging for host update arrays (4 * bcap)
@@ -837,6 +841,7 @@ struct cig_handle {
     uint64_t replay_mark = 0;
     void reset_counters() {
         presorted = false;
+        begun = false;
         CK(cudaMemsetAsync(status->counters, 0, sizeof(status->counters), stream));
         launch_mark = n_launch;
         replay_mark = graph_replays;
@@ -1637,41 +1642,44 @@ struct cig_handle {
         ps.off[4] = static_cast<uint32_t>(2 * nd + 2 * na);
         ps.f = f;
         const uint64_t total = ps.off[4];
+        SetGroups sg{};
+        sg.start[0] = gf;
+        sg.end[0] = gendf;
+        sg.count[0] = small + kGcF;
+        sg.start[1] = gr;
+        sg.end[1] = gendr;
+        sg.count[1] = small + kGcR;
+        sg.start[2] = gaf;
+        sg.end[2] = gaendf;
+        sg.count[2] = small + kGaF;
+        sg.start[3] = gar;
+        sg.end[3] = gaendr;
+        sg.count[3] = small + kGaR;
         const int p = prof_begin(CIG_STAGE_GROUP);
+        if (total && total <= kSmallSortKeys && 2 + 2 * f < 64) {
+            const SmallBatch sb{d_du, d_dv, d_au, d_av, {kf, kr, t1, t2}, small + kEpoch, small, kPhaseMask, seg_ctl};
+            if (total <= 128 * kSmallSortItems)
+                launch(small_batch<128>, 1, 128, sb, n, ps, sg, status);
+            else
+                launch(small_batch<512>, 1, 512, sb, n, ps, sg, status);
+            begun = true;
+            prof_end(p);
+            check_launch();
+            presorted = true;
+            return true;
+        }
         CK(cudaMemsetAsync(small + kGcF, 0, 2 * sizeof(uint32_t), stream));
         CK(cudaMemsetAsync(small + kGaF, 0, 2 * sizeof(uint32_t), stream));
         if (total) {
-            launch(make_keys_batch, grid_for(total), 256, d_du, d_dv, static_cast<uint32_t>(nd), d_au, d_av,
-                   static_cast<uint32_t>(na), n, ps, kc, status);
-            const unsigned long long *sorted;
+            launch(make_keys_batch, grid_for(total), 256, d_du, d_dv, d_au, d_av, n, ps, kc, status);
             size_t bytes = cub_bytes;
-            // ~0 pads the small sort's tail: keys of 2 + 2F < 64 bits sort below it.
-            if (total <= kSmallSortKeys) {
-                launch(sort_small, 1, kSmallSortThreads, kc, static_cast<uint32_t>(total), 2 + 2 * static_cast<int>(f),
-                       tc);
-                sorted = tc;
-            } else {
-                cub::DoubleBuffer<unsigned long long> db(kc, tc);
-                CK(cub::DeviceRadixSort::SortKeys(cub, bytes, db, static_cast<int>(total), 0,
-                                                  2 + 2 * static_cast<int>(f), stream));
-                sorted = db.Current();
-            }
+            cub::DoubleBuffer<unsigned long long> db(kc, tc);
+            CK(cub::DeviceRadixSort::SortKeys(cub, bytes, db, static_cast<int>(total), 0, 2 + 2 * static_cast<int>(f),
+                                              stream));
+            const unsigned long long *sorted = db.Current();
             launch(unpack_keys_batch, grid_for(total), 256, sorted, ps, kf, kr, t1, t2, gflags);
             bytes = cub_bytes;
             CK(cub::DeviceScan::ExclusiveSum(cub, bytes, gflags, gpos, static_cast<int>(total), stream));
-            SetGroups sg{};
-            sg.start[0] = gf;
-            sg.end[0] = gendf;
-            sg.count[0] = small + kGcF;
-            sg.start[1] = gr;
-            sg.end[1] = gendr;
-            sg.count[1] = small + kGcR;
-            sg.start[2] = gaf;
-            sg.end[2] = gaendf;
-            sg.count[2] = small + kGaF;
-            sg.start[3] = gar;
-            sg.end[3] = gaendr;
-            sg.count[3] = small + kGaR;
             launch(group_scatter_batch, grid_for(total), 256, sorted, ps, gflags, gpos, sg);
         }
         prof_end(p);
@@ -1916,8 +1924,8 @@ struct cig_handle {
         const InBatch ib(in_batch);
         const uint32_t *ep = small + kEpoch;
         static_assert(kSmallCount == 64, "phase_begin clears one 64-word counter block");
-        launch(phase_begin, 1, kSmallCount, small + kEpoch, small, kDeleteMask | kInsertMask | (0x3Full << kFr),
-               seg_ctl);
+        if (!begun) launch(phase_begin, 1, kSmallCount, small + kEpoch, small, kPhaseMask, seg_ctl);
+        begun = false;
         fork_arenas([&] { mutate_delete_arena(fwd, d_du, d_dv, nd, true, true); },
                     [&] { mutate_delete_arena(rev, d_du, d_dv, nd, false, false); });
         const SeedEdges seeds{d_du, d_dv, static_cast<uint32_t>(nd), n};

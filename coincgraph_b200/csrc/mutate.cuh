@@ -145,26 +145,24 @@ struct PackedSets {
     uint32_t f;  // field width F
 };
 
-__global__ void make_keys_batch(const uint32_t *du, const uint32_t *dv, uint32_t nd, const uint32_t *au,
-                                const uint32_t *av, uint32_t na, uint32_t n, PackedSets ps,
-                                unsigned long long *out, Status *st) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t total = ps.off[4];
-    if (i >= total) return;
+// Packed key of record i; counts a rejected addition once.
+__device__ __forceinline__ unsigned long long packed_key(const uint32_t *du, const uint32_t *dv, const uint32_t *au,
+                                                         const uint32_t *av, uint32_t n, const PackedSets &ps,
+                                                         uint32_t i, Status *st) {
     const uint32_t f = ps.f;
     const unsigned long long none = (1ull << f) - 1;
     uint32_t set, first, second;
     bool ok;
     if (i < ps.off[2]) {
         set = i < ps.off[1] ? 0u : 1u;
-        const uint32_t j = i - ps.off[set];
+        const uint32_t j = i - (set ? ps.off[1] : 0u);
         const uint32_t u = du[j], v = dv[j];
         ok = u < n && v < n;
         first = set == 0 ? u : v;
         second = set == 0 ? v : u;
     } else {
         set = i < ps.off[3] ? 2u : 3u;
-        const uint32_t j = i - ps.off[set];
+        const uint32_t j = i - (set == 3 ? ps.off[3] : ps.off[2]);
         const uint32_t u = au[j], v = av[j];
         ok = u < n && v < n;
         first = set == 2 ? u : v;
@@ -172,32 +170,13 @@ __global__ void make_keys_batch(const uint32_t *du, const uint32_t *dv, uint32_t
         if (!ok && set == 2) atomicAdd(&st->counters[kCntInvalid], 1ull);
     }
     const unsigned long long a = ok ? first : none, b = ok ? second : none;
-    out[i] = (static_cast<unsigned long long>(set) << (2 * f)) | (a << f) | b;
+    return (static_cast<unsigned long long>(set) << (2 * f)) | (a << f) | b;
 }
 
-// Small batches (at most kSmallSortKeys packed keys): one block sorts them
-// in shared memory, instead of a device-wide radix sort whose passes are
-// each a few microseconds of launch and latency.
-constexpr int kSmallSortThreads = 256;
-constexpr int kSmallSortItems = 16;
-constexpr uint32_t kSmallSortKeys = kSmallSortThreads * kSmallSortItems;
-
-__global__ void __launch_bounds__(kSmallSortThreads)
-    sort_small(const unsigned long long *in, uint32_t total, int end_bit, unsigned long long *out) {
-    using Sort = cub::BlockRadixSort<unsigned long long, kSmallSortThreads, kSmallSortItems>;
-    __shared__ typename Sort::TempStorage tmp;
-    unsigned long long k[kSmallSortItems];
-#pragma unroll
-    for (int j = 0; j < kSmallSortItems; ++j) {
-        const uint32_t i = threadIdx.x * kSmallSortItems + j;
-        k[j] = i < total ? in[i] : ~0ull;
-    }
-    Sort(tmp).Sort(k, 0, end_bit);
-#pragma unroll
-    for (int j = 0; j < kSmallSortItems; ++j) {
-        const uint32_t i = threadIdx.x * kSmallSortItems + j;
-        if (i < total) out[i] = k[j];
-    }
+__global__ void make_keys_batch(const uint32_t *du, const uint32_t *dv, const uint32_t *au, const uint32_t *av,
+                                uint32_t n, PackedSets ps, unsigned long long *out, Status *st) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < ps.off[4]) out[i] = packed_key(du, dv, au, av, n, ps, i, st);
 }
 
 // Sorted packed keys -> the usual (first << 32 | second) keys of each set,
@@ -246,6 +225,98 @@ __global__ void group_scatter_batch(const unsigned long long *sorted, PackedSets
     if (i + 1 == s1 || ((sorted[i + 1] >> f) & mask) == mask) {  // last valid key of the set
         sg.end[set][g + flags[i] - 1] = local + 1;
         *sg.count[set] = g + flags[i];
+    }
+}
+
+// Small batches (at most kSmallSortKeys packed keys): one block does all of it,
+// the phase's begin included.  (The device-wide sort and the kernels around it
+// are eight launches of a few microseconds each, and its passes as many
+// again; a block sort between five of those launches took 45 us on 4,000
+// keys.)
+constexpr int kSmallSortItems = 8;
+constexpr uint32_t kSmallSortKeys = 512 * kSmallSortItems;
+
+struct SmallBatch {
+    const uint32_t *du, *dv, *au, *av;
+    unsigned long long *keys[4];  // sorted keys of each set
+    uint32_t *epoch;              // phase_begin's work
+    uint32_t *counters;
+    unsigned long long mask;
+    uint32_t *seg_ctl;
+};
+
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) small_batch(SmallBatch sb, uint32_t n, PackedSets ps, SetGroups sg,
+                                                       Status *st) {
+    using Sort = cub::BlockRadixSort<unsigned long long, THREADS, kSmallSortItems>;
+    using Scan = cub::BlockScan<uint32_t, THREADS>;
+    constexpr uint32_t kItems = THREADS * kSmallSortItems;
+    __shared__ union {
+        typename Sort::TempStorage sort;
+        unsigned long long sorted[kItems];
+    } sm;
+    __shared__ typename Scan::TempStorage scan_tmp;
+    __shared__ uint32_t s_base[4];
+    begin_phase(sb.epoch, sb.counters, sb.mask, sb.seg_ctl);
+    if (threadIdx.x < 4) *sg.count[threadIdx.x] = 0u;
+    const uint32_t total = ps.off[4], f = ps.f;
+    const uint32_t i0 = threadIdx.x * kSmallSortItems;
+    unsigned long long k[kSmallSortItems];
+#pragma unroll
+    for (int j = 0; j < kSmallSortItems; ++j)  // ~0 sorts behind every key of 2 + 2 f < 64 bits
+        k[j] = i0 + j < total ? packed_key(sb.du, sb.dv, sb.au, sb.av, n, ps, i0 + j, st) : ~0ull;
+    Sort(sm.sort).Sort(k, 0, 2 + 2 * static_cast<int>(f));
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kSmallSortItems; ++j) sm.sorted[i0 + j] = k[j];
+    __syncthreads();
+    const unsigned long long mask = (1ull << f) - 1;
+    uint32_t flags = 0;
+#pragma unroll
+    for (int j = 0; j < kSmallSortItems; ++j) {
+        const uint32_t i = i0 + j;
+        const uint32_t set = i < ps.off[2] ? (i < ps.off[1] ? 0u : 1u) : (i < ps.off[3] ? 2u : 3u);
+        const uint32_t s0 = set == 0 ? 0u : set == 1 ? ps.off[1] : set == 2 ? ps.off[2] : ps.off[3];
+        const unsigned long long a = (k[j] >> f) & mask, b = k[j] & mask;
+        const bool ok = i < total && a != mask;
+        const unsigned long long prev = i == 0 ? ~k[j] : j ? k[j ? j - 1 : 0] : sm.sorted[i - 1];
+        if (ok && (i == s0 || (prev >> f) != (k[j] >> f))) flags |= 1u << j;
+        unsigned long long *dst = set == 0 ? sb.keys[0] : set == 1 ? sb.keys[1] : set == 2 ? sb.keys[2] : sb.keys[3];
+        if (i < total) dst[i - s0] = ok ? ((a << kKeyShift) | b) : kKeyNone;
+    }
+    uint32_t pos;
+    Scan(scan_tmp).ExclusiveSum(static_cast<uint32_t>(__popc(flags)), pos);
+#pragma unroll
+    for (int j = 0; j < kSmallSortItems; ++j) {
+        const uint32_t at = pos + __popc(flags & ((1u << j) - 1u));
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+            if (i0 + j == ps.off[t]) s_base[t] = at;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kSmallSortItems; ++j) {
+        const uint32_t i = i0 + j;
+        if (i >= total || ((k[j] >> f) & mask) == mask) continue;  // pad or invalid record
+        const uint32_t set = i < ps.off[2] ? (i < ps.off[1] ? 0u : 1u) : (i < ps.off[3] ? 2u : 3u);
+        const uint32_t s0 = set == 0 ? 0u : set == 1 ? ps.off[1] : set == 2 ? ps.off[2] : ps.off[3];
+        const uint32_t s1 = set == 0 ? ps.off[1] : set == 1 ? ps.off[2] : set == 2 ? ps.off[3] : total;
+        uint32_t *start = set == 0 ? sg.start[0] : set == 1 ? sg.start[1] : set == 2 ? sg.start[2] : sg.start[3];
+        uint32_t *end = set == 0 ? sg.end[0] : set == 1 ? sg.end[1] : set == 2 ? sg.end[2] : sg.end[3];
+        uint32_t *count = set == 0 ? sg.count[0] : set == 1 ? sg.count[1] : set == 2 ? sg.count[2] : sg.count[3];
+        const uint32_t head = (flags >> j) & 1u;
+        const uint32_t g = pos + __popc(flags & ((1u << j) - 1u)) - s_base[set];
+        if (head) {
+            start[g] = i - s0;
+            if (g > 0) end[g - 1] = i - s0;
+        }
+        const unsigned long long next = j + 1 < kSmallSortItems ? k[j + 1 < kSmallSortItems ? j + 1 : j]
+                                        : i + 1 < kItems        ? sm.sorted[i + 1]
+                                                                : ~0ull;
+        if (i + 1 == s1 || ((next >> f) & mask) == mask) {  // last valid key of the set
+            end[g + head - 1] = i - s0 + 1;
+            *count = g + head;
+        }
     }
 }
 

@@ -804,15 +804,9 @@ __global__ void __launch_bounds__(kTpb, 2) repair_closure(AdjView fwd, AdjView r
     }
 }
 
-// Start of a phase: advance the batch epoch (the "invalidated in this batch"
-// marker of aff_stamp, kept on the device so that a captured batch graph
-// needs no new arguments; null: keep it), clear the counters of `counters` (64
-// words) whose bit is set in `mask` and the segment table's per-batch ones
-// (null: no table), in place of one memset each.  Launched with 64 threads.
+// Start of a phase in a launch of its own (small batches: small_batch).
 __global__ void phase_begin(uint32_t *epoch, uint32_t *counters, unsigned long long mask, uint32_t *seg_ctl) {
-    if (epoch && threadIdx.x == 0) *epoch += 1u;
-    if (threadIdx.x < 64u && ((mask >> threadIdx.x) & 1u)) counters[threadIdx.x] = 0u;
-    if (seg_ctl) seg_ctl_clear(seg_ctl);
+    begin_phase(epoch, counters, mask, seg_ctl);
 }
 
 // Static-solve initialisation (InitGraph, framework.cuh:991-1041).
