@@ -288,24 +288,19 @@ __device__ __forceinline__ void warp_count(unsigned long long *counter, uint32_t
 // Grid-wide barrier for cooperatively launched kernels.  Waits are bounded:
 // after ~2 s without progress the waiting block records kErrBarrier and
 // returns false; every later barrier then returns false at once.
-// One thread per block arrives and polls the generation; the error word and
-// the clock are looked at once per kBarrierPoll polls.
+// One thread per block arrives and polls the generation, with plain volatile
+// loads: acquire loads drop the SM's L1 lines at every poll, under the warps
+// of the other block that is still at work there.
 constexpr long long kBarrierTimeoutCycles = 4000000000LL;
-constexpr uint32_t kBarrierPoll = 64;
-constexpr uint32_t kBarrierSleepNs = 20;
-
-__device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p) {
-    uint32_t v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
+constexpr uint32_t kBarrierPoll = 32;  // polls between looks at the error word and the clock
+constexpr uint32_t kBarrierSleepNs = 40;
 
 __device__ __forceinline__ bool grid_barrier(Status *st) {
     __syncthreads();
     __shared__ uint32_t ok;
     if (threadIdx.x == 0) {
         ok = 1;
-        const uint32_t gen = ld_acquire(&st->barrier_gen);
+        const uint32_t gen = ld_volatile(&st->barrier_gen);
         __threadfence();
         const uint32_t arrived = atomicAdd(&st->barrier_count, 1);
         if (arrived == gridDim.x - 1) {
@@ -315,7 +310,7 @@ __device__ __forceinline__ bool grid_barrier(Status *st) {
         } else {
             const long long start = clock64();
             uint32_t polls = 0;
-            while (ld_acquire(&st->barrier_gen) == gen) {
+            while (ld_volatile(&st->barrier_gen) == gen) {
                 if (++polls % kBarrierPoll == 0) {
                     if (ld_volatile(&st->err) & kErrBarrier) break;
                     if (clock64() - start > kBarrierTimeoutCycles) {

@@ -629,13 +629,21 @@ struct cig_handle {
     int coop_blocks(K kernel, int tpb) const {
         int per_sm = 0;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, tpb, 0));
-        per_sm = std::min(per_sm, static_cast<int>(in_batch && tune.inc_per_sm ? tune.inc_per_sm : tune.per_sm));
+        uint32_t most = in_batch && tune.inc_per_sm ? tune.inc_per_sm : tune.per_sm;
+        if (in_batch && batch_requests <= kNarrowBatch) most = std::min(most, 1u);
+        per_sm = std::min(per_sm, static_cast<int>(most));
         if (per_sm < 1) throw CigError(CIG_ERR_DEVICE, "cooperative kernel does not fit on an SM");
         return per_sm * sms;
     }
     // Set while the closures of an update batch are queued: they may use
     // their own launch shape (tune.inc_per_sm), the static solve uses per_sm.
     bool in_batch = false;
+    // Requests of the phase being queued.  Up to kNarrowBatch its closures run
+    // one block per SM: half the blocks meet at a barrier sooner (four batches
+    // of 25k + 25k on s22: 1.96 against 2.00 ms, a 511 x 511 grid 5.2 against
+    // 5.5 ms); larger batches (100k + 100k on s24) keep inc_per_sm.
+    uint64_t batch_requests = 0;
+    static constexpr uint64_t kNarrowBatch = 1u << 16;
 
     uint64_t n_launch = 0;  // kernels this engine launched (CUB sort kernels not included)
 
@@ -1412,7 +1420,10 @@ struct cig_handle {
         launch_coop(push_closure<A>, kTpb, fwd.view(), state, qstamp, tags, frontier(), seeds, parts, big_list(kPushBig),
                     n + 2, local_sweeps, seg_hot, status);
     }
-    uint32_t local_sweeps = 8;  // block-local hops per closure round (CIG_LOCAL_SWEEPS; 0 = off)
+    // Block-local hops per closure round (CIG_LOCAL_SWEEPS; 0 = off).  R-MAT
+    // batches measure the same from 1 to 32; a 511 x 511 grid 5.25 ms with 8,
+    // 4.8 with 16, 4.63 with 32, 4.75 with 64.
+    uint32_t local_sweeps = 32;
     // Share of the initially resident slots given to the last segments of the
     // arena (the smallest row classes), in percent (CIG_CACHE_SMALL_PCT); a
     // negative value: the segments of the small row classes.
@@ -1907,9 +1918,12 @@ struct cig_handle {
     }
 
     struct InBatch {
-        bool &flag;
-        explicit InBatch(bool &f) : flag(f) { flag = true; }
-        ~InBatch() { flag = false; }
+        cig_handle &h;
+        InBatch(cig_handle &handle, uint64_t requests) : h(handle) {
+            h.in_batch = true;
+            h.batch_requests = requests;
+        }
+        ~InBatch() { h.in_batch = false; }
     };
 
     // `push` false: leave the re-propagation from the repaired vertices to
@@ -1921,7 +1935,7 @@ struct cig_handle {
     // expose, are skipped.
     template <int A>
     void delete_phase_dev(const uint32_t *d_du, const uint32_t *d_dv, uint64_t nd, bool push = true) {
-        const InBatch ib(in_batch);
+        const InBatch ib(*this, nd);
         const uint32_t *ep = small + kEpoch;
         static_assert(kSmallCount == 64, "phase_begin clears one 64-word counter block");
         if (!begun) launch(phase_begin, 1, kSmallCount, small + kEpoch, small, kPhaseMask, seg_ctl);
@@ -1953,7 +1967,7 @@ struct cig_handle {
     // begin cleared the insertion counters too).
     template <int A>
     void insert_phase_dev(const uint32_t *d_au, const uint32_t *d_av, uint64_t na, bool fresh = true) {
-        const InBatch ib(in_batch);
+        const InBatch ib(*this, na);
         if (fresh) launch(phase_begin, 1, kSmallCount, nullptr, small, kInsertMask | (7ull << kFr), seg_ctl);
         fork_arenas([&] { mutate_add_arena(fwd, d_au, d_av, na, true, true); },
                     [&] { mutate_add_arena(rev, d_au, d_av, na, false, false); });

@@ -613,55 +613,73 @@ __device__ __forceinline__ void seed_deletions(const SeedEdges &e, const unsigne
     }
 }
 
+// The invalidated vertices: the closure's list, then the ones its local
+// sweeps expanded.
+struct Affected {
+    const uint32_t *list;
+    uint32_t n_list;
+    const uint32_t *done;
+    uint32_t n;
+    __device__ __forceinline__ uint32_t at(uint32_t i) const {
+        return __ldcg(i < n_list ? list + i : done + (i - n_list));
+    }
+};
+
 // Repair of the invalidated vertices: value <- initial value
 // (reset_affected_values, driver.cuh:418-433: unreached for BFS/SSSP, its own
 // id for CC), pull over their in-rows, queue every one that has a value (all
-// of them for CC).  In-rows of at least big.split entries are left to the
-// whole grid after a barrier.
+// of them for CC).  A vertex is reset by its own lane right before its row is
+// expanded: nobody else reads the value of an invalidated vertex (PullOp::peek
+// sees the stamp), so no barrier separates the resets from the pulls, and it
+// is queued when its row is done.  In-rows of at least big.split entries are
+// left to the whole grid after a barrier.
 template <int A>
 __device__ __forceinline__ void pull_repair(const AdjView &rev, unsigned long long *state, const uint32_t *aff_stamp,
-                                            uint32_t epoch, uint32_t ccs, const uint32_t *list, uint32_t n,
-                                            const Frontier &fr, const Defer &df, ExpandSmem<kTpb> &sm, Status *st) {
-    const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, gthreads = gridDim.x * blockDim.x;
-    for (uint32_t i = gtid; i < n; i += gthreads) {
-        const uint32_t v = __ldcg(list + i);
-        state[v] = (A == kCc) ? pack(v << ccs, kInf) : kInf64;
-        prefetch_l2(rev.desc + v);
-    }
-    if (!grid_barrier(st)) return;
+                                            uint32_t epoch, uint32_t ccs, const Affected &aff, const Frontier &fr,
+                                            const Defer &df, ExpandSmem<kTpb> &sm, Status *st) {
     ExpandCounters c;
     const PullOp<A> op{ccs, state, aff_stamp, epoch};
-    for (uint32_t base = 0; base < n; base += gridDim.x * kTpb) {
+    for (uint32_t base = 0; base < aff.n; base += gridDim.x * kTpb) {
         const uint32_t i = base + spread_rank<kTpb>() * gridDim.x + blockIdx.x;
-        bool has = i < n;
+        const bool mine = i < aff.n;
+        bool has = false;
         uint32_t v = 0, deg = 0;
         uint64_t off = 0;
-        if (has) {
-            v = __ldcg(list + i);
+        if (mine) {
+            v = aff.at(i);
+            state[v] = (A == kCc) ? pack(v << ccs, kInf) : kInf64;
             const RowDesc d = rev.desc[v];
             deg = d.len;
             off = d.off;
             has = deg > 0;
         }
+        __syncwarp();  // the reset, before the row's other lanes relax v
         expand_rows<kTpb>(rev, has, v, 0u, off, deg, op, sm, c, df);
-    }
-    if (!grid_barrier(st)) return;
-    const uint32_t nbig = min(ld_volatile(df.count), df.cap);
-    if (nbig) {
-        expand_deferred<kTpb>(rev, df.rows, nbig, op, c);
-        if (!grid_barrier(st)) return;
-    }
-    const uint32_t rounded = (n + 31u) & ~31u;
-    for (uint32_t i = gtid; i < rounded; i += gthreads) {
-        bool want = false;
-        uint32_t v = 0;
-        if (i < n) {
-            v = __ldcg(list + i);
-            want = (A == kCc) || val_of(__ldcg(state + v)) != kInf;
-        }
+        __syncwarp();
+        const bool later = has && deg >= df.split;
+        const bool want = mine && !later && (A == kCc || val_of(__ldcg(state + v)) != kInf);
         warp_enqueue(want, v, fr.q0, fr.cnt, fr.cap, st);
     }
     flush_counters(st, c, kCntPull);
+    if (!grid_barrier(st)) return;
+    const uint32_t nbig = min(ld_volatile(df.count), df.cap);
+    if (!nbig) return;
+    ExpandCounters cb;
+    expand_deferred<kTpb>(rev, df.rows, nbig, op, cb);
+    flush_counters(st, cb, kCntPull);
+    if (!grid_barrier(st)) return;
+    // The deferred rows' vertices; a row that found no place in the list was
+    // expanded in place above and is queued here like the others.
+    const uint32_t rounded = (aff.n + 31u) & ~31u;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < rounded; i += gridDim.x * blockDim.x) {
+        bool want = false;
+        uint32_t v = 0;
+        if (i < aff.n) {
+            v = aff.at(i);
+            want = rev.desc[v].len >= df.split && (A == kCc || val_of(__ldcg(state + v)) != kInf);
+        }
+        warp_enqueue(want, v, fr.q0, fr.cnt, fr.cap, st);
+    }
 }
 
 // The deletion phase's closure (cooperative launch): seeds, invalidation
@@ -687,7 +705,7 @@ __global__ void __launch_bounds__(kTpb, 2) repair_closure(AdjView fwd, AdjView r
     const Defer pull_df{big.rows, pull_big, big.cap, big.split};
     if (!(parts & kPartRounds)) {
         const uint32_t n = (parts & kPartPull) ? *aff_total : 0u;
-        if (n) pull_repair<A>(rev, state, aff_stamp, epoch, ccs, list, n, fr, pull_df, sm, st);
+        if (n) pull_repair<A>(rev, state, aff_stamp, epoch, ccs, Affected{list, n, list, n}, fr, pull_df, sm, st);
         return;
     }
     uint32_t lo = 0, hi = ld_volatile(cnt3 + 0);
@@ -782,12 +800,14 @@ __global__ void __launch_bounds__(kTpb, 2) repair_closure(AdjView fwd, AdjView r
         lo = hi;
         hi = hi + ld_volatile(cnt3 + ((r + 1) % 3));
     }
+    const uint32_t n_list = hi;
     if (max_sweeps) {
         // The vertices expanded by local sweeps complete the affected list.
         // Every block left the loop after the same barrier, so `done` is final.
         const uint32_t nd = ld_volatile(done_cnt);
-        for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nd && hi + i < cap; i += gridDim.x * blockDim.x)
-            list[hi + i] = __ldcg(done + i);
+        if (!(parts & kPartPull))  // for the part that follows in a launch of its own
+            for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nd && hi + i < cap; i += gridDim.x * blockDim.x)
+                list[hi + i] = __ldcg(done + i);
         if (hi + nd > cap && blockIdx.x == 0 && threadIdx.x == 0) set_error(st, kErrQueue, hi + nd);
         hi += min(nd, cap - min(hi, cap));
     }
@@ -797,11 +817,8 @@ __global__ void __launch_bounds__(kTpb, 2) repair_closure(AdjView fwd, AdjView r
         atomicAdd(&st->counters[kCntRounds], static_cast<unsigned long long>(r));
         atomicAdd(&st->counters[kCntAffected], static_cast<unsigned long long>(hi));
     }
-    if ((parts & kPartPull) && hi) {
-        // the list is complete once every block has appended its share of `done`
-        if (max_sweeps && !grid_barrier(st)) return;
-        pull_repair<A>(rev, state, aff_stamp, epoch, ccs, list, hi, fr, pull_df, sm, st);
-    }
+    if ((parts & kPartPull) && hi)
+        pull_repair<A>(rev, state, aff_stamp, epoch, ccs, Affected{list, n_list, done, hi}, fr, pull_df, sm, st);
 }
 
 // Start of a phase in a launch of its own (small batches: small_batch).
