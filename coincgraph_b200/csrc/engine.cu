@@ -221,7 +221,7 @@ enum SmallIdx : int {
     kPushBig = 44,    // 3 counters of the push closure's deferred hub rows
     kPlanDoneF = 47,  // blocks of plan_add that are done, per arena (each launch leaves 0)
     kPlanDoneR = 48,
-    kPrAct = 33,  // 3 counters of vertices consumed per PageRank sweep, then 3 of its chunks
+    kPrAct = 49,  // 3 counters of vertices consumed per PageRank sweep, then 3 of its chunks
     kSmallCount = 64
 };
 
@@ -345,7 +345,7 @@ struct cig_handle {
     double *pr_amend64 = nullptr;  // FP32 mode: per-vertex FP64 amend accumulator (pr_amend_fold)
     uint32_t *pr_hub_bits = nullptr, *pr_hub_prefix = nullptr;  // FP32 mode: FP64 residual slots (pr.cuh)
     uint32_t pr_hubs = 0;
-    double *pr_res_hub = nullptr;
+    double *pr_res_hub = nullptr, *pr_hub_more = nullptr;
     float *pr_comp = nullptr;
     BigRow *pr_chunks = nullptr;  // the sweeps' chunks of long rows (pr_chunk_cap entries)
     uint64_t pr_chunk_cap() const { return 2 * fwd.seg_total * (kSegEdges / kPrChunk); }
@@ -989,6 +989,7 @@ struct cig_handle {
         dfree(pr_hub_bits);
         dfree(pr_hub_prefix);
         dfree(pr_res_hub);
+        dfree(pr_hub_more);
         dfree(pr_comp);
         dfree(pr_chunks);
         dfree(pr_queued);
@@ -1314,6 +1315,9 @@ struct cig_handle {
                 dmalloc(pr_res_hub, std::max<uint32_t>(nh, 1));
                 CK(cudaMemset(pr_res_hub, 0, std::max<uint32_t>(nh, 1) * sizeof(double)));
                 pr_hubs = nh;
+                const size_t more = static_cast<size_t>(kHubCopies - 1) * std::max<uint32_t>(nh, 1);
+                dmalloc(pr_hub_more, more);
+                CK(cudaMemset(pr_hub_more, 0, more * sizeof(double)));
             }
             dmalloc(pr_queued, n);
             dmalloc(pr_chunks, pr_chunk_cap());
@@ -1438,7 +1442,7 @@ struct cig_handle {
     template <class T>
     PrArrays<T> pr_arrays() {
         return PrArrays<T>{static_cast<T *>(pr_rank), static_cast<T *>(pr_res), pr_hub_bits, pr_hub_prefix, pr_res_hub,
-                           pr_comp, pr_queued, q0, q1, small + kFr, static_cast<T *>(pr_contrib), small + kFinalRound,
+                           pr_hub_more, pr_hubs, pr_comp, pr_queued, q0, q1, small + kFr, static_cast<T *>(pr_contrib), small + kFinalRound,
                            n + 1};
     }
 
@@ -2981,7 +2985,7 @@ struct cig_handle {
                 const uint64_t es = pr64 ? sizeof(double) : sizeof(float);
                 vs += 2 * nn * es + (nn + 1) * es + 2 * nn * sizeof(uint32_t) + pr_chunk_cap() * sizeof(BigRow);
                 if (!pr64) vs += nn * sizeof(float) + nn * sizeof(double) + 2 * w * sizeof(uint32_t) +
-                                 std::max<uint32_t>(pr_hubs, 1) * sizeof(double);
+                                 std::max<uint32_t>(pr_hubs, 1) * kHubCopies * sizeof(double);
             } else {
                 vs += nn * sizeof(unsigned long long) + 2 * nn * sizeof(uint32_t) + (nn + 1) * sizeof(uint32_t);
             }

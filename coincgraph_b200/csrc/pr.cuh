@@ -34,6 +34,10 @@ constexpr float kAlphaF = 0.85f;
 constexpr double kAlphaD = 0.85;
 
 constexpr uint32_t kPrHubInDeg = 256;
+// Sweeps spread the adds to a hub over this many copies of its slot, by block:
+// adds to one address are served one after the other (16 thousand per sweep at
+// the largest hub of R-MAT s18), and the consumer sums the copies.
+constexpr uint32_t kHubCopies = 8;
 
 template <class T>
 struct PrArrays {
@@ -42,6 +46,8 @@ struct PrArrays {
     const uint32_t *hub_bits;    // FP32 mode: bit v set when v has an FP64 residual slot
     const uint32_t *hub_prefix;  // slots before word w of hub_bits
     double *res_hub;
+    double *hub_more;  // kHubCopies - 1 further copies of res_hub, zero outside sweeps
+    uint32_t hubs;
     float *comp;       // Kahan compensation of rank (FP32 mode only)
     uint32_t *queued;
     uint32_t *q0;
@@ -216,12 +222,17 @@ __device__ __forceinline__ void red_add(double *p, double x) {
 template <class T>
 struct PrSweepOp {
     PrArrays<T> a;
+    double *hub;  // this block's copy of the hubs' residuals
+    __device__ __forceinline__ explicit PrSweepOp(const PrArrays<T> &arr) : a(arr), hub(arr.res_hub) {
+        const uint32_t copy = blockIdx.x % kHubCopies;
+        if (copy && a.hub_more) hub = a.hub_more + static_cast<uint64_t>(copy - 1) * a.hubs;
+    }
     __device__ __forceinline__ int32_t peek(uint32_t y) const { return hub_slot(a, y); }
     __device__ __forceinline__ bool edge_peeked(bool valid, uint32_t, typename PrBits<T>::type c, uint32_t y,
                                                 int32_t h) const {
         if (valid) {
             if (h >= 0)
-                red_add(a.res_hub + h, static_cast<double>(PrBits<T>::from(c)));
+                red_add(hub + h, static_cast<double>(PrBits<T>::from(c)));
             else
                 red_add(a.res + y, PrBits<T>::from(c));
         }
@@ -232,27 +243,43 @@ struct PrSweepOp {
     }
 };
 
-// v's residual while others add to it: true when it is above epsilon.
+// v's residual while others add to it.
 template <class T>
-__device__ __forceinline__ bool res_above(const PrArrays<T> &a, uint32_t v, int32_t h, T eps, bool &finite) {
-    if (h >= 0) {
-        const double r = __ldcg(a.res_hub + h);
-        finite = isfinite(r);
-        return fabs(r) > static_cast<double>(eps);
-    }
-    const T r = __ldcg(a.res + v);
-    finite = pr_finite(r);
-    return pr_abs(r) > eps;
+__device__ __forceinline__ double res_look(const PrArrays<T> &a, uint32_t v, int32_t h) {
+    if (h < 0) return static_cast<double>(__ldcg(a.res + v));
+    double r = __ldcg(a.res_hub + h);
+#pragma unroll
+    for (uint32_t c = 0; c + 1 < kHubCopies; ++c) r += __ldcg(a.hub_more + static_cast<uint64_t>(c) * a.hubs + h);
+    return r;
 }
 
 // Take it, leaving zero.
 template <class T>
 __device__ __forceinline__ double res_exchange(const PrArrays<T> &a, uint32_t v, int32_t h) {
-    if (h >= 0)
-        return __longlong_as_double(
-            static_cast<long long>(atomicExch(reinterpret_cast<unsigned long long *>(a.res_hub + h), 0ull)));
     using B = typename PrBits<T>::type;
-    return static_cast<double>(PrBits<T>::from(atomicExch(reinterpret_cast<B *>(a.res + v), B{0})));
+    if (h < 0) return static_cast<double>(PrBits<T>::from(atomicExch(reinterpret_cast<B *>(a.res + v), B{0})));
+    auto take = [](double *p) {
+        return __longlong_as_double(static_cast<long long>(atomicExch(reinterpret_cast<unsigned long long *>(p), 0ull)));
+    };
+    double r = take(a.res_hub + h);
+#pragma unroll
+    for (uint32_t c = 0; c + 1 < kHubCopies; ++c) r += take(a.hub_more + static_cast<uint64_t>(c) * a.hubs + h);
+    return r;
+}
+
+// After the sweeps: what is left in the copies joins the hubs' own slots.
+template <class T>
+__device__ __forceinline__ void fold_hub_copies(const PrArrays<T> &a) {
+    if (!a.hub_more) return;
+    for (uint32_t h = blockIdx.x * blockDim.x + threadIdx.x; h < a.hubs; h += gridDim.x * blockDim.x) {
+        double r = __ldcg(a.res_hub + h);
+        for (uint32_t c = 0; c + 1 < kHubCopies; ++c) {
+            double *p = a.hub_more + static_cast<uint64_t>(c) * a.hubs + h;
+            r += __ldcg(p);
+            *p = 0.0;
+        }
+        a.res_hub[h] = r;
+    }
 }
 
 // An FP64 residual enters an FP32 rank as two compensated adds (its float
@@ -295,8 +322,10 @@ constexpr uint32_t kPrSweepShare = 16;
 // the whole grid after a barrier, in sweeps that have any.  (With block-wide
 // rows inside the sweep nearly half of all warp time was spent at block
 // barriers.)  Tiles shrink with n so that every warp gets a few.
-// `act` and `ch.cnt`: three counters each (sweep s uses s mod 3, clears
-// (s+1) mod 3, which was last read before the previous barrier).
+// (Tiles handed out by a counter instead: no faster at 262k vertices, a fifth
+// slower at 50k.)
+// `act` (vertices consumed) and `ch.cnt`: three counters each (sweep s uses s
+// mod 3, clears (s+1) mod 3, which was last read before the previous barrier).
 // Returns false on a barrier error; `done` tells whether it converged.
 template <class T>
 __device__ __forceinline__ bool pr_sweeps(const AdjView &fwd, const PrArrays<T> &a, T eps, uint32_t n,
@@ -323,31 +352,41 @@ __device__ __forceinline__ bool pr_sweeps(const AdjView &fwd, const PrArrays<T> 
         }
         uint32_t *ch_cnt = ch.cnt + sweeps % 3;
         uint32_t mine = 0;
-        for (uint64_t base = static_cast<uint64_t>(wid) * tile; base < n; base += static_cast<uint64_t>(warps) * tile) {
-            const uint32_t v = static_cast<uint32_t>(base) + lane;
-            const bool in = lane < tile && v < n && v >= static_cast<uint32_t>(base);
-            bool has = false;
+        // The next tile's residuals are read while this one's rows are pushed.
+        int32_t h_next = -1;
+        double r_next = 0.0;
+        auto look = [&](uint64_t t) {
+            const uint64_t at = t * tile + lane;
+            r_next = 0.0;
+            if (lane < tile && at < n) {
+                h_next = hub_slot(a, static_cast<uint32_t>(at));
+                r_next = res_look(a, static_cast<uint32_t>(at), h_next);
+            }
+        };
+        look(wid);
+        for (uint64_t t = wid; t * tile < n; t += warps) {
+            const uint32_t v = static_cast<uint32_t>(t * tile + lane);
+            const int32_t h = h_next;
+            const double seen = r_next;
+            look(t + warps);
             uint32_t deg = 0;
             uint64_t off = 0;
             T c = T(0);
-            if (in) {
-                const int32_t h = hub_slot(a, v);
-                bool finite = true;
-                has = res_above(a, v, h, eps, finite);
-                if (!finite) set_error(st, kErrNonFinite, v);
+            if (!isfinite(seen)) set_error(st, kErrNonFinite, v);
+            // (the threshold in the precision the residual is stored in)
+            bool has = h >= 0 ? fabs(seen) > static_cast<double>(eps) : pr_abs(static_cast<T>(seen)) > eps;
+            if (has) {
+                const RowDesc d = fwd.desc[v];
+                ++mine;
+                c = rank_consume(a, v, res_exchange(a, v, h), rd_live(d));
+                deg = d.len;
+                off = d.off;
+                has = deg > 0 && c != T(0);
                 if (has) {
-                    const RowDesc d = fwd.desc[v];
-                    ++mine;
-                    c = rank_consume(a, v, res_exchange(a, v, h), rd_live(d));
-                    deg = d.len;
-                    off = d.off;
-                    has = deg > 0 && c != T(0);
-                    if (has) {
-                        cnt.rows += 1;
-                        cnt.edges += deg;
-                        if (fwd.cached(off)) cnt.edges_cached += deg;
-                        if (seg_hot && sweeps == 0) atomicAdd(seg_hot + (off >> kSegShift), deg);
-                    }
+                    cnt.rows += 1;
+                    cnt.edges += deg;
+                    if (fwd.cached(off)) cnt.edges_cached += deg;
+                    if (seg_hot && sweeps == 0) atomicAdd(seg_hot + (off >> kSegShift), deg);
                 }
             }
             uint32_t bigs = __ballot_sync(kFull, has && deg >= kPrChunk);
@@ -414,6 +453,7 @@ __global__ void __launch_bounds__(kTpbPr, 4) pr_converge(AdjView fwd, PrArrays<T
                 a.queued[__ldcg(in + i)] = 0u;
             bool done = false;
             if (!pr_sweeps(fwd, a, eps, n, max_rounds - r, ch, act, seg_hot, sm.sweeps, cnt, sweeps, done, st)) break;
+            fold_hub_copies(a);
             // The pending queue: empty, or (round bound) rebuilt in q0.
             if (blockIdx.x == 0 && threadIdx.x < 3) a.cnt[threadIdx.x] = 0;
             if (!done) {
