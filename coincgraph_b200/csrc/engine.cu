@@ -183,6 +183,14 @@ __global__ void set_single(uint32_t *q, uint32_t *cnt, uint32_t value) {
     cnt[2] = 0;
 }
 
+// The four arrays of a batch one after the other (cig_handle::place_updates).
+__global__ void pack_updates(const uint32_t *du, const uint32_t *dv, uint64_t nd, const uint32_t *au,
+                             const uint32_t *av, uint64_t na, uint32_t *out) {
+    for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < 2 * (nd + na);
+         i += static_cast<uint64_t>(gridDim.x) * blockDim.x)
+        out[i] = i < nd ? du[i] : i < 2 * nd ? dv[i - nd] : i < 2 * nd + na ? au[i - 2 * nd] : av[i - 2 * nd - na];
+}
+
 enum SmallIdx : int {
     kFr = 0,        // 3 frontier counters
     kAff = 3,       // 3 affected-list counters
@@ -339,6 +347,7 @@ struct cig_handle {
     TagState *tags = nullptr;
     Status *status = nullptr;
     Status *h_status = nullptr;
+    double *h_residual = nullptr;  // PageRank: FP64 L1 residual, behind h_status in one pinned block
     uint32_t epoch = 0;
 
     void *pr_rank = nullptr, *pr_res = nullptr, *pr_contrib = nullptr, *pr_amend = nullptr;
@@ -347,13 +356,25 @@ struct cig_handle {
     uint32_t pr_hubs = 0;
     double *pr_res_hub = nullptr, *pr_hub_more = nullptr;
     float *pr_comp = nullptr;
+    uint8_t *pr_export_buf[4] = {};  // FP32 rank, residual, FP64 rank, residual (allocated by the first get_pr)
     BigRow *pr_chunks = nullptr;  // the sweeps' chunks of long rows (pr_chunk_cap entries)
     uint64_t pr_chunk_cap() const { return 2 * fwd.seg_total * (kSegEdges / kPrChunk); }
     uint32_t *pr_queued = nullptr;
     bool pr64 = false;
 
     uint64_t bcap = 0;
+    // The batch's update arrays, packed one after the other in `upd` (4 * bcap
+    // words) by place_updates, so that staged host arrays take one copy.  Their
+    // addresses depend only on the batch's shape, which a captured graph's key
+    // holds.
+    uint32_t *upd = nullptr;
     uint32_t *du = nullptr, *dv = nullptr, *au = nullptr, *av = nullptr;
+    void place_updates(uint64_t nd, uint64_t na) {
+        du = upd;
+        dv = upd + nd;
+        au = upd + 2 * nd;
+        av = upd + 2 * nd + na;
+    }
     unsigned long long *kf = nullptr, *kr = nullptr, *t1 = nullptr, *t2 = nullptr;
     uint32_t *gf = nullptr, *gr = nullptr, *mf = nullptr, *mr = nullptr, *bigf = nullptr, *bigr = nullptr;
     unsigned long long *pf = nullptr, *prr = nullptr;
@@ -736,7 +757,12 @@ struct cig_handle {
     bool capturing = false;
     uint64_t graph_gen = 1, graph_clock = 0;
     uint64_t graph_replays = 0, graph_captures = 0;
-    static constexpr size_t kMaxGraphs = 8;
+    // A stream that cycles through a few batch sizes holds three graphs per
+    // size; with 8 slots six sizes evicted one another, and every batch was
+    // captured and instantiated again (5.0 ms for six batches, 2.1 ms of it on
+    // the device).
+    static constexpr size_t kMaxGraphs = 64;
+    static constexpr size_t kMaxShapes = 256;  // shapes remembered from their first sighting
 
     static void release_graph(BatchGraph &g) {
         if (g.exec) cudaGraphExecDestroy(g.exec);
@@ -771,7 +797,7 @@ struct cig_handle {
         }
         const std::pair<int, std::pair<uint64_t, uint64_t>> shape{kind, {nd, na}};
         if (std::find(shapes_seen.begin(), shapes_seen.end(), shape) == shapes_seen.end()) {
-            if (shapes_seen.size() >= 64) shapes_seen.erase(shapes_seen.begin());
+            if (shapes_seen.size() >= kMaxShapes) shapes_seen.erase(shapes_seen.begin());
             shapes_seen.push_back(shape);
             body();
             return;
@@ -861,9 +887,12 @@ struct cig_handle {
 
     // Synchronise, read the device status, raise on device-reported errors.
     void finish() {
+        // The status word is queued behind the work: one wait, not two.
+        CK(cudaMemcpyAsync(h_status, status, sizeof(Status), cudaMemcpyDeviceToHost, stream));
+        if (opt.algo == CIG_PR)
+            CK(cudaMemcpyAsync(h_residual, small64, sizeof(double), cudaMemcpyDeviceToHost, stream));
         CK(cudaStreamSynchronize(stream));
         CK(cudaGetLastError());
-        CK(cudaMemcpy(h_status, status, sizeof(Status), cudaMemcpyDeviceToHost));
         prof_resolve();
         const uint32_t e = h_status->err;
         if (e) {
@@ -917,7 +946,8 @@ struct cig_handle {
         for (auto &e : ev) CK(cudaEventCreate(&e));
         dmalloc(status, 1);
         CK(cudaMemset(status, 0, sizeof(Status)));
-        CK(cudaHostAlloc(reinterpret_cast<void **>(&h_status), sizeof(Status), cudaHostAllocDefault));
+        CK(cudaHostAlloc(reinterpret_cast<void **>(&h_status), sizeof(Status) + sizeof(double), cudaHostAllocDefault));
+        h_residual = reinterpret_cast<double *>(h_status + 1);
         dmalloc(small, kSmallCount);
         CK(cudaMemset(small, 0, kSmallCount * sizeof(uint32_t)));
         dmalloc(small64, 4);
@@ -992,6 +1022,7 @@ struct cig_handle {
         dfree(pr_hub_more);
         dfree(pr_comp);
         dfree(pr_chunks);
+        for (auto &b : pr_export_buf) dfree(b);
         dfree(pr_queued);
         free_batch();
         dfree(tmp_u32);
@@ -1017,10 +1048,8 @@ struct cig_handle {
     }
 
     void free_batch() {
-        dfree(du);
-        dfree(dv);
-        dfree(au);
-        dfree(av);
+        dfree(upd);
+        du = dv = au = av = nullptr;
         dfree(kf);
         dfree(kr);
         dfree(t1);
@@ -1076,10 +1105,7 @@ struct cig_handle {
         CK(cudaStreamSynchronize(stream));
         free_batch();
         uint64_t cap = std::max<uint64_t>(need, std::max<uint64_t>(opt.max_batch, 1024));
-        dmalloc(du, cap);
-        dmalloc(dv, cap);
-        dmalloc(au, cap);
-        dmalloc(av, cap);
+        dmalloc(upd, 4 * cap);
         dmalloc(kf, cap);
         dmalloc(kr, cap);
         dmalloc(t1, cap);
@@ -2057,12 +2083,16 @@ struct cig_handle {
         if ((nd && (!hdu || !hdv)) || (na && (!hau || !hav))) throw CigError(CIG_ERR_ARG, "null update array");
         const uint32_t *src[4] = {hdu, hdv, hau, hav};
         const uint64_t cnt[4] = {nd, nd, na, na};
+        place_updates(nd, na);
         uint32_t *dev[4] = {du, dv, au, av};
-        // Caller arrays in page-locked host memory (cudaHostAlloc,
+        const uint64_t words = 2 * (nd + na);
+        if (!words) return;
+        // Larger caller arrays in page-locked host memory (cudaHostAlloc,
         // cudaHostRegister, a pinned torch tensor) are copied by DMA
         // straight from where they are; the call ends synchronised, so they
-        // may change again once it returns.
-        bool all_pinned = true;
+        // may change again once it returns.  Small ones are gathered like
+        // pageable ones: four copies cost more than moving 64 KiB.
+        bool all_pinned = words > (1u << 14);
         for (int a = 0; a < 4 && all_pinned; ++a) {
             if (!cnt[a]) continue;
             cudaPointerAttributes at{};
@@ -2079,22 +2109,19 @@ struct cig_handle {
                     CK(cudaMemcpyAsync(dev[a], src[a], cnt[a] * sizeof(uint32_t), cudaMemcpyHostToDevice, stream));
             return;
         }
-        uint32_t *dst[4] = {stage, stage + bcap, stage + 2 * bcap, stage + 3 * bcap};
         auto copy = [&](int part, int parts) {
             for (int a = 0; a < 4; ++a) {
                 const uint64_t q = (cnt[a] + parts - 1) / parts;
                 const uint64_t b = std::min<uint64_t>(cnt[a], static_cast<uint64_t>(part) * q);
                 const uint64_t e = std::min<uint64_t>(cnt[a], b + q);
-                if (e > b) std::memcpy(dst[a] + b, src[a] + b, (e - b) * sizeof(uint32_t));
+                if (e > b) std::memcpy(stage + (dev[a] - upd) + b, src[a] + b, (e - b) * sizeof(uint32_t));
             }
         };
         if (nd + na >= (1u << 16))
             stager_run([&](int part) { copy(part, stage_workers + 1); });
         else
             copy(0, 1);
-        for (int a = 0; a < 4; ++a)
-            if (cnt[a])
-                CK(cudaMemcpyAsync(dev[a], dst[a], cnt[a] * sizeof(uint32_t), cudaMemcpyHostToDevice, stream));
+        CK(cudaMemcpyAsync(upd, stage, words * sizeof(uint32_t), cudaMemcpyHostToDevice, stream));
     }
 
     void require_ready() {
@@ -2171,12 +2198,10 @@ struct cig_handle {
             run_cache_service();
             return;
         }
-        const uint32_t *src[4] = {d_du, d_dv, d_au, d_av};
-        uint32_t *dst[4] = {du, dv, au, av};
-        const uint64_t cnt[4] = {nd, nd, na, na};
-        for (int a = 0; a < 4; ++a)
-            if (cnt[a] && src[a] != dst[a])
-                CK(cudaMemcpyAsync(dst[a], src[a], cnt[a] * sizeof(uint32_t), cudaMemcpyDeviceToDevice, stream));
+        place_updates(nd, na);
+        if ((nd && d_du != du) || (na && d_au != au))
+            launch(pack_updates, std::min(grid_for(2 * (nd + na)), persistent_grid()), 256, d_du, d_dv, nd, d_au, d_av,
+                   na, upd);
         dispatch([&](auto tag) {
             constexpr int A = decltype(tag)::value;
             bool sorted = false;
@@ -2369,11 +2394,7 @@ struct cig_handle {
             s->ms_insert = elapsed(evs[1], evs[2]);
             s->ms_cache = elapsed(evs[2], evs[3]);
         }
-        if (opt.algo == CIG_PR) {
-            double l1 = 0;
-            cudaMemcpy(&l1, small64, sizeof(double), cudaMemcpyDeviceToHost);
-            s->pr_residual_l1 = l1;
-        }
+        if (opt.algo == CIG_PR) s->pr_residual_l1 = *h_residual;
         last_nd = nd;
         last_na = na;
     }
@@ -2393,12 +2414,17 @@ struct cig_handle {
     void get_pr(float *rank, float *res, double *rank64, double *res64) {
         require_ready();
         if (opt.algo != CIG_PR) throw CigError(CIG_ERR_ARG, "not a PageRank handle");
-        float *dr = nullptr, *ds = nullptr;
-        double *dr64 = nullptr, *ds64 = nullptr;
-        if (rank) dmalloc(dr, n);
-        if (res) dmalloc(ds, n);
-        if (rank64) dmalloc(dr64, n);
-        if (res64) dmalloc(ds64, n);
+        // Export buffers are kept for the next call: cudaMalloc and cudaFree
+        // synchronise the device.
+        auto buffer = [&](int i, bool want, size_t bytes) -> void * {
+            if (!want) return nullptr;
+            if (!pr_export_buf[i]) dmalloc(pr_export_buf[i], bytes);
+            return pr_export_buf[i];
+        };
+        float *dr = static_cast<float *>(buffer(0, rank, n * sizeof(float)));
+        float *ds = static_cast<float *>(buffer(1, res, n * sizeof(float)));
+        double *dr64 = static_cast<double *>(buffer(2, rank64, n * sizeof(double)));
+        double *ds64 = static_cast<double *>(buffer(3, res64, n * sizeof(double)));
         if (pr64)
             launch(pr_export<double>, persistent_grid(), 256, pr_arrays<double>(), n, dr, ds, dr64, ds64);
         else
@@ -2409,10 +2435,6 @@ struct cig_handle {
         if (rank64) CK(cudaMemcpyAsync(rank64, dr64, n * sizeof(double), cudaMemcpyDeviceToHost, stream));
         if (res64) CK(cudaMemcpyAsync(res64, ds64, n * sizeof(double), cudaMemcpyDeviceToHost, stream));
         CK(cudaStreamSynchronize(stream));
-        dfree(dr);
-        dfree(ds);
-        dfree(dr64);
-        dfree(ds64);
     }
 
     uint64_t digest() {
@@ -2984,6 +3006,8 @@ struct cig_handle {
             if (opt.algo == CIG_PR) {
                 const uint64_t es = pr64 ? sizeof(double) : sizeof(float);
                 vs += 2 * nn * es + (nn + 1) * es + 2 * nn * sizeof(uint32_t) + pr_chunk_cap() * sizeof(BigRow);
+                for (int i = 0; i < 4; ++i)
+                    if (pr_export_buf[i]) vs += nn * (i < 2 ? sizeof(float) : sizeof(double));
                 if (!pr64) vs += nn * sizeof(float) + nn * sizeof(double) + 2 * w * sizeof(uint32_t) +
                                  std::max<uint32_t>(pr_hubs, 1) * kHubCopies * sizeof(double);
             } else {
