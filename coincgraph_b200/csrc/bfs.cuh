@@ -309,14 +309,28 @@ __device__ __forceinline__ uint32_t bfs_bottom_up(const BfsPull &pl, uint32_t n,
             }
         }
     }
-    for (uint64_t base = static_cast<uint64_t>(wid) * 32u; base < n; base += static_cast<uint64_t>(warps) * 32u) {
-        const uint32_t v = static_cast<uint32_t>(base) + lane;
-        const bool mine = v < n && !((pl.bigbits[base >> 5] >> lane) & 1u);
-        const unsigned long long vis = mine ? __ldcg(visit + v) : full;
+    // The next tile's masks and descriptors are read while this one's rows are
+    // gathered.
+    const uint32_t words = (n + 31u) / 32u;
+    bool mine_next = false;
+    unsigned long long vis_next = full;
+    RowDesc d_next{0, 0, 0};
+    auto look = [&](uint32_t w) {
+        const uint32_t v = 32u * w + lane;
+        mine_next = w < words && v < n && !((pl.bigbits[w] >> lane) & 1u);
+        vis_next = mine_next ? __ldcg(visit + v) : full;
+        d_next = mine_next ? pl.rev.desc[v] : RowDesc{0, 0, 0};
+    };
+    look(wid);
+    for (uint32_t w = wid; w < words; w += warps) {
+        const uint32_t v = 32u * w + lane;
+        const bool mine = mine_next;
+        const unsigned long long vis = vis_next;
         const unsigned long long missing = full & ~vis;
         unsigned long long acc = 0;
-        RowDesc d{0, 0, 0};
-        if (missing) d = pl.rev.desc[v];
+        RowDesc d = d_next;
+        look(w + warps < words ? w + warps : words);
+        if (!missing) d.len = 0;
         uint32_t read = 0;
         if (d.len) {
             acc = lane_gather(pl.rev, pl.rev.at(d.off), d.len, get);
@@ -607,11 +621,22 @@ __global__ void __launch_bounds__(kTpbMs, 4) bfs_one(AdjView fwd, uint32_t n, ui
             }
             auto get = [&](uint32_t u) { return static_cast<unsigned long long>((cur[u >> 5] >> (u & 31u)) & 1u); };
             uint32_t found = 0;
+            // The next words' vertices and descriptors are read while this
+            // one's rows are looked through.
+            uint32_t seen_next = 0xFFFFFFFFu;
+            RowDesc d_next{0, 0, 0};
+            auto look = [&](uint32_t w) {
+                seen_next = 0xFFFFFFFFu;
+                if (w < words) seen_next = __ldcg(vis + w);
+                const bool open = w < words && 32u * w + lane < n && !((seen_next >> lane) & 1u);
+                d_next = open ? pl.rev.desc[32u * w + lane] : RowDesc{0, 0, 0};
+            };
+            look(wid);
             for (uint32_t w = wid; w < words; w += warps) {
-                const uint32_t seen = __ldcg(vis + w);
+                const uint32_t seen = seen_next;
                 const uint32_t v = 32u * w + lane;
-                RowDesc d{0, 0, 0};
-                if (v < n && !((seen >> lane) & 1u)) d = pl.rev.desc[v];
+                const RowDesc d = d_next;
+                look(w + warps < words ? w + warps : words);
                 uint32_t read = 0;
                 unsigned long long hit = 0;
                 // Most vertices that have a parent in the frontier find one

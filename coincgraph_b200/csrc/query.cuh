@@ -127,8 +127,11 @@ __global__ void __launch_bounds__(kTpbMs, 4) ms_closure(AdjView fwd, uint32_t *d
 // a result.  With a queue in those rounds too, the appends' atomics on its one
 // counter and the wait for every mask's old value took most of the time
 // (2.9 ms for 13 sources on R-MAT s19, a tenth of the L2's throughput).
-constexpr uint32_t kMsChunk = 256;  // rows of at least this many entries are expanded by the whole grid
-constexpr int kMsGroup = 4;         // edges per lane whose loads are in flight together
+// Short chunks and three blocks per SM with two edges per lane in flight keep
+// the warps even: 13 sources on s19 take 1.37 ms with 256-entry chunks and four
+// edges in two blocks, 1.13 with 128 and 1.05 with 64 entries.
+constexpr uint32_t kMsChunk = 64;  // rows of at least this many entries are expanded by the whole grid
+constexpr int kMsGroup = 2;        // edges per lane whose loads are in flight together
 constexpr uint32_t kMsScan = 64;    // rounds after more than n / kMsScan improvements scan the masks
 
 // Chunks of long rows met in a round (three counters, as for the frontier),
@@ -154,8 +157,9 @@ struct MsWave {
     WarpBuf buf;
 
     // Relax 32 edges, one per lane (x -> y for the sources in m; m = 0: none).
-    // Rows are read through L1: a value lowered meanwhile only costs a
-    // relaxation that fails, or one that its vertex repeats next round.
+    // x's row is read through L1 (a value lowered meanwhile is relaxed again
+    // next round), y's from L2: a stale row of a hub costs an atomic for every
+    // source, all of them on one sector.
     __device__ __forceinline__ uint32_t relax(uint32_t x, uint32_t y, unsigned long long m) const {
         constexpr int kPer = 32 / LPE;                            // edges per step
         constexpr int N = LPE < kMsGroup ? LPE : kMsGroup;        // steps in flight
@@ -178,7 +182,7 @@ struct MsWave {
             for (int j = 0; j < N; ++j)
                 if (bits[j]) {
                     dx[j] = *reinterpret_cast<const uint4 *>(dist + xs[j] * kRow + 4u * quad);
-                    dy[j] = *reinterpret_cast<const uint4 *>(dist + ys[j] * kRow + 4u * quad);
+                    dy[j] = __ldcg(reinterpret_cast<const uint4 *>(dist + ys[j] * kRow + 4u * quad));
                 }
 #pragma unroll
             for (int j = 0; j < N; ++j) {
@@ -208,7 +212,7 @@ struct MsWave {
 };
 
 template <int A, int LPE>
-__global__ void __launch_bounds__(kTpbMs, 2) ms_wave(AdjView fwd, uint32_t n, uint32_t *dist, MsFrontier fr,
+__global__ void __launch_bounds__(kTpbMs, 3) ms_wave(AdjView fwd, uint32_t n, uint32_t *dist, MsFrontier fr,
                                                      MsChunks ch, uint32_t max_rounds, Status *st) {
     __shared__ uint32_t s_scan[kTpbMs];
     __shared__ uint32_t s_x[kTpbMs];
