@@ -232,18 +232,18 @@ SEG_BYTES = 65536
 
 # Kernels of each profiler stage (the stage time covers all of them).
 STAGE_KERNELS = {
-    "group": "make_keys_batch + CUB radix sort + unpack_keys_batch + scan + group_scatter_batch",
-    "mutate": "del_classify, del_chunk_map, del_scan, del_index, del_apply, del_finish, mutate_delete(_big), "
-              "compact_rows (forward rows)",
+    "group": "make_keys_batch + CUB radix sort + unpack_keys_batch + scan + group_scatter_batch, or small_batch",
+    "mutate": "del_lane, del_wide, del_rest (forward rows; without a full position index del_classify, "
+              "del_chunk_map, del_scan, del_index, del_apply, del_finish, mutate_delete(_big), compact_rows)",
     "mutate_rev": "the same on the reverse rows",
-    "del_scan": "del_scan + del_index (inside mutate and mutate_rev)",
-    "seed": "seed_deletions, seed_insertions",
-    "inval": "inval_closure",
-    "pull": "reset_affected, pull_repair, pull_deferred, enqueue_affected",
-    "push": "push_closure",
-    "add": "plan_add, alloc_classes, seg_assign_new, mutate_add, mutate_add_big (forward rows)",
+    "del_scan": "del_lane + del_wide, or del_scan + del_index (inside mutate and mutate_rev)",
+    "seed": "the seed parts of repair_closure and push_closure",
+    "inval": "the invalidation rounds of repair_closure",
+    "pull": "the pull repair of repair_closure",
+    "push": "the rounds of push_closure",
+    "add": "plan_add, mutate_add, mutate_add_wide (forward rows)",
     "add_rev": "the same on the reverse rows",
-    "cache": "seg_rescore, seg_plan, seg_pick, seg_evict, seg_admit",
+    "cache": "seg_service",
 }
 
 # ncu DRAM bytes (read + write) per algorithmic HBM byte, measured on a
@@ -253,7 +253,7 @@ STAGE_KERNELS = {
 TRAFFIC_RATIO = {
     "push_closure": (6.58, "ncu capture of push_closure, SSSP R-MAT s22 cache 4 GiB, 100k+100k batch, "
                            "22.8 MB DRAM against 3.46 MB algorithmic"),
-    "inval_closure": (5.97, "ncu capture of inval_closure, SSSP R-MAT s22 cache 4 GiB, 100k+100k batch, "
+    "repair_closure": (5.97, "ncu capture of the invalidation rounds as a kernel of their own, SSSP R-MAT s22 cache 4 GiB, 100k+100k batch, "
                             "14.2 MB DRAM against 2.38 MB algorithmic"),
 }
 
@@ -546,12 +546,12 @@ def run_ours(args):
     stages = {n: stage_roofline(n, prof[n], hbm_peak, link_peak, nprof) for n in STAGE_KERNELS}
     stages = {n: v for n, v in stages.items() if v}
     # The dominant kernel: of the stages that are one kernel each (push:
-    # push_closure, inval: inval_closure), the one with the most time; they
+    # push_closure, inval: repair_closure), the one with the most time; they
     # are also the two largest single launches of the batch in an ncu launch
     # list of this workload.  The other stages are chains of 2-10 kernels,
     # and those of the two arenas overlap on two streams.
     dominant = max((n for n in ("push", "inval") if n in stages), key=lambda n: stages[n]["ms_per_batch"])
-    main_kernel = {"push": "push_closure", "inval": "inval_closure"}[dominant]
+    main_kernel = {"push": "push_closure", "inval": "repair_closure"}[dominant]
     rf = stages[dominant]
     hbm_launch = rf["hbm_bytes_per_batch"] * nprof / max(prof[dominant]["launches"], 1)
     ratio = TRAFFIC_RATIO.get(main_kernel)
