@@ -214,7 +214,7 @@ enum SmallIdx : int {
     kCompactCountR = 24,
     kOrderedCountR = 25,
     kIndexedCountR = 26,
-    kCoopF = 27,  // addition groups left to mutate_add_warp, per arena
+    kCoopF = 27,  // deletion groups served by a warp, per arena
     kCoopR = 28,
     kHugeF = 29,  // hub deletion groups served by the whole grid, per arena
     kHugeR = 30,
