@@ -141,8 +141,16 @@ __device__ __forceinline__ void copy_segment(uint4 *dst, const uint4 *src) {
 __global__ void __launch_bounds__(256) seg_service(SegTable t, uint32_t bump, uint32_t *cache, uint32_t *host,
                                                    Status *st) {
     __shared__ uint32_t hist[kScoreBuckets];
-    __shared__ uint32_t s_reserve, s_need, s_thr, s_extra;
+    __shared__ uint32_t s_top, s_reserve, s_need, s_thr, s_extra;
     __shared__ int32_t slot_s;
+    // Every block makes the plan below for itself, so its inputs are read
+    // before the first barrier: behind it a block with nothing to evict goes
+    // straight to the admissions, which take from kCtlFreeTop, and a later
+    // reader would plan an eviction and wait at a barrier the others skip.
+    if (threadIdx.x == 0) {
+        s_top = ld_volatile(t.ctl + kCtlFreeTop);
+        s_reserve = min(1024u, max(16u, 2u * ld_volatile(t.ctl + kCtlNewLast)));
+    }
     const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, gthreads = gridDim.x * blockDim.x;
     for (uint32_t b = threadIdx.x; b < kScoreBuckets; b += blockDim.x) hist[b] = 0;
     __syncthreads();
@@ -164,9 +172,8 @@ __global__ void __launch_bounds__(256) seg_service(SegTable t, uint32_t bump, ui
     if (!grid_barrier(st)) return;
     const uint32_t na = min(ld_volatile(t.ctl + kCtlAdmits), kMaxAdmit);
     if (threadIdx.x == 0) {  // every block comes to the same plan
-        const uint32_t reserve = min(1024u, max(16u, 2u * ld_volatile(t.ctl + kCtlNewLast)));
-        const uint32_t want = reserve + na;
-        const uint32_t top = ld_volatile(t.ctl + kCtlFreeTop);
+        const uint32_t want = s_reserve + na;
+        const uint32_t top = s_top;
         uint32_t need = min(want > top ? want - top : 0u, kMaxEvict);
         uint32_t below = 0, b = 0;
         if (need)
@@ -176,7 +183,6 @@ __global__ void __launch_bounds__(256) seg_service(SegTable t, uint32_t bump, ui
                 below += c;
             }
         if (b == static_cast<uint32_t>(kScoreBuckets)) need = below;  // fewer evictable segments than wanted
-        s_reserve = reserve;
         s_need = need;
         s_thr = b;
         s_extra = need - below;

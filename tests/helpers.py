@@ -184,6 +184,28 @@ def recurring_case() -> Case:
     return Case("recurring", n, xadj, adj, batches, source=0)
 
 
+def admission_case() -> Case:
+    """248 neighbours of the source with rows of 16,384 entries (one 64 KiB
+    segment each) or 8,192.  Batch 0 appends to the 48 shorter rows, so that
+    each moves to a segment of its own; the batches after it only delete and
+    insert edges of the source, whose subtrees then read the long rows
+    again: no new segments."""
+    rng = np.random.default_rng(41)
+    n = 40000
+    hubs = np.arange(1, 249)
+    sizes = np.where(hubs <= 200, 16384, 8192)
+    src = np.concatenate([np.zeros(len(hubs), np.int64), np.repeat(hubs, sizes)])
+    dst = np.concatenate([hubs, rng.integers(249, n, int(sizes.sum()))])
+    xadj, adj = _csr_from_edges(n, src, dst)
+    short = _u32(hubs[200:])
+    batches = [(_u32([]), _u32([]), short, _u32(rng.integers(249, n, len(short))))]
+    for k in range(3):
+        gone = _u32(hubs[60 * k:60 * k + 60])
+        back = _u32(hubs[60 * (k - 1):60 * k]) if k else _u32([])
+        batches.append((np.zeros_like(gone), gone, np.zeros_like(back), back))
+    return Case("admission", n, xadj, adj, batches, source=0)
+
+
 def grid_case(side: int = 48, batches: int = 3, size: int = 150) -> Case:
     """Road-like high-diameter case: a side x side grid, local insertions."""
     g = gen.grid(side)

@@ -13,7 +13,7 @@ import pytest
 
 import oracle
 from coincgraph_b200 import Engine
-from helpers import (ORACLE_MODE, adversarial_case, big_row_case, full_row_case, grid_case, heavy_delete_case,
+from helpers import (ORACLE_MODE, admission_case, adversarial_case, big_row_case, full_row_case, grid_case, heavy_delete_case,
                      make_engine, oracle_trace, recurring_case, rmat_case)
 
 pytestmark = pytest.mark.gpu
@@ -116,13 +116,13 @@ def test_whole_batch_equals_phases(algo):
             assert a.digest() == b.digest()
 
 
-def run_case_whole_batches(case, algo, cache_gib):
+def run_case_whole_batches(case, algo, cache_gib, **options):
     """Batches through cig_apply_batch (one key sort for the whole batch and
     the per-batch segment-table service); values and rows after every batch."""
     trace, _ = oracle_trace(case, algo)
     g = oracle.Graph(case.n, case.xadj, case.adj)
     stats = []
-    with make_engine(algo, source=case.source, cache_gib=cache_gib) as eng:
+    with make_engine(algo, source=case.source, cache_gib=cache_gib, **options) as eng:
         eng.load_csr(case.n, case.xadj, case.adj)
         eng.init()
         for i, (du, dv, au, av) in enumerate(case.batches):
@@ -166,6 +166,19 @@ def test_segment_table_churn(algo, monkeypatch):
     stats = run_case_whole_batches(rmat_case(14, 6, 2000, 2000, seed_offset=15), algo, 8 * ONE_SEGMENT_GIB)
     assert sum(s["cache_segments_evicted"] for s in stats) > 0
     assert sum(s["cache_segments_loaded"] for s in stats) > 0
+
+
+def test_admissions_without_evictions(monkeypatch):
+    """Batch 0 makes 48 segments, so its service leaves 96 slots free; the
+    batches after it make none (16 slots in reserve) and read more than 64
+    segments from host memory: their services admit up to 64 segments (the
+    limit per batch) into the free slots and evict nothing.  All blocks have
+    to take that branch together, whenever they read the free-slot counter."""
+    monkeypatch.setenv("CIG_CACHE_ADMIT_SCORE", "1")
+    stats = run_case_whole_batches(admission_case(), "bfs", 150 * ONE_SEGMENT_GIB, headroom_pct=50)
+    assert stats[0]["cache_segments_evicted"] > 0
+    # 96 free slots, 16 of them in reserve.
+    assert stats[1]["cache_segments_evicted"] == 0 and 0 < stats[1]["cache_segments_loaded"] <= 64
 
 
 @pytest.mark.parametrize("small_pct", [None, 0, 50, 100])
