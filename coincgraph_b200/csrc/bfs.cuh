@@ -53,8 +53,8 @@ struct BfsPull {
     uint32_t edges_on;
     BigRow *tasks;              // off, len, x = vertex, payload = chunks of the row << 32 | row's place in acc
     uint32_t task_cap;
-    unsigned long long *acc;    // zero between rounds
-    uint32_t *arrived;          // zero between rounds
+    unsigned long long *acc;    // cleared with the list, left zero by each round
+    uint32_t *arrived;          // cleared with the list, left zero by each round
     uint32_t *bigbits;          // bit v: v's in-row is in `tasks`
     uint32_t *ctl;              // BfsCtl, zero at launch
 };
@@ -201,7 +201,10 @@ __device__ __forceinline__ void groups_gather(const AdjView &rev, uint32_t mask,
     }
 }
 
-// List the chunks of the long in-rows and mark their vertices.
+// List the chunks of the long in-rows and mark their vertices.  A row's place
+// in `acc` and `arrived` is cleared when it is handed out, once per wave: what
+// a wave that ended in an error left there, or what the memory held before,
+// must not count as chunks that have arrived.  A grid barrier follows.
 __device__ __forceinline__ void bfs_list_tasks(const BfsPull &pl, uint32_t n, Status *st) {
     const uint32_t lane = lane_id();
     const uint32_t rounded = (n + 31u) & ~31u;
@@ -225,6 +228,8 @@ __device__ __forceinline__ void bfs_list_tasks(const BfsPull &pl, uint32_t n, St
             if (lane == 0) {
                 at = atomicAdd(pl.ctl + kBfsTasks, chunks);
                 row = atomicAdd(pl.ctl + kBfsBigRows, 1u);
+                pl.acc[row] = 0ull;
+                pl.arrived[row] = 0u;
                 if (at + chunks > pl.task_cap) set_error(st, kErrQueue, at);
             }
             at = __shfl_sync(kFull, at, 0);

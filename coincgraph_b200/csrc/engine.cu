@@ -2512,9 +2512,7 @@ struct cig_handle {
         if (rev.desc) {
             dmalloc(bfs_tasks, 2 * bfs_rows_cap());
             dmalloc(bfs_acc, bfs_rows_cap());
-            CK(cudaMemset(bfs_acc, 0, bfs_rows_cap() * sizeof(unsigned long long)));
             dmalloc(bfs_arrived, bfs_rows_cap());
-            CK(cudaMemset(bfs_arrived, 0, bfs_rows_cap() * sizeof(uint32_t)));
             dmalloc(bfs_bigbits, (n + 31) / 32);
         }
         dmalloc(ms_src, kMsWidth);

@@ -147,3 +147,26 @@ def test_sssp_wave_widths(built, k):
         got = eng.query_sssp(src)
     for j in range(k):
         np.testing.assert_array_equal(got[j], og.sssp(j, oracle.SSSP))
+
+
+def test_bfs_wave_on_used_device_memory(built):
+    """Long in-rows gathered by several warps, in buffers of a new handle that
+    the memory of this process's earlier allocations serves (all bits set):
+    the waves clear what they count in."""
+    import torch
+
+    case = big_row_case()  # vertex 5 has 6,000 in-edges: six chunks
+    og = oracle.Graph(case.n, case.xadj, case.adj)
+    src = np.concatenate([[0, 1], np.arange(7000, 7062)]).astype(np.uint32)  # 5 is two steps from 1
+    ref = np.stack([og.sssp(int(s), oracle.BFS) for s in src])
+    for _ in range(2):
+        used = [torch.full((size // 4,), -1, dtype=torch.int32, device="cuda")
+                for size in (4096, 1 << 16, 1 << 20, 1 << 24, 1 << 28) for _ in range(16)]
+        torch.cuda.synchronize()
+        del used
+        torch.cuda.empty_cache()
+        with Engine("bfs", cache_gib=1.0) as eng:
+            eng.load_csr(case.n, case.xadj, case.adj)
+            eng.init()
+            for k in (64, 5, 64):
+                np.testing.assert_array_equal(eng.query_bfs(src[:k]), ref[:k])
