@@ -86,7 +86,18 @@ struct MsBfsOp {
     }
 };
 
-// Depth `level` for the sources in m at vertex v (one thread per vertex).
+// Depth `level` for the sources in m at vertex v (one thread per vertex), as
+// ORs without a result: each waits for nothing, where a load, an OR and a
+// store per set bit of the level followed one another (five of them a round
+// at depth 800).
+__device__ __forceinline__ void planes_put(unsigned long long *planes, uint32_t n, uint32_t v, uint32_t level,
+                                           unsigned long long m) {
+    for (uint32_t b = level; b; b &= b - 1)
+        red_or(planes + static_cast<uint64_t>(__ffs(static_cast<int>(b)) - 1) * n + v, m);
+}
+
+// The same where a warp's vertices follow one another (bottom-up rounds): the
+// loads and stores of the warp are whole lines.
 __device__ __forceinline__ void planes_record(unsigned long long *planes, uint32_t n, uint32_t v, uint32_t level,
                                               unsigned long long m) {
     for (uint32_t b = level; b; b &= b - 1)
@@ -256,18 +267,15 @@ __device__ __forceinline__ void block_add(uint32_t *counter, uint32_t mine, uint
 
 // Does a top-down round over the queue hold more than pl.edges_on row
 // entries?  Looked at for queues of kBfsCount vertices and more (below, a
-// round is short anyway); one barrier, after which every block agrees.
-// `ok` false: barrier error.
+// round is short anyway).  The sum is made while the vertices are queued
+// (WarpBuf), so that the round's own barrier covers it: a counting pass with a
+// barrier of its own in every round cost a fifth to two fifths on graphs of
+// many short rounds (a 511 x 511 grid, 678 to 841 rounds: one source 6.0 ->
+// 7.4 ms, two 7.6 -> 10.7 ms), where no round can pass the limit.
+// `edges`: the sum, read together with the round's vertex count.
 constexpr uint32_t kBfsCount = 256;
-__device__ __forceinline__ bool bfs_many_edges(const BfsPull &pl, const RowDesc *desc, const uint32_t *in,
-                                               uint32_t n_in, uint32_t r, uint32_t *shared, bool &ok, Status *st) {
-    if (!pl.rev.desc || n_in < kBfsCount) return false;
-    uint32_t mine = 0;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_in; i += gridDim.x * blockDim.x)
-        mine += min(desc[__ldcg(in + i)].len, 1u << 20);
-    block_add(pl.ctl + kBfsEdges + r % 3, mine, shared);
-    ok = grid_barrier(st);
-    return ld_volatile(pl.ctl + kBfsEdges + r % 3) > pl.edges_on;
+__device__ __forceinline__ bool bfs_many_edges(const BfsPull &pl, uint32_t n_in, uint32_t edges) {
+    return pl.rev.desc && n_in >= kBfsCount && edges > pl.edges_on;
 }
 
 // Bottom-up round of a wave: every vertex that misses source bits ORs the
@@ -377,7 +385,15 @@ __device__ __forceinline__ uint32_t bfs_bottom_up(const BfsPull &pl, uint32_t n,
 
 // One wave (cooperative launch).  Round r gives depth r + 1.  `full`: the
 // wave's source bits.  Planes 0..kBfsPlanes-1 are cleared before the launch.
-__global__ void __launch_bounds__(kTpbMs, 4) bfs_wave(AdjView fwd, uint32_t n, unsigned long long full,
+// PER_SM blocks per SM: a wave of few sources on a graph of many short rounds
+// waits for its barriers, whose arrivals are atomics on one counter, so up to
+// kBfsFew sources run two (511 x 511 grid, 2 / 5 / 13 sources: 7.0 / 8.1 / 9.9
+// ms against 8.7 / 9.9 / 11.8 with four); wider waves go bottom-up and need
+// the gathers in flight (R-MAT s20: 64 sources 0.49 ms against 0.58, 13
+// sources 0.35 against 0.39).
+constexpr uint32_t kBfsFew = 16;
+template <int PER_SM>
+__global__ void __launch_bounds__(kTpbMs, PER_SM) bfs_wave(AdjView fwd, uint32_t n, unsigned long long full,
                                                       unsigned long long *visit, unsigned long long *planes,
                                                       MsFrontier fr, BigList big, uint32_t max_rounds, BfsPull pl,
                                                       Status *st) {
@@ -395,6 +411,7 @@ __global__ void __launch_bounds__(kTpbMs, 4) bfs_wave(AdjView fwd, uint32_t n, u
     uint32_t r = 0;
     for (;; ++r) {
         const uint32_t n_in = ld_volatile(fr.cnt + (r % 3));
+        const uint32_t n_edges = ld_volatile(pl.ctl + kBfsEdges + r % 3);
         if (n_in == 0) break;
         if (r >= max_rounds) {
             if (gtid == 0) set_error(st, kErrRounds, r);
@@ -403,7 +420,7 @@ __global__ void __launch_bounds__(kTpbMs, 4) bfs_wave(AdjView fwd, uint32_t n, u
         if (gtid == 0) {
             fr.cnt[(r + 2) % 3] = 0;
             big.cnt[(r + 2) % 3] = 0;
-            pl.ctl[kBfsEdges + (r + 1) % 3] = 0;
+            pl.ctl[kBfsEdges + (r + 2) % 3] = 0;
         }
         uint32_t *in = (r & 1) ? fr.q1 : fr.q0;
         uint32_t *out = (r & 1) ? fr.q0 : fr.q1;
@@ -418,17 +435,13 @@ __global__ void __launch_bounds__(kTpbMs, 4) bfs_wave(AdjView fwd, uint32_t n, u
         }
         was_pull = pull;
         pull = pl.rev.desc && n_in > (was_pull ? pl.off : pl.on);
-        if (!pull && !was_pull) {
-            bool ok = true;
-            pull = bfs_many_edges(pl, fwd.desc, in, n_in, r, &s_new, ok, st);
-            if (!ok) break;
-        }
+        if (!was_pull) pull = pull || bfs_many_edges(pl, n_in, n_edges);
         if (pull) {
             if (!was_pull) {
                 // The queued vertices are not popped: record their depth here.
                 for (uint32_t i = gtid; i < n_in; i += gthreads) {
                     const uint32_t x = __ldcg(in + i);
-                    planes_record(planes, n, x, r, __ldcg(m_in + x));
+                    planes_put(planes, n, x, r, __ldcg(m_in + x));
                 }
                 if (!listed) bfs_list_tasks(pl, n, st);
                 listed = true;
@@ -456,7 +469,9 @@ __global__ void __launch_bounds__(kTpbMs, 4) bfs_wave(AdjView fwd, uint32_t n, u
             if (gtid == 0) pl.ctl[kBfsFill] = 0;
         }
         const Defer df{big.rows, big.cnt + (r % 3), big.cap, big.split};
-        const MsBfsOp op{visit, m_out, WarpBuf{s_buf[threadIdx.x >> 5], s_held + (threadIdx.x >> 5), out, out_cnt, fr.cap, st}};
+        const MsBfsOp op{visit, m_out,
+                         WarpBuf{s_buf[threadIdx.x >> 5], s_held + (threadIdx.x >> 5), out, out_cnt, fr.cap, st,
+                                 pl.rev.desc ? fwd.desc : nullptr, pl.ctl + kBfsEdges + (r + 1) % 3}};
         for (uint32_t base = 0; base < n_in; base += gridDim.x * kTpbMs) {
             const uint32_t i = base + spread_rank<kTpbMs>() * gridDim.x + blockIdx.x;
             bool has = i < n_in;
@@ -467,9 +482,9 @@ __global__ void __launch_bounds__(kTpbMs, 4) bfs_wave(AdjView fwd, uint32_t n, u
                 x = __ldcg(in + i);
                 // Nobody writes m_in this round: take the bits and clear them.
                 m = __ldcg(m_in + x);
-                m_in[x] = 0ull;
-                planes_record(planes, n, x, r, m);
                 const RowDesc d = fwd.desc[x];
+                m_in[x] = 0ull;
+                planes_put(planes, n, x, r, m);
                 deg = d.len;
                 off = d.off;
                 has = m != 0ull && deg > 0;
@@ -573,8 +588,10 @@ __global__ void bfs_one_seed(const uint32_t *source, uint32_t *depth, uint32_t *
 
 // Single-source BFS (cooperative launch); `vis` cleared and `depth` filled
 // with kInf before it, `bm0` / `bm1` the frontier bitmaps of bottom-up rounds
-// ((n + 31) / 32 words each).
-__global__ void __launch_bounds__(kTpbMs, 4) bfs_one(AdjView fwd, uint32_t n, uint32_t *depth, uint32_t *vis,
+// ((n + 31) / 32 words each).  kBfsOnePerSm blocks per SM: see bfs_wave (the
+// grid 5.0 ms against 6.7 with four, R-MAT s20 the same).
+constexpr int kBfsOnePerSm = 2;
+__global__ void __launch_bounds__(kTpbMs, kBfsOnePerSm) bfs_one(AdjView fwd, uint32_t n, uint32_t *depth, uint32_t *vis,
                                                      uint32_t *bm0, uint32_t *bm1, MsFrontier fr, BigList big,
                                                      uint32_t max_rounds, BfsPull pl, Status *st) {
     __shared__ ExpandSmem<kTpbMs> sm;
@@ -592,6 +609,7 @@ __global__ void __launch_bounds__(kTpbMs, 4) bfs_one(AdjView fwd, uint32_t n, ui
     uint32_t r = 0;
     for (;; ++r) {
         const uint32_t n_in = ld_volatile(fr.cnt + (r % 3));
+        const uint32_t n_edges = ld_volatile(pl.ctl + kBfsEdges + r % 3);
         if (n_in == 0) break;
         if (r >= max_rounds) {
             if (gtid == 0) set_error(st, kErrRounds, r);
@@ -600,7 +618,7 @@ __global__ void __launch_bounds__(kTpbMs, 4) bfs_one(AdjView fwd, uint32_t n, ui
         if (gtid == 0) {
             fr.cnt[(r + 2) % 3] = 0;
             big.cnt[(r + 2) % 3] = 0;
-            pl.ctl[kBfsEdges + (r + 1) % 3] = 0;
+            pl.ctl[kBfsEdges + (r + 2) % 3] = 0;
         }
         uint32_t *in = (r & 1) ? fr.q1 : fr.q0;
         uint32_t *out = (r & 1) ? fr.q0 : fr.q1;
@@ -609,11 +627,7 @@ __global__ void __launch_bounds__(kTpbMs, 4) bfs_one(AdjView fwd, uint32_t n, ui
         uint32_t *next = (r & 1) ? bm0 : bm1;
         was_pull = pull;
         pull = pl.rev.desc && n_in > (was_pull ? pl.off : pl.on);
-        if (!pull && !was_pull) {
-            bool ok = true;
-            pull = bfs_many_edges(pl, fwd.desc, in, n_in, r, &s_new, ok, st);
-            if (!ok) break;
-        }
+        if (!was_pull) pull = pull || bfs_many_edges(pl, n_in, n_edges);
         if (pull) {
             if (!was_pull) {  // the queue as a bitmap
                 for (uint32_t w = gtid; w < words; w += gthreads) cur[w] = 0u;
@@ -695,7 +709,8 @@ __global__ void __launch_bounds__(kTpbMs, 4) bfs_one(AdjView fwd, uint32_t n, ui
         }
         const Defer df{big.rows, big.cnt + (r % 3), big.cap, big.split};
         const OneBfsOp op{vis, depth, r + 1,
-                          WarpBuf{s_buf[threadIdx.x >> 5], s_held + (threadIdx.x >> 5), out, out_cnt, fr.cap, st}};
+                          WarpBuf{s_buf[threadIdx.x >> 5], s_held + (threadIdx.x >> 5), out, out_cnt, fr.cap, st,
+                                  pl.rev.desc ? fwd.desc : nullptr, pl.ctl + kBfsEdges + (r + 1) % 3}};
         for (uint32_t base = 0; base < n_in; base += gridDim.x * kTpbMs) {
             const uint32_t i = base + spread_rank<kTpbMs>() * gridDim.x + blockIdx.x;
             bool has = i < n_in;

@@ -185,6 +185,11 @@ __device__ __forceinline__ void report_bounds(Status *st, uint64_t index) {
     if (st) set_error(st, kErrBounds, static_cast<uint32_t>(index));
 }
 
+// OR in memory without a result.
+__device__ __forceinline__ void red_or(unsigned long long *p, unsigned long long x) {
+    asm volatile("red.relaxed.gpu.global.or.b64 [%0], %1;" ::"l"(p), "l"(x) : "memory");
+}
+
 // Warp-aggregated append: one atomicAdd per warp.  All 32 lanes must call.
 __device__ __forceinline__ void warp_enqueue(bool want, uint32_t item, uint32_t *queue, uint32_t *count,
                                              uint32_t capacity, Status *st) {
@@ -209,6 +214,7 @@ __device__ __forceinline__ void warp_enqueue(bool want, uint32_t item, uint32_t 
 // warps' atomics on the queue's one counter were what the round waited for.
 // All 32 lanes call; flush() once at the end of the warp's work.
 constexpr uint32_t kWarpBuf = 96;
+constexpr uint32_t kCountRow = 16;
 struct WarpBuf {
     uint32_t *items;  // kWarpBuf words of this warp
     uint32_t *held;   // items in it
@@ -216,6 +222,11 @@ struct WarpBuf {
     uint32_t *count;
     uint32_t capacity;
     Status *st;
+    // Sum of the queued vertices' row lengths, rows of at least kCountRow
+    // entries (desc null: not wanted).  The descriptors are read while the
+    // append waits for its place; a warp without such rows adds nothing.
+    const RowDesc *desc = nullptr;
+    uint32_t *edges = nullptr;
 
     __device__ __forceinline__ void flush() const {
         __syncwarp();
@@ -223,6 +234,15 @@ struct WarpBuf {
         if (!c) return;
         uint32_t base = 0;
         if (lane_id() == 0) base = atomicAdd(count, c);
+        if (desc) {
+            uint32_t sum = 0;
+            for (uint32_t i = lane_id(); i < c; i += 32u) {
+                const uint32_t len = desc[items[i]].len;
+                if (len >= kCountRow) sum += min(len, 1u << 20);
+            }
+            sum = __reduce_add_sync(kFull, sum);
+            if (lane_id() == 0 && sum) atomicAdd(edges, sum);
+        }
         base = __shfl_sync(kFull, base, 0);
         for (uint32_t i = lane_id(); i < c; i += 32u) {
             if (base + i < capacity)

@@ -647,12 +647,12 @@ struct cig_handle {
     BigList big_list(int counter) const { return BigList{big_rows, small + counter, kBigRowCap, tune.split}; }
 
     template <class K>
-    int coop_blocks(K kernel, int tpb) const {
+    int coop_blocks(K kernel, int tpb, uint32_t limit = ~0u) const {
         int per_sm = 0;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, tpb, 0));
         uint32_t most = in_batch && tune.inc_per_sm ? tune.inc_per_sm : tune.per_sm;
         if (in_batch && batch_requests <= kNarrowBatch) most = std::min(most, 1u);
-        per_sm = std::min(per_sm, static_cast<int>(most));
+        per_sm = std::min(per_sm, static_cast<int>(std::min(most, limit)));
         if (per_sm < 1) throw CigError(CIG_ERR_DEVICE, "cooperative kernel does not fit on an SM");
         return per_sm * sms;
     }
@@ -718,10 +718,12 @@ struct cig_handle {
         ++n_launch;
     }
 
+    // At most per_sm blocks per SM.
     template <class... P>
-    void launch_coop_on(cudaStream_t st, void (*kernel)(P...), int tpb, typename Identity<P>::type... args) {
+    void launch_coop_on(cudaStream_t st, uint32_t per_sm, void (*kernel)(P...), int tpb,
+                        typename Identity<P>::type... args) {
         void *argv[] = {static_cast<void *>(&args)...};
-        const int blocks = coop_blocks(kernel, tpb);
+        const int blocks = coop_blocks(kernel, tpb, per_sm);
         CK(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kernel), dim3(blocks), dim3(tpb), argv, 0, st));
         ++n_launch;
     }
@@ -2573,7 +2575,7 @@ struct cig_handle {
         if (kw == 1) {  // distances straight into the result
             CK(cudaMemsetAsync(wout, 0xFF, static_cast<size_t>(n) * sizeof(uint32_t), qstream));
             ms_seed<<<1, kMsWidth, 0, qstream>>>(ms_src, 1u, wout, 1u, nullptr, fr, qstatus);
-            launch_coop_on(qstream, ms_closure<A>, kTpbMs, query_view(), wout, fr, bl, n + 2, qstatus);
+            launch_coop_on(qstream, ~0u, ms_closure<A>, kTpbMs, query_view(), wout, fr, bl, n + 2, qstatus);
             --n_launch;  // no transpose
         } else if (kw <= 4) {
             sssp_wave_n<A, 1>(kw, fr, wout);
@@ -2594,7 +2596,7 @@ struct cig_handle {
         ms_seed<<<1, kMsWidth, 0, qstream>>>(ms_src, kw, ms_dist, row, nullptr, fr, qstatus);
         const MsChunks ch{ms_chunks, ms_small + 3, static_cast<uint32_t>(ms_chunk_cap()), ms_small + 8,
                           ms_small + 11};
-        launch_coop_on(qstream, ms_wave<A, LPE>, kTpbMs, query_view(), n, ms_dist, fr, ch, n + 2, qstatus);
+        launch_coop_on(qstream, ~0u, ms_wave<A, LPE>, kTpbMs, query_view(), n, ms_dist, fr, ch, n + 2, qstatus);
         constexpr uint32_t rows = 512 / LPE;
         ms_transpose<LPE><<<(n + rows - 1) / rows, 256, 0, qstream>>>(ms_dist, n, kw, wout);
     }
@@ -2628,7 +2630,7 @@ struct cig_handle {
                 CK(cudaMemsetAsync(wout, 0xFF, static_cast<size_t>(n) * sizeof(uint32_t), qstream));
                 CK(cudaMemsetAsync(vis, 0, words * sizeof(uint32_t), qstream));
                 bfs_one_seed<<<1, 1, 0, qstream>>>(ms_src, wout, vis, ms_q0, ms_small);
-                launch_coop_on(qstream, bfs_one, kTpbMs, query_view(), n, wout, vis,
+                launch_coop_on(qstream, kBfsOnePerSm, bfs_one, kTpbMs, query_view(), n, wout, vis,
                                reinterpret_cast<uint32_t *>(ms_mask0), reinterpret_cast<uint32_t *>(ms_mask1), fr, bl,
                                n + 2, bfs_pull(kw), qstatus);
                 ++n_launch;
@@ -2647,8 +2649,9 @@ struct cig_handle {
                 CK(cudaMemsetAsync(ms_visit, 0, n * sizeof(unsigned long long), qstream));
                 ms_seed<<<1, kMsWidth, 0, qstream>>>(ms_src, kw, nullptr, 0u, ms_visit, fr, qstatus);
                 const unsigned long long full = kw >= 64 ? ~0ull : ((1ull << kw) - 1);
-                launch_coop_on(qstream, bfs_wave, kTpbMs, query_view(), n, full, ms_visit, planes, fr, bl, n + 2,
-                               bfs_pull(kw), qstatus);
+                const bool few = kw <= kBfsFew;
+                launch_coop_on(qstream, few ? 2u : 4u, few ? bfs_wave<2> : bfs_wave<4>, kTpbMs, query_view(), n, full,
+                               ms_visit, planes, fr, bl, n + 2, bfs_pull(kw), qstatus);
                 bfs_depths<<<sms * 8, 256, 0, qstream>>>(ms_visit, planes, n, kw, ms_small + 8, wout);
             } else if (opt.flags & CIG_FLAG_WEIGHT_U255) {
                 sssp_wave<kSsspU>(kw, fr, bl, wout);

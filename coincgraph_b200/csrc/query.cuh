@@ -145,10 +145,6 @@ struct MsChunks {
     uint32_t *tiles;  // three counters (TileFeed)
 };
 
-__device__ __forceinline__ void red_or(unsigned long long *p, unsigned long long x) {
-    asm volatile("red.relaxed.gpu.global.or.b64 [%0], %1;" ::"l"(p), "l"(x) : "memory");
-}
-
 template <int A, int LPE>
 struct MsWave {
     uint32_t *dist;

@@ -170,3 +170,35 @@ def test_bfs_wave_on_used_device_memory(built):
             eng.init()
             for k in (64, 5, 64):
                 np.testing.assert_array_equal(eng.query_bfs(src[:k]), ref[:k])
+
+
+@pytest.mark.parametrize("k", [1, 2, 16, 17])
+def test_bfs_switches_on_the_queued_rows(built, k):
+    """Two steps from the sources lie 300 rows of 200 entries, a queue far
+    below n / 32 vertices whose rows hold more than n entries: the round goes
+    bottom-up by the lengths added up while the vertices were queued (short
+    rows are not counted), on both sides of the blocks-per-SM rule.  Beside it
+    a chain of 600 vertices, so that the wave ends in several hundred queue
+    rounds below the limit."""
+    rng = np.random.default_rng(9)
+    n = 50000
+    mid = np.arange(100, 400)
+    chain = np.arange(1000, 1600)
+    src = np.concatenate([np.repeat(np.arange(20), 300), np.repeat(mid, 200), chain[:-1], np.arange(20)])
+    dst = np.concatenate([np.tile(mid, 20), rng.integers(2000, n, 300 * 200), chain[1:], np.full(20, 1000)])
+    g = gen.graph_from_edges(n, src, dst)
+    sources = np.arange(k, dtype=np.uint32)
+    og = oracle.Graph(g.n, g.xadj, g.adj)
+    import torch
+
+    with Engine("bfs", cache_gib=1.0) as eng:
+        eng.load_csr(g.n, g.xadj, g.adj)
+        eng.init()
+        out = torch.empty((k, n), dtype=torch.int32, device="cuda")
+        st = eng.query_device("bfs", sources, out, width=64)
+        got = out.cpu().numpy().view(np.uint32)
+    for j, s in enumerate(sources):
+        np.testing.assert_array_equal(got[j], og.sssp(int(s), oracle.BFS))
+    # Top-down rounds expand the sources, the 300 rows and the chain; a
+    # bottom-up round looks through the in-row of every unreached vertex.
+    assert st["rows_expanded"] > 10000
