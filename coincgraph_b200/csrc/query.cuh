@@ -132,7 +132,10 @@ __global__ void __launch_bounds__(kTpbMs, 4) ms_closure(AdjView fwd, uint32_t *d
 // edges in two blocks, 1.13 with 128 and 1.05 with 64 entries.
 constexpr uint32_t kMsChunk = 64;  // rows of at least this many entries are expanded by the whole grid
 constexpr int kMsGroup = 2;        // edges per lane whose loads are in flight together
-constexpr uint32_t kMsScan = 64;    // rounds after more than n / kMsScan improvements scan the masks
+// A scan round hands out n / 32 tiles whatever it finds in them, so few
+// improvements are better queued (511 x 511 grid, 13 sources: 12.3 ms with
+// scans from n / 64 on, 9.2 from n / 16; R-MAT s19: 1.31, 1.30).
+constexpr uint32_t kMsScan = 16;  // rounds after more than n / kMsScan improvements scan the masks
 
 // Chunks of long rows met in a round (three counters, as for the frontier),
 // and the entries of a queue rebuilt from the masks (three counters).  A warp
@@ -152,56 +155,112 @@ struct MsWave {
     bool queue;  // append improved vertices
     WarpBuf buf;
 
+    // N 16-byte pieces of edges per lane: sources 4 quad .. 4 quad + 3 of edge
+    // xs -> ys, those of `bits` (0: none).  xs's row is read through L1 (a
+    // value lowered meanwhile is relaxed again next round), ys's from L2: a
+    // stale row of a hub costs an atomic for every source, all of them on one
+    // sector.
+    template <int N>
+    __device__ __forceinline__ uint32_t pieces(const uint32_t (&xs)[N], const uint32_t (&ys)[N],
+                                               const uint32_t (&quad)[N], const uint32_t (&bits)[N]) const {
+        constexpr uint64_t kRow = 4 * LPE;
+        uint4 dx[N], dy[N];
+        uint32_t hits = 0;
+#pragma unroll
+        for (int j = 0; j < N; ++j)
+            if (bits[j]) {
+                dx[j] = *reinterpret_cast<const uint4 *>(dist + xs[j] * kRow + 4u * quad[j]);
+                dy[j] = __ldcg(reinterpret_cast<const uint4 *>(dist + ys[j] * kRow + 4u * quad[j]));
+            }
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            uint32_t add = 0;
+            if (bits[j]) {
+                const uint32_t w = edge_weight<A>(xs[j], ys[j]);
+                const uint32_t nd[4] = {dx[j].x + w, dx[j].y + w, dx[j].z + w, dx[j].w + w};
+                const uint32_t od[4] = {dy[j].x, dy[j].y, dy[j].z, dy[j].w};
+                uint32_t *row = dist + ys[j] * kRow + 4u * quad[j];
+                uint32_t old[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    old[i] = ((bits[j] >> i) & 1u) && nd[i] < od[i] ? atomicMin(row + i, nd[i]) : 0u;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) add |= nd[i] < old[i] ? 1u << i : 0u;
+                hits += add ? 1u : 0u;
+            }
+            const unsigned long long add64 = static_cast<unsigned long long>(add) << (4u * quad[j]);
+            if (queue)
+                buf.add(add && atomicOr(mask_out + ys[j], add64) == 0ull, ys[j]);
+            else if (add)
+                red_or(mask_out + ys[j], add64);
+        }
+        return hits;
+    }
+
     // Relax 32 edges, one per lane (x -> y for the sources in m; m = 0: none).
-    // x's row is read through L1 (a value lowered meanwhile is relaxed again
-    // next round), y's from L2: a stale row of a hub costs an atomic for every
-    // source, all of them on one sector.
     __device__ __forceinline__ uint32_t relax(uint32_t x, uint32_t y, unsigned long long m) const {
         constexpr int kPer = 32 / LPE;                            // edges per step
         constexpr int N = LPE < kMsGroup ? LPE : kMsGroup;        // steps in flight
-        constexpr uint64_t kRow = 4 * LPE;
-        const uint32_t lane = lane_id(), quad = lane % LPE;
+        const uint32_t lane = lane_id();
         uint32_t hits = 0;
+        if constexpr (LPE >= 8) {
+            // Few sources per edge (high-diameter graphs: one or two of 64):
+            // the pieces that hold any are dealt out instead of all of them,
+            // up to half of what the steps below would go through (511 x 511
+            // grid, 64 sources: 31.4 -> 16.0 ms, with kMsScan; R-MAT s20:
+            // 9.4 -> 8.4).  Rows of up to four pieces are two such steps.
+            unsigned long long nz = m | (m >> 1);
+            nz = (nz | (nz >> 2)) & 0x1111111111111111ull;
+            const uint32_t mine = __popcll(nz);
+            const uint32_t total = __reduce_add_sync(kFull, mine);
+            if (total <= 16u * LPE) {
+                uint32_t incl = mine;
+#pragma unroll
+                for (uint32_t o = 1; o < 32u; o <<= 1) {
+                    const uint32_t t = __shfl_up_sync(kFull, incl, o);
+                    if (lane >= o) incl += t;
+                }
+                const uint32_t excl = incl - mine;
+                for (uint32_t base = 0; base < total; base += 32u * kMsGroup) {
+                    uint32_t xs[kMsGroup], ys[kMsGroup], quad[kMsGroup], bits[kMsGroup];
+#pragma unroll
+                    for (int j = 0; j < kMsGroup; ++j) {
+                        const uint32_t e = base + 32u * j + lane;
+                        uint32_t lo = 0, hi = 32;  // the last lane whose pieces start at or before e
+#pragma unroll
+                        for (int step = 0; step < 5; ++step) {
+                            const uint32_t mid = (lo + hi) >> 1;
+                            if (__shfl_sync(kFull, excl, mid) <= e)
+                                lo = mid;
+                            else
+                                hi = mid;
+                        }
+                        xs[j] = __shfl_sync(kFull, x, lo);
+                        ys[j] = __shfl_sync(kFull, y, lo);
+                        const unsigned long long ms = __shfl_sync(kFull, m, lo);
+                        unsigned long long z = __shfl_sync(kFull, nz, lo);
+                        for (uint32_t k = e - __shfl_sync(kFull, excl, lo); k && z; --k) z &= z - 1;
+                        quad[j] = z ? static_cast<uint32_t>(__ffsll(static_cast<long long>(z)) - 1) >> 2 : 0u;
+                        bits[j] = e < total ? static_cast<uint32_t>(ms >> (4u * quad[j])) & 15u : 0u;
+                    }
+                    hits += pieces<kMsGroup>(xs, ys, quad, bits);
+                }
+                return hits;
+            }
+        }
 #pragma unroll
         for (int s0 = 0; s0 < LPE; s0 += N) {
-            uint32_t xs[N], ys[N], bits[N];
-            uint4 dx[N], dy[N];
+            uint32_t xs[N], ys[N], bits[N], quad[N];
 #pragma unroll
             for (int j = 0; j < N; ++j) {
                 const int src = (s0 + j) * kPer + static_cast<int>(lane / LPE);
                 xs[j] = LPE == 1 ? x : __shfl_sync(kFull, x, src);
                 ys[j] = LPE == 1 ? y : __shfl_sync(kFull, y, src);
                 const unsigned long long ms = LPE == 1 ? m : __shfl_sync(kFull, m, src);
-                bits[j] = static_cast<uint32_t>(ms >> (4u * quad)) & 15u;
+                quad[j] = lane % LPE;
+                bits[j] = static_cast<uint32_t>(ms >> (4u * quad[j])) & 15u;
             }
-#pragma unroll
-            for (int j = 0; j < N; ++j)
-                if (bits[j]) {
-                    dx[j] = *reinterpret_cast<const uint4 *>(dist + xs[j] * kRow + 4u * quad);
-                    dy[j] = __ldcg(reinterpret_cast<const uint4 *>(dist + ys[j] * kRow + 4u * quad));
-                }
-#pragma unroll
-            for (int j = 0; j < N; ++j) {
-                uint32_t add = 0;
-                if (bits[j]) {
-                    const uint32_t w = edge_weight<A>(xs[j], ys[j]);
-                    const uint32_t nd[4] = {dx[j].x + w, dx[j].y + w, dx[j].z + w, dx[j].w + w};
-                    const uint32_t od[4] = {dy[j].x, dy[j].y, dy[j].z, dy[j].w};
-                    uint32_t *row = dist + ys[j] * kRow + 4u * quad;
-                    uint32_t old[4];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        old[i] = ((bits[j] >> i) & 1u) && nd[i] < od[i] ? atomicMin(row + i, nd[i]) : 0u;
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) add |= nd[i] < old[i] ? 1u << i : 0u;
-                    hits += add ? 1u : 0u;
-                }
-                const unsigned long long add64 = static_cast<unsigned long long>(add) << (4u * quad);
-                if (queue)
-                    buf.add(add && atomicOr(mask_out + ys[j], add64) == 0ull, ys[j]);
-                else if (add)
-                    red_or(mask_out + ys[j], add64);
-            }
+            hits += pieces<N>(xs, ys, quad, bits);
         }
         return hits;
     }
@@ -261,9 +320,12 @@ __global__ void __launch_bounds__(kTpbMs, 3) ms_wave(AdjView fwd, uint32_t n, ui
         uint32_t tile = 32;  // items per warp and step: few items spread over all warps
         while (tile > (scan ? 8u : 1u) && items <= static_cast<uint64_t>(warps) * (scan ? 4u : 1u) * (tile / 2))
             tile >>= 1;
+        // A round whose tiles go round once asks for no further ones: a
+        // thousand warps' requests on one counter take as long as their work.
+        const bool more = items > static_cast<uint64_t>(warps) * tile;
         TileFeed feed(ch.tiles + r % 3, warps);
-        for (uint64_t t = wid; t * tile < items; t = feed.take()) {
-            feed.ask();
+        for (uint64_t t = wid; t * tile < items; t = more ? feed.take() : items) {
+            if (more) feed.ask();
             const uint64_t i = t * tile + lane;
             uint32_t x = 0, deg = 0;
             uint64_t off = 0;

@@ -202,3 +202,21 @@ def test_bfs_switches_on_the_queued_rows(built, k):
     # Top-down rounds expand the sources, the 300 rows and the chain; a
     # bottom-up round looks through the in-row of every unreached vertex.
     assert st["rows_expanded"] > 10000
+
+
+@pytest.mark.parametrize("k", [4, 8, 16, 17, 32, 33, 64])
+@pytest.mark.parametrize("spread", [True, False])
+def test_sssp_waves_of_sparse_and_dense_masks(built, k, spread):
+    """A grid, where sources far apart leave a vertex one or two bits of the
+    wave (their 16-byte pieces are dealt out), and neighbouring sources leave
+    it all of them; queue rounds, scan rounds and the changes between them."""
+    case = grid_case(70, 1, 20)
+    rng = np.random.default_rng(k)
+    src = (rng.integers(0, case.n, k) if spread else 2000 + np.arange(k) // 4).astype(np.uint32)
+    og = oracle.Graph(case.n, case.xadj, case.adj)
+    with Engine("sssp", cache_gib=1.0) as eng:
+        eng.load_csr(case.n, case.xadj, case.adj)
+        eng.init()
+        got = eng.query_sssp(src)
+    for j, s in enumerate(src):
+        np.testing.assert_array_equal(got[j], og.sssp(int(s), oracle.SSSP))
