@@ -202,63 +202,60 @@ struct MsWave {
         constexpr int kPer = 32 / LPE;                            // edges per step
         constexpr int N = LPE < kMsGroup ? LPE : kMsGroup;        // steps in flight
         const uint32_t lane = lane_id();
-        uint32_t hits = 0;
-        if constexpr (LPE >= 8) {
-            // Few sources per edge (high-diameter graphs: one or two of 64):
-            // the pieces that hold any are dealt out instead of all of them,
-            // up to half of what the steps below would go through (511 x 511
-            // grid, 64 sources: 31.4 -> 16.0 ms, with kMsScan; R-MAT s20:
-            // 9.4 -> 8.4).  Rows of up to four pieces are two such steps.
-            unsigned long long nz = m | (m >> 1);
+        // Few sources per edge (high-diameter graphs: one or two of 64): the
+        // pieces that hold any are dealt out instead of all of them, up to
+        // half of what the steps would go through (511 x 511 grid, 64
+        // sources: 31.4 -> 16.0 ms, with kMsScan; R-MAT s20: 9.4 -> 8.4).
+        // Rows of up to four pieces are two such steps.
+        constexpr bool kDeal = LPE >= 8;
+        unsigned long long nz = 0;
+        uint32_t excl = 0, total = 0;
+        bool deal = false;
+        if constexpr (kDeal) {
+            nz = m | (m >> 1);
             nz = (nz | (nz >> 2)) & 0x1111111111111111ull;
             const uint32_t mine = __popcll(nz);
-            const uint32_t total = __reduce_add_sync(kFull, mine);
-            if (total <= 16u * LPE) {
+            total = __reduce_add_sync(kFull, mine);
+            deal = total <= 16u * LPE;
+            if (deal) {
                 uint32_t incl = mine;
 #pragma unroll
                 for (uint32_t o = 1; o < 32u; o <<= 1) {
                     const uint32_t t = __shfl_up_sync(kFull, incl, o);
                     if (lane >= o) incl += t;
                 }
-                const uint32_t excl = incl - mine;
-                for (uint32_t base = 0; base < total; base += 32u * kMsGroup) {
-                    uint32_t xs[kMsGroup], ys[kMsGroup], quad[kMsGroup], bits[kMsGroup];
-#pragma unroll
-                    for (int j = 0; j < kMsGroup; ++j) {
-                        const uint32_t e = base + 32u * j + lane;
-                        uint32_t lo = 0, hi = 32;  // the last lane whose pieces start at or before e
-#pragma unroll
-                        for (int step = 0; step < 5; ++step) {
-                            const uint32_t mid = (lo + hi) >> 1;
-                            if (__shfl_sync(kFull, excl, mid) <= e)
-                                lo = mid;
-                            else
-                                hi = mid;
-                        }
-                        xs[j] = __shfl_sync(kFull, x, lo);
-                        ys[j] = __shfl_sync(kFull, y, lo);
-                        const unsigned long long ms = __shfl_sync(kFull, m, lo);
-                        unsigned long long z = __shfl_sync(kFull, nz, lo);
-                        for (uint32_t k = e - __shfl_sync(kFull, excl, lo); k && z; --k) z &= z - 1;
-                        quad[j] = z ? static_cast<uint32_t>(__ffsll(static_cast<long long>(z)) - 1) >> 2 : 0u;
-                        bits[j] = e < total ? static_cast<uint32_t>(ms >> (4u * quad[j])) & 15u : 0u;
-                    }
-                    hits += pieces<kMsGroup>(xs, ys, quad, bits);
-                }
-                return hits;
+                excl = incl - mine;
             }
         }
-#pragma unroll
-        for (int s0 = 0; s0 < LPE; s0 += N) {
+        const int steps = deal ? static_cast<int>((total + 31u) / 32u) : LPE;
+        uint32_t hits = 0;
+#pragma unroll(kDeal ? 1 : LPE)
+        for (int s0 = 0; s0 < steps; s0 += N) {
             uint32_t xs[N], ys[N], bits[N], quad[N];
 #pragma unroll
             for (int j = 0; j < N; ++j) {
-                const int src = (s0 + j) * kPer + static_cast<int>(lane / LPE);
+                uint32_t src = LPE == 1 ? lane : (s0 + j) * kPer + lane / LPE;
+                const uint32_t e = 32u * (s0 + j) + lane;
+                quad[j] = lane % LPE;
+                if (kDeal && deal) {
+                    uint32_t lo = 0, hi = 32;  // the last lane whose pieces start at or before e
+#pragma unroll
+                    for (int step = 0; step < 5; ++step) {
+                        const uint32_t mid = (lo + hi) >> 1;
+                        if (__shfl_sync(kFull, excl, mid) <= e)
+                            lo = mid;
+                        else
+                            hi = mid;
+                    }
+                    src = lo;
+                    unsigned long long z = __shfl_sync(kFull, nz, src);
+                    for (uint32_t k = e - __shfl_sync(kFull, excl, src); k && z; --k) z &= z - 1;
+                    quad[j] = z ? static_cast<uint32_t>(__ffsll(static_cast<long long>(z)) - 1) >> 2 : 0u;
+                }
                 xs[j] = LPE == 1 ? x : __shfl_sync(kFull, x, src);
                 ys[j] = LPE == 1 ? y : __shfl_sync(kFull, y, src);
                 const unsigned long long ms = LPE == 1 ? m : __shfl_sync(kFull, m, src);
-                quad[j] = lane % LPE;
-                bits[j] = static_cast<uint32_t>(ms >> (4u * quad[j])) & 15u;
+                bits[j] = kDeal && deal && e >= total ? 0u : static_cast<uint32_t>(ms >> (4u * quad[j])) & 15u;
             }
             hits += pieces<N>(xs, ys, quad, bits);
         }
