@@ -358,7 +358,7 @@ struct cig_handle {
     float *pr_comp = nullptr;
     uint8_t *pr_export_buf[4] = {};  // FP32 rank, residual, FP64 rank, residual (allocated by the first get_pr)
     BigRow *pr_chunks = nullptr;  // the sweeps' chunks of long rows (pr_chunk_cap entries)
-    uint64_t pr_chunk_cap() const { return 2 * fwd.seg_total * (kSegEdges / kPrChunk); }
+    uint32_t pr_chunk_cap = 0;
     uint32_t *pr_queued = nullptr;
     bool pr64 = false;
 
@@ -972,6 +972,7 @@ struct cig_handle {
             index_headroom = std::max<uint64_t>(64, std::strtoull(e, nullptr, 10));
         if (const char *e = std::getenv("CIG_POS_INDEX_SPARE")) index_spare = std::max(0.0, std::atof(e));
         if (const char *e = std::getenv("CIG_PULL_ON")) tune.pull_on = static_cast<uint32_t>(std::max(0, std::atoi(e)));
+        if (const char *e = std::getenv("CIG_CHUNK_CAP")) chunk_cap = std::strtoull(e, nullptr, 10);
         if (const char *e = std::getenv("CIG_PULL_OFF")) tune.pull_off = static_cast<uint32_t>(std::max(1, std::atoi(e)));
     }
 
@@ -1348,7 +1349,7 @@ struct cig_handle {
                 CK(cudaMemset(pr_hub_more, 0, more * sizeof(double)));
             }
             dmalloc(pr_queued, n);
-            dmalloc(pr_chunks, pr_chunk_cap());
+            pr_chunk_cap = alloc_chunks(pr_chunks, kPrChunk);
             dmalloc(aff_stamp, n);
             CK(cudaMemset(aff_stamp, 0, n * sizeof(uint32_t)));
         } else {
@@ -1490,7 +1491,7 @@ struct cig_handle {
         const T eps = static_cast<T>(opt.pr_epsilon);
         const int p = prof_begin(CIG_STAGE_PR);
         CK(cudaMemsetAsync(small + kPrAct, 0, 6 * sizeof(uint32_t), stream));
-        const PrChunks ch{pr_chunks, small + kPrAct + 3, static_cast<uint32_t>(pr_chunk_cap())};
+        const PrChunks ch{pr_chunks, small + kPrAct + 3, pr_chunk_cap};
         launch_coop(pr_converge<T>, kTpbPr, fwd.view(), a, eps, n, static_cast<uint32_t>(opt.pr_max_rounds), ch,
                     small + kPrAct, seg_hot, status);
         prof_end(p);
@@ -2471,15 +2472,56 @@ struct cig_handle {
     unsigned long long *bfs_acc = nullptr;
     uint32_t *bfs_arrived = nullptr, *bfs_bigbits = nullptr;
     BigRow *ms_chunks = nullptr;  // chunks of long rows of SSSP waves
-    uint64_t ms_chunk_cap() const { return 2 * fwd.seg_total * (kSegEdges / kMsChunk); }
-    uint64_t bfs_rows_cap() const { return rev.desc ? rev.seg_total * (kSegEdges / kBfsChunk) : 0; }
+    uint32_t ms_chunk_cap = 0;
+    bool ms_chunks_made = false, bfs_pull_made = false;
+    // Long in-rows, and their chunks: a row of d >= kBfsChunk entries lies in a
+    // power-of-two block of at least d slots, so either is at most one per
+    // kBfsChunk slots of the reverse arena.
+    uint64_t bfs_rows_cap() const { return rev.seg_total * (kSegEdges / kBfsChunk); }
+
+    // Entries for the chunks of `chunk` entries of rows at least as long.  One
+    // per `chunk` slots covers the whole arena (a row lies in a power-of-two
+    // block at least as long as itself); but the arena is host memory, which
+    // may exceed the device's many times, so the list stays below 6 bytes per
+    // vertex (24 MiB for small graphs), and further below where the device has
+    // no room: the kernels go through what finds no place in it where they
+    // met it.  CIG_CHUNK_CAP (at creation) sets the entries.
+    uint64_t chunk_cap = ~0ull;
+    uint32_t alloc_chunks(BigRow *&rows, uint32_t chunk) {
+        uint64_t want = std::min<uint64_t>(fwd.seg_total * (kSegEdges / chunk), std::max<uint64_t>(1u << 20, n / 4));
+        want = std::min<uint64_t>(want, chunk_cap);
+        for (; want; want /= 2) {
+            if (cudaMalloc(reinterpret_cast<void **>(&rows), want * sizeof(BigRow)) == cudaSuccess)
+                return static_cast<uint32_t>(want);
+            cudaGetLastError();
+            rows = nullptr;
+        }
+        return 0;
+    }
+    // The buffers of bottom-up rounds of waves, at the first wave; without
+    // room for them waves stay top-down.
+    void alloc_bfs_pull() {
+        if (bfs_pull_made || !rev.desc) return;
+        bfs_pull_made = true;
+        try {
+            dmalloc(bfs_tasks, bfs_rows_cap());
+            dmalloc(bfs_acc, bfs_rows_cap());
+            dmalloc(bfs_arrived, bfs_rows_cap());
+            dmalloc(bfs_bigbits, (n + 31) / 32);
+        } catch (const CigError &) {
+            dfree(bfs_tasks);
+            dfree(bfs_acc);
+            dfree(bfs_arrived);
+            dfree(bfs_bigbits);
+        }
+    }
 
     // Bottom-up switch of a BFS query: frontier above n/pull_on vertices
     // (then at least n/pull_off); needs the device in-edge arena.
     BfsPull bfs_pull(uint32_t kw) const {
         BfsPull p{};
         p.ctl = ms_small + 8;
-        if (opt.algo == CIG_PR || !rev.desc || !tune.pull_on) return p;
+        if (opt.algo == CIG_PR || !rev.desc || !tune.pull_on || (kw > 1 && !bfs_bigbits)) return p;
         p.rev = rev.view();
 #ifdef CIG_BOUNDS_CHECK
         p.rev.bst = qstatus;
@@ -2490,7 +2532,7 @@ struct cig_handle {
         // most in-rows); a top-down edge costs about four times a vertex.
         p.edges_on = kw == 1 ? n / 4 : n;
         p.tasks = bfs_tasks;
-        p.task_cap = static_cast<uint32_t>(2 * bfs_rows_cap());
+        p.task_cap = static_cast<uint32_t>(bfs_rows_cap());
         p.acc = bfs_acc;
         p.arrived = bfs_arrived;
         p.bigbits = bfs_bigbits;
@@ -2510,13 +2552,6 @@ struct cig_handle {
         dmalloc(ms_q0, n + 1);
         dmalloc(ms_q1, n + 1);
         dmalloc(ms_small, 16);
-        dmalloc(ms_chunks, ms_chunk_cap());
-        if (rev.desc) {
-            dmalloc(bfs_tasks, 2 * bfs_rows_cap());
-            dmalloc(bfs_acc, bfs_rows_cap());
-            dmalloc(bfs_arrived, bfs_rows_cap());
-            dmalloc(bfs_bigbits, (n + 31) / 32);
-        }
         dmalloc(ms_src, kMsWidth);
         dmalloc(ms_big, kBigRowCap);
     }
@@ -2540,6 +2575,7 @@ struct cig_handle {
         dfree(bfs_acc);
         dfree(bfs_arrived);
         dfree(bfs_bigbits);
+        ms_chunks_made = bfs_pull_made = false;
         dfree(ms_src);
         dfree(ms_big);
         dfree(ms_out);
@@ -2594,8 +2630,9 @@ struct cig_handle {
         constexpr uint32_t row = 4 * LPE;
         CK(cudaMemsetAsync(ms_dist, 0xFF, static_cast<size_t>(n) * row * sizeof(uint32_t), qstream));
         ms_seed<<<1, kMsWidth, 0, qstream>>>(ms_src, kw, ms_dist, row, nullptr, fr, qstatus);
-        const MsChunks ch{ms_chunks, ms_small + 3, static_cast<uint32_t>(ms_chunk_cap()), ms_small + 8,
-                          ms_small + 11};
+        if (!ms_chunks_made) ms_chunk_cap = alloc_chunks(ms_chunks, kMsChunk);
+        ms_chunks_made = true;
+        const MsChunks ch{ms_chunks, ms_small + 3, ms_chunk_cap, ms_small + 8, ms_small + 11};
         launch_coop_on(qstream, ~0u, ms_wave<A, LPE>, kTpbMs, query_view(), n, ms_dist, fr, ch, n + 2, qstatus);
         constexpr uint32_t rows = 512 / LPE;
         ms_transpose<LPE><<<(n + rows - 1) / rows, 256, 0, qstream>>>(ms_dist, n, kw, wout);
@@ -2649,6 +2686,7 @@ struct cig_handle {
                 CK(cudaMemsetAsync(ms_visit, 0, n * sizeof(unsigned long long), qstream));
                 ms_seed<<<1, kMsWidth, 0, qstream>>>(ms_src, kw, nullptr, 0u, ms_visit, fr, qstatus);
                 const unsigned long long full = kw >= 64 ? ~0ull : ((1ull << kw) - 1);
+                alloc_bfs_pull();
                 const bool few = kw <= kBfsFew;
                 launch_coop_on(qstream, few ? 2u : 4u, few ? bfs_wave<2> : bfs_wave<4>, kTpbMs, query_view(), n, full,
                                ms_visit, planes, fr, bl, n + 2, bfs_pull(kw), qstatus);
@@ -3006,7 +3044,7 @@ struct cig_handle {
             if (inval_done) vs += (nn + 1) * sizeof(uint32_t);
             if (opt.algo == CIG_PR) {
                 const uint64_t es = pr64 ? sizeof(double) : sizeof(float);
-                vs += 2 * nn * es + (nn + 1) * es + 2 * nn * sizeof(uint32_t) + pr_chunk_cap() * sizeof(BigRow);
+                vs += 2 * nn * es + (nn + 1) * es + 2 * nn * sizeof(uint32_t) + pr_chunk_cap * sizeof(BigRow);
                 for (int i = 0; i < 4; ++i)
                     if (pr_export_buf[i]) vs += nn * (i < 2 ? sizeof(float) : sizeof(double));
                 if (!pr64) vs += nn * sizeof(float) + nn * sizeof(double) + 2 * w * sizeof(uint32_t) +
@@ -3031,8 +3069,8 @@ struct cig_handle {
         if (qstream)
             m->query_buffers = nn * kMsWidth * sizeof(uint32_t) + 3 * nn * sizeof(unsigned long long) +
                                2 * (nn + 1) * sizeof(uint32_t) + sizeof(Status) + (16 + kMsWidth) * sizeof(uint32_t) +
-                               (kBigRowCap + ms_chunk_cap()) * sizeof(BigRow) +
-                               (rev.desc ? bfs_rows_cap() * (2 * sizeof(BigRow) + 12) + w * sizeof(uint32_t) : 0);
+                               (kBigRowCap + (ms_chunks ? ms_chunk_cap : 0)) * sizeof(BigRow) +
+                               (bfs_bigbits ? bfs_rows_cap() * (sizeof(BigRow) + 12) + w * sizeof(uint32_t) : 0);
         m->total = m->edge_cache + m->segment_table + m->descriptors + m->reverse_arena + m->position_index +
                    m->vertex_state + m->batch_buffers + m->query_buffers;
         m->pinned_host = segs * kSegEdges * sizeof(uint32_t) + 4 * bcap * sizeof(uint32_t);

@@ -300,8 +300,8 @@ __device__ __forceinline__ T rank_consume(const PrArrays<T> &a, uint32_t v, doub
 // 4.93, 128 4.77; 50k vertices, FP64: 1.59, 1.55, 1.56).
 constexpr uint32_t kPrChunk = 128;
 
-// The chunks a sweep leaves to the whole grid; `cap` covers every slot of the
-// arena (2 * slots / kPrChunk), so it cannot run out.
+// The chunks a sweep leaves to the whole grid; what finds no place in the
+// list is pushed by the warp that met it.
 struct PrChunks {
     BigRow *rows;
     uint32_t *cnt;  // 3 counters
@@ -401,14 +401,14 @@ __device__ __forceinline__ bool pr_sweeps(const AdjView &fwd, const PrArrays<T> 
                 uint32_t at = 0;
                 if (lane == 0) at = atomicAdd(ch_cnt, k);
                 at = __shfl_sync(kFull, at, 0);
-                for (uint32_t i = lane; i < k; i += 32u) {
-                    if (at + i < ch.cap)
-                        ch.rows[at + i] = BigRow{loff + static_cast<uint64_t>(i) * kPrChunk,
-                                                 static_cast<unsigned long long>(lc), lv,
-                                                 min(kPrChunk, ldeg - i * kPrChunk)};
-                    else
-                        set_error(st, kErrQueue, at + i);
-                }
+                const uint32_t fit = at < ch.cap ? min(k, ch.cap - at) : 0u;
+                for (uint32_t i = lane; i < fit; i += 32u)
+                    ch.rows[at + i] = BigRow{loff + static_cast<uint64_t>(i) * kPrChunk,
+                                             static_cast<unsigned long long>(lc), lv,
+                                             min(kPrChunk, ldeg - i * kPrChunk)};
+                for (uint32_t i = fit; i < k; ++i)
+                    sweep_row<32u>(fwd, fwd.at(loff + static_cast<uint64_t>(i) * kPrChunk),
+                                   min(kPrChunk, ldeg - i * kPrChunk), lane, lv, lc, op, cnt);
             }
             expand_rows_warp<kTpbPr>(fwd, has && deg < kPrChunk, v, PrBits<T>::to(c), off, deg, op, sm, cnt);
         }

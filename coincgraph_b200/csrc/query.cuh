@@ -139,7 +139,8 @@ constexpr uint32_t kMsScan = 16;  // rounds after more than n / kMsScan improvem
 
 // Chunks of long rows met in a round (three counters, as for the frontier),
 // and the entries of a queue rebuilt from the masks (three counters).  A warp
-// per chunk: short, since the longest warp decides a round's time.
+// per chunk: short, since the longest warp decides a round's time.  What finds
+// no place in the list is relaxed by the warp that met it.
 struct MsChunks {
     BigRow *rows;
     uint32_t *cnt;
@@ -263,6 +264,24 @@ struct MsWave {
     }
 };
 
+// The entries of a chunk (it lies in one segment) of x's row for the sources
+// in m, by one warp; the next step's are read while this one's are relaxed.
+template <int A, int LPE>
+__device__ __forceinline__ uint32_t ms_chunk(const AdjView &fwd, const MsWave<A, LPE> &op, uint64_t off, uint32_t len,
+                                             uint32_t x, unsigned long long m) {
+    const uint32_t lane = lane_id();
+    const uint32_t *rp = fwd.at(off);
+    uint32_t hits = 0;
+    uint32_t y_next = lane < len ? __ldg(rp + lane) : kTomb;
+    for (uint32_t e0 = 0; e0 < len; e0 += 32u) {
+        const uint32_t y = fwd.vid(y_next);
+        y_next = e0 + 32u + lane < len ? __ldg(rp + e0 + 32u + lane) : kTomb;
+        const bool live = y != kTomb;
+        hits += op.relax(x, live ? y : 0u, live ? m : 0ull);
+    }
+    return hits;
+}
+
 template <int A, int LPE>
 __global__ void __launch_bounds__(kTpbMs, 3) ms_wave(AdjView fwd, uint32_t n, uint32_t *dist, MsFrontier fr,
                                                      MsChunks ch, uint32_t max_rounds, Status *st) {
@@ -355,52 +374,58 @@ __global__ void __launch_bounds__(kTpbMs, 3) ms_wave(AdjView fwd, uint32_t n, ui
                 uint32_t at = 0;
                 if (lane == 0) at = atomicAdd(ch_cnt, k);
                 at = __shfl_sync(kFull, at, 0);
-                for (uint32_t c = lane; c < k; c += 32u) {
-                    if (at + c < ch.cap)
-                        ch.rows[at + c] = BigRow{loff + static_cast<uint64_t>(c) * kMsChunk, lm, lx,
-                                                 min(kMsChunk, ldeg - c * kMsChunk)};
-                    else
-                        set_error(st, kErrQueue, at + c);
+                const uint32_t fit = at < ch.cap ? min(k, ch.cap - at) : 0u;
+                for (uint32_t c = lane; c < fit; c += 32u)
+                    ch.rows[at + c] = BigRow{loff + static_cast<uint64_t>(c) * kMsChunk, lm, lx,
+                                             min(kMsChunk, ldeg - c * kMsChunk)};
+                if (lane == l) {
+                    off += static_cast<uint64_t>(fit) * kMsChunk;
+                    deg = fit < k ? deg - fit * kMsChunk : 0u;
                 }
             }
-            // The warp's rows concatenated, 32 edges per step; the next
-            // step's entries are read while this one's are relaxed.
-            const uint32_t mine = deg < kMsChunk ? deg : 0u;
-            uint32_t incl = mine;
+            // What is left of the warp's rows concatenated (short rows; of
+            // rows that found no place in the list a chunk at a time, which
+            // lies in one segment), 32 edges per step; the next step's entries
+            // are read while this one's are relaxed.
+            while (__any_sync(kFull, deg != 0u)) {
+                const uint32_t mine = min(deg, kMsChunk);
+                uint32_t incl = mine;
 #pragma unroll
-            for (uint32_t o = 1; o < 32u; o <<= 1) {
-                const uint32_t t = __shfl_up_sync(kFull, incl, o);
-                if (lane >= o) incl += t;
-            }
-            const uint32_t total = __shfl_sync(kFull, incl, 31);
-            if (!total) continue;
-            s_scan[wb + lane] = incl - mine;
-            s_x[wb + lane] = x;
-            s_m[wb + lane] = m;
-            s_ptr[wb + lane] = mine ? fwd.at(off) : nullptr;
-            __syncwarp();
-            auto fetch = [&](uint32_t e, uint32_t &owner) -> uint32_t {
-                owner = 0;
-                if (e >= total) return kTomb;
-                uint32_t lo = 0, hi = 32;  // the last lane whose edges start at or before e
-                while (hi - lo > 1) {
-                    const uint32_t mid = (lo + hi) >> 1;
-                    if (s_scan[wb + mid] <= e)
-                        lo = mid;
-                    else
-                        hi = mid;
+                for (uint32_t o = 1; o < 32u; o <<= 1) {
+                    const uint32_t t = __shfl_up_sync(kFull, incl, o);
+                    if (lane >= o) incl += t;
                 }
-                owner = lo;
-                return __ldg(s_ptr[wb + lo] + (e - s_scan[wb + lo]));
-            };
-            uint32_t o_next, y_next = fetch(lane, o_next);
-            for (uint32_t e0 = 0; e0 < total; e0 += 32u) {
-                const uint32_t y = fwd.vid(y_next), o = o_next;
-                y_next = fetch(e0 + 32u + lane, o_next);
-                const bool live = y != kTomb;
-                hits += op.relax(s_x[wb + o], live ? y : 0u, live ? s_m[wb + o] : 0ull);
+                const uint32_t total = __shfl_sync(kFull, incl, 31);
+                s_scan[wb + lane] = incl - mine;
+                s_x[wb + lane] = x;
+                s_m[wb + lane] = m;
+                s_ptr[wb + lane] = mine ? fwd.at(off) : nullptr;
+                deg -= mine;
+                off += mine;
+                __syncwarp();
+                auto fetch = [&](uint32_t e, uint32_t &owner) -> uint32_t {
+                    owner = 0;
+                    if (e >= total) return kTomb;
+                    uint32_t lo = 0, hi = 32;  // the last lane whose edges start at or before e
+                    while (hi - lo > 1) {
+                        const uint32_t mid = (lo + hi) >> 1;
+                        if (s_scan[wb + mid] <= e)
+                            lo = mid;
+                        else
+                            hi = mid;
+                    }
+                    owner = lo;
+                    return __ldg(s_ptr[wb + lo] + (e - s_scan[wb + lo]));
+                };
+                uint32_t o_next, y_next = fetch(lane, o_next);
+                for (uint32_t e0 = 0; e0 < total; e0 += 32u) {
+                    const uint32_t y = fwd.vid(y_next), o = o_next;
+                    y_next = fetch(e0 + 32u + lane, o_next);
+                    const bool live = y != kTomb;
+                    hits += op.relax(s_x[wb + o], live ? y : 0u, live ? s_m[wb + o] : 0ull);
+                }
+                __syncwarp();
             }
-            __syncwarp();
         }
         op.buf.flush();
         if (scan) block_add(out_cnt, min(hits, 1024u), &s_new);
@@ -411,14 +436,7 @@ __global__ void __launch_bounds__(kTpbMs, 3) ms_wave(AdjView fwd, uint32_t n, ui
             hits = 0;
             for (uint32_t i = wid; i < nch; i += warps) {
                 const BigRow c = ch.rows[i];
-                const uint32_t *rp = fwd.at(c.off);  // a chunk lies in one segment
-                uint32_t y_next = lane < c.deg ? __ldg(rp + lane) : kTomb;
-                for (uint32_t e0 = 0; e0 < c.deg; e0 += 32u) {
-                    const uint32_t y = fwd.vid(y_next);
-                    y_next = e0 + 32u + lane < c.deg ? __ldg(rp + e0 + 32u + lane) : kTomb;
-                    const bool live = y != kTomb;
-                    hits += op.relax(c.x, live ? y : 0u, live ? c.payload : 0ull);
-                }
+                hits += ms_chunk(fwd, op, c.off, c.deg, c.x, c.payload);
             }
             op.buf.flush();
             if (scan) block_add(out_cnt, min(hits, 1024u), &s_new);

@@ -51,3 +51,35 @@ def test_index_budget_bounds_the_tables_and_keeps_results():
             sizes[budget] = eng.memory()["position_index"]
     assert sizes[1.0 / 1024] <= (1 << 20)
     assert sizes[0.0] > sizes[1.0 / 1024]
+
+
+def test_query_buffers_follow_the_vertices_not_the_arena():
+    """Query buffers of a graph whose rows take far more memory than its
+    vertices: the lists of row chunks stay below 24 MiB (or 6 bytes per
+    vertex), are made by the first wave that uses them, and the memory
+    report follows."""
+    import torch
+
+    rng = np.random.default_rng(5)
+    n = 4096
+    deg = 16384  # 256 MiB of rows, over a million chunks of 64 entries, on 4,096 vertices
+    xadj = np.arange(n + 1, dtype=np.uint64) * deg
+    adj = rng.integers(0, n, n * deg, dtype=np.uint32)
+    base = n * (64 * 4 + 3 * 8) + 2 * (n + 1) * 4 + 65536 * 24 + 8192
+    with Engine("sssp", cache_gib=1.0) as eng:
+        eng.load_csr(n, xadj, adj)
+        eng.init()
+        assert eng.memory()["query_buffers"] == 0
+        eng.query_bfs([1])
+        assert eng.memory()["query_buffers"] <= base
+        bfs = eng.query_bfs([1, 2, 3])
+        waves = eng.memory()["query_buffers"]
+        slots = eng.memory()["reverse_arena"] // 4
+        assert waves <= base + slots // 1024 * 36 + n // 8 + 8
+        free0 = torch.cuda.mem_get_info()[0]
+        sssp = eng.query_sssp([1, 2, 3])
+        grown = eng.memory()["query_buffers"] - waves
+        assert 0 < grown <= 24 << 20
+        # the report against the device (3 n result words beside; 2 MiB granules)
+        assert free0 - torch.cuda.mem_get_info()[0] <= grown + (8 << 20)
+        assert (bfs != 0xFFFFFFFF).all() and (sssp <= 128 * bfs).all() and (sssp >= bfs).all()

@@ -87,3 +87,23 @@ def test_pr_round_bound_keeps_the_pending_queue(make, fp64):
             s = eng.apply_batch([], [], [], [])
         assert s["pr_residual_l1"] <= case.n * 1e-9 * 1.01
         assert max_rel(eng.pagerank(fp64=fp64)[0], x) <= 1e-6
+
+
+@pytest.mark.parametrize("fp64", [False, True])
+@pytest.mark.parametrize("cap", ["0", "1", "77"])
+def test_pr_with_a_full_chunk_list(fp64, cap, monkeypatch):
+    """Sweeps over rows of up to 20,000 entries (several segments) when the
+    list of their chunks holds none, one, or some of them."""
+    monkeypatch.setenv("CIG_CHUNK_CAP", cap)
+    case = big_row_case()
+    g = oracle.Graph(case.n, case.xadj, case.adj)
+    with Engine("pr", pr_epsilon=1e-9, pr_max_rounds=100000, flags=FLAG_PR_FP64 if fp64 else 0) as eng:
+        eng.load_csr(case.n, case.xadj, case.adj)
+        eng.init()
+        for du, dv, au, av in case.batches:
+            g.delete(du, dv)
+            g.add(au, av)
+            s = eng.apply_batch(du, dv, au, av)
+        assert s["pr_residual_l1"] <= case.n * 1e-9 * 1.01
+        x, ok = g.pagerank(1e-15, 100000)
+        assert ok and max_rel(eng.pagerank(fp64=fp64)[0], x) <= (1e-6 if fp64 else 1e-5)

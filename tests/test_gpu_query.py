@@ -220,3 +220,20 @@ def test_sssp_waves_of_sparse_and_dense_masks(built, k, spread):
         got = eng.query_sssp(src)
     for j, s in enumerate(src):
         np.testing.assert_array_equal(got[j], og.sssp(int(s), oracle.SSSP))
+
+
+@pytest.mark.parametrize("cap", ["0", "1", "77"])
+@pytest.mark.parametrize("k", [3, 13, 64])
+def test_sssp_waves_with_a_full_chunk_list(built, k, cap, monkeypatch):
+    """Rows of up to 20,000 entries when the list of their chunks holds none,
+    one, or some of them: the rest is relaxed by the warps that met it."""
+    monkeypatch.setenv("CIG_CHUNK_CAP", cap)
+    case = big_row_case()
+    og = oracle.Graph(case.n, case.xadj, case.adj)
+    src = np.concatenate([[0, 1], np.arange(7000, 7000 + k - 2)]).astype(np.uint32)
+    with Engine("sssp", cache_gib=65536 / 2**30) as eng:
+        eng.load_csr(case.n, case.xadj, case.adj)
+        eng.init()
+        got = eng.query_sssp(src)
+    for j, s in enumerate(src):
+        np.testing.assert_array_equal(got[j], og.sssp(int(s), oracle.SSSP))
