@@ -2498,6 +2498,10 @@ struct cig_handle {
         }
         return 0;
     }
+    void alloc_sssp_chunks() {
+        if (!ms_chunks_made) ms_chunk_cap = alloc_chunks(ms_chunks, kMsChunk);
+        ms_chunks_made = true;
+    }
     // The buffers of bottom-up rounds of waves, at the first wave; without
     // room for them waves stay top-down.
     void alloc_bfs_pull() {
@@ -2539,27 +2543,36 @@ struct cig_handle {
         return p;
     }
 
+    // The buffers of the first query; all of them or (out of memory: the call
+    // fails, a later one may try again) none.
     void alloc_queries() {
         if (qstream) return;
-        CK(cudaStreamCreateWithFlags(&qstream, cudaStreamNonBlocking));
-        for (auto &e : q_ev) CK(cudaEventCreate(&e));
-        dmalloc(qstatus, 1);
-        CK(cudaHostAlloc(reinterpret_cast<void **>(&h_qstatus), sizeof(Status), cudaHostAllocDefault));
-        dmalloc(ms_dist, static_cast<size_t>(n) * kMsWidth);
-        dmalloc(ms_visit, n);
-        dmalloc(ms_mask0, n);
-        dmalloc(ms_mask1, n);
-        dmalloc(ms_q0, n + 1);
-        dmalloc(ms_q1, n + 1);
-        dmalloc(ms_small, 16);
-        dmalloc(ms_src, kMsWidth);
-        dmalloc(ms_big, kBigRowCap);
+        try {
+            for (auto &e : q_ev) CK(cudaEventCreate(&e));
+            dmalloc(qstatus, 1);
+            CK(cudaHostAlloc(reinterpret_cast<void **>(&h_qstatus), sizeof(Status), cudaHostAllocDefault));
+            dmalloc(ms_dist, static_cast<size_t>(n) * kMsWidth);
+            dmalloc(ms_visit, n);
+            dmalloc(ms_mask0, n);
+            dmalloc(ms_mask1, n);
+            dmalloc(ms_q0, n + 1);
+            dmalloc(ms_q1, n + 1);
+            dmalloc(ms_small, 16);
+            dmalloc(ms_src, kMsWidth);
+            dmalloc(ms_big, kBigRowCap);
+            CK(cudaStreamCreateWithFlags(&qstream, cudaStreamNonBlocking));
+        } catch (...) {
+            free_queries();
+            throw;
+        }
     }
 
     void free_queries() {
         if (qstream) cudaStreamSynchronize(qstream);
-        for (auto &e : q_ev)
+        for (auto &e : q_ev) {
             if (e) cudaEventDestroy(e);
+            e = nullptr;
+        }
         dfree(qstatus);
         if (h_qstatus) cudaFreeHost(h_qstatus);
         h_qstatus = nullptr;
@@ -2579,6 +2592,7 @@ struct cig_handle {
         dfree(ms_src);
         dfree(ms_big);
         dfree(ms_out);
+        ms_out_cap = 0;
         if (qstream) cudaStreamDestroy(qstream);
         qstream = nullptr;
     }
@@ -2630,8 +2644,7 @@ struct cig_handle {
         constexpr uint32_t row = 4 * LPE;
         CK(cudaMemsetAsync(ms_dist, 0xFF, static_cast<size_t>(n) * row * sizeof(uint32_t), qstream));
         ms_seed<<<1, kMsWidth, 0, qstream>>>(ms_src, kw, ms_dist, row, nullptr, fr, qstatus);
-        if (!ms_chunks_made) ms_chunk_cap = alloc_chunks(ms_chunks, kMsChunk);
-        ms_chunks_made = true;
+        alloc_sssp_chunks();
         const MsChunks ch{ms_chunks, ms_small + 3, ms_chunk_cap, ms_small + 8, ms_small + 11};
         launch_coop_on(qstream, ~0u, ms_wave<A, LPE>, kTpbMs, query_view(), n, ms_dist, fr, ch, n + 2, qstatus);
         constexpr uint32_t rows = 512 / LPE;
@@ -2738,6 +2751,7 @@ struct cig_handle {
         const uint64_t need = static_cast<uint64_t>(std::min<uint32_t>(k, kMsWidth)) * n;
         if (need > ms_out_cap) {
             dfree(ms_out);
+            ms_out_cap = 0;  // until the allocation has succeeded
             dmalloc(ms_out, need);
             ms_out_cap = need;
         }
@@ -2790,6 +2804,11 @@ struct cig_handle {
         if (o) sv->opt = *o;
         if (sv->opt.max_wave == 0 || sv->opt.max_wave > kMsWidth) sv->opt.max_wave = kMsWidth;
         if (sv->opt.max_pending == 0) sv->opt.max_pending = 4096;
+        // The waves' own buffers first: the budget is a share of what they
+        // leave free.
+        alloc_queries();
+        alloc_bfs_pull();
+        alloc_sssp_chunks();
         uint64_t budget = sv->opt.budget_bytes;
         if (!budget) {
             size_t fr = 0, tot = 0;
@@ -2800,7 +2819,6 @@ struct cig_handle {
         sv->chunk_cap = std::max<uint64_t>(1024, std::min<uint64_t>(0x40000000ull, budget / 2 / kBytesPerBatchSlot));
         const uint64_t rows = budget / 2 / (static_cast<uint64_t>(n) * sizeof(uint32_t));
         sv->wave_cap = static_cast<uint32_t>(std::max<uint64_t>(1, std::min<uint64_t>(sv->opt.max_wave, rows)));
-        alloc_queries();
         dmalloc(sv->digests, kMsWidth);
         dmalloc(sv->rows, static_cast<size_t>(sv->wave_cap) * n);
         sv->t0 = std::chrono::steady_clock::now();

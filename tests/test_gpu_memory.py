@@ -83,3 +83,40 @@ def test_query_buffers_follow_the_vertices_not_the_arena():
         # the report against the device (3 n result words beside; 2 MiB granules)
         assert free0 - torch.cuda.mem_get_info()[0] <= grown + (8 << 20)
         assert (bfs != 0xFFFFFFFF).all() and (sssp <= 128 * bfs).all() and (sssp >= bfs).all()
+
+
+def test_queries_answer_after_a_failed_allocation():
+    """A query without device memory for its buffers (or its result) fails
+    with the out-of-memory error and takes nothing; once there is memory, the
+    same handle answers."""
+    import torch
+
+    import oracle
+    from coincgraph_b200 import CigError, gen
+
+    rng = np.random.default_rng(6)
+    n = 1 << 20  # 256 bytes of query buffers per vertex
+    g = gen.graph_from_edges(n, rng.integers(0, 2000, 200000), rng.integers(0, 2000, 200000))
+    ref = oracle.Graph(g.n, g.xadj, g.adj).sssp(5, oracle.BFS)
+
+    def fails(eng, leave):
+        torch.cuda.empty_cache()
+        hog = torch.empty(torch.cuda.mem_get_info()[0] - leave, dtype=torch.uint8, device="cuda")
+        with pytest.raises(CigError) as err:
+            eng.query_bfs(np.arange(64))
+        assert err.value.code == -2, err.value  # CIG_ERR_NOMEM
+        del hog
+        torch.cuda.empty_cache()
+
+    # 256 MiB for 64 results, then 300 MiB of buffers: the first, then the
+    # second does not fit.
+    for leave in (64 << 20, 400 << 20):
+        with Engine("bfs", cache_gib=1.0) as eng:
+            eng.load_csr(g.n, g.xadj, g.adj)
+            eng.init()
+            fails(eng, leave)
+            assert eng.memory()["query_buffers"] == 0
+            np.testing.assert_array_equal(eng.query_bfs([5])[0], ref)
+            fails(eng, 64 << 20)  # the result buffer cannot grow
+            np.testing.assert_array_equal(eng.query_bfs([5])[0], ref)
+            np.testing.assert_array_equal(eng.query_bfs(np.full(64, 5))[63], ref)
