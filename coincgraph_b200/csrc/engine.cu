@@ -1483,6 +1483,16 @@ struct cig_handle {
         CK(cudaMemcpyAsync(small + kFr, counts, sizeof(counts), cudaMemcpyHostToDevice, stream));
         check_launch();
         pr_run_converge<T>();
+        if constexpr (sizeof(T) == 4) {
+            uint32_t pending = 0;
+            CK(cudaMemcpyAsync(&pending, small + kFr, sizeof(pending), cudaMemcpyDeviceToHost, stream));
+            CK(cudaStreamSynchronize(stream));
+            if (pending) return;  // cut off by the round bound
+            launch(pr_refine_scatter, persistent_grid(), kTpbPr, fwd.view(), a, n, pr_amend64, status);
+            launch(pr_refine_diff, persistent_grid(), 256, a, n, pr_amend64);
+            launch(pr_amend_fold<T>, persistent_grid(), 256, a, pr_amend64, n, static_cast<T>(opt.pr_epsilon), status);
+            pr_run_converge<T>();
+        }
     }
 
     template <class T>

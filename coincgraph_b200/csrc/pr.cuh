@@ -300,6 +300,12 @@ __device__ __forceinline__ T rank_consume(const PrArrays<T> &a, uint32_t v, doub
 // 4.93, 128 4.77; 50k vertices, FP64: 1.59, 1.55, 1.56).
 constexpr uint32_t kPrChunk = 128;
 
+// Sweeps stop below epsilon: with epsilon itself as their threshold they left
+// FP64 ranks at 50k vertices 2.5e-9 off (relative 2-norm, epsilon 1e-9) where
+// queue rounds leave 2.2e-9 (8k vertices: 2.5e-9, 2.55e-9); with 0.7 of it
+// 1.8e-9 at either size, for 3 % more time at a million vertices.
+constexpr double kPrSweepEps = 0.7;
+
 // The chunks a sweep leaves to the whole grid; what finds no place in the
 // list is pushed by the warp that met it.
 struct PrChunks {
@@ -335,6 +341,7 @@ __device__ __forceinline__ bool pr_sweeps(const AdjView &fwd, const PrArrays<T> 
                                           uint32_t &sweeps, bool &done, Status *st) {
     using B = typename PrBits<T>::type;
     const PrSweepOp<T> op{a};
+    eps *= static_cast<T>(kPrSweepEps);
     const uint32_t lane = lane_id();
     const uint32_t warps = (gridDim.x * kTpbPr) >> 5;
     const uint32_t wid = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
@@ -671,6 +678,54 @@ __global__ void pr_amend_fold(PrArrays<T> a, double *acc, uint32_t n, T eps, Sta
             }
         }
         warp_enqueue(want, v, a.q0, a.cnt, a.cap, st);
+    }
+}
+
+// FP32 mode, after the static solve: the residual that the ranks really leave,
+// 0.15 + alpha P^T x - x in FP64, takes the place of the FP32 one (one step of
+// iterative refinement).  The solve starts from 0.15 rounded to FP32 (4e-8 off
+// at every vertex) and adds equal contributions up in FP32, whose roundings
+// have one sign; sweeps add up more between two consumptions than queue
+// rounds, which made the ranks of a 262k-vertex R-MAT 3.1e-8 off instead of
+// 2.8e-8 (relative 2-norm), and of smaller ones up to 1.2e-7.
+__device__ __forceinline__ double rank_exact(const PrArrays<float> &a, uint32_t v) {
+    return static_cast<double>(__ldcg(a.rank + v)) - static_cast<double>(__ldcg(a.comp + v));
+}
+
+struct PrRefineOp {
+    double *acc;
+    __device__ __forceinline__ bool edge(bool valid, uint32_t, unsigned long long c, uint32_t y) const {
+        if (valid) red_add(acc + y, PrBits<double>::from(c));
+        return valid;
+    }
+};
+
+// acc += alpha P^T x.
+__global__ void __launch_bounds__(kTpbPr, 4) pr_refine_scatter(AdjView fwd, PrArrays<float> a, uint32_t n, double *acc,
+                                                               Status *st) {
+    __shared__ ExpandSmem<kTpbPr, unsigned long long> sm;
+    ExpandCounters cnt;
+    const PrRefineOp op{acc};
+    for (uint32_t base = 0; base < n; base += gridDim.x * kTpbPr) {
+        const uint32_t v = base + spread_rank<kTpbPr>() * gridDim.x + blockIdx.x;
+        RowDesc d{0, 0, 0};
+        unsigned long long c = 0;
+        if (v >= base && v < n) {
+            d = fwd.desc[v];
+            const uint32_t deg = rd_live(d);
+            if (deg) c = PrBits<double>::to(kAlphaD * rank_exact(a, v) / static_cast<double>(deg));
+        }
+        expand_rows<kTpbPr>(fwd, d.len > 0u, v, c, d.off, d.len, op, sm, cnt);
+    }
+    flush_counters(st, cnt, kCntPr);
+}
+
+// acc = 0.15 + acc - x - r: what the residual lacks, for pr_amend_fold.
+__global__ void pr_refine_diff(PrArrays<float> a, uint32_t n, double *acc) {
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+        const int32_t h = hub_slot(a, v);
+        const double r = h >= 0 ? a.res_hub[h] : static_cast<double>(a.res[v]);
+        acc[v] = 0.15 + acc[v] - rank_exact(a, v) - r;
     }
 }
 

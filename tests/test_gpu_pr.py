@@ -107,3 +107,30 @@ def test_pr_with_a_full_chunk_list(fp64, cap, monkeypatch):
         assert s["pr_residual_l1"] <= case.n * 1e-9 * 1.01
         x, ok = g.pagerank(1e-15, 100000)
         assert ok and max_rel(eng.pagerank(fp64=fp64)[0], x) <= (1e-6 if fp64 else 1e-5)
+
+
+@pytest.mark.parametrize("fp64", [False, True])
+def test_pr_error_of_sweeps(fp64):
+    """The ranks' error against 64 bits after a static solve by sweeps and
+    after a batch.  FP64, epsilon 1e-9: what the sweeps leave, residuals of
+    either sign up to 0.7 epsilon, makes 1.8e-9 (relative 2-norm; with epsilon
+    itself as their threshold 2.5e-9, by queue rounds 2.2e-9 to 2.6e-9).  FP32:
+    one rounding of the result, 2^-24, and that remainder, at most 0.7e-9 / 0.15
+    on ranks of at least 0.15 (summed up in FP32 alone: 2e-7 to 4e-7)."""
+    case = rmat_case(13, 1, 200, 200, seed_offset=23)
+    g = oracle.Graph(case.n, case.xadj, case.adj)
+    with Engine("pr", pr_epsilon=1e-9, pr_max_rounds=100000, flags=FLAG_PR_FP64 if fp64 else 0) as eng:
+        eng.load_csr(case.n, case.xadj, case.adj)
+        eng.init()
+        for batch in [None, *case.batches]:
+            if batch is not None:
+                g.delete(*batch[:2])
+                g.add(*batch[2:])
+                eng.apply_batch(*batch)
+            x, ok = g.pagerank(1e-15, 100000)
+            assert ok
+            rank = eng.pagerank(fp64=fp64)[0].astype(np.float64)
+            if fp64:
+                assert np.linalg.norm(rank - x) <= 2.1e-9 * np.linalg.norm(x)
+            else:
+                assert max_rel(rank, x) <= 2.0**-24 + 0.7e-9 / 0.15 / 0.15
