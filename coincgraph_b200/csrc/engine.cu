@@ -659,8 +659,9 @@ struct cig_handle {
     // Set while the closures of an update batch are queued: they may use
     // their own launch shape (tune.inc_per_sm), the static solve uses per_sm.
     bool in_batch = false;
-    // Requests of the phase being queued.  Up to kNarrowBatch its closures run
-    // one block per SM: half the blocks meet at a barrier sooner (four batches
+    // Requests that the closure being queued follows: the phase's, or the whole
+    // batch's for the push that both phases share.  Up to kNarrowBatch the
+    // closures run one block per SM: half the blocks meet at a barrier sooner (four batches
     // of 25k + 25k on s22: 1.96 against 2.00 ms, a 511 x 511 grid 5.2 against
     // 5.5 ms); larger batches (100k + 100k on s24) keep inc_per_sm.
     uint64_t batch_requests = 0;
@@ -2006,11 +2007,13 @@ struct cig_handle {
         if (push) run_push<A>();
     }
 
-    // `fresh` false: keep the frontier the deletion phase left queued (its
-    // begin cleared the insertion counters too).
+    // `carried` (not null): keep the frontier that the batch's deletion phase
+    // left queued for this push (its begin cleared the insertion counters too);
+    // its requests count towards the push closure's launch shape.
     template <int A>
-    void insert_phase_dev(const uint32_t *d_au, const uint32_t *d_av, uint64_t na, bool fresh = true) {
-        const InBatch ib(*this, na);
+    void insert_phase_dev(const uint32_t *d_au, const uint32_t *d_av, uint64_t na, const uint64_t *carried = nullptr) {
+        const InBatch ib(*this, na + (carried ? *carried : 0));
+        const bool fresh = !carried;
         if (fresh) launch(phase_begin, 1, kSmallCount, nullptr, small, kInsertMask | (7ull << kFr), seg_ctl);
         fork_arenas([&] { mutate_add_arena(fwd, d_au, d_av, na, true, true); },
                     [&] { mutate_add_arena(rev, d_au, d_av, na, false, false); });
@@ -2204,7 +2207,7 @@ struct cig_handle {
                 if (mutation_after) CK(cudaStreamWaitEvent(stream, mutation_after, 0));
                 delete_phase_dev<A>(d_du, d_dv, nd, !merge_push);
                 CK(cudaEventRecord(e1, stream));
-                insert_phase_dev<A>(d_au, d_av, na, !merge_push);
+                insert_phase_dev<A>(d_au, d_av, na, merge_push ? &nd : nullptr);
                 CK(cudaEventRecord(e2, stream));
                 presorted = false;
             });
@@ -2226,7 +2229,7 @@ struct cig_handle {
             // a function of the shape.
             presorted = sorted || presort_fits(nd, na);
             CK(cudaEventRecord(e1, stream));
-            run_graphed(4, nd, na, [&] { insert_phase_dev<A>(au, av, na, !merge_push); });
+            run_graphed(4, nd, na, [&] { insert_phase_dev<A>(au, av, na, merge_push ? &nd : nullptr); });
             presorted = false;
             CK(cudaEventRecord(e2, stream));
         });
