@@ -1845,14 +1845,16 @@ struct cig_handle {
         uint32_t *wcount = small + (forward ? kCoopF : kCoopR);
         uint32_t *hcount = small + (forward ? kHugeF : kHugeR);
         if (ix.keys && ixb[forward ? 0 : 1].cls <= kIdxCls) {
-            // Every row above kIdxCls at the last build is indexed: no flat
-            // scan.  Grids follow the batch: at most one group per request.
-            const DelLists dl{wide, wcount, huge, hcount, big, bcount};
+            // Every row above kIdxCls at the last build is indexed: rows that
+            // grew since are scanned by del_wide (at least a block per SM).
+            // Grids follow the batch: at most one group per request.
+            const DelLists dl{wide,           wcount, huge,      hcount, big,    bcount,
+                              indexed_groups, ocount, chunk_map, icount, chunks, firstpos};
             uint32_t *hot = forward ? seg_hot : nullptr;
             const int ps = prof_begin(CIG_STAGE_DEL_SCAN);
             launch(del_lane, std::min(grid_for(nd), persistent_grid()), 256, A.view(), A.desc, sorted, grp, ix, dl, cl,
                    matched, hot, stats, status->counters, status);
-            launch(del_wide, std::min(grid_for(nd, kMutWarps), sms * 3), kMutWarps * 32, A.view(), A.desc, sorted, grp,
+            launch(del_wide, std::min(std::max(grid_for(nd, kMutWarps), sms), sms * 3), kMutWarps * 32, A.view(), A.desc, sorted, grp,
                    ix, dl, cl, matched, hot, stats, status->counters, status);
             prof_end(ps);
             launch(del_rest, std::min(grid_for(nd, kMutWarps), sms * 4), kTpbMut, A.view(), A.desc, sorted, grp, ix,

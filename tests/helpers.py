@@ -169,6 +169,45 @@ def full_row_case() -> Case:
     return Case("fullrow", n, xadj, adj, batches, source=0)
 
 
+def grown_row_case() -> Case:
+    """Rows that are short when the position index is built and grow past the
+    longest row one warp serves (4096): 0 to 40,000 entries (several
+    segments), 1 to 6,000, some of them parallel edges; vertex 2's in-row to
+    20,000.  Then deletions of a few, many and missing entries, repeated
+    requests, and enough for a compaction; the rows go on growing between."""
+    rng = np.random.default_rng(53)
+    n = 45000
+    src = np.concatenate([[0, 0, 1, 1], rng.integers(0, n, 3000)])
+    dst = np.concatenate([[5, 6, 7, 8], rng.integers(0, n, 3000)])
+    xadj, adj = _csr_from_edges(n, src, dst)
+    row0 = list(rng.permutation(np.arange(10, n))[:40000])
+    row1 = list(rng.integers(10, 5000, 6000))
+    in2 = list(rng.permutation(np.arange(10, n))[:20000])
+
+    def take(row, k):
+        got = [row.pop(i) for i in sorted(rng.choice(len(row), k, replace=False), reverse=True)]
+        return got
+
+    def batch(d0, d1, d2, a0, a1, extra=()):
+        du = [0] * len(d0) + [1] * len(d1) + list(d2) + [e[0] for e in extra]
+        dv = list(d0) + list(d1) + [2] * len(d2) + [e[1] for e in extra]
+        order = rng.permutation(len(du))
+        return (_u32(du)[order], _u32(dv)[order], _u32([0] * len(a0) + [1] * len(a1)), _u32(list(a0) + list(a1)))
+
+    batches = [(_u32([]), _u32([]), _u32([0] * 40000 + [1] * 6000 + in2),
+                _u32(row0 + row1 + [2] * 20000))]
+    # few keys per row, two of them missing; a lane's worth, 32 and 300 of them
+    batches.append(batch(take(row0, 3), [row1[0]], take(in2, 4), [], [], extra=[(0, 1), (1, 4)]))
+    batches.append(batch(take(row0, 32), take(row1, 9), take(in2, 300), [11, 12], [13]))
+    # repeated requests on both out-rows, and more keys than a group of shared memory holds
+    twice = [row1[3], row1[3], row1[5]]
+    batches.append(batch(take(row0, 1) * 2, twice, take(in2, 2500), [], row1[:50]))
+    # a quarter and more: compactions
+    batches.append(batch(take(row0, 12000), sorted(set(row1))[:1500], take(in2, 6000), row0[:100], []))
+    batches.append(batch(take(row0, 5), [], take(in2, 5), [], []))
+    return Case("grownrow", n, xadj, adj, batches, source=0)
+
+
 def recurring_case() -> Case:
     """The same edges deleted and inserted again, batch after batch, some of
     them twice in the row and some requested when they are absent, in an

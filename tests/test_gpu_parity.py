@@ -13,8 +13,8 @@ import pytest
 
 import oracle
 from coincgraph_b200 import Engine
-from helpers import (ORACLE_MODE, admission_case, adversarial_case, big_row_case, full_row_case, grid_case, heavy_delete_case,
-                     make_engine, oracle_trace, recurring_case, rmat_case)
+from helpers import (ORACLE_MODE, admission_case, adversarial_case, big_row_case, full_row_case, grid_case,
+                     grown_row_case, heavy_delete_case, make_engine, oracle_trace, recurring_case, rmat_case)
 
 pytestmark = pytest.mark.gpu
 
@@ -179,6 +179,13 @@ def test_admissions_without_evictions(monkeypatch):
     assert stats[0]["cache_segments_evicted"] > 0
     # 96 free slots, 16 of them in reserve.
     assert stats[1]["cache_segments_evicted"] == 0 and 0 < stats[1]["cache_segments_loaded"] <= 64
+
+
+@pytest.mark.parametrize("algo", ["bfs", "cc"])
+@pytest.mark.parametrize("cache", list(CACHES))
+def test_deletions_in_rows_grown_since_the_index_build(algo, cache):
+    run_case(grown_row_case(), algo, CACHES[cache])
+    run_case_whole_batches(grown_row_case(), algo, CACHES[cache])
 
 
 @pytest.mark.parametrize("small_pct", [None, 0, 50, 100])
