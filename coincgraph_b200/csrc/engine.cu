@@ -679,8 +679,12 @@ struct cig_handle {
         // than 4).
         uint32_t inc_per_sm = 2;
         uint32_t split = kSplitDeg; // rows of at least this many entries are expanded by the whole grid
-        uint32_t pull_on = 32;      // BFS waves go bottom-up above n/pull_on frontier vertices (0: never)
-        uint32_t pull_off = 64;     // ... and stay while at least n/pull_off
+        uint32_t pull_on = 32;      // one-source BFS goes bottom-up above n/pull_on frontier vertices (0: never)
+        uint32_t pull_off = 64;     // ... and stays while at least n/pull_off
+        // The same for waves of several sources, which run a kernel of their
+        // own: not touched by the autotuner, which times single sources.
+        uint32_t wave_on = 32;
+        uint32_t wave_off = 64;
     } tune;
 
     template <class... P>
@@ -972,9 +976,11 @@ struct cig_handle {
         if (const char *e = std::getenv("CIG_POS_INDEX_HEADROOM"))
             index_headroom = std::max<uint64_t>(64, std::strtoull(e, nullptr, 10));
         if (const char *e = std::getenv("CIG_POS_INDEX_SPARE")) index_spare = std::max(0.0, std::atof(e));
-        if (const char *e = std::getenv("CIG_PULL_ON")) tune.pull_on = static_cast<uint32_t>(std::max(0, std::atoi(e)));
+        if (const char *e = std::getenv("CIG_PULL_ON"))
+            tune.pull_on = tune.wave_on = static_cast<uint32_t>(std::max(0, std::atoi(e)));
         if (const char *e = std::getenv("CIG_CHUNK_CAP")) chunk_cap = std::strtoull(e, nullptr, 10);
-        if (const char *e = std::getenv("CIG_PULL_OFF")) tune.pull_off = static_cast<uint32_t>(std::max(1, std::atoi(e)));
+        if (const char *e = std::getenv("CIG_PULL_OFF"))
+            tune.pull_off = tune.wave_off = static_cast<uint32_t>(std::max(1, std::atoi(e)));
     }
 
     void destroy() {
@@ -1611,7 +1617,7 @@ struct cig_handle {
         tune = best;
         dispatch([&](auto tag) { static_solve<decltype(tag)::value>(); });
         finish();
-        // Push/pull threshold of the BFS query waves: time single-source waves
+        // Push/pull threshold of one-source BFS queries: time single-source waves
         // (the first 8 vertices with out-edges) for each divisor.
         uint32_t pull_best = tune.pull_on;
         if (rev.desc) {
@@ -2540,13 +2546,14 @@ struct cig_handle {
     BfsPull bfs_pull(uint32_t kw) const {
         BfsPull p{};
         p.ctl = ms_small + 8;
-        if (opt.algo == CIG_PR || !rev.desc || !tune.pull_on || (kw > 1 && !bfs_bigbits)) return p;
+        const uint32_t on = kw == 1 ? tune.pull_on : tune.wave_on, off = kw == 1 ? tune.pull_off : tune.wave_off;
+        if (opt.algo == CIG_PR || !rev.desc || !on || (kw > 1 && !bfs_bigbits)) return p;
         p.rev = rev.view();
 #ifdef CIG_BOUNDS_CHECK
         p.rev.bst = qstatus;
 #endif
-        p.on = std::max<uint32_t>(1, n / tune.pull_on);
-        p.off = std::max<uint32_t>(1, n / tune.pull_off);
+        p.on = std::max<uint32_t>(1, n / on);
+        p.off = std::max<uint32_t>(1, n / off);
         // A bottom-up round passes over every vertex (and, in a wave, over
         // most in-rows); a top-down edge costs about four times a vertex.
         p.edges_on = kw == 1 ? n / 4 : n;

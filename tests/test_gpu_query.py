@@ -237,3 +237,22 @@ def test_sssp_waves_with_a_full_chunk_list(built, k, cap, monkeypatch):
         got = eng.query_sssp(src)
     for j, s in enumerate(src):
         np.testing.assert_array_equal(got[j], og.sssp(int(s), oracle.SSSP))
+
+
+def test_autotune_leaves_wide_waves_alone(built):
+    """The autotuner times one-source queries; a wave of 64 takes the same
+    rounds in the same directions after it as before."""
+    import torch
+
+    case = grid_case(64, 1, 20)
+    src = np.random.default_rng(2).integers(0, case.n, 64).astype(np.uint32)
+    out = torch.empty((64, case.n), dtype=torch.int32, device="cuda")
+    with Engine("bfs", cache_gib=1.0) as eng:
+        eng.load_csr(case.n, case.xadj, case.adj)
+        eng.init()
+        before = eng.query_device("bfs", src, out, width=64)
+        for _ in range(3):
+            eng.autotune()
+            after = eng.query_device("bfs", src, out, width=64)
+            for key in ("rounds", "edges_scanned", "rows_expanded"):
+                assert after[key] == before[key], key
