@@ -1998,7 +1998,7 @@ struct cig_handle {
         auto closure = [&](uint32_t parts) {
             launch_coop(repair_closure<A>, kTpb, fwd.view(), rev.view(), seeds, parts, state, aff_stamp, ep, list,
                         small + kAff, n + 1, big_list(kBigRows), small + kPullBig, n + 2, local_sweeps, inval_done,
-                        small + kInvalDone, small + kAffTotal, frontier(), seg_hot, status);
+                        small + kInvalDone, small + kAffTotal, qstamp, tags, frontier(), seg_hot, status);
         };
         if (prof_on) {  // stage by stage (the rows are mutated by now; the seeds read only values)
             const std::pair<int, uint32_t> stages[] = {

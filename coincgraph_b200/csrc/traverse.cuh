@@ -631,12 +631,14 @@ struct Affected {
 // of them for CC).  A vertex is reset by its own lane right before its row is
 // expanded: nobody else reads the value of an invalidated vertex (PullOp::peek
 // sees the stamp), so no barrier separates the resets from the pulls, and it
-// is queued when its row is done.  In-rows of at least big.split entries are
-// left to the whole grid after a barrier.
+// is queued when its row is done, with the tag of the push closure's seeds, so
+// that an insertion of the same batch that improves it does not queue it again
+// (the frontier has room for every vertex once).  In-rows of at least
+// big.split entries are left to the whole grid after a barrier.
 template <int A>
 __device__ __forceinline__ void pull_repair(const AdjView &rev, unsigned long long *state, const uint32_t *aff_stamp,
-                                            uint32_t epoch, uint32_t ccs, const Affected &aff, const Frontier &fr,
-                                            const Defer &df, ExpandSmem<kTpb> &sm, Status *st) {
+                                            uint32_t epoch, uint32_t ccs, const Affected &aff, uint32_t *qstamp,
+                                            uint32_t tag, const Frontier &fr, const Defer &df, ExpandSmem<kTpb> &sm, Status *st) {
     ExpandCounters c;
     const PullOp<A> op{ccs, state, aff_stamp, epoch};
     for (uint32_t base = 0; base < aff.n; base += gridDim.x * kTpb) {
@@ -658,6 +660,7 @@ __device__ __forceinline__ void pull_repair(const AdjView &rev, unsigned long lo
         __syncwarp();
         const bool later = has && deg >= df.split;
         const bool want = mine && !later && (A == kCc || val_of(__ldcg(state + v)) != kInf);
+        if (want) qstamp[v] = tag;
         warp_enqueue(want, v, fr.q0, fr.cnt, fr.cap, st);
     }
     flush_counters(st, c, kCntPull);
@@ -677,6 +680,7 @@ __device__ __forceinline__ void pull_repair(const AdjView &rev, unsigned long lo
         if (i < aff.n) {
             v = aff.at(i);
             want = rev.desc[v].len >= df.split && (A == kCc || val_of(__ldcg(state + v)) != kInf);
+            if (want) qstamp[v] = tag;
         }
         warp_enqueue(want, v, fr.q0, fr.cnt, fr.cap, st);
     }
@@ -690,8 +694,9 @@ __global__ void __launch_bounds__(kTpb, 2) repair_closure(AdjView fwd, AdjView r
                                                           const uint32_t *epoch_p, uint32_t *list, uint32_t *cnt3,
                                                           uint32_t cap, BigList big, uint32_t *pull_big,
                                                           uint32_t max_rounds, uint32_t max_sweeps, uint32_t *done,
-                                                          uint32_t *done_cnt, uint32_t *aff_total, Frontier fr,
-                                                          uint32_t *seg_hot, Status *st) {
+                                                          uint32_t *done_cnt, uint32_t *aff_total, uint32_t *qstamp,
+                                                          const TagState *tags, Frontier fr, uint32_t *seg_hot,
+                                                          Status *st) {
     __shared__ ExpandSmem<kTpb> sm;
     __shared__ uint32_t lq[2][kLocalCap];
     __shared__ uint32_t lq_n[2];
@@ -705,7 +710,8 @@ __global__ void __launch_bounds__(kTpb, 2) repair_closure(AdjView fwd, AdjView r
     const Defer pull_df{big.rows, pull_big, big.cap, big.split};
     if (!(parts & kPartRounds)) {
         const uint32_t n = (parts & kPartPull) ? *aff_total : 0u;
-        if (n) pull_repair<A>(rev, state, aff_stamp, epoch, ccs, Affected{list, n, list, n}, fr, pull_df, sm, st);
+        if (n) pull_repair<A>(rev, state, aff_stamp, epoch, ccs, Affected{list, n, list, n}, qstamp, tags->next_tag, fr,
+                                  pull_df, sm, st);
         return;
     }
     uint32_t lo = 0, hi = ld_volatile(cnt3 + 0);
@@ -818,7 +824,8 @@ __global__ void __launch_bounds__(kTpb, 2) repair_closure(AdjView fwd, AdjView r
         atomicAdd(&st->counters[kCntAffected], static_cast<unsigned long long>(hi));
     }
     if ((parts & kPartPull) && hi)
-        pull_repair<A>(rev, state, aff_stamp, epoch, ccs, Affected{list, n_list, done, hi}, fr, pull_df, sm, st);
+        pull_repair<A>(rev, state, aff_stamp, epoch, ccs, Affected{list, n_list, done, hi}, qstamp, tags->next_tag, fr,
+                       pull_df, sm, st);
 }
 
 // Start of a phase in a launch of its own (small batches: small_batch).

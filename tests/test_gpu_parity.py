@@ -485,3 +485,29 @@ def _value_digest(values):
         z = (z ^ (z >> np.uint64(27))) * np.uint64(0x94D049BB133111EB)
         z = z ^ (z >> np.uint64(31))
         return int(np.sum(z, dtype=np.uint64))
+
+
+@pytest.mark.parametrize("algo", ["bfs", "cc"])
+def test_repaired_vertices_that_the_insertions_improve(algo):
+    """Nearly every vertex is invalidated by the deletion, repaired and queued,
+    and then improved by an inserted edge of the same batch: it is queued
+    once (the frontier holds each vertex once)."""
+    n = 64
+    k = np.arange(n - 1, dtype=np.uint32)
+    chain_u, chain_v = k, k + 1
+    # a detour that still reaches every vertex of the chain when (0, 1) is gone
+    u = np.concatenate([chain_u, np.zeros(8, np.uint32), np.full(1, 40, np.uint32)])
+    v = np.concatenate([chain_v, np.full(8, 40, np.uint32), np.ones(1, np.uint32)])
+    from coincgraph_b200 import gen
+
+    g = gen.graph_from_edges(n, u, v)
+    og = oracle.Graph(g.n, g.xadj, g.adj)
+    du, dv = np.array([0], np.uint32), np.array([1], np.uint32)
+    au, av = np.zeros(n - 2, np.uint32), np.arange(2, n, dtype=np.uint32)
+    with make_engine(algo, cache_gib=1.0) as eng:
+        eng.load_csr(g.n, g.xadj, g.adj)
+        eng.init()
+        eng.apply_batch(du, dv, au, av)
+        og.delete(du, dv)
+        og.add(au, av)
+        assert np.array_equal(eng.values(), og.cc() if algo == "cc" else og.sssp(0, ORACLE_MODE[algo]))
