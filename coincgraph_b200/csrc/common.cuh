@@ -40,7 +40,8 @@ enum : uint32_t {
 // A deleted entry is overwritten with kTomb (never a vertex id: ids are
 // below n <= 2^32 - 1).  Survivors keep their relative order, so a row with
 // its tombstones removed is exactly the row the reference keeps; tombstones
-// are dropped when the row is compacted or relocated.
+// are dropped when the row is compacted, or moves to a block that would not
+// hold them.
 constexpr uint32_t kTomb = 0xFFFFFFFFu;
 constexpr uint32_t kMaxTombs = (1u << 26) - 1;
 

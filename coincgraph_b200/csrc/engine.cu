@@ -737,7 +737,7 @@ struct cig_handle {
 
     // ------------------------------------------------------------ CUDA graphs of the batch path
     // A batch (or one phase) of the traversal algorithms is a fixed chain of
-    // ~60 launches and memsets on the engine stream whose arguments depend
+    // launches on the engine stream (about 20) whose arguments depend
     // only on the batch shape (deletions, insertions) and on device buffers
     // that stay put between reallocations; everything that changes per batch
     // (epoch, tags, counts) lives on the device.  So the chain is captured

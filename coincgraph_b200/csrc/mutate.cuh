@@ -19,8 +19,10 @@
 //     the rest of the row; the scan of a row stops once every requested
 //     deletion of that row has been found, so a batch reads about half of
 //     each touched row and writes one word per deletion;
-//   - a row is compacted (tombstones dropped, order kept) when it relocates
-//     or when tombstones reach a quarter of its length;
+//   - a row is compacted (tombstones dropped, order kept) when tombstones
+//     reach a quarter of its length, or when its block would overflow: in
+//     place if the live entries then fit, else into the larger block (which
+//     it enters as it is, tombstones and all, where they fit);
 //   - grouping, matching, allocation and appends all run on the GPU.
 #pragma once
 
@@ -189,7 +191,7 @@ __global__ void unpack_keys_batch(const unsigned long long *sorted, PackedSets p
     const uint32_t f = ps.f;
     const unsigned long long mask = (1ull << f) - 1;
     const unsigned long long k = sorted[i];
-    const uint32_t set = static_cast<uint32_t>(k >> (2 * f)) & 3u;  // & 3: a small-sort pad (~0) reads as set 3
+    const uint32_t set = static_cast<uint32_t>(k >> (2 * f)) & 3u;
     const unsigned long long a = (k >> f) & mask, b = k & mask;
     const bool ok = a != mask;
     unsigned long long *dst = set == 0 ? k0 : set == 1 ? k1 : set == 2 ? k2 : k3;
@@ -213,7 +215,7 @@ __global__ void group_scatter_batch(const unsigned long long *sorted, PackedSets
     const unsigned long long mask = (1ull << f) - 1;
     const unsigned long long k = sorted[i];
     if (((k >> f) & mask) == mask) return;  // invalid record
-    const uint32_t set = static_cast<uint32_t>(k >> (2 * f)) & 3u;  // & 3: a small-sort pad (~0) reads as set 3
+    const uint32_t set = static_cast<uint32_t>(k >> (2 * f)) & 3u;
     const uint32_t s0 = ps.off[set], s1 = ps.off[set + 1];
     const uint32_t base = pos[s0];
     const uint32_t local = i - s0;
@@ -1869,7 +1871,8 @@ __global__ void plan_add(const RowDesc *desc, const unsigned long long *keys, Gr
 // kWarpMove that must drop its tombstones).  Serving them inside the warp that found them left the
 // busiest warps a serial queue of up to 32 row copies while most of the grid
 // had no group at all.  `vals` is add_v for the forward arena and add_u for
-// the reverse arena.  A moving row is copied without its tombstones.
+// the reverse arena.  A moving row keeps its tombstones where the new block
+// holds them (moves_whole); the short rows that a lane moves drop theirs.
 constexpr uint32_t kLaneAdds = 8;
 constexpr uint32_t kLaneRow = 8;
 

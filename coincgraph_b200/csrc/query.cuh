@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(kTpbMs, 4) ms_closure(AdjView fwd, uint32_t *d
 // the non-zero masks: a round scans them, and an improved bit is an OR without
 // a result.  With a queue in those rounds too, the appends' atomics on its one
 // counter and the wait for every mask's old value took most of the time
-// (2.9 ms for 13 sources on R-MAT s19, a tenth of the L2's throughput).
+// (2.9 ms for 13 sources on R-MAT s19, 6 % of the L2's throughput).
 // Short chunks and three blocks per SM with two edges per lane in flight keep
 // the warps even: 13 sources on s19 take 1.37 ms with 256-entry chunks and four
 // edges in two blocks, 1.13 with 128 and 1.05 with 64 entries.

@@ -206,7 +206,7 @@ typedef struct {
     uint32_t split_degree;
     double best_ms;           /* static solve with the chosen shape */
     uint32_t candidates;
-    uint32_t pull_divisor;    /* 0: BFS waves stay top-down */
+    uint32_t pull_divisor;    /* one-source BFS queries; 0: they stay top-down */
 } cig_tune_result;
 
 int cig_autotune(cig_handle *h, cig_tune_result *res);

@@ -511,3 +511,26 @@ def test_repaired_vertices_that_the_insertions_improve(algo):
         og.delete(du, dv)
         og.add(au, av)
         assert np.array_equal(eng.values(), og.cc() if algo == "cc" else og.sssp(0, ORACLE_MODE[algo]))
+
+
+@pytest.mark.parametrize("keys", [2, 1022, 1024, 1026, 4094, 4096, 4098])
+@pytest.mark.parametrize("mix", ["deletions", "additions", "both"])
+def test_batches_beside_the_one_block_sort_limits(keys, mix):
+    """Whole batches of so many packed keys (two per record): the block sorts
+    of 1,024 and 4,096 keys, full and one record to either side, and the
+    device sort after them; one set of keys or all four; records out of range
+    at the end of a set, which sort behind its other keys (and, in a full
+    block, leave no padding behind them)."""
+    case = rmat_case(11, 1, 3000, 3000, seed_offset=40)
+    du, dv, au, av = case.batches[0]
+    half = keys // 2
+    nd = {"deletions": half, "additions": 0, "both": half // 2}[mix]
+    na = half - nd
+    du, dv, au, av = (x.copy() for x in (du[:nd], dv[:nd], au[:na], av[:na]))
+    if nd > 1:
+        du[-1], dv[nd // 2] = case.n, 0xFFFFFFFF
+        du[: nd // 4], dv[: nd // 4] = du[nd // 4 : 2 * (nd // 4)], dv[nd // 4 : 2 * (nd // 4)]  # requested twice
+    if na > 1:
+        av[-1], au[na // 3] = case.n, 0xFFFFFFFF
+    case.batches = [(du, dv, au, av), (au, av, du, dv)]
+    run_case_whole_batches(case, "sssp", 1.0)
