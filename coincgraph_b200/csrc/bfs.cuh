@@ -10,12 +10,15 @@
 // al., "The More the Merrier: Efficient Multi-Source Graph Traversal", VLDB
 // 2014).
 //
-// Depths of a wave are kept bit-sliced: plane p of vertex v holds, for every
-// source, bit p of its depth, so recording a level for any number of sources
-// is one OR per set bit of the level, and the k x n result is written once,
-// in rows, from a few planes (depths stay below 16, four planes, on R-MAT).
-// A word per vertex and source instead took a 4 n k byte fill, scattered
-// 4-byte stores and a transpose that read it all again.
+// Depths of a wave below 16 are kept bit-sliced: plane p of vertex v holds, for
+// every source, bit p of its depth, so recording a level for any number of
+// sources is one OR per set bit of the level, and the k x n result is written
+// once, in rows, from four planes (depths stay below 16 on R-MAT).  A word per
+// vertex and source instead took a 4 n k byte fill, scattered 4-byte stores and
+// a transpose that read it all again.  Deeper levels, on graphs whose rounds
+// carry few sources per vertex, go straight to the result, one word per source,
+// and a fifth plane marks them (in further planes a vertex took an OR for every
+// set bit of a depth of up to twelve bits).
 #pragma once
 
 #include "common.cuh"
@@ -26,10 +29,10 @@ namespace cig {
 
 constexpr uint32_t kMsWidth = 64;
 constexpr int kTpbMs = 256;
-constexpr uint32_t kBfsPlanes = 4;      // planes cleared before the wave; the kernel clears further ones as levels need them
+constexpr uint32_t kBfsPlanes = 4;      // depth bits of the planes; plane kBfsPlanes marks deeper levels
+constexpr uint32_t kBfsDeep = 1u << kBfsPlanes;
 constexpr uint32_t kBfsChunk = 1024;     // in-rows of at least this many entries are gathered by several warps
 constexpr uint32_t kBfsWarpRow = 256;    // ... of at least this many by a warp, shorter ones by eight lanes
-constexpr uint32_t kBfsMaxPlanes = 32;  // depths are below 2^32
 
 struct MsFrontier {
     uint32_t *q0;
@@ -58,7 +61,14 @@ struct BfsPull {
     uint32_t *bigbits;          // bit v: v's in-row is in `tasks`
     uint32_t *ctl;              // BfsCtl, zero at launch
 };
-enum BfsCtl : int { kBfsTasks = 0, kBfsBigRows = 1, kBfsFill = 2, kBfsRounds = 3, kBfsEdges = 4 /* 3 counters */ };
+enum BfsCtl : int {
+    kBfsTasks = 0,
+    kBfsBigRows = 1,
+    kBfsFill = 2,
+    kBfsRounds = 3,
+    kBfsEdges = 4,  // 3 counters
+    kBfsGoOn = 7    // bits 0: deep rounds follow, 1: bottom-up, 2: tasks listed
+};
 
 // Top-down edge of a wave: the bits that have not reached y do so now.
 struct MsBfsOp {
@@ -86,23 +96,42 @@ struct MsBfsOp {
     }
 };
 
-// Depth `level` for the sources in m at vertex v (one thread per vertex), as
-// ORs without a result: each waits for nothing, where a load, an OR and a
-// store per set bit of the level followed one another (five of them a round
-// at depth 800).
-__device__ __forceinline__ void planes_put(unsigned long long *planes, uint32_t n, uint32_t v, uint32_t level,
-                                           unsigned long long m) {
-    for (uint32_t b = level; b; b &= b - 1)
-        red_or(planes + static_cast<uint64_t>(__ffs(static_cast<int>(b)) - 1) * n + v, m);
-}
+// Where a wave's depths go.  DEEP: levels of kBfsDeep and more, whose rounds run
+// in a kernel of their own (in one kernel with the others the deep part took
+// registers from those: 3 to 8 % on R-MAT).
+template <bool DEEP>
+struct BfsDepths {
+    unsigned long long *planes;
+    uint32_t *out;  // source-major result
+    uint32_t n;
 
-// The same where a warp's vertices follow one another (bottom-up rounds): the
-// loads and stores of the warp are whole lines.
-__device__ __forceinline__ void planes_record(unsigned long long *planes, uint32_t n, uint32_t v, uint32_t level,
-                                              unsigned long long m) {
-    for (uint32_t b = level; b; b &= b - 1)
-        planes[static_cast<uint64_t>(__ffs(static_cast<int>(b)) - 1) * n + v] |= m;
-}
+    __device__ __forceinline__ void deep(uint32_t v, uint32_t level, unsigned long long m) const {
+        red_or(planes + static_cast<uint64_t>(kBfsPlanes) * n + v, m);
+        for (unsigned long long b = m; b; b &= b - 1)
+            out[static_cast<uint64_t>(__ffsll(static_cast<long long>(b)) - 1) * n + v] = level;
+    }
+    // Depth `level` for the sources in m at vertex v (one thread per vertex), as
+    // ORs without a result: each waits for nothing, where a load, an OR and a
+    // store per set bit of the level followed one another.
+    __device__ __forceinline__ void put(uint32_t v, uint32_t level, unsigned long long m) const {
+        if (DEEP && level >= kBfsDeep) {
+            deep(v, level, m);
+            return;
+        }
+        for (uint32_t b = level; b; b &= b - 1)
+            red_or(planes + static_cast<uint64_t>(__ffs(static_cast<int>(b)) - 1) * n + v, m);
+    }
+    // The same where a warp's vertices follow one another (bottom-up rounds):
+    // the loads and stores of the warp are whole lines.
+    __device__ __forceinline__ void record(uint32_t v, uint32_t level, unsigned long long m) const {
+        if (DEEP && level >= kBfsDeep) {
+            deep(v, level, m);
+            return;
+        }
+        for (uint32_t b = level; b; b &= b - 1)
+            planes[static_cast<uint64_t>(__ffs(static_cast<int>(b)) - 1) * n + v] |= m;
+    }
+};
 
 // Warp-wide OR.
 __device__ __forceinline__ unsigned long long warp_or(unsigned long long x) {
@@ -284,8 +313,9 @@ __device__ __forceinline__ bool bfs_many_edges(const BfsPull &pl, uint32_t n_in,
 // below kBfsWarpRow by eight lanes, below kBfsChunk by a warp, longer ones by a
 // warp per chunk.  Bound by the gathers: 8 bytes of a 32-byte L2 sector per
 // entry.  Returns the new frontier vertices found by this thread.
+template <class D>
 __device__ __forceinline__ uint32_t bfs_bottom_up(const BfsPull &pl, uint32_t n, unsigned long long full,
-                                                  unsigned long long *visit, unsigned long long *planes,
+                                                  unsigned long long *visit, const D &depths,
                                                   const unsigned long long *m_in, unsigned long long *m_out,
                                                   uint32_t level, ExpandCounters &cnt, unsigned long long &src_edges) {
     const uint32_t lane = lane_id();
@@ -315,7 +345,7 @@ __device__ __forceinline__ uint32_t bfs_bottom_up(const BfsPull &pl, uint32_t n,
                 m_out[t.x] = nb;
                 if (nb) {
                     visit[t.x] = vis | nb;
-                    planes_record(planes, n, t.x, level, nb);
+                    depths.record(t.x, level, nb);
                     ++found;
                     ++cnt.hits;
                 }
@@ -375,7 +405,7 @@ __device__ __forceinline__ uint32_t bfs_bottom_up(const BfsPull &pl, uint32_t n,
         if (mine) m_out[v] = nb;
         if (nb) {
             visit[v] = vis | nb;
-            planes_record(planes, n, v, level, nb);
+            depths.record(v, level, nb);
             ++found;
             ++cnt.hits;
         }
@@ -383,39 +413,43 @@ __device__ __forceinline__ uint32_t bfs_bottom_up(const BfsPull &pl, uint32_t n,
     return found;
 }
 
-// One wave (cooperative launch).  Round r gives depth r + 1.  `full`: the
-// wave's source bits.  Planes 0..kBfsPlanes-1 are cleared before the launch.
-// PER_SM blocks per SM: a wave of few sources on a graph of many short rounds
-// waits for its barriers, whose arrivals are atomics on one counter, so up to
-// kBfsFew sources run two (511 x 511 grid, 2 / 5 / 13 sources: 7.0 / 8.1 / 9.9
-// ms against 8.7 / 9.9 / 11.8 with four); wider waves go bottom-up and need
-// the gathers in flight (R-MAT s20: 64 sources 0.49 ms against 0.58, 13
-// sources 0.35 against 0.39).
-constexpr uint32_t kBfsFew = 16;
-template <int PER_SM>
-__global__ void __launch_bounds__(kTpbMs, PER_SM) bfs_wave(AdjView fwd, uint32_t n, unsigned long long full,
-                                                      unsigned long long *visit, unsigned long long *planes,
-                                                      MsFrontier fr, BigList big, uint32_t max_rounds, BfsPull pl,
-                                                      Status *st) {
-    __shared__ ExpandSmem<kTpbMs, unsigned long long> sm;
-    __shared__ uint32_t s_new;
-    __shared__ uint32_t s_buf[kTpbMs / 32][kWarpBuf];
-    __shared__ uint32_t s_held[kTpbMs / 32];
-    if (threadIdx.x < kTpbMs / 32) s_held[threadIdx.x] = 0;
-    __syncthreads();
+// The rounds of a wave: those before the first deep level (true: go on to the
+// deep ones), or, DEEP, from there on.
+struct BfsLoop {
+    uint32_t r = 0;
+    bool pull = false, listed = false;  // every block takes the same decisions from the same counts
     ExpandCounters cnt;
     unsigned long long src_edges = 0;
-    // every block takes the same decisions from the same counts
-    bool pull = false, was_pull = false, listed = false;
+};
+struct BfsWaveSmem {
+    ExpandSmem<kTpbMs, unsigned long long> expand;
+    uint32_t fresh;
+    uint32_t buf[kTpbMs / 32][kWarpBuf];
+    uint32_t held[kTpbMs / 32];
+};
+template <bool DEEP>
+__device__ __forceinline__ bool bfs_rounds(const AdjView &fwd, uint32_t n, unsigned long long full,
+                                           unsigned long long *visit, const BfsDepths<DEEP> &depths,
+                                           const MsFrontier &fr, const BigList &big, uint32_t max_rounds,
+                                           const BfsPull &pl, BfsWaveSmem &ws, BfsLoop &lp, Status *st) {
+    auto &sm = ws.expand;
+    uint32_t &s_new = ws.fresh;
+    auto &s_buf = ws.buf;
+    auto &s_held = ws.held;
+    ExpandCounters &cnt = lp.cnt;
+    unsigned long long &src_edges = lp.src_edges;
     const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, gthreads = gridDim.x * blockDim.x;
-    uint32_t r = 0;
+    uint32_t &r = lp.r;
+    bool &pull = lp.pull, &listed = lp.listed;
+    bool was_pull = false;
     for (;; ++r) {
+        if (!DEEP && r + 1 == kBfsDeep) return true;
         const uint32_t n_in = ld_volatile(fr.cnt + (r % 3));
         const uint32_t n_edges = ld_volatile(pl.ctl + kBfsEdges + r % 3);
-        if (n_in == 0) break;
+        if (n_in == 0) return false;
         if (r >= max_rounds) {
             if (gtid == 0) set_error(st, kErrRounds, r);
-            break;
+            return false;
         }
         if (gtid == 0) {
             fr.cnt[(r + 2) % 3] = 0;
@@ -428,10 +462,10 @@ __global__ void __launch_bounds__(kTpbMs, PER_SM) bfs_wave(AdjView fwd, uint32_t
         unsigned long long *m_in = (r & 1) ? fr.mask1 : fr.mask0;
         unsigned long long *m_out = (r & 1) ? fr.mask0 : fr.mask1;
         const uint32_t level = r + 1;
-        if (level >= (1u << kBfsPlanes) && (level & (level - 1)) == 0) {  // the first level that sets this plane
-            unsigned long long *plane = planes + static_cast<uint64_t>(31 - __clz(level)) * n;
-            for (uint32_t v = gtid; v < n; v += gthreads) plane[v] = 0ull;
-            if (!grid_barrier(st)) break;
+        if (DEEP && level == kBfsDeep) {  // the first deep level
+            unsigned long long *mark = depths.planes + static_cast<uint64_t>(kBfsPlanes) * n;
+            for (uint32_t v = gtid; v < n; v += gthreads) mark[v] = 0ull;
+            if (!grid_barrier(st)) return false;
         }
         was_pull = pull;
         pull = pl.rev.desc && n_in > (was_pull ? pl.off : pl.on);
@@ -441,16 +475,16 @@ __global__ void __launch_bounds__(kTpbMs, PER_SM) bfs_wave(AdjView fwd, uint32_t
                 // The queued vertices are not popped: record their depth here.
                 for (uint32_t i = gtid; i < n_in; i += gthreads) {
                     const uint32_t x = __ldcg(in + i);
-                    planes_put(planes, n, x, r, __ldcg(m_in + x));
+                    depths.put(x, r, __ldcg(m_in + x));
                 }
                 if (!listed) bfs_list_tasks(pl, n, st);
                 listed = true;
-                if (!grid_barrier(st)) break;
+                if (!grid_barrier(st)) return false;
             }
             const uint32_t found =
-                bfs_bottom_up(pl, n, full, visit, planes, m_in, m_out, level, cnt, src_edges);
+                bfs_bottom_up(pl, n, full, visit, depths, m_in, m_out, level, cnt, src_edges);
             block_add(out_cnt, found, &s_new);
-            if (!grid_barrier(st)) break;
+            if (!grid_barrier(st)) return false;
             continue;
         }
         if (was_pull) {
@@ -465,7 +499,7 @@ __global__ void __launch_bounds__(kTpbMs, PER_SM) bfs_wave(AdjView fwd, uint32_t
                 }
                 warp_enqueue(want, v, in, pl.ctl + kBfsFill, fr.cap, st);
             }
-            if (!grid_barrier(st)) break;
+            if (!grid_barrier(st)) return false;
             if (gtid == 0) pl.ctl[kBfsFill] = 0;
         }
         const Defer df{big.rows, big.cnt + (r % 3), big.cap, big.split};
@@ -484,7 +518,7 @@ __global__ void __launch_bounds__(kTpbMs, PER_SM) bfs_wave(AdjView fwd, uint32_t
                 m = __ldcg(m_in + x);
                 const RowDesc d = fwd.desc[x];
                 m_in[x] = 0ull;
-                planes_put(planes, n, x, r, m);
+                depths.put(x, r, m);
                 deg = d.len;
                 off = d.off;
                 has = m != 0ull && deg > 0;
@@ -493,65 +527,135 @@ __global__ void __launch_bounds__(kTpbMs, PER_SM) bfs_wave(AdjView fwd, uint32_t
             expand_rows<kTpbMs>(fwd, has, x, m, off, deg, op, sm, cnt, df);
         }
         op.buf.flush();
-        if (!grid_barrier(st)) break;
+        if (!grid_barrier(st)) return false;
         const uint32_t nbig = min(ld_volatile(big.cnt + (r % 3)), big.cap);
         if (nbig) {
             expand_deferred<kTpbMs, unsigned long long>(fwd, big.rows, nbig, op, cnt);
             op.buf.flush();
-            if (!grid_barrier(st)) break;
+            if (!grid_barrier(st)) return false;
         }
     }
-    flush_counters(st, cnt, kCntPush);
+}
+
+// Counters at the end of a wave's kernel, which began at round `before`.
+__device__ __forceinline__ void bfs_wave_end(const BfsPull &pl, const BfsLoop &lp, uint32_t before, Status *st) {
+    flush_counters(st, lp.cnt, kCntPush);
+    unsigned long long src_edges = lp.src_edges;
     for (int o = 16; o > 0; o >>= 1) src_edges += __shfl_down_sync(kFull, src_edges, o);
     if (lane_id() == 0 && src_edges) atomicAdd(&st->counters[kCntSrcEdges], src_edges);
-    if (gtid == 0) {
-        pl.ctl[kBfsRounds] = r;
-        atomicAdd(&st->counters[kCntRounds], static_cast<unsigned long long>(r));
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        pl.ctl[kBfsRounds] = lp.r;
+        atomicAdd(&st->counters[kCntRounds], static_cast<unsigned long long>(lp.r - before));
     }
+}
+
+// One wave (cooperative launch), up to the deep levels.  Round r gives depth
+// r + 1.  `full`: the wave's source bits.  Planes 0..kBfsPlanes-1 are cleared
+// before the launch, the mark of deep levels by the round that reaches them.
+// PER_SM blocks per SM: rounds of few vertices wait for their barriers, which
+// cost with the blocks, long ones for the gathers in flight.  Two, except for
+// waves of more than kBfsFew sources and for graphs of many and long rows
+// (bfs_blocks in engine.cu).  511 x 511 grid, 2 / 5 / 13 sources: 7.0 / 8.1 /
+// 9.9 ms with two blocks, 8.7 / 9.9 / 11.8 with four; R-MAT s16, 1 / 13 / 64
+// sources: 0.094 / 0.147 / 0.160 and 0.115 / 0.175 / 0.160; s22, 1 / 13 / 64:
+// 0.36 / 1.23 / 1.35 and 0.30 / 0.94 / 1.35.
+constexpr uint32_t kBfsFew = 16;
+template <int PER_SM>
+__global__ void __launch_bounds__(kTpbMs, PER_SM) bfs_wave(AdjView fwd, uint32_t n, unsigned long long full,
+                                                           unsigned long long *visit, unsigned long long *planes,
+                                                           MsFrontier fr, BigList big, uint32_t max_rounds,
+                                                           BfsPull pl, Status *st) {
+    __shared__ BfsWaveSmem ws;
+    if (threadIdx.x < kTpbMs / 32) ws.held[threadIdx.x] = 0;
+    __syncthreads();
+    BfsLoop lp;
+    const bool more =
+        bfs_rounds(fwd, n, full, visit, BfsDepths<false>{planes, nullptr, n}, fr, big, max_rounds, pl, ws, lp, st);
+    bfs_wave_end(pl, lp, 0u, st);
+    if (more && blockIdx.x == 0 && threadIdx.x == 0)
+        pl.ctl[kBfsGoOn] = 1u | (lp.pull ? 2u : 0u) | (lp.listed ? 4u : 0u);
 }
 
 // Source-major depths from the planes: out[j * n + v], four vertices per
 // thread and 512-byte stores per warp where the rows are 16-byte aligned (n a
 // multiple of 4 and an aligned result), one vertex per thread otherwise; one
-// pass over `visit` and the planes in use.
-template <int V>
+// pass over `visit` and the planes in use.  Deep entries are there already.
+template <int V, bool DEEP>
 __device__ __forceinline__ void bfs_depths_of(const unsigned long long *visit, const unsigned long long *planes,
                                               uint32_t n, uint32_t k, uint32_t used, uint32_t v, uint32_t *out) {
-    unsigned long long vis[V], p[kBfsPlanes][V];
+    unsigned long long vis[V], p[kBfsPlanes][V], mark[DEEP ? V : 1];
 #pragma unroll
     for (int i = 0; i < V; ++i) vis[i] = visit[v + i];
 #pragma unroll
     for (uint32_t b = 0; b < kBfsPlanes; ++b)
 #pragma unroll
         for (int i = 0; i < V; ++i) p[b][i] = b < used ? planes[static_cast<uint64_t>(b) * n + v + i] : 0ull;
+    if constexpr (DEEP)
+#pragma unroll
+        for (int i = 0; i < V; ++i) mark[i] = planes[static_cast<uint64_t>(kBfsPlanes) * n + v + i];
     for (uint32_t j = 0; j < k; ++j) {
         uint32_t d[V];
+        bool there = false;
 #pragma unroll
         for (int i = 0; i < V; ++i) {
             d[i] = 0;
 #pragma unroll
             for (uint32_t b = 0; b < kBfsPlanes; ++b) d[i] |= (static_cast<uint32_t>(p[b][i] >> j) & 1u) << b;
-            for (uint32_t b = kBfsPlanes; b < used; ++b)
-                d[i] |= (static_cast<uint32_t>(planes[static_cast<uint64_t>(b) * n + v + i] >> j) & 1u) << b;
             if (!((vis[i] >> j) & 1ull)) d[i] = kInf;
+            if constexpr (DEEP) there = there || ((mark[i] >> j) & 1ull);
         }
         uint32_t *to = out + static_cast<uint64_t>(j) * n + v;
-        if constexpr (V == 4)
+        if (DEEP && there) {
+#pragma unroll
+            for (int i = 0; i < V; ++i)
+                if (!((mark[DEEP ? i : 0] >> j) & 1ull)) to[i] = d[i];
+        } else if constexpr (V == 4) {
             __stcs(reinterpret_cast<uint4 *>(to), make_uint4(d[0], d[1], d[2], d[3]));
-        else
+        } else {
             __stcs(to, d[0]);
+        }
     }
 }
 
-__global__ void bfs_depths(const unsigned long long *visit, const unsigned long long *planes, uint32_t n, uint32_t k,
-                           const uint32_t *ctl, uint32_t *out) {
-    const uint32_t used = 32u - __clz(ctl[kBfsRounds]);
+template <bool DEEP>
+__device__ __forceinline__ void bfs_depths_all(const unsigned long long *visit, const unsigned long long *planes,
+                                               uint32_t n, uint32_t k, uint32_t used, uint32_t *out) {
     const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, gthreads = gridDim.x * blockDim.x;
     if ((n & 3u) == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
-        for (uint32_t q = gtid; q < n / 4; q += gthreads) bfs_depths_of<4>(visit, planes, n, k, used, 4 * q, out);
+        for (uint32_t q = gtid; q < n / 4; q += gthreads)
+            bfs_depths_of<4, DEEP>(visit, planes, n, k, used, 4 * q, out);
     } else {
-        for (uint32_t v = gtid; v < n; v += gthreads) bfs_depths_of<1>(visit, planes, n, k, used, v, out);
+        for (uint32_t v = gtid; v < n; v += gthreads) bfs_depths_of<1, DEEP>(visit, planes, n, k, used, v, out);
     }
+}
+
+// Waves without deep levels (the others' depths: bfs_wave_deep).
+__global__ void bfs_depths(const unsigned long long *visit, const unsigned long long *planes, uint32_t n, uint32_t k,
+                           const uint32_t *ctl, uint32_t *out) {
+    if (!ctl[kBfsGoOn]) bfs_depths_all<false>(visit, planes, n, k, 32u - __clz(ctl[kBfsRounds]), out);
+}
+
+// The rounds from the first deep level on, if bfs_wave left any, and the depths
+// of such a wave: few vertices a round, so two blocks per SM (cooperative
+// launch).  511 x 511 grid, 64 sources: 11.5 ms with every level in planes,
+// 8.9 so; 2048 x 2048: 264 and 214 ms.
+__global__ void __launch_bounds__(kTpbMs, 2) bfs_wave_deep(AdjView fwd, uint32_t n, unsigned long long full,
+                                                           unsigned long long *visit, unsigned long long *planes,
+                                                           uint32_t *out, uint32_t k, MsFrontier fr, BigList big,
+                                                           uint32_t max_rounds, BfsPull pl, Status *st) {
+    const uint32_t go_on = pl.ctl[kBfsGoOn];
+    if (!go_on) return;
+    __shared__ BfsWaveSmem ws;
+    if (threadIdx.x < kTpbMs / 32) ws.held[threadIdx.x] = 0;
+    __syncthreads();
+    BfsLoop lp;
+    const uint32_t before = lp.r = kBfsDeep - 1;
+    lp.pull = go_on & 2u;
+    lp.listed = go_on & 4u;
+    bfs_rounds(fwd, n, full, visit, BfsDepths<true>{planes, out, n}, fr, big, max_rounds, pl, ws, lp, st);
+    bfs_wave_end(pl, lp, before, st);
+    // Every block left the rounds after the same barrier.
+    bfs_depths_all<true>(visit, planes, n, k, 32u - __clz(lp.r), out);
 }
 
 // ---------------------------------------------------------------- one source
@@ -588,10 +692,9 @@ __global__ void bfs_one_seed(const uint32_t *source, uint32_t *depth, uint32_t *
 
 // Single-source BFS (cooperative launch); `vis` cleared and `depth` filled
 // with kInf before it, `bm0` / `bm1` the frontier bitmaps of bottom-up rounds
-// ((n + 31) / 32 words each).  kBfsOnePerSm blocks per SM: see bfs_wave (the
-// grid 5.0 ms against 6.7 with four, R-MAT s20 the same).
-constexpr int kBfsOnePerSm = 2;
-__global__ void __launch_bounds__(kTpbMs, kBfsOnePerSm) bfs_one(AdjView fwd, uint32_t n, uint32_t *depth, uint32_t *vis,
+// ((n + 31) / 32 words each).  PER_SM blocks per SM as for bfs_wave.
+template <int PER_SM>
+__global__ void __launch_bounds__(kTpbMs, PER_SM) bfs_one(AdjView fwd, uint32_t n, uint32_t *depth, uint32_t *vis,
                                                      uint32_t *bm0, uint32_t *bm1, MsFrontier fr, BigList big,
                                                      uint32_t max_rounds, BfsPull pl, Status *st) {
     __shared__ ExpandSmem<kTpbMs> sm;

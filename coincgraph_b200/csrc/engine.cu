@@ -641,6 +641,7 @@ struct cig_handle {
 
     Frontier frontier() const { return Frontier{q0, q1, small + kFr, n + 1}; }
 
+    uint64_t loaded_edges = 0;  // of the graph as it was loaded
     BigRow *big_rows = nullptr;
     // Deferred hub rows; the counters (three from `counter` on) are cleared by
     // the phase's begin.
@@ -1219,6 +1220,7 @@ struct cig_handle {
         });
         if (bad) throw CigError(CIG_ERR_ARG, "edge destination out of range");
         n = nv;
+        loaded_edges = m;
         source = std::min<uint32_t>(opt.source, n - 1);
         if (opt.algo == CIG_CC) {
             // Depth bits below the label (labels are vertex ids < n).
@@ -2541,6 +2543,15 @@ struct cig_handle {
         }
     }
 
+    // Blocks per SM of a BFS query of kw sources (bfs_wave): four where rounds
+    // are long, which is to say for many sources, and for graphs of many edges
+    // (2^23) whose rows are not those of a grid or a road network (eight
+    // entries on average), by the edges of the loaded graph.
+    uint32_t bfs_blocks(uint32_t kw) const {
+        const bool long_rounds = loaded_edges >= (1ull << 23) && loaded_edges >= 8ull * n;
+        return kw > kBfsFew || long_rounds ? 4u : 2u;
+    }
+
     // Bottom-up switch of a BFS query: frontier above n/pull_on vertices
     // (then at least n/pull_off); needs the device in-edge arena.
     BfsPull bfs_pull(uint32_t kw) const {
@@ -2702,7 +2713,8 @@ struct cig_handle {
                 CK(cudaMemsetAsync(wout, 0xFF, static_cast<size_t>(n) * sizeof(uint32_t), qstream));
                 CK(cudaMemsetAsync(vis, 0, words * sizeof(uint32_t), qstream));
                 bfs_one_seed<<<1, 1, 0, qstream>>>(ms_src, wout, vis, ms_q0, ms_small);
-                launch_coop_on(qstream, kBfsOnePerSm, bfs_one, kTpbMs, query_view(), n, wout, vis,
+                const uint32_t per_sm = bfs_blocks(kw);
+                launch_coop_on(qstream, per_sm, per_sm == 2 ? bfs_one<2> : bfs_one<4>, kTpbMs, query_view(), n, wout, vis,
                                reinterpret_cast<uint32_t *>(ms_mask0), reinterpret_cast<uint32_t *>(ms_mask1), fr, bl,
                                n + 2, bfs_pull(kw), qstatus);
                 ++n_launch;
@@ -2712,9 +2724,8 @@ struct cig_handle {
             CK(cudaMemsetAsync(ms_mask0, 0, n * sizeof(unsigned long long), qstream));
             CK(cudaMemsetAsync(ms_mask1, 0, n * sizeof(unsigned long long), qstream));
             if (algo == CIG_BFS) {
-                // The planes live in the distance buffer (32 planes of 8 n
-                // bytes = 64 words per vertex).
-                static_assert(kBfsMaxPlanes * sizeof(unsigned long long) <= kMsWidth * sizeof(uint32_t),
+                // The planes live in the distance buffer (64 words per vertex).
+                static_assert((kBfsPlanes + 1) * sizeof(unsigned long long) <= kMsWidth * sizeof(uint32_t),
                               "planes fit the distance buffer");
                 unsigned long long *planes = reinterpret_cast<unsigned long long *>(ms_dist);
                 CK(cudaMemsetAsync(planes, 0, kBfsPlanes * n * sizeof(unsigned long long), qstream));
@@ -2722,9 +2733,11 @@ struct cig_handle {
                 ms_seed<<<1, kMsWidth, 0, qstream>>>(ms_src, kw, nullptr, 0u, ms_visit, fr, qstatus);
                 const unsigned long long full = kw >= 64 ? ~0ull : ((1ull << kw) - 1);
                 alloc_bfs_pull();
-                const bool few = kw <= kBfsFew;
-                launch_coop_on(qstream, few ? 2u : 4u, few ? bfs_wave<2> : bfs_wave<4>, kTpbMs, query_view(), n, full,
+                const uint32_t per_sm = bfs_blocks(kw);
+                launch_coop_on(qstream, per_sm, per_sm == 2 ? bfs_wave<2> : bfs_wave<4>, kTpbMs, query_view(), n, full,
                                ms_visit, planes, fr, bl, n + 2, bfs_pull(kw), qstatus);
+                launch_coop_on(qstream, 2, bfs_wave_deep, kTpbMs, query_view(), n, full, ms_visit, planes, wout, kw, fr,
+                               bl, n + 2, bfs_pull(kw), qstatus);
                 bfs_depths<<<sms * 8, 256, 0, qstream>>>(ms_visit, planes, n, kw, ms_small + 8, wout);
             } else if (opt.flags & CIG_FLAG_WEIGHT_U255) {
                 sssp_wave<kSsspU>(kw, fr, bl, wout);
