@@ -505,7 +505,7 @@ __device__ __forceinline__ bool bfs_rounds(const AdjView &fwd, uint32_t n, unsig
         const Defer df{big.rows, big.cnt + (r % 3), big.cap, big.split};
         const MsBfsOp op{visit, m_out,
                          WarpBuf{s_buf[threadIdx.x >> 5], s_held + (threadIdx.x >> 5), out, out_cnt, fr.cap, st,
-                                 pl.rev.desc ? fwd.desc : nullptr, pl.ctl + kBfsEdges + (r + 1) % 3}};
+                                 fwd.desc, pl.ctl + kBfsEdges + (r + 1) % 3}};
         for (uint32_t base = 0; base < n_in; base += gridDim.x * kTpbMs) {
             const uint32_t i = base + spread_rank<kTpbMs>() * gridDim.x + blockIdx.x;
             bool has = i < n_in;
@@ -813,7 +813,7 @@ __global__ void __launch_bounds__(kTpbMs, PER_SM) bfs_one(AdjView fwd, uint32_t 
         const Defer df{big.rows, big.cnt + (r % 3), big.cap, big.split};
         const OneBfsOp op{vis, depth, r + 1,
                           WarpBuf{s_buf[threadIdx.x >> 5], s_held + (threadIdx.x >> 5), out, out_cnt, fr.cap, st,
-                                  pl.rev.desc ? fwd.desc : nullptr, pl.ctl + kBfsEdges + (r + 1) % 3}};
+                                  fwd.desc, pl.ctl + kBfsEdges + (r + 1) % 3}};
         for (uint32_t base = 0; base < n_in; base += gridDim.x * kTpbMs) {
             const uint32_t i = base + spread_rank<kTpbMs>() * gridDim.x + blockIdx.x;
             bool has = i < n_in;
