@@ -256,3 +256,26 @@ def test_autotune_leaves_wide_waves_alone(built):
             after = eng.query_device("bfs", src, out, width=64)
             for key in ("rounds", "edges_scanned", "rows_expanded"):
                 assert after[key] == before[key], key
+
+
+@pytest.mark.parametrize("last", [14, 15, 16, 17, 40])
+@pytest.mark.parametrize("pull", ["0", "1000000"])
+def test_bfs_depths_beside_the_plane_limit(built, last, pull, monkeypatch):
+    """Chains whose deepest level lies on either side of 16, where depths go
+    from the planes to the result directly, top-down and bottom-up; the four
+    vertices of a 16-byte store hold planes', direct and unreached entries."""
+    monkeypatch.setenv("CIG_PULL_ON", pull)
+    monkeypatch.setenv("CIG_PULL_OFF", "2000000")
+    for n in (64, 65):
+        chain = np.arange(last + 1)
+        ends = np.arange(last + 1, n - 4)  # one step behind the chain's middle and end, in turn
+        src = np.concatenate([chain[:-1], np.where(ends % 2, last, last // 2)])
+        g = gen.graph_from_edges(n, src, np.concatenate([chain[1:], ends]))
+        og = oracle.Graph(g.n, g.xadj, g.adj)
+        sources = np.array([0, 3, n - 1], dtype=np.uint32)
+        with Engine("bfs", cache_gib=1.0) as eng:
+            eng.load_csr(g.n, g.xadj, g.adj)
+            eng.init()
+            got = eng.query_bfs(sources)
+        for j, s in enumerate(sources):
+            np.testing.assert_array_equal(got[j], og.sssp(int(s), oracle.BFS))
